@@ -15,12 +15,21 @@ order — no degree counting, no dictionary keyed by tensors.
 """
 from __future__ import annotations
 
+import operator
+
 
 class _Node:
     __slots__ = ("name", "inputs", "outputs", "helpers", "seq")
 
     def __init__(self, name, inputs, outputs, helpers, seq):
-        self.name, self.inputs, self.outputs, self.helpers, self.seq = name, inputs, outputs, helpers, seq
+        self.name = name
+        self.inputs = inputs
+        self.outputs = outputs
+        self.helpers = helpers
+        self.seq = seq
+
+
+_creation = operator.attrgetter("seq")
 
 
 class DAGTracker:
@@ -60,25 +69,22 @@ class DAGTracker:
 
     def add_node(self, name, input_args, output_tensors, helper_tensors=None):
         self._seq += 1
-        node = _Node(name, list(input_args), list(output_tensors), list(helper_tensors or []), self._seq)
+        node = _Node(name, tuple(input_args), tuple(output_tensors), tuple(helper_tensors) if helper_tensors else (), self._seq)
         for t in output_tensors:
             t._grad_node = node
 
     def _upstream(self, root):
         from mytorch_b200.tensor import Tensor
 
-        seen, stack, nodes = set(), [root], []
+        seen, stack = {root}, [root]
         while stack:
-            node = stack.pop()
-            if id(node) in seen:
-                continue
-            seen.add(id(node))
-            nodes.append(node)
-            for arg in node.inputs:
-                if isinstance(arg, Tensor) and arg._grad_node is not None:
-                    stack.append(arg._grad_node)
-        nodes.sort(key=lambda n: -n.seq)
-        return nodes
+            for arg in stack.pop().inputs:
+                if isinstance(arg, Tensor):
+                    node = arg._grad_node
+                    if node is not None and node not in seen:
+                        seen.add(node)
+                        stack.append(node)
+        return sorted(seen, key=_creation, reverse=True)
 
     def backward(self, tensor):
         from mytorch_b200.tensor import MismatchShapesError, Tensor, shape_size
@@ -92,7 +98,7 @@ class DAGTracker:
         seed.fill_(1)
         tensor.grad = seed
 
-        hook = self.leaf_grad_final_hook
+        hook, join = self.leaf_grad_final_hook, self.join_hook
         pending = {}
         if hook is not None:  # how many contributions every leaf will receive
             for node in order:
@@ -101,39 +107,38 @@ class DAGTracker:
                         pending[id(arg)] = pending.get(id(arg), 0) + 1
 
         for node in order:
-            func = self._backward_funcs[node.name]
+            name, inputs = node.name, node.inputs
             fused = None  # the input whose gradient so far is handed to the operator
-            slot = self.fused_accumulate.get(node.name)
+            extra = {}
+            slot = self.fused_accumulate.get(name)
             if slot is not None:
-                cand = node.inputs[slot]
+                cand = inputs[slot]
                 if isinstance(cand, Tensor) and cand.requires_grad and cand.grad is not None:
                     fused = cand
-            extra = {}
-            if fused is not None:
-                extra["accumulate_dx"] = fused.grad
-            if node.name in self.deferrable and self.join_hook is not None:
+                    extra["accumulate_dx"] = cand.grad
+            if join is not None and name in self.deferrable:
                 extra["defer_weight_gradient"] = True
-            grads = list(func(*[t.grad for t in node.outputs], *node.helpers, *node.inputs, **extra))
-            grads += [None] * (len(node.inputs) - len(grads))
-            for arg, grad in zip(node.inputs, grads):
-                if arg is None or not isinstance(arg, Tensor) or not arg.requires_grad:
+            grads = self._backward_funcs[name](*[t.grad for t in node.outputs], *node.helpers, *inputs, **extra)
+            for k, (arg, grad) in enumerate(zip(inputs, grads)):  # operators may return fewer gradients than they have inputs
+                if grad is None or not isinstance(arg, Tensor) or not arg.requires_grad:
                     continue
-                if grad is not None:
-                    if arg.grad is None or (arg is fused and grad is grads[slot]):
-                        arg.grad = grad
-                    else:
-                        if arg.grad.shape != grad.shape:
-                            raise MismatchShapesError([arg.grad.shape, grad.shape])
-                        if self.join_hook is not None and arg._grad_node is None:  # a leaf: its gradient may come from there
-                            self.join_hook()
-                        arg.grad = arg.grad + grad
-                if hook is not None and id(arg) in pending:
-                    pending[id(arg)] -= 1
-                    if pending[id(arg)] == 0 and arg.grad is not None:
-                        hook(arg)  # the gradient may still be in flight on the backend's side stream: the hook orders itself after it
+                if arg.grad is None or (arg is fused and k == slot):
+                    arg.grad = grad
+                else:
+                    if arg.grad.shape != grad.shape:
+                        raise MismatchShapesError([arg.grad.shape, grad.shape])
+                    if join is not None and arg._grad_node is None:  # a leaf: its gradient may come from there
+                        join()
+                    arg.grad = arg.grad + grad
+            if hook is not None:
+                for arg in inputs:
+                    if isinstance(arg, Tensor) and arg.requires_grad and id(arg) in pending:
+                        pending[id(arg)] -= 1
+                        if pending[id(arg)] == 0 and arg.grad is not None:
+                            hook(arg)  # the gradient may still be in flight on the backend's side stream: the hook orders itself after it
 
-        if self.join_hook is not None:
-            self.join_hook()
+        if join is not None:
+            join()
 
         for node in order:
             for t in node.outputs:

@@ -1,4 +1,4 @@
-"""CUDA runtime glue: the kernel library (ctypes over its C ABI), device memory, streams, events.
+"""CUDA runtime glue: the kernel library (a CPython binding of its C ABI), device memory, streams, events.
 
 Plays the role of the reference's ``mytorch/backends/cuda/env.py`` (library loader
 ``:341-393``, ``CudaMemory`` ``:524-561``, ``allocate_memory`` / ``transfer_memory``
@@ -14,166 +14,62 @@ operation raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import numpy as np
 
 from mytorch_b200.backends.backend_dispatcher import BackendDispatcher
 
-_P, _I, _L, _F, _D = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_double
-
-_CONV = [_I] * 11
-_POOL = [_I] * 10
-_SIGNATURES = {
-    "mtb_version": ([], _I),
-    "mtb_device_check": ([], _I),
-    "mtb_fill_f32": ([_P, _L, _F, _P], _I),
-    "mtb_copy_f32": ([_P, _P, _L, _P], _I),
-    "mtb_scale_f32": ([_P, _P, _L, _F, _P], _I),
-    "mtb_relu_forward_f32": ([_P, _P, _L, _P], _I),
-    "mtb_relu_backward_f32": ([_P, _P, _P, _L, _P], _I),
-    "mtb_add_f32": ([_P, _P, _P, _L, _F, _P], _I),
-    "mtb_mul_f32": ([_P, _P, _P, _L, _P], _I),
-    "mtb_add_bias_rows_f32": ([_P, _P, _P, _L, _I, _F, _P], _I),
-    "mtb_binary_strided_f32": ([_I, _I, _P, _P, _P, _P, _P, _P, _P, _F, _P], _I),
-    "mtb_resize_channels_f32": ([_P, _P, _L, _I, _I, _P], _I),
-    "mtb_nchw_to_nhwc_f32": ([_P, _P, _I, _I, _I, _I, _P], _I),
-    "mtb_nhwc_to_nchw_f32": ([_P, _P, _I, _I, _I, _I, _P], _I),
-    "mtb_cast": ([_I, _P, _P, _L, _P], _I),
-    "mtb_batch_norm2d_workspace_bytes": ([_I, _I, _I, _I], _L),
-    "mtb_batch_norm2d_forward_f32": ([_I, _I, _I, _I, _P, _P, _P, _D, _I, _D, _P, _P, _P, _P, _P, _I, _P, _L, _P], _I),
-    "mtb_batch_norm2d_backward_f32": ([_I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _D, _I, _P, _P, _P, _P, _L, _P], _I),
-    "mtb_batch_norm2d_add_relu_forward_f32": ([_I, _I, _I, _I, _P, _P, _P, _P, _D, _I, _D, _P, _P, _P, _P, _P, _P, _I, _P, _L, _P], _I),
-    "mtb_batch_norm2d_add_relu_backward_f32": ([_I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _D, _P, _P, _P, _P, _P, _L, _P], _I),
-    "mtb_add_relu_f32": ([_P, _P, _P, _L, _P], _I),
-    "mtb_add_relu_backward_f32": ([_P, _P, _P, _P, _L, _P], _I),
-    "mtb_colsum_workspace_bytes": ([_I], _L),
-    "mtb_colsum_f32": ([_P, _L, _I, _F, _P, _P, _L, _P], _I),
-    "mtb_colsum_noalloc_f32": ([_P, _L, _I, _F, _P, _P], _I),
-    "mtb_nhwc_spatial_sum_f32": ([_P, _P, _I, _I, _I, _F, _P], _I),
-    "mtb_nhwc_spatial_bcast_f32": ([_P, _P, _I, _I, _I, _F, _P], _I),
-    "mtb_sum_strided_f32": ([_P, _P, _I, _P, _P, _I, _P, _P, _F, _P], _I),
-    "mtb_max_strided_f32": ([_P, _P, _P, _I, _P, _P, _L, _L, _P], _I),
-    "mtb_max_backward_f32": ([_P, _P, _P, _L, _I, _P, _P, _L, _P], _I),
-    "mtb_eq_strided": ([_I, _I, _P, _P, _P, _P, _P, _P, _P], _I),
-    "mtb_max_pool2d_forward_f32": (_POOL + [_P, _P, _P, _P], _I),
-    "mtb_max_pool2d_backward_f32": (_POOL + [_P, _P, _P, _P, _P, _P], _I),
-    "mtb_max_pool2d_argmax_u8": ([_P, _P, _L, _P], _I),
-    "mtb_cross_entropy_workspace_bytes": ([_I], _L),
-    "mtb_cross_entropy_forward_f32": ([_I, _I, _P, _P, _P, _P, _L, _P], _I),
-    "mtb_cross_entropy_backward_f32": ([_I, _I, _P, _P, _P, _P, _P], _I),
-    "mtb_sgd_f32": ([_P, _P, _P, _L, _I, _D, _D, _D, _D, _I, _I, _D, _P], _I),
-    "mtb_sgd_multi_f32": ([_I, _P, _P, _P, _P, _P, _D, _D, _D, _D, _I, _I, _D, _P], _I),
-    "mtb_pack_scale_f32": ([_I, _P, _P, _P, _P, _D, _P], _I),
-    "mtb_conv2d_workspace_bytes": (_CONV, _L),
-    "mtb_conv2d_plan_f32": (_CONV + [_P], _I),
-    "mtb_conv2d_forward_f32": (_CONV + [_P, _P, _P, _P, _I, _P, _L, _P], _I),
-    "mtb_conv2d_stats_max_rows": ([], _I),
-    "mtb_conv2d_forward_stats_f32": (_CONV + [_P, _P, _P, _P, _I, _P, _P, _P, _L, _P], _I),
-    "mtb_batch_norm2d_forward_prestats_f32": ([_I, _I, _I, _I, _P, _P, _P, _D, _D, _P, _P, _P, _P, _P, _I, _P, _I, _P, _L, _P], _I),
-    "mtb_conv2d_dgrad_f32": (_CONV + [_P, _P, _P, _P, _L, _P], _I),
-    "mtb_conv2d_dgrad_add_f32": (_CONV + [_P, _P, _P, _P, _P, _L, _P], _I),
-    "mtb_conv2d_dgrad_accumulates_in_place": (_CONV + [_P, _P, _P], _I),
-    "mtb_conv2d_wgrad_f32": (_CONV + [_P, _P, _P, _P, _L, _P], _I),
-    "mtb_gemm_f32": ([_I, _I, _I, _P, _I, _P, _I, _P, _I, _P, _P], _I),
-    "mtb_tc_status": ([_P], _I),
-    # runtime
-    "mtb_malloc": ([_L], _P),
-    "mtb_free": ([_P], _I),
-    "mtb_pool_reserved_bytes": ([], _L),
-    "mtb_pool_in_use_bytes": ([], _L),
-    "mtb_pool_trim": ([], _I),
-    "mtb_set_device": ([_I], _I),
-    "mtb_get_device": ([_P], _I),
-    "mtb_device_count": ([_P], _I),
-    "mtb_device_synchronize": ([], _I),
-    "mtb_mem_get_info": ([_P, _P], _I),
-    "mtb_memcpy_h2d_async": ([_P, _P, _L, _P], _I),
-    "mtb_memcpy_d2h_async": ([_P, _P, _L, _P], _I),
-    "mtb_memcpy_d2d_async": ([_P, _P, _L, _P], _I),
-    "mtb_memset_async": ([_P, _I, _L, _P], _I),
-    "mtb_host_alloc_pinned": ([_L], _P),
-    "mtb_host_free_pinned": ([_P], _I),
-    "mtb_stream_create": ([], _P),
-    "mtb_stream_destroy": ([_P], _I),
-    "mtb_stream_synchronize": ([_P], _I),
-    "mtb_stream_wait_event": ([_P, _P], _I),
-    "mtb_event_create": ([_I], _P),
-    "mtb_event_destroy": ([_P], _I),
-    "mtb_event_record": ([_P, _P], _I),
-    "mtb_event_synchronize": ([_P], _I),
-    "mtb_event_elapsed_ms": ([_P, _P, _P], _I),
-    "mtb_graph_begin_capture": ([_P], _I),
-    "mtb_graph_end_capture": ([_P, _P], _I),
-    "mtb_graph_launch": ([_P, _P], _I),
-    "mtb_graph_destroy": ([_P], _I),
-    "mtb_tc_wait_selftest": ([_L, _I, _P], _I),
-}
-
 LIBRARY_PATH = os.environ.get(
     "MYTORCH_B200_LIB",
     os.path.join(os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__)))), "lib", "libmytorch_b200.so"),
 )
-
-# entry points that only enqueue or bookkeep: not counted as kernel launches
-_NOT_LAUNCHES = {"mtb_free", "mtb_pool_trim", "mtb_set_device", "mtb_get_device", "mtb_device_count", "mtb_device_synchronize", "mtb_mem_get_info",
-                 "mtb_memcpy_h2d_async", "mtb_memcpy_d2h_async", "mtb_memcpy_d2d_async", "mtb_memset_async", "mtb_host_free_pinned",
-                 "mtb_stream_destroy", "mtb_stream_synchronize", "mtb_stream_wait_event", "mtb_event_destroy", "mtb_event_record",
-                 "mtb_event_synchronize", "mtb_event_elapsed_ms", "mtb_graph_begin_capture", "mtb_graph_end_capture", "mtb_graph_launch",
-                 "mtb_graph_destroy", "mtb_tc_status", "mtb_device_check", "mtb_conv2d_plan_f32"}
+BINDING_PATH = os.path.join(os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__)))), "lib", "_mtb_binding.so")
 
 
 class NativeError(RuntimeError):
     pass
 
 
+def _load_binding():
+    """The CPython binding of the C ABI (``csrc/binding.cpp``), or None when it has not been built."""
+    if not os.path.exists(BINDING_PATH):
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_mtb_binding", BINDING_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_mtb_binding", loader))
+    loader.exec_module(module)
+    return module
+
+
+_binding = _load_binding()
+# every entry point the Python layer binds (argument types come from the public header, compiled into the binding)
+_SIGNATURES = _binding.entry_points if _binding is not None else ()
+
+
 class NativeLibrary:
-    """ctypes view of ``libmytorch_b200.so``; every wrapped call raises on a non-zero status (or a
-    NULL pointer from the entry points that return one)."""
+    """The entry points of ``libmytorch_b200.so`` as attributes, without their ``mtb_`` prefix; a call raises on a
+    non-zero status (or a NULL pointer from the entry points that return one).  Pointer arguments are None,
+    addresses, ``CudaMemory`` blocks or ctypes objects (host arrays, ``byref``)."""
 
     def __init__(self, path=LIBRARY_PATH):
-        if not os.path.exists(path):
+        if not os.path.exists(path) or _binding is None:
+            missing = path if not os.path.exists(path) else BINDING_PATH
             raise NativeError(
-                f"kernel library not found at {path}; build it with `python -m mytorch_b200.build` "
+                f"kernel library not found at {missing}; build it with `python -m mytorch_b200.build` "
                 "(there is no fallback implementation)")
-        self._dll = ctypes.CDLL(path)
-        self._dll.mtb_last_error.restype = ctypes.c_char_p
-        self._dll.mtb_last_error.argtypes = []
-        self.launches = 0
-        for name, (argtypes, restype) in _SIGNATURES.items():
-            fn = getattr(self._dll, name)
-            fn.argtypes = argtypes
-            fn.restype = restype
-            if restype is _P:
-                wrapped = self._pointer(name, fn)
-            elif restype is _I and name not in ("mtb_version", "mtb_conv2d_stats_max_rows", "mtb_conv2d_dgrad_accumulates_in_place"):
-                wrapped = self._checked(name, fn, name not in _NOT_LAUNCHES)
-            else:
-                wrapped = fn
-            setattr(self, name[4:], wrapped)
+        _binding.load(path, NativeError)
+        for name in _SIGNATURES:
+            setattr(self, name[4:], getattr(_binding, name[4:]))
 
-    def _checked(self, name, fn, counts):
-        def call(*args):
-            rc = fn(*args)
-            if rc != 0:
-                raise NativeError(f"{name} failed ({rc}): {self._dll.mtb_last_error().decode()}")
-            if counts:
-                self.launches += 1
-            return rc
-
-        return call
-
-    def _pointer(self, name, fn):
-        def call(*args):
-            p = fn(*args)
-            if not p:
-                raise NativeError(f"{name} failed: {self._dll.mtb_last_error().decode()}")
-            return p
-
-        return call
+    @property
+    def launches(self):
+        """Calls so far of entry points that enqueue kernels."""
+        return _binding.launches()
 
     def exported(self, name):
-        return hasattr(self._dll, name)
+        return name in _SIGNATURES
 
 
 class Event:
@@ -249,6 +145,7 @@ class CudaEnv:
         self._side_scratch = {}
         self._side_keepalive = []
         self._side_busy = set()
+        self._fork_events, self._join_events = {}, {}
         self.overlap_weight_gradients = not os.environ.get("MTB_SERIAL_WGRAD")
         from mytorch_b200.autograd import DAGTracker
 
@@ -256,17 +153,15 @@ class CudaEnv:
 
     # ---- devices, streams
     def current_device(self):
-        dev = ctypes.c_int(0)
-        self.lib.get_device(ctypes.byref(dev))
-        return dev.value
+        return _binding.current_device()
 
     def set_device(self, index):
-        if index is not None and index != self.current_device():
+        if index is not None and index != _binding.current_device():
             self.lib.set_device(int(index))
 
     def stream(self):
         """The compute stream of the current device: every operator enqueues its work there."""
-        dev = self.current_device()
+        dev = _binding.current_device()
         s = self._streams.get(dev)
         if s is None:
             s = self._streams[dev] = self.lib.stream_create()
@@ -303,8 +198,11 @@ class CudaEnv:
         side = self._side_streams.get(dev)
         if side is None:
             side = self._side_streams[dev] = self.lib.stream_create()
-        ev = Event()
-        ev.record(self.stream())
+        # one event per device is enough: a wait refers to the record that precedes it, later records do not move it
+        ev = self._fork_events.get(dev)
+        if ev is None:
+            ev = self._fork_events[dev] = Event()
+        self.lib.event_record(ev.handle, self.stream())
         self.lib.stream_wait_event(side, ev.handle)
         self._side_keepalive.extend(keepalive)
         self._side_busy.add(dev)
@@ -328,8 +226,10 @@ class CudaEnv:
         current = self.current_device()
         for dev in list(self._side_busy):
             self.set_device(dev)
-            ev = Event()
-            ev.record(self._side_streams[dev])
+            ev = self._join_events.get(dev)
+            if ev is None:
+                ev = self._join_events[dev] = Event()
+            self.lib.event_record(ev.handle, self._side_streams[dev])
             self.lib.stream_wait_event(self.stream(), ev.handle)
         self.set_device(current)
         self._side_busy.clear()
@@ -358,17 +258,17 @@ class CudaEnv:
         return buf.ptr, buf.nbytes
 
 
-class CudaMemory:
-    """A device allocation from the library's pool. ``ptr`` is the raw device address; ``read`` /
-    ``write`` move bytes between it and NumPy arrays without interpreting any layout."""
+if _binding is not None:
+    _binding.on_first_use(CudaEnv.instance)
 
-    def __init__(self, device_index, nbytes):
-        env = CudaEnv.instance()
-        self.device_index = env.current_device() if device_index is None else device_index
-        env.set_device(self.device_index)
-        self.nbytes = int(nbytes)
-        self._lib = env.lib
-        self.ptr = env.lib.malloc(max(self.nbytes, 1))
+
+class CudaMemory(_binding.Block if _binding is not None else object):
+    """A device allocation from the library's pool (``CudaMemory(device_index, nbytes)``; allocation, ``destroy`` and
+    the release when the object goes away are native, see ``csrc/binding.cpp``). ``ptr`` is the raw device address,
+    ``nbytes`` and ``device_index`` say how much and where; ``read`` / ``write`` move bytes between it and NumPy
+    arrays without interpreting any layout."""
+
+    __slots__ = ()
 
     def read(self, shape, np_dtype):
         env = CudaEnv.instance()
@@ -401,17 +301,6 @@ class CudaMemory:
         env.set_device(self.device_index)
         env.lib.memcpy_d2d_async(self.ptr, other.ptr, self.nbytes if nbytes is None else nbytes, env.stream())
 
-    def destroy(self):
-        if self.ptr:
-            self._lib.free(self.ptr)
-            self.ptr = 0
-
-    def __del__(self):
-        try:
-            self.destroy()
-        except Exception:
-            pass
-
 
 def host_pointer(host):
     """(address, bytes) of a contiguous host buffer: NumPy array or an object with ``data_ptr()``."""
@@ -436,11 +325,10 @@ class CudaMemoryView(CudaMemory):
     """A window into another allocation (used for gradient tensors that live inside one flat
     all-reduce buffer). Keeps the parent alive; frees nothing."""
 
+    __slots__ = ("_parent",)
+
     def __init__(self, parent, offset_bytes, nbytes, device_index):
-        self.device_index = device_index
+        self.device_index = parent.device_index if device_index is None else device_index
         self.nbytes = int(nbytes)
         self._parent = parent
         self.ptr = parent.ptr + int(offset_bytes)
-
-    def destroy(self):
-        self.ptr = 0

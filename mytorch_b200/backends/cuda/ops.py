@@ -12,6 +12,8 @@ the logical-dimension strides of either layout to the generic strided kernels.
 from __future__ import annotations
 
 import ctypes
+import math
+from array import array
 
 import numpy as np
 
@@ -19,26 +21,22 @@ from mytorch_b200.backends.backend_dispatcher import BackendDispatcher
 from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory
 from mytorch_b200.backends.utils import calculate_broadcast_shape, calculate_reduce_shape, calculate_reshaped_shape
 from mytorch_b200.dtype import float32, int32, int64
+from mytorch_b200.tensor import InvalidDataTypeError, MismatchShapesError, Tensor
 
 _reg = BackendDispatcher.instance().register_backend_function
 _LL = ctypes.c_longlong
+_on_device = Tensor._on_device
 
 
-def _T():
-    from mytorch_b200.tensor import Tensor
-
-    return Tensor
-
-
-def _env(t=None):
-    env = CudaEnv.instance()
-    if t is not None:
-        env.set_device(t.device.index)
+def _env(t):
+    env = CudaEnv._instance or CudaEnv.instance()
+    env.set_device(t.device.index)
     return env
 
 
 def _ptr(t):
-    return None if t is None else t._native_array.ptr
+    """A tensor as a pointer argument (the binding takes blocks as they are)."""
+    return None if t is None else t._native_array
 
 
 def _numel(shape):
@@ -49,7 +47,11 @@ def _numel(shape):
 
 
 def _new(shape, like, dtype=None):
-    return _T()(shape=tuple(shape), dtype=dtype or like.dtype, device=like.device)
+    dtype = dtype or like.dtype
+    n = dtype._itemsize
+    for s in shape:
+        n *= s
+    return _on_device(shape, dtype, like.device, CudaMemory(like.device.index, n))
 
 
 def _grad_buffer(param):
@@ -60,14 +62,10 @@ def _grad_buffer(param):
     slot = getattr(param, "_grad_slot", None)
     if slot is None or param.grad is not None:
         return _new(param.shape, param)
-    g = _T()(tensor=param)
-    g._native_array = slot
-    return g
+    return _on_device(param.shape, param.dtype, param.device, slot)
 
 
 def _f32(*tensors):
-    from mytorch_b200.tensor import InvalidDataTypeError
-
     for t in tensors:
         if t is not None and t.dtype is not float32:
             raise InvalidDataTypeError(t.dtype)
@@ -152,9 +150,7 @@ def _conv_args(x, w, stride, padding, cin=None):
         cin2 = cin
     cin = cin_x
     if cin != cin2:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([x.shape, w.shape])
+            raise MismatchShapesError([x.shape, w.shape])
     return (n, cin, h, wd, kh, kw, stride[0], stride[1], padding[0], padding[1], cout)
 
 
@@ -299,9 +295,7 @@ def cuda_linear(x, weight, bias):
     b, fin = x.shape
     fout = weight.shape[0]
     if weight.shape[1] != fin:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([x.shape, weight.shape])
+            raise MismatchShapesError([x.shape, weight.shape])
     y = _new((b, fout), x)
     _gemm(env, b, fout, fin, x, 0, weight, 1, bias, 0, y)
     return y
@@ -330,9 +324,7 @@ def cuda_mm(x, y):
     env = _env(x)
     (m, k), (k2, n) = x.shape, y.shape
     if k != k2:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([x.shape, y.shape])
+            raise MismatchShapesError([x.shape, y.shape])
     z = _new((m, n), x)
     _gemm(env, m, n, k, x, 0, y, 0, None, 0, z)
     return z
@@ -376,9 +368,7 @@ def cuda_batch_norm2d_add_relu(x, residual, weight, bias, eps, training, momentu
     """max(0, batch_norm2d(x) + residual) in one normalise pass; returns (y, mean, var)."""
     _f32(x, residual, weight, bias, running_mean, running_var)
     if x.shape != residual.shape:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([x.shape, residual.shape])
+            raise MismatchShapesError([x.shape, residual.shape])
     env = _env(x)
     n, c, h, w = x.shape
     y, mean, var = _new(x.shape, x), _new((c,), x), _new((c,), x)
@@ -504,9 +494,7 @@ def cuda_add_relu(x, y):
     """max(0, x + y) for same-shape operands (residual connection followed by ReLU)."""
     _f32(x, y)
     if x.shape != y.shape:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([x.shape, y.shape])
+            raise MismatchShapesError([x.shape, y.shape])
     env = _env(x)
     z = _new(x.shape, x)
     env.lib.add_relu_f32(_ptr(x), _ptr(y), _ptr(z), _numel(x.shape), env.stream())
@@ -552,9 +540,7 @@ def cuda_normal(x, seed, mean, stddev):
 def cuda_copy(dst, src):
     env = _env(dst)
     if dst.shape != src.shape:
-        from mytorch_b200.tensor import MismatchShapesError
-
-        raise MismatchShapesError([dst.shape, src.shape])
+            raise MismatchShapesError([dst.shape, src.shape])
     if dst.dtype is float32:
         env.lib.copy_f32(_ptr(dst), _ptr(src), _numel(dst.shape), env.stream())
     else:
@@ -711,8 +697,8 @@ def cuda_max(tensor, dim, keepdim):
         red_len, red_stride = tensor.shape[dim], st[dim]
         out_shape = calculate_reduce_shape(tensor.shape, (dim,), keepdim)
     n_out = _numel(out_shape)
-    values = _T()(shape=(n_out,), dtype=tensor.dtype, device=tensor.device)
-    indices = _T()(shape=tuple(out_shape), dtype=int64, device=tensor.device)
+    values = Tensor(shape=(n_out,), dtype=tensor.dtype, device=tensor.device)
+    indices = Tensor(shape=tuple(out_shape), dtype=int64, device=tensor.device)
     env.lib.max_strided_f32(_ptr(src), _ptr(values), _ptr(indices), len(kept_shape), _ll(kept_shape), _ll(kept_strides), red_len, red_stride,
                             env.stream())
     return cuda_reshape(values, tuple(out_shape)), indices
@@ -727,7 +713,7 @@ def cuda_max_backward(output_grad, indices_tensor, tensor, dim, keepdim):
     if _nontrivial_nhwc(g):  # the kernel reads dy in logical (dense) order, like the indices
         g = cuda_reshape(g, (_numel(g.shape),))
     if dim is None:
-        flat = _T()(shape=(_numel(tensor.shape),), dtype=tensor.dtype, device=tensor.device)
+        flat = Tensor(shape=(_numel(tensor.shape),), dtype=tensor.dtype, device=tensor.device)
         env.lib.max_backward_f32(_ptr(g), _ptr(indices_tensor), _ptr(flat), _numel(tensor.shape), 0, _ll([]), _ll([]), 1, env.stream())
         return [cuda_reshape(flat, tensor.shape)]
     dim = dim + nd if dim < 0 else dim
@@ -742,15 +728,13 @@ def cuda_max_backward(output_grad, indices_tensor, tensor, dim, keepdim):
 def cuda_eq(x, y):
     """int8 tensor of element-wise equality (``mytorch/backends/cuda/ops/eq.py:9``)."""
     from mytorch_b200.dtype import int8
-    from mytorch_b200.tensor import InvalidDataTypeError, MismatchShapesError
-
     if x.shape != y.shape:
         raise MismatchShapesError([x.shape, y.shape])
     kinds = {float32: 0, int64: 1}
     if x.dtype not in kinds or y.dtype is not x.dtype:
         raise InvalidDataTypeError(x.dtype)
     env = _env(x)
-    out = _T()(shape=x.shape, dtype=int8, device=x.device)
+    out = Tensor(shape=x.shape, dtype=int8, device=x.device)
     env.lib.eq_strided(kinds[x.dtype], len(x.shape), _ll(x.shape), _ll(_strides(x)), _ll(_strides(y)), _ptr(x), _ptr(y), _ptr(out), env.stream())
     return out
 
@@ -758,16 +742,15 @@ def cuda_eq(x, y):
 def _bmm_into(env, batch, m, n, k, a, ta, b, tb, c):
     """c[i] = op(a[i]) op(b[i]) for i < batch; dense 3-D operands, one GEMM per batch entry."""
     sa, sb, sc = 4 * (a.shape[1] * a.shape[2]), 4 * (b.shape[1] * b.shape[2]), 4 * m * n
+    pa, pb, pc = a._native_array.ptr, b._native_array.ptr, c._native_array.ptr
     for i in range(batch):
-        env.lib.gemm_f32(m, n, k, _ptr(a) + i * sa, ta, _ptr(b) + i * sb, tb, None, 0, _ptr(c) + i * sc, env.stream())
+        env.lib.gemm_f32(m, n, k, pa + i * sa, ta, pb + i * sb, tb, None, 0, pc + i * sc, env.stream())
 
 
 @_reg("cuda", "bmm")
 def cuda_bmm(x, y):
     """[B,M,K] x [B,K,N] -> [B,M,N] (``mytorch/backends/cuda/ops/mm.py:131-138``)."""
     _f32(x, y)
-    from mytorch_b200.tensor import MismatchShapesError
-
     if len(x.shape) != 3 or len(y.shape) != 3 or x.shape[0] != y.shape[0] or x.shape[2] != y.shape[1]:
         raise MismatchShapesError([x.shape, y.shape])
     env = _env(x)
@@ -811,7 +794,7 @@ def cuda_sum_scale(x, dim, keepdim, scale):
     xs = _strides(x)
     kept = [i for i in range(len(x.shape)) if i not in dim]
     red = list(dim)
-    dense = out if not _nontrivial_nhwc(out) else _T()(shape=(_numel(out_shape),), dtype=x.dtype, device=x.device)
+    dense = out if not _nontrivial_nhwc(out) else Tensor(shape=(_numel(out_shape),), dtype=x.dtype, device=x.device)
     env.lib.sum_strided_f32(_ptr(x), _ptr(dense), len(kept), _ll([x.shape[i] for i in kept]), _ll([xs[i] for i in kept]),
                             len(red), _ll([x.shape[i] for i in red]), _ll([xs[i] for i in red]), float(scale), st)
     if dense is not out:
@@ -847,28 +830,24 @@ def _dense_copy(env, t):
     """Logical row-major copy of a channels-last tensor."""
     n, c, h, w = t.shape
     out = CudaMemory(t.device.index, t._native_array.nbytes)
-    env.lib.nhwc_to_nchw_f32(_ptr(t), out.ptr, n, c, h, w, env.stream())
+    env.lib.nhwc_to_nchw_f32(_ptr(t), out, n, c, h, w, env.stream())
     return out
 
 
 @_reg("cuda", "reshape")
 def cuda_reshape(x, shape):
-    from mytorch_b200.tensor import channels_last
-
     env = _env(x)
     new_shape = calculate_reshaped_shape(x.shape, shape)
-    out = _T()(tensor=x)
-    out.shape = tuple(new_shape)
-    out._nhwc = channels_last(out.shape, out.dtype, "cuda")
+    new_shape = tuple(new_shape)
     mem = x._native_array
     if _nontrivial_nhwc(x):
         mem = _dense_copy(env, x)
+    out = _on_device(new_shape, x.dtype, x.device, mem)
     if _nontrivial_nhwc(out):
-        n, c, h, w = out.shape
+        n, c, h, w = new_shape
         dst = CudaMemory(x.device.index, mem.nbytes)
-        env.lib.nchw_to_nhwc_f32(mem.ptr, dst.ptr, n, c, h, w, env.stream())
-        mem = dst
-    out._native_array = mem
+        env.lib.nchw_to_nhwc_f32(mem, dst, n, c, h, w, env.stream())
+        out._native_array = dst
     return out
 
 
@@ -876,7 +855,7 @@ def cuda_reshape(x, shape):
 def cuda_permute(x, dims):
     _f32(x)
     env = _env(x)
-    out = _new([x.shape[d] for d in dims], x)
+    out = _new(tuple(x.shape[d] for d in dims), x)
     xs = _strides(x)
     src = [xs[d] for d in dims]
     env.lib.binary_strided_f32(5, len(dims), _ll(out.shape), _ll(src), _ll(src), _ll(_strides(out)), _ptr(x), None, _ptr(out), 1.0,
@@ -896,8 +875,6 @@ def cuda_permute_backward(output_grad, x, dims):
 
 @_reg("cuda", "cross_entropy")
 def cuda_cross_entropy(input, target):
-    from mytorch_b200.tensor import InvalidDataTypeError
-
     if target.dtype is not int64:
         raise InvalidDataTypeError(target.dtype)
     _f32(input)
@@ -941,13 +918,12 @@ def cuda_sgd_multi(entries, lr, weight_decay, momentum, dampening, nesterov, max
     if not entries:
         return
     env = _env(entries[0][0])
-    _refuse_first_step_in_capture(env, any(f for _, _, f in entries))
-    k = len(entries)
-    vp = ctypes.c_void_p
-    params = (vp * k)(*[_ptr(p) for p, _, _ in entries])
-    grads = (vp * k)(*[_ptr(p.grad) for p, _, _ in entries])
-    bufs = (vp * k)(*[_ptr(b) for _, b, _ in entries])
-    sizes = (_LL * k)(*[_numel(p.shape) for p, _, _ in entries])
-    first = (ctypes.c_int * k)(*[int(bool(f)) for _, _, f in entries])
-    env.lib.sgd_multi_f32(k, params, grads, bufs, sizes, first, float(lr), float(weight_decay), float(momentum), float(dampening),
+    _refuse_first_step_in_capture(env, any([f for _, _, f in entries]))
+    # host tables as the C side reads them (the binding passes the arrays' storage)
+    params = array("Q", [p._native_array.ptr for p, _, _ in entries])
+    grads = array("Q", [p.grad._native_array.ptr for p, _, _ in entries])
+    bufs = array("Q", [b._native_array.ptr for _, b, _ in entries])
+    sizes = array("q", [math.prod(p.shape) for p, _, _ in entries])
+    first = array("i", [1 if f else 0 for _, _, f in entries])
+    env.lib.sgd_multi_f32(len(entries), params, grads, bufs, sizes, first, float(lr), float(weight_decay), float(momentum), float(dampening),
                           int(bool(nesterov)), int(bool(maximize)), float(grad_scale), env.stream())

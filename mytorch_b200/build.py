@@ -1,4 +1,5 @@
-"""Builds the sm_100a kernel library in-tree: ``mytorch_b200/lib/libmytorch_b200.so``.
+"""Builds the sm_100a kernel library in-tree: ``mytorch_b200/lib/libmytorch_b200.so``, and beside it the CPython
+binding of its C ABI, ``_mtb_binding.so`` (``csrc/binding.cpp``, host compiler).
 
     python -m mytorch_b200.build [--force] [--verbose]
 
@@ -12,12 +13,14 @@ import concurrent.futures
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(HERE, "build")
 LIB = os.path.join(LIBDIR, "libmytorch_b200.so")
+BINDING = os.path.join(LIBDIR, "_mtb_binding.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -78,6 +81,14 @@ def build_library(force=False, verbose=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    src = os.path.join(CSRC, "binding.cpp")
+    if force or _stale(BINDING, [src, os.path.join(os.path.dirname(HERE), "include", "mytorch_b200.h")]):
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"],
+               src, "-o", BINDING, "-ldl"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("the binding did not compile")
     return LIB
 
 

@@ -1,0 +1,314 @@
+// CPython binding of the C ABI: one vectorcall function per entry point, and the device-memory object.
+//
+// What bounds it: a training step issued operator by operator makes about 300 library calls, and a step of a
+// small network is over in a fraction of a millisecond on the GPU, so the host's cost per call IS the step time.
+// Through ctypes one call of the convolution entry points (18 arguments) took 3-4 us, an allocation plus its
+// release 3.5 us.  Here the argument conversion is compiled per signature (taken from the public header, so the
+// two cannot drift apart), and a device block is a C object whose constructor and destructor call the pool
+// directly.  Host time to enqueue a step, before and after: the MNIST example at 64 images 1100 -> 616 us, ResNet-18
+// training 3230 -> 1530 us, ResNet-18 inference 1070 -> 408 us (with leaner tensor construction and tape loops).
+//
+// Nothing here touches CUDA: the kernel library is opened at run time (load()), so importing this module needs
+// neither a GPU nor the driver.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <dlfcn.h>
+#include <structmember.h>
+
+#include <string>
+#include <cstring>
+#include <tuple>
+#include <type_traits>
+#include <utility>
+
+#include "../../include/mytorch_b200.h"
+
+namespace {
+
+PyObject* g_error = nullptr;  // NativeError, handed over by load()
+PyObject* g_first_use = nullptr;  // called when memory is asked for before load(): sets the CUDA state up or raises
+const char* (*g_last_error)() = nullptr;
+long long g_launches = 0;
+
+// ------------------------------------------------------------------ device memory
+
+struct Block {
+  PyObject_HEAD
+  unsigned long long ptr;
+  long long nbytes;
+  int device_index;
+  char owned;  // a view of another block owns nothing
+};
+PyTypeObject BlockType = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+// ------------------------------------------------------------------ argument conversion
+
+inline bool from_py(PyObject* o, int& v) {
+  const long x = PyLong_AsLong(o);
+  if (x == -1 && PyErr_Occurred()) return false;
+  if (x != (int)x) { PyErr_SetString(PyExc_OverflowError, "argument does not fit a C int"); return false; }
+  v = (int)x;
+  return true;
+}
+inline bool from_py(PyObject* o, long long& v) {
+  v = PyLong_AsLongLong(o);
+  return !(v == -1 && PyErr_Occurred());
+}
+inline bool from_py(PyObject* o, double& v) {
+  v = PyFloat_AsDouble(o);
+  return !(v == -1.0 && PyErr_Occurred());
+}
+inline bool from_py(PyObject* o, float& v) {
+  double d;
+  if (!from_py(o, d)) return false;
+  v = (float)d;
+  return true;
+}
+
+// An address that is neither None, an integer nor a block: a ctypes byref(), array or scalar (its storage), or a
+// ctypes pointer value.
+bool address_of(PyObject* o, void*& v) {
+  PyObject* target = PyObject_GetAttrString(o, "_obj");  // byref(x)
+  const bool by_reference = target != nullptr;
+  if (!target) { PyErr_Clear(); Py_INCREF(o); target = o; }
+  if (!by_reference && !strcmp(Py_TYPE(o)->tp_name, "c_void_p")) {
+    PyObject* value = PyObject_GetAttrString(o, "value");
+    Py_DECREF(target);
+    if (!value) return false;
+    v = value == Py_None ? nullptr : PyLong_AsVoidPtr(value);
+    Py_DECREF(value);
+    return !PyErr_Occurred();
+  }
+  Py_buffer view;
+  const int rc = PyObject_GetBuffer(target, &view, PyBUF_SIMPLE);
+  Py_DECREF(target);  // the caller's argument keeps the storage alive during the call
+  if (rc) return false;
+  v = view.buf;
+  PyBuffer_Release(&view);
+  return true;
+}
+template <class T>
+inline bool from_py(PyObject* o, T*& v) {
+  if (o == Py_None) { v = nullptr; return true; }
+  if (PyLong_CheckExact(o)) {
+    v = (T*)PyLong_AsVoidPtr(o);
+    return !(v == nullptr && PyErr_Occurred());
+  }
+  if (PyObject_TypeCheck(o, &BlockType)) { v = (T*)((Block*)o)->ptr; return true; }
+  void* p = nullptr;
+  if (!address_of(o, p)) return false;
+  v = (T*)p;
+  return true;
+}
+
+inline PyObject* to_py(int v) { return PyLong_FromLong(v); }
+inline PyObject* to_py(long long v) { return PyLong_FromLongLong(v); }
+inline PyObject* to_py(void* v) { return PyLong_FromVoidPtr(v); }
+
+// ------------------------------------------------------------------ one function per entry point
+
+enum Kind {
+  LAUNCH,   // status; counted as work enqueued on the GPU
+  STATUS,   // status; bookkeeping
+  POINTER,  // NULL means failure
+  VALUE,    // host arithmetic: the result itself
+};
+
+PyObject* raise_native(const char* name, int rc) {
+  if (rc) PyErr_Format(g_error, "%s failed (%d): %s", name, rc, g_last_error());
+  else PyErr_Format(g_error, "%s failed: %s", name, g_last_error());
+  return nullptr;
+}
+
+template <int ID, Kind K, class Sig>
+struct Entry;
+template <int ID, Kind K, class R, class... A>
+struct Entry<ID, K, R(A...)> {
+  static inline R (*fn)(A...) = nullptr;
+  static inline const char* name = nullptr;
+
+  template <size_t... I>
+  static PyObject* invoke(PyObject* const* args, std::index_sequence<I...>) {
+    std::tuple<A...> a;
+    if (!(from_py(args[I], std::get<I>(a)) && ... && true)) return nullptr;
+    if constexpr (K == VALUE) {
+      return to_py(fn(std::get<I>(a)...));
+    } else {
+      // released: a launch waits when the stream's queue is full, and other Python threads feed it meanwhile
+      R r;
+      Py_BEGIN_ALLOW_THREADS
+      r = fn(std::get<I>(a)...);
+      Py_END_ALLOW_THREADS
+      if constexpr (K == POINTER) {
+        if (!r) return raise_native(name, 0);
+      } else {
+        if (r) return raise_native(name, r);
+        if (K == LAUNCH) ++g_launches;
+      }
+      return to_py(r);
+    }
+  }
+  static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (!fn) { PyErr_SetString(PyExc_RuntimeError, "the kernel library is not loaded"); return nullptr; }
+    if (n != (Py_ssize_t)sizeof...(A)) {
+      PyErr_Format(PyExc_TypeError, "%s takes %zu arguments (%zd given)", name, sizeof...(A), n);
+      return nullptr;
+    }
+    return invoke(args, std::index_sequence_for<A...>{});
+  }
+};
+
+#define MTB_ENTRIES(X) \
+  X(version, VALUE) X(device_check, STATUS) X(fill_f32, LAUNCH) X(copy_f32, LAUNCH) X(scale_f32, LAUNCH) X(relu_forward_f32, LAUNCH) \
+  X(relu_backward_f32, LAUNCH) X(add_f32, LAUNCH) X(mul_f32, LAUNCH) X(add_bias_rows_f32, LAUNCH) X(binary_strided_f32, LAUNCH) \
+  X(resize_channels_f32, LAUNCH) X(nchw_to_nhwc_f32, LAUNCH) X(nhwc_to_nchw_f32, LAUNCH) X(cast, LAUNCH) \
+  X(batch_norm2d_workspace_bytes, VALUE) X(batch_norm2d_forward_f32, LAUNCH) X(batch_norm2d_backward_f32, LAUNCH) \
+  X(batch_norm2d_add_relu_forward_f32, LAUNCH) X(batch_norm2d_add_relu_backward_f32, LAUNCH) X(add_relu_f32, LAUNCH) \
+  X(add_relu_backward_f32, LAUNCH) X(colsum_workspace_bytes, VALUE) X(colsum_f32, LAUNCH) X(colsum_noalloc_f32, LAUNCH) \
+  X(nhwc_spatial_sum_f32, LAUNCH) X(nhwc_spatial_bcast_f32, LAUNCH) X(sum_strided_f32, LAUNCH) X(max_strided_f32, LAUNCH) \
+  X(max_backward_f32, LAUNCH) X(eq_strided, LAUNCH) X(max_pool2d_forward_f32, LAUNCH) X(max_pool2d_backward_f32, LAUNCH) \
+  X(max_pool2d_argmax_u8, LAUNCH) X(cross_entropy_workspace_bytes, VALUE) X(cross_entropy_forward_f32, LAUNCH) \
+  X(cross_entropy_backward_f32, LAUNCH) X(sgd_f32, LAUNCH) X(sgd_multi_f32, LAUNCH) X(pack_scale_f32, LAUNCH) \
+  X(conv2d_workspace_bytes, VALUE) X(conv2d_plan_f32, STATUS) X(conv2d_forward_f32, LAUNCH) X(conv2d_stats_max_rows, VALUE) \
+  X(conv2d_forward_stats_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
+  X(conv2d_dgrad_add_f32, LAUNCH) X(conv2d_dgrad_accumulates_in_place, VALUE) X(conv2d_wgrad_f32, LAUNCH) X(gemm_f32, LAUNCH) \
+  X(tc_status, STATUS) X(tc_wait_selftest, LAUNCH) \
+  X(malloc, POINTER) X(free, STATUS) X(pool_reserved_bytes, VALUE) X(pool_in_use_bytes, VALUE) X(pool_trim, STATUS) X(set_device, STATUS) \
+  X(get_device, STATUS) X(device_count, STATUS) X(device_synchronize, STATUS) X(mem_get_info, STATUS) X(memcpy_h2d_async, STATUS) \
+  X(memcpy_d2h_async, STATUS) X(memcpy_d2d_async, STATUS) X(memset_async, STATUS) X(host_alloc_pinned, POINTER) X(host_free_pinned, STATUS) \
+  X(stream_create, POINTER) X(stream_destroy, STATUS) X(stream_synchronize, STATUS) X(stream_wait_event, STATUS) X(event_create, POINTER) \
+  X(event_destroy, STATUS) X(event_record, STATUS) X(event_synchronize, STATUS) X(event_elapsed_ms, STATUS) X(graph_begin_capture, STATUS) \
+  X(graph_end_capture, STATUS) X(graph_launch, STATUS) X(graph_destroy, STATUS)
+
+#define X(n, k) ID_##n,
+enum EntryId { MTB_ENTRIES(X) kEntries };
+#undef X
+#define X(n, k) using E_##n = Entry<ID_##n, k, std::remove_pointer_t<decltype(&mtb_##n)>>;
+MTB_ENTRIES(X)
+#undef X
+
+// ------------------------------------------------------------------ Block
+
+int block_init(PyObject* self, PyObject* args, PyObject* kwargs) {
+  static const char* names[] = {"device_index", "nbytes", nullptr};
+  PyObject* device = nullptr;
+  long long nbytes = 0;
+  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "OL", (char**)names, &device, &nbytes)) return -1;
+  if (!E_malloc::fn) {
+    PyObject* r = g_first_use ? PyObject_CallNoArgs(g_first_use) : nullptr;
+    if (!r) return -1;
+    Py_DECREF(r);
+    if (!E_malloc::fn) { PyErr_SetString(PyExc_RuntimeError, "the kernel library is not loaded"); return -1; }
+  }
+  Block* b = (Block*)self;
+  int current = 0;
+  if (int rc = E_get_device::fn(&current)) { raise_native("mtb_get_device", rc); return -1; }
+  int want = current;
+  if (device != Py_None && !from_py(device, want)) return -1;
+  if (want != current)
+    if (int rc = E_set_device::fn(want)) { raise_native("mtb_set_device", rc); return -1; }
+  void* p = E_malloc::fn(nbytes > 0 ? nbytes : 1);
+  if (!p) { raise_native("mtb_malloc", 0); return -1; }
+  if (b->owned && b->ptr) E_free::fn((void*)b->ptr);
+  b->ptr = (unsigned long long)p;
+  b->nbytes = nbytes;
+  b->device_index = want;
+  b->owned = 1;
+  return 0;
+}
+void block_release(Block* b) {
+  if (b->owned && b->ptr && E_free::fn) E_free::fn((void*)b->ptr);
+  b->ptr = 0;
+  b->owned = 0;
+}
+void block_dealloc(PyObject* self) {
+  block_release((Block*)self);
+  Py_TYPE(self)->tp_free(self);
+}
+PyObject* block_destroy(PyObject* self, PyObject*) {
+  block_release((Block*)self);
+  Py_RETURN_NONE;
+}
+PyMemberDef block_members[] = {
+    {"ptr", T_ULONGLONG, offsetof(Block, ptr), 0, "device address"},
+    {"nbytes", T_LONGLONG, offsetof(Block, nbytes), 0, "size in bytes"},
+    {"device_index", T_INT, offsetof(Block, device_index), 0, "device the block lives on"},
+    {nullptr, 0, 0, 0, nullptr}};
+PyMethodDef block_methods[] = {{"destroy", block_destroy, METH_NOARGS, "Give the block back to the pool now."}, {nullptr, nullptr, 0, nullptr}};
+
+// ------------------------------------------------------------------ module
+
+// load(path, error_class): open the kernel library and resolve every entry point.
+PyObject* load(PyObject*, PyObject* args) {
+  const char* path;
+  PyObject* error;
+  if (!PyArg_ParseTuple(args, "sO", &path, &error)) return nullptr;
+  void* dll = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (!dll) { PyErr_Format(error, "cannot open %s: %s", path, dlerror()); return nullptr; }
+  Py_INCREF(error);
+  Py_XSETREF(g_error, error);
+  auto find = [&](const char* name) {
+    void* p = dlsym(dll, name);
+    if (!p) PyErr_Format(error, "%s does not export %s", path, name);
+    return p;
+  };
+  if (!(g_last_error = (decltype(g_last_error))find("mtb_last_error"))) return nullptr;
+#define X(n, k) \
+  E_##n::name = "mtb_" #n; \
+  if (!(E_##n::fn = (decltype(E_##n::fn))find("mtb_" #n))) return nullptr;
+  MTB_ENTRIES(X)
+#undef X
+  Py_RETURN_NONE;
+}
+
+PyObject* on_first_use(PyObject*, PyObject* f) {
+  Py_INCREF(f);
+  Py_XSETREF(g_first_use, f);
+  Py_RETURN_NONE;
+}
+
+// Entry-point calls so far that enqueue kernels.
+PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
+
+PyObject* current_device(PyObject*, PyObject*) {
+  int device = 0;
+  if (!E_get_device::fn) { PyErr_SetString(PyExc_RuntimeError, "the kernel library is not loaded"); return nullptr; }
+  if (int rc = E_get_device::fn(&device)) return raise_native("mtb_get_device", rc);
+  return PyLong_FromLong(device);
+}
+
+PyMethodDef methods[] = {
+    {"load", load, METH_VARARGS, nullptr},
+    {"on_first_use", on_first_use, METH_O, nullptr},
+    {"launches", launches, METH_NOARGS, nullptr},
+    {"current_device", current_device, METH_NOARGS, nullptr},
+#define X(n, k) {#n, (PyCFunction)(void (*)())E_##n::call, METH_FASTCALL, nullptr},
+    MTB_ENTRIES(X)
+#undef X
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_mtb_binding", "C ABI of libmytorch_b200.so", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__mtb_binding() {
+  BlockType.tp_name = "mytorch_b200.Block";
+  BlockType.tp_basicsize = sizeof(Block);
+  BlockType.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE;
+  BlockType.tp_doc = "A device allocation from the library's pool.";
+  BlockType.tp_new = PyType_GenericNew;
+  BlockType.tp_init = block_init;
+  BlockType.tp_dealloc = block_dealloc;
+  BlockType.tp_members = block_members;
+  BlockType.tp_methods = block_methods;
+  if (PyType_Ready(&BlockType) < 0) return nullptr;
+  PyObject* m = PyModule_Create(&module);
+  if (!m) return nullptr;
+  PyObject* names = PyTuple_New(kEntries);
+#define X(n, k) PyTuple_SET_ITEM(names, ID_##n, PyUnicode_FromString("mtb_" #n));
+  MTB_ENTRIES(X)
+#undef X
+  Py_INCREF(&BlockType);
+  if (PyModule_AddObject(m, "entry_points", names) < 0 || PyModule_AddObject(m, "Block", (PyObject*)&BlockType) < 0) return nullptr;
+  return m;
+}

@@ -10,13 +10,14 @@ class DType:
         self.np_dtype = np_dtype
         self.cuda_dtype = cuda_dtype
         self.is_floating = is_floating
+        self._itemsize = np.dtype(np_dtype).itemsize
         DType._registry[name] = self
 
     def __repr__(self):
         return self.name
 
     def itemsize(self):
-        return np.dtype(self.np_dtype).itemsize
+        return self._itemsize
 
     @staticmethod
     def from_np_dtype(np_dtype):

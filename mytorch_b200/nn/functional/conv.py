@@ -7,11 +7,10 @@ def conv2d(input: Tensor, weight: Tensor, bias=None, stride=1, padding=0, bn_sta
     """``bn_stats`` (no counterpart in the reference): the result goes straight into a BatchNorm layer
     in training mode; the CUDA backend then lets the convolution reduce the batch statistics of its
     own output, which BatchNorm picks up instead of re-reading the tensor.  Results are unchanged."""
-    tensors = [input, weight] + ([bias] if bias is not None else [])
-    if any(t.device != input.device for t in tensors):
-        raise MismatchDevicesError([t.device for t in tensors])
-    if any(t.dtype != input.dtype for t in tensors):
-        raise MismatchDataTypesError([t.dtype for t in tensors])
+    if weight.device is not input.device or (bias is not None and bias.device is not input.device):
+        raise MismatchDevicesError([t.device for t in (input, weight, bias) if t is not None])
+    if weight.dtype is not input.dtype or (bias is not None and bias.dtype is not input.dtype):
+        raise MismatchDataTypesError([t.dtype for t in (input, weight, bias) if t is not None])
     stride = (stride, stride) if isinstance(stride, int) else tuple(stride)
     padding = (padding, padding) if isinstance(padding, int) else tuple(padding)
     if bn_stats and input.device.type == "cuda":

@@ -6,11 +6,17 @@ tracker = DAGTracker.instance()
 
 
 def dispatch(device, name):
-    return BackendDispatcher.instance().dispatch(device.type, name)
+    registry = BackendDispatcher._instance or BackendDispatcher.instance()
+    return registry.dispatch(device.type, name)
 
 
 def grad_enabled(*tensors):
-    return any(t is not None and t.requires_grad for t in tensors) and not tracker.no_grad
+    if tracker.no_grad:
+        return False
+    for t in tensors:
+        if t is not None and t.requires_grad:
+            return True
+    return False
 
 
 def record(name, inputs, output, helpers=None):

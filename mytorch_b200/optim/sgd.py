@@ -16,18 +16,22 @@ class SGD(Optimizer):
     def step(self):
         dispatcher = BackendDispatcher.instance()
         for group in self.param_groups:
-            entries = []
+            entries, states = [], self.state
+            devices = set()
             for param in group["params"]:
                 if param.shape != param.grad.shape:
                     raise RuntimeError(f"Mismatched shape between param and param.grad: {param}, {param.grad}")
-                state = self.state.setdefault(param, {})
-                first = state.get("momentum_buffer") is None
+                state = states.get(param)
+                if state is None:
+                    state = states[param] = {}
+                buffer = state.get("momentum_buffer")
+                first = buffer is None
                 if first:
-                    state["momentum_buffer"] = Tensor(shape=param.shape, device=param.device, dtype=param.dtype)
-                entries.append((param, state["momentum_buffer"], first))
+                    buffer = state["momentum_buffer"] = Tensor(shape=param.shape, device=param.device, dtype=param.dtype)
+                entries.append((param, buffer, first))
+                devices.add(param.device)
             hyper = (group["lr"], group["weight_decay"], group["momentum"], group["dampening"], group["nesterov"], group["maximize"])
-            devices = {(p.device.type, p.device.index) for p, _, _ in entries}
-            if len(devices) == 1 and next(iter(devices))[0] == "cuda":
+            if len(devices) == 1 and next(iter(devices)).type == "cuda":
                 dispatcher.dispatch("cuda", "sgd_multi")(entries, *hyper, self.grad_scale)
             else:
                 for param, buf, first in entries:

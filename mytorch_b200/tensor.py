@@ -52,22 +52,30 @@ def shape_size(shape):
 
 
 class Device:
-    """``"cpu"``, ``"cuda"`` or ``"cuda:<index>"`` (mytorch/tensor.py:52-81)."""
+    """``"cpu"``, ``"cuda"`` or ``"cuda:<index>"`` (mytorch/tensor.py:52-81).  One object per device: equality is
+    identity, so the checks every operator makes cost nothing."""
 
-    def __init__(self, device):
+    _known = {}
+
+    def __new__(cls, device=None):
+        if device is None:  # unpickling: the state follows, and Device(that object) is the known one
+            return object.__new__(cls)
         if isinstance(device, Device):
-            self.type, self.index = device.type, device.index
-            return
-        text = device.strip()
-        head, sep, tail = text.partition(":")
-        self.type = head.strip()
-        self.index = int(tail) if sep else None
+            return cls._known.setdefault((device.type, device.index), device)
+        found = cls._known.get(device)
+        if found is None:
+            head, sep, tail = device.strip().partition(":")
+            key = (head.strip(), int(tail) if sep else None)
+            found = cls._known.get(key)
+            if found is None:
+                found = object.__new__(cls)
+                found.type, found.index = key
+                found = cls._known.setdefault(key, found)
+            cls._known[device] = found
+        return found
 
-    def __eq__(self, other):
-        return isinstance(other, Device) and self.type == other.type and self.index == other.index
-
-    def __hash__(self):
-        return hash((self.type, self.index))
+    def __reduce__(self):
+        return (Device, (repr(self),))
 
     def __repr__(self):
         return self.type if self.index is None else f"{self.type}:{self.index}"
@@ -82,6 +90,9 @@ def channels_last(shape, dtype, device_type):
     return device_type == "cuda" and len(shape) == 4 and dtype is float32
 
 
+_new_object = object.__new__
+
+
 def tensor(data, dtype=None, device=None, requires_grad=False):
     data = np.array(data)
     if dtype is not None:
@@ -90,11 +101,27 @@ def tensor(data, dtype=None, device=None, requires_grad=False):
 
 
 class Tensor:
+    # what most tensors are; instances only store what differs (every operator of a training step makes some)
+    requires_grad = False
+    grad = None
+    _grad_node = None
+    _cpu_array = None
+
+    @staticmethod
+    def _on_device(shape, dtype, device, memory):
+        """A CUDA tensor over ``memory``: what the operators make their results with.  Nothing is parsed or
+        checked: ``shape`` is a tuple of ints, ``device`` a CUDA ``Device`` (shared, never modified)."""
+        t = _new_object(Tensor)
+        t.shape = shape
+        t.dtype = dtype
+        t.device = device
+        t._nhwc = dtype is float32 and len(shape) == 4
+        t._native_array = memory
+        return t
+
     def __init__(self, cpu_array=None, dtype: Optional[DType] = None, shape=None, device=None,
                  tensor: Optional["Tensor"] = None, requires_grad: bool = False):
         self.requires_grad = requires_grad
-        self.grad = None
-        self._grad_node = None
 
         if tensor is not None:  # alias: shares storage with `tensor`
             self._cpu_array = tensor._cpu_array
