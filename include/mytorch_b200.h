@@ -127,6 +127,11 @@ int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, i
  * C[M,N] = op(A) op(B) (+ bias[N]) (relu). A is [M,K] (trans_a 0) or [K,M]; B is [K,N] (trans_b 0) or [N,K]. */
 int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                  void* stream);
+/* The same with scratch of mtb_gemm_workspace_bytes() (0 = none needed): products with few output tiles and a long
+ * reduction split it across CTAs, the partials are added in a fixed order. */
+long long mtb_gemm_workspace_bytes(int m, int n, int k);
+int mtb_gemm_ws_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
+                    void* workspace, long long workspace_bytes, void* stream);
 
 /* ---- BatchNorm2d (replaces batch_norm2d_reference_<dt> and its backward,
  *      mytorch/native/cuda/batch_norm.cu/source.cu:134-166 and :269-289) ---- */

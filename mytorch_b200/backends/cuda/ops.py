@@ -285,7 +285,8 @@ def _colsum(env, mat, rows, cols, like, scale=1.0, out=None):
 # ---------------------------------------------------------------------------- linear / mm
 
 def _gemm(env, m, n, k, a, ta, b, tb, bias, relu, c):
-    env.lib.gemm_f32(m, n, k, _ptr(a), ta, _ptr(b), tb, _ptr(bias), relu, _ptr(c), env.stream())
+    ws, ws_bytes = env.workspace(env.lib.gemm_workspace_bytes(m, n, k))
+    env.lib.gemm_ws_f32(m, n, k, _ptr(a), ta, _ptr(b), tb, _ptr(bias), relu, _ptr(c), ws, ws_bytes, env.stream())
 
 
 @_reg("cuda", "linear")

@@ -172,6 +172,7 @@ struct Entry<ID, K, R(A...)> {
   X(conv2d_workspace_bytes, VALUE) X(conv2d_plan_f32, STATUS) X(conv2d_forward_f32, LAUNCH) X(conv2d_stats_max_rows, VALUE) \
   X(conv2d_forward_stats_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
   X(conv2d_dgrad_add_f32, LAUNCH) X(conv2d_dgrad_accumulates_in_place, VALUE) X(conv2d_wgrad_f32, LAUNCH) X(gemm_f32, LAUNCH) \
+  X(gemm_workspace_bytes, VALUE) X(gemm_ws_f32, LAUNCH) \
   X(tc_status, STATUS) X(tc_wait_selftest, LAUNCH) \
   X(malloc, POINTER) X(free, STATUS) X(pool_reserved_bytes, VALUE) X(pool_in_use_bytes, VALUE) X(pool_trim, STATUS) X(set_device, STATUS) \
   X(get_device, STATUS) X(device_count, STATUS) X(device_synchronize, STATUS) X(mem_get_info, STATUS) X(memcpy_h2d_async, STATUS) \

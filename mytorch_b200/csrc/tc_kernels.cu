@@ -549,15 +549,15 @@ int pick_bn_for(int n, long long rows) {
 // (tiles x splits <= SMs) and every unit keeps at least eight reduction blocks.
 struct GemmPlan { int bn, splits, kb_per_split; };
 
-GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, int force_bn = 0) {
+GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, int force_bn = 0, int min_kb = 64) {
   const int sms = mtb_sm_count();
   const long long m_tiles = (rows + 127) / 128;
-  static const int kSplits[] = {1, 2, 3, 4, 6, 8};
+  static const int kSplits[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
   GemmPlan best{force_bn ? force_bn : pick_bn_for(n, rows), 1, num_kb};
   // Measured: the split only pays when even 64-wide tiles leave half the GPU idle (the 4x4 layers at 64
   // images: 41 -> 24 us for the data gradient of 512 -> 512); with more tiles than that the last unit's pass
   // over the partials costs more than the idle SMs did (256 -> 256 on 8x8 at 64 images: 20 -> 40 us).
-  if (m_tiles * ((n + 63) / 64) > sms / 2 || num_kb < 64) may_split = false;  // short reductions gain nothing either
+  if (m_tiles * ((n + 63) / 64) > sms / 2 || num_kb < min_kb) may_split = false;  // short reductions gain nothing either
   if (!may_split || getenv("MTB_DISABLE_SPLITK")) return best;
   double best_ns = 1e30;
   for (int bn = force_bn ? force_bn : pick_bn(n); bn >= (force_bn ? force_bn : 64); bn >>= 1) {
@@ -658,10 +658,18 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
   return true;
 }
 
+// Tile width and split of a plain GEMM.  A Linear layer over few samples has one or two output tiles and a long
+// reduction ([64 x 9216] x [9216 x 128]: two CTAs walked 288 blocks each, 57 us); with scratch its reduction is split.
+static GemmPlan plan_dense(int m, int n, int k) { return plan_gemm(n, m, (k + 31) / 32, true, 0, 32); }
+
+long long mtb_tc_gemm_workspace_bytes(int m, int n, int k) { return split_partial_bytes(plan_dense(m, n, k), m, n); }
+
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* stream) {
+                    void* workspace, long long workspace_bytes, void* stream) {
   CUtensorMap mapA, mapB;
-  int bn = pick_bn_for(n, m);
+  GemmPlan gp = plan_dense(m, n, k);
+  if (!workspace || split_partial_bytes(gp, m, n) > workspace_bytes) gp = GemmPlan{pick_bn_for(n, m), 1, (k + 31) / 32};
+  const int bn = gp.bn;
   int rc;
   if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, 128);
   else rc = tc::encode_tiled_2d(&mapA, a, k, m, m, 32, 32, true);
@@ -670,7 +678,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   else rc = tc::encode_tiled_2d(&mapB, b, k, n, n, 32, 32, true);
   if (rc) return rc;
   GemmParams p{};
-  p.splits = 1; p.kb_per_split = (k + 31) / 32;
+  p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
   p.M = m; p.N = n; p.num_kb = (k + 31) / 32;
   p.m_tiles = (m + 127) / 128; p.n_tiles = (n + bn - 1) / bn;
   p.out = c; p.ldo = n; p.bias = bias; p.relu = relu;
