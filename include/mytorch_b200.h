@@ -127,11 +127,6 @@ int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, i
  * C[M,N] = op(A) op(B) (+ bias[N]) (relu). A is [M,K] (trans_a 0) or [K,M]; B is [K,N] (trans_b 0) or [N,K]. */
 int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                  void* stream);
-/* The same with scratch of mtb_gemm_workspace_bytes() (0 = none needed): products with few output tiles and a long
- * reduction split it across CTAs, the partials are added in a fixed order. */
-long long mtb_gemm_workspace_bytes(int m, int n, int k);
-int mtb_gemm_ws_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* workspace, long long workspace_bytes, void* stream);
 
 /* ---- BatchNorm2d (replaces batch_norm2d_reference_<dt> and its backward,
  *      mytorch/native/cuda/batch_norm.cu/source.cu:134-166 and :269-289) ---- */
@@ -196,6 +191,9 @@ int mtb_binary_strided_f32(int op, int ndim, const long long* shape, const long 
 /* dst[rows][c_dst] from src[rows][c_src]: extra channels are zero, surplus channels are dropped (channel
  * padding of the image stem for the tensor-core convolution; no counterpart in the reference) */
 int mtb_resize_channels_f32(const float* src, float* dst, long long rows, int c_src, int c_dst, void* stream);
+/* out[N][OH][OW][32]: the kh*kw*c (<= 32) input values each output pixel's filter sees, in filter order, then zeros: a
+ * convolution over few input channels becomes one over a block of 32 channels (no counterpart in the reference) */
+int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, const float* x, float* out, void* stream);
 int mtb_nchw_to_nhwc_f32(const float* src, float* dst, int n, int c, int h, int w, void* stream);
 int mtb_nhwc_to_nchw_f32(const float* src, float* dst, int n, int c, int h, int w, void* stream);
 /* kind: 0 int32->int64, 1 int64->float32, 2 float32->int64, 3 int8->float32 (replaces cast_reference, cast.cu/source.cu:5-14) */

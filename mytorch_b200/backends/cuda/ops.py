@@ -17,12 +17,14 @@ from array import array
 
 import numpy as np
 
+from mytorch_b200.autograd import DAGTracker
 from mytorch_b200.backends.backend_dispatcher import BackendDispatcher
 from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory
 from mytorch_b200.backends.utils import calculate_broadcast_shape, calculate_reduce_shape, calculate_reshaped_shape
 from mytorch_b200.dtype import float32, int32, int64
 from mytorch_b200.tensor import InvalidDataTypeError, MismatchShapesError, Tensor
 
+_tracker = DAGTracker.instance()
 _reg = BackendDispatcher.instance().register_backend_function
 _LL = ctypes.c_longlong
 _on_device = Tensor._on_device
@@ -141,29 +143,59 @@ def cuda_download(t):
 
 # ---------------------------------------------------------------------------- convolution
 
-def _conv_args(x, w, stride, padding, cin=None):
-    """(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout); `cin` overrides the filter's channel count when
-    the activation has been padded to a channel block but the filter has not."""
-    n, cin_x, h, wd = x.shape
+def _conv_args(x, w, stride, padding):
+    """(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout)"""
+    n, cin, h, wd = x.shape
     cout, cin2, kh, kw = w.shape
-    if cin is not None:
-        cin2 = cin
-    cin = cin_x
     if cin != cin2:
-            raise MismatchShapesError([x.shape, w.shape])
+        raise MismatchShapesError([x.shape, w.shape])
     return (n, cin, h, wd, kh, kw, stride[0], stride[1], padding[0], padding[1], cout)
 
 
 _TC_CHANNELS = 32  # the tensor-core convolution reads activations in blocks of 32 channels
 
 
-def _wants_channel_padding(x):
-    """Image stems (1 or 3 input channels) would otherwise run on the CUDA-core kernels; padding
-    their few channels with zeros up to one 32-channel block lets them use the tensor-core path
-    (extra zero FLOPs are far cheaper than the FFMA kernel) when the padded tensor is large enough
-    for that path to accept it."""
+def _stem_form(x_shape, w_shape, stride, padding):
+    """How a convolution over fewer than 32 channels (an image stem) reaches the tensor-core kernels, or None when it
+    does not (too small for them, or an output width they do not take).
+
+    ``(pack, args)``: ``mtb_pack_patches_f32`` with the window ``pack`` = (kh, kw, sh, sw, ph, pw) turns the input into
+    blocks of 32 channels, on which the convolution has the arguments ``args``.  Where the whole filter fits 32 entries (3x3
+    over 3 channels) the window disappears and each output reads one block; where one filter row does (7x7 over 3
+    channels: 21) a window of a single column stays, 7 blocks instead of the 49 of zero-padded channels.
+    ``pack`` is None where not even a row fits: the channels are padded with zeros to one block."""
+    n, c, h, w = x_shape
+    cout, _, kh, kw = w_shape
+    (sh, sw), (ph, pw) = stride, padding
+    if c >= _TC_CHANNELS or cout % 4 or n * h * w * _TC_CHANNELS * 4 < (1 << 17):
+        return None
+    oh, ow = (h + 2 * ph - kh) // sh + 1, (w + 2 * pw - kw) // sw + 1
+    if c == 1:  # 28x28 digits: no gain was measured from fewer blocks (the step is all launches), so the form stays
+        return None, (n, _TC_CHANNELS, h, w, kh, kw, sh, sw, ph, pw, cout)
+    if kh * kw * c <= _TC_CHANNELS:
+        return (kh, kw, sh, sw, ph, pw), (n, _TC_CHANNELS, oh, ow, 1, 1, 1, 1, 0, 0, cout)
+    if kw * c <= _TC_CHANNELS:
+        return (1, kw, 1, sw, 0, pw), (n, _TC_CHANNELS, h, ow, kh, 1, sh, 1, ph, 0, cout)
+    return None, (n, _TC_CHANNELS, h, w, kh, kw, sh, sw, ph, pw, cout)
+
+
+def _stem_input(env, x, form):
+    """The input in the form the convolution reads."""
+    pack, args = form
+    if pack is None:
+        return _pad_channels(env, x, _TC_CHANNELS)
     n, c, h, w = x.shape
-    return c < _TC_CHANNELS and n * h * w * _TC_CHANNELS * 4 >= (1 << 17)
+    out = _new((n, _TC_CHANNELS, args[2], args[3]), x)
+    env.lib.pack_patches_f32(n, c, h, w, *pack, _ptr(x), _ptr(out), env.stream())
+    return out
+
+
+def _stem_filter_rows(w_shape, form):
+    """(rows, entries per row) of the filter as that form reads it: a row is widened to one block of 32."""
+    cout, c, kh, kw = w_shape
+    if form[0] is None:
+        return cout * kh * kw, c
+    return cout * form[1][4], form[0][0] * kw * c
 
 
 def _pad_channels(env, t, channels):
@@ -190,12 +222,19 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
     _f32(input, weight, bias)
     env = _env(input)
     x, wt = input, weight
-    if _wants_channel_padding(input):
-        x, wt = _pad_channels(env, input, _TC_CHANNELS), _pad_channels(env, weight, _TC_CHANNELS)
-        input._padded_for_conv = x  # backward of this convolution reuses it (the weight gradient reads x again)
     a = _conv_args(x, wt, stride, padding)
     n, cin, h, w, kh, kw, sh, sw, ph, pw, cout = a
     oh, ow = (h + 2 * ph - kh) // sh + 1, (w + 2 * pw - kw) // sw + 1
+    form = _stem_form(x.shape, wt.shape, stride, padding) if cin < _TC_CHANNELS else None
+    if form is not None:
+        a = form[1]
+        x = _stem_input(env, input, form)
+        if weight.requires_grad and not _tracker.no_grad:
+            input._stem_held = (form, x)  # the weight gradient of this convolution reads it again
+        rows, entries = _stem_filter_rows(weight.shape, form)
+        block = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
+        env.lib.resize_channels_f32(_ptr(weight), block, rows, entries, _TC_CHANNELS, env.stream())
+        wt = _on_device((rows, _TC_CHANNELS), float32, weight.device, block)
     out = _new((n, cout, oh, ow), input)
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     if bn_stats:
@@ -220,17 +259,14 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
     _f32(output_grad, input, weight)
     env = _env(input)
     want_dx, want_dw, cin = input.requires_grad, weight.requires_grad, input.shape[1]
-    padded = _wants_channel_padding(input)
+    form = _stem_form(input.shape, weight.shape, stride, padding) if cin < _TC_CHANNELS else None
     x, wt = input, weight
+    a = _conv_args(x, weight, stride, padding)
+    # a data gradient of 1 or 3 channels fits no tensor-core tile: 32 are computed (the filter padded with zeros) and the first taken
+    padded = want_dx and form is not None and cin % 4 != 0 and a[-1] % 32 == 0
     if padded:
-        x = getattr(input, "_padded_for_conv", None)
-        if x is None:
-            x = _pad_channels(env, input, _TC_CHANNELS)
-        else:
-            del input._padded_for_conv
-        if want_dx:  # the data gradient reads the (padded) filter; the weight gradient only needs its shape
-            wt = _pad_channels(env, weight, _TC_CHANNELS)
-    a = _conv_args(x, weight, stride, padding, cin=x.shape[1])
+        wt = _pad_channels(env, weight, _TC_CHANNELS)
+        a = (a[0], _TC_CHANNELS) + a[2:]
     st = env.stream()
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     dx = dw = db = None
@@ -245,7 +281,7 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
             dx = _new(x.shape, x)
             env.lib.conv2d_dgrad_add_f32(*a, _ptr(output_grad), _ptr(wt), _ptr(accumulate_dx), _ptr(dx), ws, ws_bytes, st)
         else:
-            dx = _new(x.shape, x)
+            dx = _new((a[0], a[1], a[2], a[3]), x)
             env.lib.conv2d_dgrad_f32(*a, _ptr(output_grad), _ptr(wt), _ptr(dx), ws, ws_bytes, st)
             if padded:
                 dx = _take_channels(env, dx, cin, dx)
@@ -256,15 +292,26 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         # stream, beside the data-gradient / BatchNorm chain that the next layer waits for, and is
         # joined when backward ends (or before anything touches the gradient: see DAGTracker.backward).
         # A weight that already holds a gradient (shared weights) accumulates on the compute stream.
+        wa = a
+        if form is not None:
+            held = getattr(input, "_stem_held", None)
+            if held is not None and held[0] == form:
+                x = held[1]
+                del input._stem_held
+            else:
+                x = _stem_input(env, input, form)
+            wa = form[1]
+            ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*wa))
         wst, wws, wws_bytes = st, ws, ws_bytes
         if defer_weight_gradient and env.overlap_weight_gradients and weight.grad is None:
             wst = env.fork_side((x, output_grad))
-            wws, wws_bytes = env.side_workspace(env.lib.conv2d_workspace_bytes(*a))
-        if padded:
-            wide = _new((weight.shape[0], _TC_CHANNELS) + tuple(weight.shape[2:]), weight)
-            env.lib.conv2d_wgrad_f32(*a, _ptr(x), _ptr(output_grad), _ptr(wide), wws, wws_bytes, wst)
+            wws, wws_bytes = env.side_workspace(env.lib.conv2d_workspace_bytes(*wa))
+        if form is not None:
+            rows, entries = _stem_filter_rows(weight.shape, form)
+            wide = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
+            env.lib.conv2d_wgrad_f32(*wa, _ptr(x), _ptr(output_grad), wide, wws, wws_bytes, wst)
             dw = _grad_buffer(weight)
-            env.lib.resize_channels_f32(_ptr(wide), _ptr(dw), weight.shape[0] * weight.shape[2] * weight.shape[3], _TC_CHANNELS, cin, wst)
+            env.lib.resize_channels_f32(wide, _ptr(dw), rows, _TC_CHANNELS, entries, wst)
             if wst is not st:
                 env._side_keepalive.append(wide)
         else:
@@ -285,8 +332,7 @@ def _colsum(env, mat, rows, cols, like, scale=1.0, out=None):
 # ---------------------------------------------------------------------------- linear / mm
 
 def _gemm(env, m, n, k, a, ta, b, tb, bias, relu, c):
-    ws, ws_bytes = env.workspace(env.lib.gemm_workspace_bytes(m, n, k))
-    env.lib.gemm_ws_f32(m, n, k, _ptr(a), ta, _ptr(b), tb, _ptr(bias), relu, _ptr(c), ws, ws_bytes, env.stream())
+    env.lib.gemm_f32(m, n, k, _ptr(a), ta, _ptr(b), tb, _ptr(bias), relu, _ptr(c), env.stream())
 
 
 @_reg("cuda", "linear")

@@ -161,7 +161,7 @@ struct Entry<ID, K, R(A...)> {
 #define MTB_ENTRIES(X) \
   X(version, VALUE) X(device_check, STATUS) X(fill_f32, LAUNCH) X(copy_f32, LAUNCH) X(scale_f32, LAUNCH) X(relu_forward_f32, LAUNCH) \
   X(relu_backward_f32, LAUNCH) X(add_f32, LAUNCH) X(mul_f32, LAUNCH) X(add_bias_rows_f32, LAUNCH) X(binary_strided_f32, LAUNCH) \
-  X(resize_channels_f32, LAUNCH) X(nchw_to_nhwc_f32, LAUNCH) X(nhwc_to_nchw_f32, LAUNCH) X(cast, LAUNCH) \
+  X(resize_channels_f32, LAUNCH) X(pack_patches_f32, LAUNCH) X(nchw_to_nhwc_f32, LAUNCH) X(nhwc_to_nchw_f32, LAUNCH) X(cast, LAUNCH) \
   X(batch_norm2d_workspace_bytes, VALUE) X(batch_norm2d_forward_f32, LAUNCH) X(batch_norm2d_backward_f32, LAUNCH) \
   X(batch_norm2d_add_relu_forward_f32, LAUNCH) X(batch_norm2d_add_relu_backward_f32, LAUNCH) X(add_relu_f32, LAUNCH) \
   X(add_relu_backward_f32, LAUNCH) X(colsum_workspace_bytes, VALUE) X(colsum_f32, LAUNCH) X(colsum_noalloc_f32, LAUNCH) \
@@ -172,7 +172,6 @@ struct Entry<ID, K, R(A...)> {
   X(conv2d_workspace_bytes, VALUE) X(conv2d_plan_f32, STATUS) X(conv2d_forward_f32, LAUNCH) X(conv2d_stats_max_rows, VALUE) \
   X(conv2d_forward_stats_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
   X(conv2d_dgrad_add_f32, LAUNCH) X(conv2d_dgrad_accumulates_in_place, VALUE) X(conv2d_wgrad_f32, LAUNCH) X(gemm_f32, LAUNCH) \
-  X(gemm_workspace_bytes, VALUE) X(gemm_ws_f32, LAUNCH) \
   X(tc_status, STATUS) X(tc_wait_selftest, LAUNCH) \
   X(malloc, POINTER) X(free, STATUS) X(pool_reserved_bytes, VALUE) X(pool_in_use_bytes, VALUE) X(pool_trim, STATUS) X(set_device, STATUS) \
   X(get_device, STATUS) X(device_count, STATUS) X(device_synchronize, STATUS) X(mem_get_info, STATUS) X(memcpy_h2d_async, STATUS) \

@@ -80,17 +80,9 @@ MTB_API int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, i
   return mtb_conv2d_wgrad_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream);
 }
 
-MTB_API long long mtb_gemm_workspace_bytes(int m, int n, int k) { return mtb_tc_gemm_workspace_bytes(m, n, k); }
-
-// workspace (may be NULL): scratch of mtb_gemm_workspace_bytes(); see mtb_conv2d_forward_f32.
-MTB_API int mtb_gemm_ws_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                            void* workspace, long long workspace_bytes, void* stream) {
-  if (mtb_tc_gemm_supported(m, n, k, a, trans_a, b, trans_b, c))
-    return mtb_tc_gemm_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, workspace, workspace_bytes, stream);
-  return mtb_gemm_simt_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream);
-}
-
 MTB_API int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                          void* stream) {
-  return mtb_gemm_ws_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, nullptr, 0, stream);
+  if (mtb_tc_gemm_supported(m, n, k, a, trans_a, b, trans_b, c))
+    return mtb_tc_gemm_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream);
+  return mtb_gemm_simt_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream);
 }

@@ -193,7 +193,52 @@ __global__ void __launch_bounds__(256) resize_channels_kernel(const float* __res
   }
 }
 
+// out[n][oh][ow][32]: the first k_h * KW * C entries of a pixel are the input pixels its filter rows see, as one run of
+// (kh, kw, c); the rest is zero.  A thread writes four entries (16 bytes; eight threads write a pixel's 128 bytes).
+// Bound by those writes: the input is C / 32 of their size and its re-reads hit L1.
+struct PatchRuns {
+  int N, C, H, W, KH, KW, SH, SW, PH, PW, OH, OW;
+};
+__global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restrict__ x, float4* __restrict__ out, PatchRuns d, unsigned total) {
+  const int run = d.KW * d.C, used = d.KH * run;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned pixel = i >> 3;
+    const int k0 = (int)(i & 7u) * 4;
+    const unsigned ow = pixel % (unsigned)d.OW, t = pixel / (unsigned)d.OW;
+    const int oh = (int)(t % (unsigned)d.OH), n = (int)(t / (unsigned)d.OH);
+    const int h0 = oh * d.SH - d.PH, w0 = (int)ow * d.SW - d.PW;
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = k0 + q;
+      v[q] = 0.f;
+      if (k < used) {
+        const int kh = k / run, r = k - kh * run, kw = r / d.C;  // constant divisors per launch, small numbers
+        const int h = h0 + kh, w = w0 + kw;
+        if ((unsigned)h < (unsigned)d.H && (unsigned)w < (unsigned)d.W) v[q] = __ldg(x + (((long long)n * d.H + h) * d.W + w) * d.C + (r - kw * d.C));
+      }
+    }
+    out[i] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
 }  // namespace
+
+// Gathers what a filter of few input channels sees into runs of 32 floats per output pixel: out[N][OH][OW][32] with
+// entry (kh * KW + kw) * C + c, zero beyond the edges and from KH * KW * C on (KH * KW * C <= 32).  A convolution with
+// few input channels then is one with 32 channels and no window (or, with KH = 1 here, one whose window is a single
+// column): a 7x7 filter over 3 channels reads 7 blocks of 32 instead of 49.  No counterpart in the reference.
+MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, const float* x, float* out, void* stream) {
+  MTB_REQUIRE(x && out && n > 0 && c > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0 && ph >= 0 && pw >= 0, "pack_patches: bad arguments");
+  MTB_REQUIRE((long long)kh * kw * c <= 32, "pack_patches: the filter has more than 32 entries");
+  PatchRuns d{n, c, h, w, kh, kw, sh, sw, ph, pw, (h + 2 * ph - kh) / sh + 1, (w + 2 * pw - kw) / sw + 1};
+  MTB_REQUIRE(d.OH > 0 && d.OW > 0 && mtb_aligned16(out), "pack_patches: empty or unaligned output");
+  const long long total = (long long)n * d.OH * d.OW * 8;
+  MTB_REQUIRE(total < (1LL << 32) - (1LL << 24), "pack_patches: too many pixels");
+  pack_patches_kernel<<<mtb_stream_grid(total, 256), 256, 0, (cudaStream_t)stream>>>(x, (float4*)out, d, (unsigned)total);
+  MTB_LAUNCH_CHECK("pack_patches_kernel");
+  return MTB_OK;
+}
 
 // Copy a row-major [rows, c_src] matrix into [rows, c_dst]: extra columns are zero, surplus columns are
 // dropped.  Pads the 1- or 3-channel image stem (and its filter) to one 32-channel block for the

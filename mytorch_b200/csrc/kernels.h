@@ -32,7 +32,6 @@ bool mtb_tc_conv2d_wgrad_supported(int n, int cin, int h, int w, int kh, int kw,
 int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                             const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream);
 bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* c);
-long long mtb_tc_gemm_workspace_bytes(int m, int n, int k);
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* workspace, long long workspace_bytes, void* stream);
+                    void* stream);
 

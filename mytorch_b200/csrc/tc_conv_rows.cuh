@@ -873,6 +873,10 @@ __global__ void __launch_bounds__(1024) wgrad_reduce_many_kernel(const float* __
   if (r < Kw && c < Cout) {
     const float* q = partial + (long long)r * Cout + c;
     int z = z0;
+    for (; z + 24 < splits; z += 32) {  // four loads in flight; the grouping is fixed
+      const float a = q[z * plane], b = q[(z + 8) * plane], d = q[(z + 16) * plane], e = q[(z + 24) * plane];
+      s0 += a; s1 += b; s0 += d; s1 += e;
+    }
     for (; z + 8 < splits; z += 16) { s0 += q[z * plane]; s1 += q[(z + 8) * plane]; }
     if (z < splits) s0 += q[z * plane];
   }

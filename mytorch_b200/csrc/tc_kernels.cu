@@ -108,9 +108,9 @@ struct GemmParams {
   float* out;
   long long ldo;
   const float* bias;
-  // optional: out += result instead of out = result (the rows of `out` already hold a value this launch adds
-  // to; a thread reads the very elements it then writes, so accumulating in place is safe)
-  int accumulate;
+  // optional tensor laid out like `out`: out = result + addend (gradient accumulation).  May be `out` itself: a
+  // thread reads the very elements it then writes.
+  const float* addend;
   int relu;
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
@@ -152,11 +152,15 @@ struct Cfg {
   static constexpr uint32_t kTmemCols = 2 * BN;
 };
 
-template <int BN, int AMODE, int BMODE, bool STATS>
+// What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, or add a tensor.
+enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2 };
+
+template <int BN, int AMODE, int BMODE, int EPI>
 __global__ void __launch_bounds__(192, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p) {
   using C = Cfg<BN>;
   constexpr int STAGES = C::kStages;
+  constexpr bool STATS = EPI == EPI_STATS, ADD = EPI == EPI_ADD;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
   __shared__ uint32_t tmem_slot;
@@ -319,10 +323,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       const int buf = t & 1;
       const uint32_t use = (uint32_t)(t >> 1);
       // one lane polls (128 threads spinning on the barrier slow the other roles' barrier traffic down)
-      bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull[buf]), use & 1u, abort_ptr, 4);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
+      auto wait_for_accumulator = [&]() {
+        bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull[buf]), use & 1u, abort_ptr, 4);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      if constexpr (!ADD) {
+        if (!wait_for_accumulator()) break;
+      }
       const int row = m0 + quarter * 32 + lane;
       long long orow_index = row;
       if (p.o_strided && row < p.M) {
@@ -331,9 +340,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         orow_index = ((long long)nn * p.o_H + p.o_h0 + p.o_sh * i) * p.o_W + p.o_w0 + p.o_sw * j;
       }
       float* orow = p.out + orow_index * p.ldo;
+      const float* arow = ADD ? p.addend + orow_index * p.ldo : nullptr;
       const bool valid = row < p.M;
       const float cnt = STATS ? (float)__popc(__ballot_sync(0xffffffffu, valid)) : 0.f;
-      // r: this lane's row of the finished accumulator, columns c0 .. c0+31 of the tile
+      // r: this lane's row of the finished accumulator, columns c0 .. c0+31 of the tile; add: the same columns of the
+      // addend, fetched one chunk ahead (a memory round trip per chunk in front of the stores would make the epilogue
+      // of a short reduction several times longer than its main loop)
+      const bool adds = ADD && valid && vec_ok && n0 + BN <= p.N;
+      auto fetch_addend = [&](int c0, float4 (&add)[8]) {
+        if (adds) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) add[j] = *reinterpret_cast<const float4*>(arow + n0 + c0 + 4 * j);
+        }
+      };
+      float4 add[8];
+      if constexpr (ADD) {
+        fetch_addend(0, add);
+        if (!wait_for_accumulator()) break;
+      }
       auto finish = [&](int c0, const uint32_t (&r)[32]) {
         const int col0 = n0 + c0;
         if constexpr (STATS) {
@@ -368,8 +392,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + jj);
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
-                  if (p.accumulate) {
-                    const float4 b = *reinterpret_cast<const float4*>(orow + col0 + jj);
+                  if constexpr (ADD) {
+                    const float4 b = adds ? add[jj / 4] : *reinterpret_cast<const float4*>(arow + col0 + jj);
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
                   if (p.relu) { v[h].x = fmaxf(v[h].x, 0.f); v[h].y = fmaxf(v[h].y, 0.f); v[h].z = fmaxf(v[h].z, 0.f); v[h].w = fmaxf(v[h].w, 0.f); }
@@ -382,7 +406,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (col0 + j < p.N) {
                   float v = __uint_as_float(r[j]);
                   if (p.bias) v += p.bias[col0 + j];
-                  if (p.accumulate) v += orow[col0 + j];
+                  if constexpr (ADD) v += arow[col0 + j];
                   if (p.relu) v = fmaxf(v, 0.f);
                   orow[col0 + j] = v;
                 }
@@ -414,8 +438,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
           for (int c0 = 0; c0 < BN; c0 += 32) {
             uint32_t r[32];
             tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), r);
-            tmem_ld_wait();
-            finish(c0, r);
+            if constexpr (ADD) {
+              float4 next[8];
+              if (c0 + 32 < BN) fetch_addend(c0 + 32, next);
+              tmem_ld_wait();
+              finish(c0, r);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) add[j] = next[j];
+            } else {
+              tmem_ld_wait();
+              finish(c0, r);
+            }
           }
         }
         count_rows();
@@ -468,6 +501,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c) {
           uint32_t r[32];
+          if constexpr (ADD) {
+            if (c > 0) fetch_addend(c * 32, add);
+          }
           reduce_chunk(c, r);
           finish(c * 32, r);
         }
@@ -501,15 +537,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   }
 }
 
-template <int BN, int AMODE, int BMODE, bool STATS = false>
+template <int BN, int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
   using C = Cfg<BN>;
-  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, STATS>;
+  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI>;
   static unsigned long long configured = 0;
   if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
   int tiles = p.m_tiles * p.n_tiles * p.splits;  // work units
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
-  if (STATS && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
+  if (EPI == EPI_STATS && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
   kernel<<<grid, 192, C::kSmemBytes, st>>>(mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
@@ -521,11 +557,11 @@ int stats_rows_for(int tiles, int n_tiles) {
   return grid / n_tiles * 4;
 }
 
-template <int AMODE, int BMODE>
+template <int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc_bn(int bn, const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
-  if (bn == 64) return launch_tc<64, AMODE, BMODE>(mapA, mapB, p, st);
-  if (bn == 128) return launch_tc<128, AMODE, BMODE>(mapA, mapB, p, st);
-  return launch_tc<256, AMODE, BMODE>(mapA, mapB, p, st);
+  if (bn == 64) return launch_tc<64, AMODE, BMODE, EPI>(mapA, mapB, p, st);
+  if (bn == 128) return launch_tc<128, AMODE, BMODE, EPI>(mapA, mapB, p, st);
+  return launch_tc<256, AMODE, BMODE, EPI>(mapA, mapB, p, st);
 }
 
 int pick_bn(int n) { return n <= 64 ? 64 : (n <= 128 ? 128 : 256); }
@@ -549,15 +585,15 @@ int pick_bn_for(int n, long long rows) {
 // (tiles x splits <= SMs) and every unit keeps at least eight reduction blocks.
 struct GemmPlan { int bn, splits, kb_per_split; };
 
-GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, int force_bn = 0, int min_kb = 64) {
+GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, int force_bn = 0) {
   const int sms = mtb_sm_count();
   const long long m_tiles = (rows + 127) / 128;
-  static const int kSplits[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
+  static const int kSplits[] = {1, 2, 3, 4, 6, 8};
   GemmPlan best{force_bn ? force_bn : pick_bn_for(n, rows), 1, num_kb};
   // Measured: the split only pays when even 64-wide tiles leave half the GPU idle (the 4x4 layers at 64
   // images: 41 -> 24 us for the data gradient of 512 -> 512); with more tiles than that the last unit's pass
   // over the partials costs more than the idle SMs did (256 -> 256 on 8x8 at 64 images: 20 -> 40 us).
-  if (m_tiles * ((n + 63) / 64) > sms / 2 || num_kb < min_kb) may_split = false;  // short reductions gain nothing either
+  if (m_tiles * ((n + 63) / 64) > sms / 2 || num_kb < 64) may_split = false;  // short reductions gain nothing either
   if (!may_split || getenv("MTB_DISABLE_SPLITK")) return best;
   double best_ns = 1e30;
   for (int bn = force_bn ? force_bn : pick_bn(n); bn >= (force_bn ? force_bn : 64); bn >>= 1) {
@@ -658,18 +694,10 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
   return true;
 }
 
-// Tile width and split of a plain GEMM.  A Linear layer over few samples has one or two output tiles and a long
-// reduction ([64 x 9216] x [9216 x 128]: two CTAs walked 288 blocks each, 57 us); with scratch its reduction is split.
-static GemmPlan plan_dense(int m, int n, int k) { return plan_gemm(n, m, (k + 31) / 32, true, 0, 32); }
-
-long long mtb_tc_gemm_workspace_bytes(int m, int n, int k) { return split_partial_bytes(plan_dense(m, n, k), m, n); }
-
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* workspace, long long workspace_bytes, void* stream) {
+                    void* stream) {
   CUtensorMap mapA, mapB;
-  GemmPlan gp = plan_dense(m, n, k);
-  if (!workspace || split_partial_bytes(gp, m, n) > workspace_bytes) gp = GemmPlan{pick_bn_for(n, m), 1, (k + 31) / 32};
-  const int bn = gp.bn;
+  int bn = pick_bn_for(n, m);
   int rc;
   if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, 128);
   else rc = tc::encode_tiled_2d(&mapA, a, k, m, m, 32, 32, true);
@@ -678,7 +706,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   else rc = tc::encode_tiled_2d(&mapB, b, k, n, n, 32, 32, true);
   if (rc) return rc;
   GemmParams p{};
-  p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
+  p.splits = 1; p.kb_per_split = (k + 31) / 32;
   p.M = m; p.N = n; p.num_kb = (k + 31) / 32;
   p.m_tiles = (m + 127) / 128; p.n_tiles = (n + bn - 1) / bn;
   p.out = c; p.ldo = n; p.bias = bias; p.relu = relu;
@@ -735,14 +763,13 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   // ... unless the output is small: then BatchNorm's own pass is all launch latency, and the epilogue is cheaper
   // (measured on the three 1x1 shortcuts of ResNet-18: 1.782 -> 1.770 ms per step at 64 images, but
   // 6.37 -> 6.41 ms at 512, where their outputs are 17 to 67 MB)
+  // 64-wide tiles keep plain per-lane sums, cheap enough to hide behind the stores whatever the reduction.
   const bool small_output = (long long)M * cout * 4 <= (12ll << 20);
-  if (want_stats && (p.num_kb >= 16 || small_output)) {
+  if (want_stats && (p.num_kb >= 16 || small_output || bn == 64)) {
     p.stats = stats;
     *stats_rows = gp.splits > 1 ? p.m_tiles * 4 : stats_rows_for(p.m_tiles * p.n_tiles, p.n_tiles);
     cudaStream_t st = (cudaStream_t)stream;
-    if (bn == 64) return launch_tc<64, A_IM2COL, B_KMAJOR, true>(mapA, mapB, p, st);
-    if (bn == 128) return launch_tc<128, A_IM2COL, B_KMAJOR, true>(mapA, mapB, p, st);
-    return launch_tc<256, A_IM2COL, B_KMAJOR, true>(mapA, mapB, p, st);
+    return launch_tc_bn<A_IM2COL, B_KMAJOR, EPI_STATS>(bn, mapA, mapB, p, st);
   }
   return launch_tc_bn<A_IM2COL, B_KMAJOR>(bn, mapA, mapB, p, (cudaStream_t)stream);
 }
@@ -810,6 +837,10 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   // addend == dx: dx already holds the gradient to add to; every class adds its own pixels in its epilogue
   // and the pixels of classes without taps stay as they are.
   const bool in_place = addend != nullptr && addend == dx;
+  // A 1x1 filter's data gradient is bound by writing dx, so its epilogue also reads the tensor to add and the separate
+  // pass (read twice, write once) goes: 64 <- 256 channels on 128 x 56 x 56, see the measurements of the bottleneck step.
+  // Filters with more taps are bound by the tensor pipe, which pays for every load in the epilogue (measured slower).
+  const bool fused_add = addend != nullptr && !in_place && al16(addend) && kh * kw == 1 && sh * sw == 1;
   if (need_zero && !in_place) MTB_CUDA(cudaMemsetAsync(dx, 0, (size_t)n * h * w * cin * 4, st));
   // The classes write disjoint pixels.  When one class fills only part of the GPU they run side by side on
   // separate lanes (then without split reductions, whose tickets and partials one launch at a time owns).
@@ -842,7 +873,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
       p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
       p.m_tiles = (int)((M + 127) / 128); p.n_tiles = (cin + bn - 1) / bn;
       p.out = dx; p.ldo = cin; p.bias = nullptr; p.relu = 0;
-      p.accumulate = in_place ? 1 : 0;
+      p.addend = in_place || fused_add ? addend : nullptr;
       p.OW = aw.count; p.OH = ah.count; p.SW = 1; p.SH = 1; p.PW = -aw.lower; p.PH = -ah.lower; p.KW = aw.taps; p.KH = ah.taps;
       p.cchunks = cout / 32;
       p.b_per_tap = 1;
@@ -852,13 +883,13 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
           p.b_tap_x[jh * aw.taps + jw] = (fkh * kw + fkw) * cin;
         }
       p.o_strided = 1; p.o_Hc = ah.count; p.o_Wc = aw.count; p.o_H = h; p.o_W = w; p.o_h0 = ah.start; p.o_w0 = aw.start; p.o_sh = sh; p.o_sw = sw;
-      rc = launch_tc_bn<A_IM2COL, B_MNMAJOR>(bn, mapA, mapB, p, cst);
+      rc = p.addend ? launch_tc_bn<A_IM2COL, B_MNMAJOR, EPI_ADD>(bn, mapA, mapB, p, cst) : launch_tc_bn<A_IM2COL, B_MNMAJOR>(bn, mapA, mapB, p, cst);
       if (rc) return rc;
     }
   }
   rc = mtb_join_lanes(st, lanes);
   if (rc) return rc;
-  if (addend && !in_place) return mtb_add_f32(dx, addend, dx, (long long)n * h * w * cin, 1.0f, st);
+  if (addend && !in_place && !fused_add) return mtb_add_f32(dx, addend, dx, (long long)n * h * w * cin, 1.0f, st);
   return MTB_OK;
 }
 
@@ -1087,30 +1118,38 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
   }
 }
 
-// dw[co][r] = sum_s partial[s][r][co]: a CTA takes 32 rows x 128 output channels, reads float4
-// along co (splits added in index order), transposes through shared memory and writes 128-byte
-// runs along r.
-__global__ void __launch_bounds__(1024) wgrad_reduce_transpose_kernel(const float* __restrict__ partial, float* __restrict__ dw, int Kw, int Cout,
-                                                                       int splits) {
-  __shared__ float tile[128][33];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 128;
+// dw[co][r] = sum_s partial[s][r][co]: a CTA takes 8 rows x 128 output channels, reads float4 along co (even and odd
+// splits in one sum each, in index order), transposes through shared memory and writes 32-byte runs along r.
+// Bound by latency where there is little to read: a 1x1 layer or a stem has one split per SM and a few thousand outputs,
+// and blocks of 32 rows with two loads in flight took 25 us over 148 planes; with 8 rows and sixteen loads in flight
+// four times as many CTAs take a quarter of the round trips each.
+constexpr int kReduceRows = 8;
+__global__ void __launch_bounds__(32 * kReduceRows) wgrad_reduce_transpose_kernel(const float* __restrict__ partial, float* __restrict__ dw, int Kw,
+                                                                                   int Cout, int splits) {
+  __shared__ float tile[128][kReduceRows + 1];
+  const int r0 = blockIdx.x * kReduceRows, c0 = blockIdx.y * 128;
   const long long plane = (long long)Kw * Cout;
   {
     const int r = r0 + threadIdx.y, c = c0 + 4 * threadIdx.x;
     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
     if (r < Kw && c < Cout) {  // Cout % 4 == 0 on this path, so the four channels are in range together
       const float* q = partial + (long long)r * Cout + c;
+      auto add = [](float4& s, const float4& a) { s.x += a.x; s.y += a.y; s.z += a.z; s.w += a.w; };
+      constexpr int AHEAD = 16;
       int z = 0;
-      for (; z + 1 < splits; z += 2) {  // two independent loads in flight; the grouping is fixed
-        const float4 a = *reinterpret_cast<const float4*>(q + z * plane);
-        const float4 b = *reinterpret_cast<const float4*>(q + (z + 1) * plane);
-        s0.x += a.x; s0.y += a.y; s0.z += a.z; s0.w += a.w;
-        s1.x += b.x; s1.y += b.y; s1.z += b.z; s1.w += b.w;
+      for (; z + AHEAD <= splits; z += AHEAD) {
+        float4 v[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) v[u] = *reinterpret_cast<const float4*>(q + (z + u) * plane);
+#pragma unroll
+        for (int u = 0; u < AHEAD; u += 2) { add(s0, v[u]); add(s1, v[u + 1]); }
       }
-      if (z < splits) {
-        const float4 a = *reinterpret_cast<const float4*>(q + z * plane);
-        s0.x += a.x; s0.y += a.y; s0.z += a.z; s0.w += a.w;
+      for (; z + 1 < splits; z += 2) {
+        const float4 a = *reinterpret_cast<const float4*>(q + z * plane), b = *reinterpret_cast<const float4*>(q + (z + 1) * plane);
+        add(s0, a);
+        add(s1, b);
       }
+      if (z < splits) add(s0, *reinterpret_cast<const float4*>(q + z * plane));
     }
     tile[4 * threadIdx.x + 0][threadIdx.y] = s0.x + s1.x;
     tile[4 * threadIdx.x + 1][threadIdx.y] = s0.y + s1.y;
@@ -1118,11 +1157,11 @@ __global__ void __launch_bounds__(1024) wgrad_reduce_transpose_kernel(const floa
     tile[4 * threadIdx.x + 3][threadIdx.y] = s0.w + s1.w;
   }
   __syncthreads();
-  const int r = r0 + threadIdx.x;
+  const int t = threadIdx.y * 32 + threadIdx.x, r = r0 + t % kReduceRows;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int cc = threadIdx.y + 32 * k, c = c0 + cc;
-    if (r < Kw && c < Cout) dw[(long long)c * Kw + r] = tile[cc][threadIdx.x];
+    const int cc = t / kReduceRows + 32 * k, c = c0 + cc;
+    if (r < Kw && c < Cout) dw[(long long)c * Kw + r] = tile[cc][t % kReduceRows];
   }
 }
 
@@ -1271,8 +1310,8 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   else MTB_LAUNCH_WGRAD(256, 64);
 #undef MTB_LAUNCH_WGRAD
   MTB_LAUNCH_CHECK("tc_wgrad_kernel");
-  dim3 rgrid((unsigned)((q.Kw + 31) / 32), (unsigned)((cout + 127) / 128));
-  wgrad_reduce_transpose_kernel<<<rgrid, dim3(32, 32), 0, st>>>((const float*)workspace, dw, (int)q.Kw, cout, q.splits);
+  dim3 rgrid((unsigned)((q.Kw + kReduceRows - 1) / kReduceRows), (unsigned)((cout + 127) / 128));
+  wgrad_reduce_transpose_kernel<<<rgrid, dim3(32, kReduceRows), 0, st>>>((const float*)workspace, dw, (int)q.Kw, cout, q.splits);
   MTB_LAUNCH_CHECK("wgrad_reduce_transpose_kernel");
   return MTB_OK;
 }

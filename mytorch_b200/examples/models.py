@@ -95,30 +95,27 @@ class ResNet18Cifar(nn.Module):
 
 
 class Bottleneck(nn.Module):
-    """1x1 reduce, 3x3 (carries the stride), 1x1 expand x4."""
+    """1x1 reduce, 3x3 (carries the stride), 1x1 expand x4; the ReLUs and the shortcut addition run inside the
+    BatchNorm operators (same arithmetic and state-dict keys as the separate layers)."""
 
     def __init__(self, cin, mid, stride, device="cpu"):
         super().__init__()
         cout = mid * 4
         self.conv1 = nn.Conv2d(cin, mid, 1, 1, 0, bias=False, device=device)
-        self.bn1 = nn.BatchNorm2d(mid, device=device)
+        self.bn1 = nn.BatchNormReLU2d(mid, device=device)
         self.conv2 = nn.Conv2d(mid, mid, 3, stride, 1, bias=False, device=device)
-        self.bn2 = nn.BatchNorm2d(mid, device=device)
+        self.bn2 = nn.BatchNormReLU2d(mid, device=device)
         self.conv3 = nn.Conv2d(mid, cout, 1, 1, 0, bias=False, device=device)
-        self.bn3 = nn.BatchNorm2d(cout, device=device)
+        self.bn3 = nn.BatchNormAddReLU2d(cout, device=device)
         self.downsample = None
         if stride != 1 or cin != cout:
             self.downsample = nn.Sequential(nn.Conv2d(cin, cout, 1, stride, 0, bias=False, device=device),
                                             nn.BatchNorm2d(cout, device=device))
-        self.relu = nn.ReLU()
         _feed_batch_norm(self.conv1, self.conv2, self.conv3, *([self.downsample._modules["0"]] if self.downsample is not None else []))
 
     def forward(self, x):
-        y = self.relu(self.bn1(self.conv1(x)))
-        y = self.relu(self.bn2(self.conv2(y)))
-        y = self.bn3(self.conv3(y))
-        shortcut = x if self.downsample is None else self.downsample(x)
-        return self.relu(y + shortcut)
+        shortcut = x if self.downsample is None else self.downsample(x)  # first: see BasicBlock
+        return self.bn3(self.conv3(self.bn2(self.conv2(self.bn1(self.conv1(x))))), shortcut)
 
 
 class ResNet50(nn.Module):
@@ -128,8 +125,7 @@ class ResNet50(nn.Module):
         super().__init__()
         self.conv1 = nn.Conv2d(3, 64, 7, 2, 3, bias=False, device=device)
         _feed_batch_norm(self.conv1)
-        self.bn1 = nn.BatchNorm2d(64, device=device)
-        self.relu = nn.ReLU()
+        self.bn1 = nn.BatchNormReLU2d(64, device=device)
         self.maxpool = nn.MaxPool2d(3, 2, 1)
         cin = 64
         for si, (mid, count) in enumerate(zip((64, 128, 256, 512), (3, 4, 6, 3))):
@@ -141,7 +137,7 @@ class ResNet50(nn.Module):
         self.fc = nn.Linear(cin, num_classes, device=device)
 
     def forward(self, x):
-        x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
+        x = self.maxpool(self.bn1(self.conv1(x)))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(x.mean(dim=(2, 3)))
 
