@@ -99,6 +99,13 @@ int mtb_conv2d_stats_max_rows(void);
 int mtb_conv2d_forward_stats_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                  const float* wt, const float* bias, float* y, int relu, float* stats, int* stats_rows, void* workspace,
                                  long long workspace_bytes, void* stream);
+/* Inference: y = batch_norm(conv(x) + bias) (+ residual) (ReLU) with running statistics, in one launch (the reference runs
+ * conv2d, batch_norm2d, add and relu: mytorch/nn/conv.py:71, mytorch/nn/batch_norm.py:123-135, mytorch/nn/relu.py:5-10).
+ * gamma, beta, bias and residual (shape of y) may be NULL; the bits are those of the separate operators. */
+int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
+                              const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
+                              const float* running_var, double eps, const float* residual, int relu, float* y, void* workspace,
+                              long long workspace_bytes, void* stream);
 /* dx[N,H,W,Cin]: every element is written (zeros where no window reaches); no atomics */
 int mtb_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                          const float* wt, float* dx, void* workspace, long long workspace_bytes, void* stream);

@@ -214,13 +214,8 @@ def _take_channels(env, t, channels, like, out=None):
     return out
 
 
-@_reg("cuda", "conv2d")
-def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
-    """``bn_stats``: the output feeds a BatchNorm layer in training mode; where the kernel allows, the
-    convolution's epilogue also reduces the per-channel batch statistics of the output and leaves them
-    on the result (``_bn_partials``) for ``batch_norm2d``, which then skips its own pass over the tensor."""
-    _f32(input, weight, bias)
-    env = _env(input)
+def _conv_operands(env, input, weight, stride, padding):
+    """(arguments, input, filter, output tensor) of a forward convolution, the operands in the form its kernel reads."""
     x, wt = input, weight
     a = _conv_args(x, wt, stride, padding)
     n, cin, h, w, kh, kw, sh, sw, ph, pw, cout = a
@@ -235,10 +230,34 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
         block = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
         env.lib.resize_channels_f32(_ptr(weight), block, rows, entries, _TC_CHANNELS, env.stream())
         wt = _on_device((rows, _TC_CHANNELS), float32, weight.device, block)
-    out = _new((n, cout, oh, ow), input)
+    return a, x, wt, _new((n, cout, oh, ow), input)
+
+
+@_reg("cuda", "conv2d_batch_norm")
+def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps, relu, residual=None):
+    """Inference: relu?(batch_norm2d(conv2d(input)) + residual) with running statistics, in the convolution's launch."""
+    _f32(input, weight, bias, gamma, beta, running_mean, running_var, residual)
+    env = _env(input)
+    a, x, wt, out = _conv_operands(env, input, weight, stride, padding)
+    if residual is not None and residual.shape != out.shape:
+        raise MismatchShapesError([out.shape, residual.shape])
+    ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
+    env.lib.conv2d_bn_forward_f32(*a, _ptr(x), _ptr(wt), _ptr(bias), _ptr(gamma), _ptr(beta), _ptr(running_mean), _ptr(running_var), float(eps),
+                                  _ptr(residual), int(bool(relu)), _ptr(out), ws, ws_bytes, env.stream())
+    return out
+
+
+@_reg("cuda", "conv2d")
+def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
+    """``bn_stats``: the output feeds a BatchNorm layer in training mode; where the kernel allows, the
+    convolution's epilogue also reduces the per-channel batch statistics of the output and leaves them
+    on the result (``_bn_partials``) for ``batch_norm2d``, which then skips its own pass over the tensor."""
+    _f32(input, weight, bias)
+    env = _env(input)
+    a, x, wt, out = _conv_operands(env, input, weight, stride, padding)
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     if bn_stats:
-        partials = CudaMemory(input.device.index, env.lib.conv2d_stats_max_rows() * 3 * cout * 4)
+        partials = CudaMemory(input.device.index, env.lib.conv2d_stats_max_rows() * 3 * a[-1] * 4)
         rows = ctypes.c_int(0)
         env.lib.conv2d_forward_stats_f32(*a, _ptr(x), _ptr(wt), _ptr(bias), _ptr(out), 0, partials.ptr, ctypes.byref(rows), ws, ws_bytes,
                                          env.stream())

@@ -4,6 +4,7 @@
 // partials (shifted sums, Chan merge) combined in a fixed order by a one-CTA-per-256-channels
 // finalise kernel, so results are bit-reproducible.
 #include "colreduce.cuh"
+#include "kernels.h"
 
 MTB_API long long mtb_batch_norm2d_workspace_bytes(int n, int c, int h, int w);
 
@@ -159,12 +160,13 @@ __global__ void bn_eval_prep_kernel(int C, const float* __restrict__ gamma, floa
 
 // ---------------------------------------------------------------- forward: normalise
 
+// With var != NULL (running statistics) `scale` holds gamma, or is NULL, and the scale is computed here.
 // MODE 0: y = bn(x); 1: y = max(0, bn(x)); 2: y = max(0, bn(x) + res) (res has the shape of x)
 template <int V, int MODE>
-__global__ void __launch_bounds__(256) bn_normalize_kernel(const float* __restrict__ x, float* __restrict__ y, long long rows, int C, int L,
+__global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float* y, long long rows, int C, int L,
                                                             long long rows_per_block, const float* __restrict__ mean,
                                                             const float* __restrict__ scale, const float* __restrict__ beta,
-                                                            const float* __restrict__ res) {
+                                                            const float* __restrict__ res, const float* __restrict__ var, float eps) {
   const int lane = threadIdx.x & (L - 1);
   const int rsub = threadIdx.x / L;
   const int R = 256 / L;
@@ -174,7 +176,12 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* __restri
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     mu[i] = mean[cg * V + i];
-    g[i] = scale[cg * V + i];
+    if (var) {
+      const float rstd = 1.0f / sqrtf(var[cg * V + i] + eps);
+      g[i] = scale ? scale[cg * V + i] * rstd : rstd;
+    } else {
+      g[i] = scale[cg * V + i];
+    }
     b[i] = beta ? beta[cg * V + i] : 0.f;
   }
   long long r0 = blockIdx.y * rows_per_block;
@@ -366,10 +373,10 @@ ColCfg stream_cfg(long long rows, int C, bool aligned) {
 }
 
 int launch_normalize(const float* x, float* y, long long rows, int c, bool aligned, const float* mean, const float* scale, const float* beta,
-                     int mode, const float* res, cudaStream_t st) {
+                     int mode, const float* res, cudaStream_t st, const float* var = nullptr, float eps = 0.f) {
   ColCfg s = stream_cfg(rows, c, aligned);
   dim3 grid(s.col_blocks, s.row_blocks);
-#define MTB_BN_NORM(V_, M_) bn_normalize_kernel<V_, M_><<<grid, 256, 0, st>>>(x, y, rows, c, s.lanes, s.rows_per_block, mean, scale, beta, res)
+#define MTB_BN_NORM(V_, M_) bn_normalize_kernel<V_, M_><<<grid, 256, 0, st>>>(x, y, rows, c, s.lanes, s.rows_per_block, mean, scale, beta, res, var, eps)
   if (s.vec == 4) { if (mode == 2) MTB_BN_NORM(4, 2); else if (mode == 1) MTB_BN_NORM(4, 1); else MTB_BN_NORM(4, 0); }
   else { if (mode == 2) MTB_BN_NORM(1, 2); else if (mode == 1) MTB_BN_NORM(1, 1); else MTB_BN_NORM(1, 0); }
 #undef MTB_BN_NORM
@@ -445,6 +452,11 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
 }
 
 }  // namespace
+
+int mtb_bn_eval_apply(const float* x, float* y, long long rows, int c, const MtbBnEval& bn, const float* residual, int relu, cudaStream_t st) {
+  const bool aligned = mtb_aligned16(x) && mtb_aligned16(y) && mtb_aligned16(residual);
+  return launch_normalize(x, y, rows, c, aligned, bn.mean, bn.gamma, bn.beta, residual ? 2 : (relu ? 1 : 0), residual, st, bn.var, bn.eps);
+}
 
 // Scratch the forward and backward entry points need, in bytes (an upper bound for the shape).
 MTB_API long long mtb_batch_norm2d_workspace_bytes(int n, int c, int h, int w) {

@@ -170,7 +170,7 @@ struct Entry<ID, K, R(A...)> {
   X(max_pool2d_argmax_u8, LAUNCH) X(cross_entropy_workspace_bytes, VALUE) X(cross_entropy_forward_f32, LAUNCH) \
   X(cross_entropy_backward_f32, LAUNCH) X(sgd_f32, LAUNCH) X(sgd_multi_f32, LAUNCH) X(pack_scale_f32, LAUNCH) \
   X(conv2d_workspace_bytes, VALUE) X(conv2d_plan_f32, STATUS) X(conv2d_forward_f32, LAUNCH) X(conv2d_stats_max_rows, VALUE) \
-  X(conv2d_forward_stats_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
+  X(conv2d_forward_stats_f32, LAUNCH) X(conv2d_bn_forward_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
   X(conv2d_dgrad_add_f32, LAUNCH) X(conv2d_dgrad_accumulates_in_place, VALUE) X(conv2d_wgrad_f32, LAUNCH) X(gemm_f32, LAUNCH) \
   X(tc_status, STATUS) X(tc_wait_selftest, LAUNCH) \
   X(malloc, POINTER) X(free, STATUS) X(pool_reserved_bytes, VALUE) X(pool_in_use_bytes, VALUE) X(pool_trim, STATUS) X(set_device, STATUS) \

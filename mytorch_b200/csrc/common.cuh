@@ -15,6 +15,13 @@ enum MtbStatus {
   MTB_ERR_DEVICE = 5,       // a kernel reported a device-side problem (bounded wait ran out)
 };
 
+// BatchNorm with running statistics, applied where a convolution stores its output (inference): (v - mean) * scale + beta
+// with scale = gamma / sqrt(var + eps); mean == NULL: none.  gamma / beta may be NULL.
+struct MtbBnEval {
+  const float *mean, *var, *gamma, *beta;
+  float eps;
+};
+
 int mtb_fail(int code, const char* fmt, ...);
 int mtb_sm_count();
 // Opt a kernel in to `bytes` of dynamic shared memory on the CURRENT device.  The attribute is kept

@@ -39,6 +39,22 @@ MTB_API int mtb_conv2d_forward_stats_f32(int n, int cin, int h, int w, int kh, i
   return mtb_conv2d_forward_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, stream);
 }
 
+// Inference: y = relu?(batch_norm(conv(x)) + residual), BatchNorm with running statistics, in one launch.  The epilogue applies
+// the BatchNorm kernels' own expression to the value it would have stored, so the bits are those of the separate
+// operators; what goes is the write and the read of the convolution's output and two launches.
+MTB_API int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
+                                      const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
+                                      const float* running_var, double eps, const float* residual, int relu, float* y, void* workspace,
+                                      long long workspace_bytes, void* stream) {
+  MTB_REQUIRE(running_mean && running_var, "conv2d_bn_forward: running statistics are required");
+  MTB_REQUIRE(!residual || relu, "conv2d_bn_forward: an addition goes with a ReLU");
+  const MtbBnEval bn{running_mean, running_var, gamma, beta, (float)eps};
+  if (mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, y) && (!residual || mtb_aligned16(residual)))
+    return mtb_tc_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream, nullptr,
+                                     nullptr, &bn, residual);
+  return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, &bn, residual, stream);
+}
+
 MTB_API int mtb_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                                  const float* wt, float* dx, void* workspace, long long workspace_bytes, void* stream) {
   if (mtb_tc_conv2d_dgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx))

@@ -1,6 +1,7 @@
 // Convolution on the CUDA cores (FP32) for the shapes the tensor-core kernels do not take: channel counts that are no
 // multiple of 32, activations under 128 KiB.  Forward, data gradient and weight gradient as implicit matrix
 // products over channels-last tensors (see simt_tile.cuh for the kernel).
+#include "kernels.h"
 #include "simt_tile.cuh"
 
 namespace {
@@ -35,8 +36,8 @@ Choice wgrad_choice(const ConvDims& d) {
 
 }  // namespace
 
-MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
-                                        const float* wt, const float* bias, float* y, int relu, void* stream) {
+int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
+                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream) {
   ConvDims d;
   int rc = conv_dims(d, n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (rc) return rc;
@@ -45,10 +46,24 @@ MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, in
   Out o{};
   o.out = y; o.ld = cout; o.bias = bias; o.relu = relu;
   const Choice c = choose(M, cout, K, 1, 1);
+  if (bn_eval) {
+    if (tile_info(c.tile).cluster) {  // small tiles: BatchNorm in the store
+      o.bn = *bn_eval;
+      o.residual = residual;
+    } else {
+      const int rc2 = mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, 0, nullptr, nullptr, stream);
+      return rc2 ? rc2 : mtb_bn_eval_apply(y, y, M, cout, *bn_eval, residual, relu, (cudaStream_t)stream);
+    }
+  }
   const DenseK filter{wt, K};
   if (cin % 4 == 0 && mtb_aligned16(x) && mtb_aligned16(wt))
     return launch<PatchK, 4, DenseK, 4>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt");
   return launch<PatchK, 1, DenseK, 1>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt");
+}
+
+MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
+                                        const float* wt, const float* bias, float* y, int relu, void* stream) {
+  return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream);
 }
 
 MTB_API int mtb_conv2d_dgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,

@@ -5,6 +5,11 @@
 // general CUDA-core family (gemm_simt.cu, conv_simt.cu)
 MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                         const float* wt, const float* bias, float* y, int relu, void* stream);
+// the same, followed by BatchNorm with running statistics and an optional addition before the ReLU
+int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
+                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream);
+// y = relu?(batch_norm(x) + residual) over [rows, c] with running statistics; x == y is allowed (batch_norm.cu)
+int mtb_bn_eval_apply(const float* x, float* y, long long rows, int c, const MtbBnEval& bn, const float* residual, int relu, cudaStream_t st);
 MTB_API int mtb_conv2d_dgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                                       const float* wt, float* dx, void* stream);
 MTB_API long long mtb_conv2d_wgrad_simt_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
@@ -19,7 +24,8 @@ bool mtb_tc_conv2d_forward_supported(int n, int cin, int h, int w, int kh, int k
                                      const float* wt, const float* y);
 int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                               const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes, void* stream,
-                              float* stats = nullptr, int* stats_rows = nullptr);
+                              float* stats = nullptr, int* stats_rows = nullptr, const MtbBnEval* bn_eval = nullptr,
+                              const float* residual = nullptr);
 bool mtb_tc_conv2d_dgrad_supported(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                                    const float* wt, const float* dx);
 bool mtb_tc_conv2d_dgrad_in_place(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,

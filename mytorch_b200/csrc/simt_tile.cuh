@@ -304,6 +304,8 @@ struct Out {
   float* out;
   long long ld;
   const float* bias;
+  MtbBnEval bn;              // mean != NULL: BatchNorm with running statistics after the bias (cluster kernels only)
+  const float* residual;     // laid out like out: added before the ReLU (cluster kernels only)
   int relu;
   long long split_plane;     // > 0: every slice of the reduction writes its own plane of partials
   const DgradClass* cls;     // data gradient: row -> pixel of the residue class
@@ -320,11 +322,21 @@ __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
   return o.out + r * o.ld;
 }
 
+// TAIL: with BatchNorm and the residual of Out (the cluster kernels, whose store is one loop)
+template <bool TAIL>
 __device__ __forceinline__ void store4(const Out& o, float* row, int j, int N, bool vec, float4 v) {
   float t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     if (o.bias && j + q < N) t[q] += o.bias[j + q];
+    if constexpr (TAIL) {
+      if (o.bn.mean && j + q < N) {
+        const float rstd = 1.0f / sqrtf(o.bn.var[j + q] + o.bn.eps);
+        const float scale = o.bn.gamma ? o.bn.gamma[j + q] * rstd : rstd, beta = o.bn.beta ? o.bn.beta[j + q] : 0.f;
+        t[q] = (t[q] - o.bn.mean[j + q]) * scale + beta;
+      }
+      if (o.residual && j + q < N) t[q] += o.residual[row - o.out + j + q];
+    }
     if (o.relu) t[q] = fmaxf(t[q], 0.f);
   }
   if (vec && j + 3 < N) {
@@ -457,7 +469,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
         const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], q));
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
       }
-      if (m0 + r < M) store4(o, out_row(o, m0 + r, z), n0 + c, N, vec, s);
+      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>>(o, out_row(o, m0 + r, z), n0 + c, N, vec, s);
     }
     cluster.sync();  // nobody leaves while its tile is being read
   } else {
@@ -468,7 +480,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
       float* row = out_row(o, i, z) + slice * o.split_plane;
 #pragma unroll
       for (int g = 0; g < GN; ++g)
-        store4(o, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
+        store4<false>(o, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
     }
   }
 }
@@ -553,16 +565,16 @@ int launch_tile(const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& tab
 template <class SA, int VA, class SB, int VB>
 int launch(const Choice& c, const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, cudaStream_t st,
            const char* name) {
-  const bool planes = o.split_plane > 0;
+  const bool cluster = (c.slices > 1 && o.split_plane == 0) || o.bn.mean;
   switch (c.tile) {
     case XL: return launch_tile<TileXL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
     case L: return launch_tile<TileL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
     case MD: return launch_tile<TileM, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
     case SM:
-      if (c.slices > 1 && !planes) return launch_tile<TileS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
+      if (cluster) return launch_tile<TileS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
       return launch_tile<TileS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
     default:
-      if (c.slices > 1 && !planes) return launch_tile<TileXS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
+      if (cluster) return launch_tile<TileXS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
       return launch_tile<TileXS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
   }
 }

@@ -345,6 +345,26 @@ struct LaneColSums {
   }
 };
 
+// ---- BatchNorm with running statistics in an epilogue (inference) ----
+//
+// y = (v - mean) * scale + beta, the expression of the BatchNorm kernels (same bits).  The grid makes a CTA stay on one
+// column tile, whose coefficients all its threads put into shared memory before the roles part.
+template <int BN>
+struct BnColumns {
+  float mean[BN], scale[BN], beta[BN];
+};
+template <int BN>
+__device__ __forceinline__ void load_bn_columns(BnColumns<BN>& t, const MtbBnEval& b, int n0, int N) {
+  for (int c = threadIdx.x; c < BN; c += blockDim.x) {
+    const int col = n0 + c;
+    const bool in = col < N;
+    const float rstd = in ? 1.0f / sqrtf(b.var[col] + b.eps) : 0.f;
+    t.mean[c] = in ? b.mean[col] : 0.f;
+    t.scale[c] = in ? (b.gamma ? b.gamma[col] * rstd : rstd) : 0.f;
+    t.beta[c] = in && b.beta ? b.beta[col] : 0.f;
+  }
+}
+
 // ---- host: tensor maps ----
 // fp32 matrix [rows][cols] row-major (row pitch `pitch_elems`), boxes of box_cols x box_rows
 // elements, 128-byte swizzle, zero fill outside the matrix.

@@ -38,6 +38,7 @@ struct RowConvParams {
   long long ldo;
   const float* bias;
   const float* addend;     // optional [same shape as out]: out = conv + addend (gradient accumulation)
+  MtbBnEval bn;            // EPI_BN: out = BatchNorm(conv) (+ addend)
   int relu;
   int issuers;             // issuing warps at work (1 or 2)
   int b_tap_x[64];         // MN-major B only: first column of tap j in the weight matrix
@@ -59,11 +60,13 @@ constexpr int kRowThreads = 32 * (1 + kRowIssuers + 4);  // producer, issuers, f
 // MT = tiles of 128 positions per work item.  With streamed weights two tiles share every weight
 // stage (two accumulators), which halves the L2 -> shared-memory weight traffic per MMA; that traffic,
 // at ~47 B/cycle/SM, is what bounds the 128-channel layers.
-template <int BN, int BMODE, int FK, int MT, bool STATS>
+template <int BN, int BMODE, int FK, int MT, int EPI>
 __global__ void __launch_bounds__(kRowThreads, 1)
 tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const RowConvParams p) {
   constexpr uint32_t kTapBytes = BN * 128;
+  constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN;
   extern __shared__ uint8_t smem_raw[];
+  __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
   __shared__ uint64_t bar_afull[kRowAStages], bar_aempty[kRowAStages], bar_bfull[8], bar_bempty[8], bar_tfull[2], bar_tempty[2], bar_bres;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -103,6 +106,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     tmem_alloc(smem_u32(&tmem_slot), 2 * MT * BN);
     tmem_relinquish();
   }
+  if constexpr (BNORM) load_bn_columns<BN>(bn_columns, p.bn, (int)(blockIdx.x % p.n_tiles) * BN, p.N);
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
@@ -326,6 +330,10 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     WarpColStats<(STATS && !LANE_SUMS) ? BN / 32 : 1> stats;
     LaneColSums<LANE_SUMS ? BN / 32 : 1> sums;
     if constexpr (LANE_SUMS) sums.reset(); else stats.reset();
+    auto bn_apply = [&](float v, int c) {
+      if constexpr (BNORM) return (v - bn_columns.mean[c]) * bn_columns.scale[c] + bn_columns.beta[c];
+      else return v;
+    };
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
       const int q_item = (tile / p.n_tiles) * (128 * MT) + quarter * 32 + lane;
       const int n0 = (tile % p.n_tiles) * BN;
@@ -372,7 +380,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
               float o[8];
 #pragma unroll
               for (int k = 0; k < 8; ++k) {
-                o[k] = __uint_as_float(r[j + k]) + (p.bias ? __ldg(p.bias + n0 + c0 + j + k) : 0.f);
+                o[k] = bn_apply(__uint_as_float(r[j + k]) + (p.bias ? __ldg(p.bias + n0 + c0 + j + k) : 0.f), c0 + j + k);
                 if (p.relu) o[k] = fmaxf(o[k], 0.f);
               }
               st_global_v8(orow + c0 + j, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]);
@@ -465,6 +473,10 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                     const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + jj);
                     o[h].x += b.x; o[h].y += b.y; o[h].z += b.z; o[h].w += b.w;
                   }
+                  if constexpr (BNORM) {
+                    o[h].x = bn_apply(o[h].x, c0 + jj); o[h].y = bn_apply(o[h].y, c0 + jj + 1);
+                    o[h].z = bn_apply(o[h].z, c0 + jj + 2); o[h].w = bn_apply(o[h].w, c0 + jj + 3);
+                  }
                   if (arow) {
                     const float4 b = prefetched ? pre[kPre > 1 ? (c0 + jj) / 4 : 0] : *reinterpret_cast<const float4*>(arow + col0 + jj);
                     o[h].x += b.x; o[h].y += b.y; o[h].z += b.z; o[h].w += b.w;
@@ -479,6 +491,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                 if (col0 + j < p.N) {
                   float o = __uint_as_float(r[j]);
                   if (p.bias) o += p.bias[col0 + j];
+                  o = bn_apply(o, c0 + j);
                   if (arow) o += arow[col0 + j];
                   if (p.relu) o = fmaxf(o, 0.f);
                   orow[col0 + j] = o;
@@ -520,12 +533,12 @@ struct RowConvPlan {
 };
 
 // One candidate layout: mt tiles per work item.
-static bool row_conv_layout(RowConvPlan& r, int mt, int ph, int pw, int taps, int kc, int nout, int bn, bool allow_resident) {
+static bool row_conv_layout(RowConvPlan& r, int mt, int ph, int pw, int taps, int kc, int nout, int bn, bool allow_resident, uint32_t reserve) {
   r.mt = mt;
   r.nr_max = (r.Wp - 1 + 128 * mt - 1) / r.Wp + 1 + 2 * ph;
   const uint32_t need = kRowLead + (uint32_t)(r.nr_max * r.Wp + pw + 8) * 128u;
   r.a_stage_bytes = (need + 1023u) & ~1023u;
-  const uint32_t budget = 227u * 1024u - 2048u;
+  const uint32_t budget = 227u * 1024u - 2048u - reserve;
   const uint32_t fixed = 1024u + kRowAStages * r.a_stage_bytes;
   const uint32_t tap_bytes = (uint32_t)bn * 128u;
   if (fixed + 3u * tap_bytes > budget) return false;
@@ -550,7 +563,8 @@ static bool row_conv_layout(RowConvPlan& r, int mt, int ph, int pw, int taps, in
   return true;
 }
 
-RowConvPlan row_conv_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout, int bn) {
+// reserve: shared memory the kernel needs beside the stages (BatchNorm coefficients)
+RowConvPlan row_conv_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout, int bn, uint32_t reserve = 0) {
   RowConvPlan r{};
   if (getenv("MTB_DISABLE_ROWCONV")) return r;
   if (sh != 1 || sw != 1 || kh != 2 * ph + 1 || kw != 2 * pw + 1 || kh * kw < 2 || kh * kw > 64 || pw > 7 || kc % 32) return r;
@@ -560,38 +574,39 @@ RowConvPlan row_conv_plan(int n, int h, int w, int kh, int kw, int sh, int sw, i
   if ((double)w * h < 0.8 * (double)r.Wp * r.Hv) return r;  // too much padding: the im2col kernel wastes nothing
   if ((long long)n * r.Hv * r.Wp > 0x7ffff000LL) return r;   // the kernel indexes positions with 32-bit integers
   const int taps = kh * kw;
-  if (!row_conv_layout(r, 1, ph, pw, taps, kc, nout, bn, true)) return r;
+  if (!row_conv_layout(r, 1, ph, pw, taps, kc, nout, bn, true, reserve)) return r;
   r.ok = true;
   // Streamed weights: let two tiles share every weight stage when that still fills the GPU.
   if (!r.resident && bn <= 128 && !getenv("MTB_ROWCONV_MT1")) {
     const long long items = (((long long)n * r.Hv * r.Wp + 255) / 256) * ((nout + bn - 1) / bn);
     RowConvPlan r2 = r;
     const long long min_items = getenv("MTB_ROWCONV_MIN_ITEMS") ? atoll(getenv("MTB_ROWCONV_MIN_ITEMS")) : 2LL * mtb_sm_count();
-    if (items >= min_items && row_conv_layout(r2, 2, ph, pw, taps, kc, nout, bn, false) && r2.tps >= 2) r = r2;
+    if (items >= min_items && row_conv_layout(r2, 2, ph, pw, taps, kc, nout, bn, false, reserve) && r2.tps >= 2) r = r2;
   }
   return r;
 }
 
-template <int BN, int BMODE, int FK, int MT, bool STATS>
+template <int BN, int BMODE, int FK, int MT, int EPI>
 int launch_row_conv_kernel(const CUtensorMap& mapA, const CUtensorMap& mapB, const RowConvParams& p, uint32_t smem_bytes, cudaStream_t st) {
-  auto kernel = tc_conv_rows_kernel<BN, BMODE, FK, MT, STATS>;
+  auto kernel = tc_conv_rows_kernel<BN, BMODE, FK, MT, EPI>;
   static unsigned long long configured = 0;
-  if (int rc = mtb_opt_in_smem((const void*)kernel, 227 * 1024 - 1024, &configured)) return rc;
+  if (int rc = mtb_opt_in_smem((const void*)kernel, 227 * 1024 - (EPI == EPI_BN ? 1024 + 12 * BN : 1024), &configured)) return rc;
   const int items = ((p.m_tiles + MT - 1) / MT) * p.n_tiles;
   int grid = items < mtb_sm_count() ? items : mtb_sm_count();
-  if (STATS) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one output-channel tile
+  if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one output-channel tile
   kernel<<<grid, kRowThreads, smem_bytes, st>>>(mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_conv_rows_kernel");
   return MTB_OK;
 }
 
-// the statistics variant exists for the forward role only (K-major weights)
+// the statistics and BatchNorm variants exist for the forward role only (K-major weights)
 template <int BN, int BMODE, int FK, int MT>
 int launch_row_conv(const CUtensorMap& mapA, const CUtensorMap& mapB, const RowConvParams& p, uint32_t smem_bytes, cudaStream_t st) {
   if constexpr (BMODE == B_KMAJOR) {
-    if (p.stats) return launch_row_conv_kernel<BN, BMODE, FK, MT, true>(mapA, mapB, p, smem_bytes, st);
+    if (p.stats) return launch_row_conv_kernel<BN, BMODE, FK, MT, EPI_STATS>(mapA, mapB, p, smem_bytes, st);
+    if (p.bn.mean) return launch_row_conv_kernel<BN, BMODE, FK, MT, EPI_BN>(mapA, mapB, p, smem_bytes, st);
   }
-  return launch_row_conv_kernel<BN, BMODE, FK, MT, false>(mapA, mapB, p, smem_bytes, st);
+  return launch_row_conv_kernel<BN, BMODE, FK, MT, EPI_PLAIN>(mapA, mapB, p, smem_bytes, st);
 }
 
 // Partial-statistics rows the STATS variant writes (see RowConvParams::stats).
@@ -615,7 +630,7 @@ int launch_row_conv_bn(int bn, int mt, const CUtensorMap& mapA, const CUtensorMa
 template <int BMODE>
 int run_row_conv(const RowConvPlan& plan, int bn, int n, int h, int w, int kc, int kh, int kw, int ph, int pw, int nout, const float* act,
                  const CUtensorMap& mapB, const int* b_tap_x, const float* bias, const float* addend, int relu, float* out, cudaStream_t st,
-                 float* stats = nullptr) {
+                 float* stats = nullptr, const MtbBnEval* bn_eval = nullptr) {
   CUtensorMap mapA;
   int rc = tc::encode_rows_4d(&mapA, act, n, h, w, kc, 32, plan.Wp);
   if (rc) return rc;
@@ -628,6 +643,7 @@ int run_row_conv(const RowConvPlan& plan, int bn, int n, int h, int w, int kc, i
   p.out = out; p.ldo = nout; p.bias = bias; p.addend = addend; p.relu = relu;
   p.issuers = getenv("MTB_ROWCONV_ONE_ISSUER") ? 1 : kRowIssuers;
   p.stats = stats;
+  if (bn_eval) p.bn = *bn_eval;
   if (b_tap_x) for (int j = 0; j < kh * kw; ++j) p.b_tap_x[j] = b_tap_x[j];
   return launch_row_conv_bn<BMODE>(bn, plan.mt, mapA, mapB, p, plan.smem_bytes, st);
 }

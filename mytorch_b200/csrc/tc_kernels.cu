@@ -111,6 +111,7 @@ struct GemmParams {
   // optional tensor laid out like `out`: out = result + addend (gradient accumulation).  May be `out` itself: a
   // thread reads the very elements it then writes.
   const float* addend;
+  MtbBnEval bn;  // EPI_BN
   int relu;
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
@@ -152,20 +153,22 @@ struct Cfg {
   static constexpr uint32_t kTmemCols = 2 * BN;
 };
 
-// What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, or add a tensor.
-enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2 };
+// What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, add a tensor, or BatchNorm
+// with running statistics (then optionally add a tensor).
+enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3 };
 
 template <int BN, int AMODE, int BMODE, int EPI>
 __global__ void __launch_bounds__(192, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p) {
   using C = Cfg<BN>;
   constexpr int STAGES = C::kStages;
-  constexpr bool STATS = EPI == EPI_STATS, ADD = EPI == EPI_ADD;
+  constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN, ADD = EPI == EPI_ADD || BNORM;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ int split_last;
+  __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -187,6 +190,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     tmem_alloc(smem_u32(&tmem_slot), C::kTmemCols);
     tmem_relinquish();
   }
+  if constexpr (BNORM) load_bn_columns<BN>(bn_columns, p.bn, (blockIdx.x / p.splits) % p.n_tiles * BN, p.N);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -340,13 +344,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         orow_index = ((long long)nn * p.o_H + p.o_h0 + p.o_sh * i) * p.o_W + p.o_w0 + p.o_sw * j;
       }
       float* orow = p.out + orow_index * p.ldo;
-      const float* arow = ADD ? p.addend + orow_index * p.ldo : nullptr;
+      const float* arow = ADD && (!BNORM || p.addend) ? p.addend + orow_index * p.ldo : nullptr;
       const bool valid = row < p.M;
       const float cnt = STATS ? (float)__popc(__ballot_sync(0xffffffffu, valid)) : 0.f;
       // r: this lane's row of the finished accumulator, columns c0 .. c0+31 of the tile; add: the same columns of the
       // addend, fetched one chunk ahead (a memory round trip per chunk in front of the stores would make the epilogue
       // of a short reduction several times longer than its main loop)
-      const bool adds = ADD && valid && vec_ok && n0 + BN <= p.N;
+      const bool adds = ADD && arow && valid && vec_ok && n0 + BN <= p.N;
       auto fetch_addend = [&](int c0, float4 (&add)[8]) {
         if (adds) {
 #pragma unroll
@@ -392,7 +396,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + jj);
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
-                  if constexpr (ADD) {
+                  if constexpr (BNORM) {
+                    const float4 mu = *reinterpret_cast<const float4*>(&bn_columns.mean[c0 + jj]);
+                    const float4 g = *reinterpret_cast<const float4*>(&bn_columns.scale[c0 + jj]);
+                    const float4 b = *reinterpret_cast<const float4*>(&bn_columns.beta[c0 + jj]);
+                    v[h].x = (v[h].x - mu.x) * g.x + b.x; v[h].y = (v[h].y - mu.y) * g.y + b.y;
+                    v[h].z = (v[h].z - mu.z) * g.z + b.z; v[h].w = (v[h].w - mu.w) * g.w + b.w;
+                  }
+                  if (ADD && arow) {
                     const float4 b = adds ? add[jj / 4] : *reinterpret_cast<const float4*>(arow + col0 + jj);
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
@@ -406,7 +417,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (col0 + j < p.N) {
                   float v = __uint_as_float(r[j]);
                   if (p.bias) v += p.bias[col0 + j];
-                  if constexpr (ADD) v += arow[col0 + j];
+                  if constexpr (BNORM) v = (v - bn_columns.mean[c0 + j]) * bn_columns.scale[c0 + j] + bn_columns.beta[c0 + j];
+                  if (ADD && arow) v += arow[col0 + j];
                   if (p.relu) v = fmaxf(v, 0.f);
                   orow[col0 + j] = v;
                 }
@@ -545,7 +557,7 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
   if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
   int tiles = p.m_tiles * p.n_tiles * p.splits;  // work units
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
-  if (EPI == EPI_STATS && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
+  if ((EPI == EPI_STATS || EPI == EPI_BN) && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
   kernel<<<grid, 192, C::kSmemBytes, st>>>(mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
@@ -733,23 +745,23 @@ bool mtb_tc_conv2d_forward_supported(int n, int cin, int h, int w, int kh, int k
 // *stats_rows == 0 means this launch did not produce statistics.
 int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                               const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes, void* stream,
-                              float* stats, int* stats_rows) {
+                              float* stats, int* stats_rows, const MtbBnEval* bn_eval, const float* residual) {
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   const long long M = (long long)n * oh * ow, K = (long long)kh * kw * cin;
-  const bool rows_path = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, pick_bn_for(cout, M)).ok;
-  GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), !rows_path && workspace != nullptr);
-  if (split_partial_bytes(gp, M, cout) > workspace_bytes) gp = GemmPlan{pick_bn_for(cout, M), 1, (int)(K / 32)};
-  const int bn = rows_path ? pick_bn_for(cout, M) : gp.bn;
+  const int row_bn = pick_bn_for(cout, M);
+  const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, row_bn, bn_eval ? 12u * row_bn : 0u);
+  GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), !plan.ok && workspace != nullptr);
+  if (split_partial_bytes(gp, M, cout) > workspace_bytes) gp = GemmPlan{row_bn, 1, (int)(K / 32)};
+  const int bn = plan.ok ? row_bn : gp.bn;
   if (stats_rows) *stats_rows = 0;
   const bool want_stats = stats && stats_rows && !relu && cout % 32 == 0 && (!bias || al16(bias)) && !getenv("MTB_DISABLE_CONV_STATS");
   CUtensorMap mapA, mapB;
   int rc = tc::encode_tiled_2d(&mapB, wt, cout, K, K, 32, bn);
   if (rc) return rc;
-  const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, bn);
   if (plan.ok) {
     if (want_stats) *stats_rows = row_conv_stats_rows(plan, (long long)n * plan.Hv * plan.Wp, cout, bn);
-    return run_row_conv<B_KMAJOR>(plan, bn, n, h, w, cin, kh, kw, ph, pw, cout, x, mapB, nullptr, bias, nullptr, relu, y, (cudaStream_t)stream,
-                                  want_stats ? stats : nullptr);
+    return run_row_conv<B_KMAJOR>(plan, bn, n, h, w, cin, kh, kw, ph, pw, cout, x, mapB, nullptr, bias, residual, relu, y, (cudaStream_t)stream,
+                                  want_stats ? stats : nullptr, bn_eval);
   }
   rc = tc::encode_im2col_4d(&mapA, x, n, h, w, cin, -pw, -ph, pw - (kw - 1), ph - (kh - 1), sw, sh, 32, 128);
   if (rc) return rc;
@@ -770,6 +782,11 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
     *stats_rows = gp.splits > 1 ? p.m_tiles * 4 : stats_rows_for(p.m_tiles * p.n_tiles, p.n_tiles);
     cudaStream_t st = (cudaStream_t)stream;
     return launch_tc_bn<A_IM2COL, B_KMAJOR, EPI_STATS>(bn, mapA, mapB, p, st);
+  }
+  if (bn_eval) {
+    p.bn = *bn_eval;
+    p.addend = residual;
+    return launch_tc_bn<A_IM2COL, B_KMAJOR, EPI_BN>(bn, mapA, mapB, p, (cudaStream_t)stream);
   }
   return launch_tc_bn<A_IM2COL, B_KMAJOR>(bn, mapA, mapB, p, (cudaStream_t)stream);
 }

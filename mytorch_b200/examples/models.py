@@ -7,6 +7,7 @@ initialisation consumes one random draw per weight / bias tensor in creation ord
 """
 import mytorch_b200.nn as nn
 import mytorch_b200.nn.functional as F
+from mytorch_b200.nn.batch_norm import inference_conv_norm
 
 
 class Flatten(nn.Module):
@@ -30,6 +31,16 @@ def _feed_batch_norm(*convs):
     """Mark convolutions whose output goes straight into a BatchNorm layer (see ``nn.Conv2d.feeds_batch_norm``)."""
     for conv in convs:
         conv.feeds_batch_norm = True
+
+
+def _conv_norm(conv, norm, x, *residual):
+    """norm(conv(x), *residual), in the convolution's launch where nothing is differentiated."""
+    kind = type(norm)
+    if not norm.training and (kind is not nn.BatchNorm2d or not residual):
+        y = inference_conv_norm(conv, norm, x, kind is not nn.BatchNorm2d, *residual)
+        if y is not None:
+            return y
+    return norm(conv(x), *residual)
 
 
 class BasicBlock(nn.Module):
@@ -57,12 +68,10 @@ class BasicBlock(nn.Module):
         # gradient for every pixel of x, and the 1x1 / stride-2 convolution adds its own in place to the
         # pixels it reaches (instead of a zero-filled tensor that has to be added afterwards).
         shortcut = x if self.downsample is None else self.downsample(x)
-        y = self.bn1(self.conv1(x))
-        if not self.fused:
-            y = self.relu(y)
+        y = _conv_norm(self.conv1, self.bn1, x)
         if self.fused:
-            return self.bn2(self.conv2(y), shortcut)
-        return self.relu(self.bn2(self.conv2(y)) + shortcut)
+            return _conv_norm(self.conv2, self.bn2, y, shortcut)
+        return self.relu(self.bn2(self.conv2(self.relu(y))) + shortcut)
 
 
 class ResNet18Cifar(nn.Module):
@@ -87,7 +96,7 @@ class ResNet18Cifar(nn.Module):
             _feed_batch_norm(self.conv1)
 
     def forward(self, x):
-        x = self.bn1(self.conv1(x))
+        x = _conv_norm(self.conv1, self.bn1, x)
         if not self.fused:
             x = self.relu(x)
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
@@ -115,7 +124,8 @@ class Bottleneck(nn.Module):
 
     def forward(self, x):
         shortcut = x if self.downsample is None else self.downsample(x)  # first: see BasicBlock
-        return self.bn3(self.conv3(self.bn2(self.conv2(self.bn1(self.conv1(x))))), shortcut)
+        y = _conv_norm(self.conv2, self.bn2, _conv_norm(self.conv1, self.bn1, x))
+        return _conv_norm(self.conv3, self.bn3, y, shortcut)
 
 
 class ResNet50(nn.Module):
@@ -137,7 +147,7 @@ class ResNet50(nn.Module):
         self.fc = nn.Linear(cin, num_classes, device=device)
 
     def forward(self, x):
-        x = self.maxpool(self.bn1(self.conv1(x)))
+        x = self.maxpool(_conv_norm(self.conv1, self.bn1, x))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(x.mean(dim=(2, 3)))
 

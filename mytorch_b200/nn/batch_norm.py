@@ -5,6 +5,7 @@ from mytorch_b200.dtype import float32
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d, _batch_norm2d_add_relu, _batch_norm2d_relu
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.parameter import Parameter
+from mytorch_b200.ops._common import dispatch, tracker
 from mytorch_b200.tensor import Tensor
 
 
@@ -69,3 +70,21 @@ class BatchNorm1d(BatchNorm2d):
         y = _batch_norm2d(x.reshape((n, c, length, 1)), self.weight, self.bias, self.eps, self.training, self.momentum, self.running_mean,
                           self.running_var)
         return y.reshape(x.shape)
+
+
+def inference_conv_norm(conv, norm, x, relu=False, residual=None):
+    """``norm(conv(x))``, then optionally ``+ residual``, then optionally ReLU, as one operator where that is possible: a
+    convolution and a BatchNorm layer that normalises with its running statistics, on CUDA, with no gradient to record.
+    None elsewhere.  Same bits as the separate layers."""
+    if norm.training or norm.running_mean is None or x.device.type != "cuda":
+        return None
+    if not tracker.no_grad and (x.requires_grad or conv.weight.requires_grad or norm.weight is not None and norm.weight.requires_grad
+                                or residual is not None and residual.requires_grad):
+        return None
+    channels = (norm.num_features,)
+    tensors = [conv.weight, norm.running_mean, norm.running_var] + [t for t in (conv.bias, norm.weight, norm.bias, residual) if t is not None]
+    if (conv.weight.shape[0],) != channels or any(t.device is not x.device or t.dtype is not x.dtype for t in tensors):
+        return None  # the separate operators say what is wrong
+    affine = norm.weight is not None and norm.bias is not None
+    return dispatch(x.device, "conv2d_batch_norm")(x, conv.weight, conv.bias, conv.stride, conv.padding, norm.weight if affine else None,
+                                                   norm.bias if affine else None, norm.running_mean, norm.running_var, norm.eps, relu, residual)
