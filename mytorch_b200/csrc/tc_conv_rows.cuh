@@ -41,6 +41,7 @@ struct RowConvParams {
   MtbBnEval bn;            // EPI_BN: out = BatchNorm(conv) (+ addend)
   int relu;
   int issuers;             // issuing warps at work (1 or 2)
+  int b_blocks;            // MN-major B through one copy per tap (encode_blocks_3d) instead of one per 32 columns
   int b_tap_x[64];         // MN-major B only: first column of tap j in the weight matrix
   // STATS kernels only: partial rows [(blockIdx.x / n_tiles) * 4 + epilogue warp][3][N] of per-channel
   // (count, mean, M2) over the pixels this CTA produced (grid is a multiple of n_tiles)
@@ -135,8 +136,12 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             if (BMODE == B_KMAJOR) {
               tma_load_2d(b_dst, &mapB, bres, tap * p.kc_total + cc * 32, 0);
             } else {
+              if (p.b_blocks) {
+                tma_load_3d(b_dst, &mapB, bres, 0, cc * 32, p.b_tap_x[tap] / 32);
+              } else {
 #pragma unroll
-              for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, bres, p.b_tap_x[tap] + 32 * j, cc * 32);
+                for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, bres, p.b_tap_x[tap] + 32 * j, cc * 32);
+              }
             }
           }
       }
@@ -170,8 +175,12 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
               if (BMODE == B_KMAJOR) {
                 tma_load_2d(b_dst, &mapB, bfull, tap * p.kc_total + cc * 32, n0);
               } else {
+              if (p.b_blocks) {
+                  tma_load_3d(b_dst, &mapB, bfull, 0, cc * 32, (p.b_tap_x[tap] + n0) / 32);
+                } else {
 #pragma unroll
-                for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, bfull, p.b_tap_x[tap] + n0 + 32 * j, cc * 32);
+                  for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, bfull, p.b_tap_x[tap] + n0 + 32 * j, cc * 32);
+                }
               }
             }
             if (++bs == BST) { bs = 0; bphase ^= 1u; }
@@ -563,6 +572,25 @@ static bool row_conv_layout(RowConvPlan& r, int mt, int ph, int pw, int taps, in
   return true;
 }
 
+// What a launch takes, in ns: waves x tiles per item x reduction blocks x the measured time of a block.  The 64-wide kernel is
+// bound by reading 6 KB of operands per 48-cycle MMA from shared memory, the 128-wide one by 8 KB per 64 cycles plus what the
+// copies write; a 256-wide tile waits for its weights (one tap per stage).
+double row_conv_ns(const RowConvPlan& r, int bn, long long positions, int nout, int num_kb) {
+  const long long items = ((positions + 128 * r.mt - 1) / (128 * r.mt)) * ((nout + bn - 1) / bn);
+  const long long waves = (items + mtb_sm_count() - 1) / mtb_sm_count();
+  const double block = bn == 64 ? (r.resident ? 150 : r.mt == 2 ? 162 : 200) : bn == 128 ? (r.mt == 2 ? 222 : 290) : 479;
+  return (double)waves * r.mt * num_kb * block + 2000.0;
+}
+
+// Whether to take the row-staged kernel where it fits.  Up to 64 output channels always: the im2col kernel gathers every pixel
+// nine times for MMAs of half the rate (64 -> 64 on 512 x 32x32: 134 us against 87).  Wider layers go by price: with 128 and
+// more columns per gathered pixel the im2col kernel is near the MMA rate and wastes nothing on padding positions (128 -> 128 on
+// 128 x 16x16: 26 us against 33; 256 -> 256 on 128 x 14x14: 55 against 73; but 128 -> 128 on 128 x 28x28: 65 against 54).
+bool row_conv_pays(const RowConvPlan& r, int bn, long long positions, int nout, int num_kb, double im2col_ns) {
+  if (!r.ok) return false;
+  return nout <= 64 || getenv("MTB_ROWCONV_MIN_ITEMS") || row_conv_ns(r, bn, positions, nout, num_kb) <= im2col_ns;
+}
+
 // reserve: shared memory the kernel needs beside the stages (BatchNorm coefficients)
 RowConvPlan row_conv_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout, int bn, uint32_t reserve = 0) {
   RowConvPlan r{};
@@ -576,12 +604,16 @@ RowConvPlan row_conv_plan(int n, int h, int w, int kh, int kw, int sh, int sw, i
   const int taps = kh * kw;
   if (!row_conv_layout(r, 1, ph, pw, taps, kc, nout, bn, true, reserve)) return r;
   r.ok = true;
-  // Streamed weights: let two tiles share every weight stage when that still fills the GPU.
+  // Streamed weights: two tiles may share every weight stage.
   if (!r.resident && bn <= 128 && !getenv("MTB_ROWCONV_MT1")) {
-    const long long items = (((long long)n * r.Hv * r.Wp + 255) / 256) * ((nout + bn - 1) / bn);
+    const long long positions = (long long)n * r.Hv * r.Wp;
     RowConvPlan r2 = r;
-    const long long min_items = getenv("MTB_ROWCONV_MIN_ITEMS") ? atoll(getenv("MTB_ROWCONV_MIN_ITEMS")) : 2LL * mtb_sm_count();
-    if (items >= min_items && row_conv_layout(r2, 2, ph, pw, taps, kc, nout, bn, false, reserve) && r2.tps >= 2) r = r2;
+    if (row_conv_layout(r2, 2, ph, pw, taps, kc, nout, bn, false, reserve) && r2.tps >= 2) {
+      const char* least = getenv("MTB_ROWCONV_MIN_ITEMS");
+      const bool two = least ? ((positions + 255) / 256) * ((nout + bn - 1) / bn) >= atoll(least)
+                             : row_conv_ns(r2, bn, positions, nout, taps * kc / 32) < row_conv_ns(r, bn, positions, nout, taps * kc / 32);
+      if (two) r = r2;
+    }
   }
   return r;
 }
@@ -630,7 +662,7 @@ int launch_row_conv_bn(int bn, int mt, const CUtensorMap& mapA, const CUtensorMa
 template <int BMODE>
 int run_row_conv(const RowConvPlan& plan, int bn, int n, int h, int w, int kc, int kh, int kw, int ph, int pw, int nout, const float* act,
                  const CUtensorMap& mapB, const int* b_tap_x, const float* bias, const float* addend, int relu, float* out, cudaStream_t st,
-                 float* stats = nullptr, const MtbBnEval* bn_eval = nullptr) {
+                 float* stats = nullptr, const MtbBnEval* bn_eval = nullptr, bool b_blocks = false) {
   CUtensorMap mapA;
   int rc = tc::encode_rows_4d(&mapA, act, n, h, w, kc, 32, plan.Wp);
   if (rc) return rc;
@@ -644,6 +676,7 @@ int run_row_conv(const RowConvPlan& plan, int bn, int n, int h, int w, int kc, i
   p.issuers = getenv("MTB_ROWCONV_ONE_ISSUER") ? 1 : kRowIssuers;
   p.stats = stats;
   if (bn_eval) p.bn = *bn_eval;
+  p.b_blocks = b_blocks;
   if (b_tap_x) for (int j = 0; j < kh * kw; ++j) p.b_tap_x[j] = b_tap_x[j];
   return launch_row_conv_bn<BMODE>(bn, plan.mt, mapA, mapB, p, plan.smem_bytes, st);
 }
@@ -952,6 +985,16 @@ WgradRowsPlan wgrad_rows_plan(int n, int cin, int h, int w, int kh, int kw, int 
   r.splits = (r.kb_total + r.kb_per_split - 1) / r.kb_per_split;
   r.ok = true;
   return r;
+}
+
+// Whether to take the row-staged weight gradient where it fits.  It stages X and dY once for all taps but its tiles are 64
+// columns wide and a quarter of every MMA is dropped; the im2col form, one copy per stage for dY, overtakes it as soon as the
+// layer is wider than 64 channels (128 -> 128 on 512 x 16x16: 76 us against 123; 256 -> 256 on 128 x 14x14: 60 against 115), and
+// on 64 channels where a CTA has only a few position blocks (64 images of 32x32, 4 blocks: 27 us against 31; at 23 and 31
+// blocks: 92 against 94, 110 against 126).  With one block of 32 input channels the two are level (32 -> 32 on 512 x 28x28: 62
+// against 64).
+bool wgrad_rows_pay(const WgradRowsPlan& r, int cin, int cout) {
+  return r.ok && (cin <= 32 || (cin <= 64 && cout <= 64 && r.kb_per_split >= 16));
 }
 
 template <int BN, int FIX>

@@ -60,6 +60,20 @@ int encode_tiled_2d(CUtensorMap* map, const float* base, long long rows, long lo
   return MTB_OK;
 }
 
+int encode_blocks_3d(CUtensorMap* map, const float* base, long long rows, long long cols, long long pitch_elems, int box_rows, int blocks) {
+  int rc = load_driver_entry_points();
+  if (rc) return rc;
+  cuuint64_t dims[3] = {32, (cuuint64_t)rows, (cuuint64_t)(cols / 32)};
+  cuuint64_t strides[2] = {(cuuint64_t)pitch_elems * 4, 128};
+  cuuint32_t box[3] = {32, (cuuint32_t)box_rows, (cuuint32_t)blocks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = g_encode_tiled(map, tma_dtype(), 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return mtb_fail(MTB_ERR_CUDA, "cuTensorMapEncodeTiled (blocks) failed (%d) rows=%lld cols=%lld pitch=%lld box=%d blocks=%d", (int)r, rows, cols, pitch_elems, box_rows, blocks);
+  return MTB_OK;
+}
+
 int encode_rows_4d(CUtensorMap* map, const float* base, int n, int h, int w, int c, int channels, int box_w, bool mn_major) {
   int rc = load_driver_entry_points();
   if (rc) return rc;
@@ -115,6 +129,8 @@ struct GemmParams {
   int relu;
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
+  // MN-major operands through one copy per reduction block (encode_blocks_3d) instead of one per 32 columns
+  int a_blocks, b_blocks;
   // B operand addressed per filter tap (data gradient: weights read in place).  When set, the
   // k-block (tap, cc) reads B at inner coordinate b_tap_x[tap] + n0 (+32j), outer cc*32.
   int b_per_tap;
@@ -234,8 +250,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             if (AMODE == A_KMAJOR) {
               tma_load_2d(a_dst, &mapA, full, kbh * 32, m0);
             } else if (AMODE == A_MNMAJOR) {
+              if (p.a_blocks) {
+                tma_load_3d(a_dst, &mapA, full, 0, kbh * 32, m0 / 32);
+              } else {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) tma_load_2d(a_dst + j * 4096, &mapA, full, m0 + 32 * j, kbh * 32);
+                for (int j = 0; j < 4; ++j) tma_load_2d(a_dst + j * 4096, &mapA, full, m0 + 32 * j, kbh * 32);
+              }
             } else {
               tma_load_im2col_4d(a_dst, &mapA, full, cc * 32, pix_w, pix_h, pix_n, (uint16_t)kw, (uint16_t)kh);
             }
@@ -244,8 +264,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             } else {
               int bx = n0, by = kbh * 32;
               if (p.b_per_tap) { bx = p.b_tap_x[tap] + n0; by = cc * 32; }
+              if (p.b_blocks) {
+                tma_load_3d(b_dst, &mapB, full, 0, by, bx / 32);
+              } else {
 #pragma unroll
-              for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, full, bx + 32 * j, by);
+                for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * 4096, &mapB, full, bx + 32 * j, by);
+              }
             }
             if (++cc == p.cchunks) {
               cc = 0;
@@ -589,6 +613,26 @@ int pick_bn_for(int n, long long rows) {
   return bn;
 }
 
+// What a launch of the im2col kernel without split takes, in ns: waves x (reduction blocks x the time of one block + about
+// 900 ns for filling the pipeline and the first stores).  The block times were measured (weights K-major in forward,
+// MN-major in the data gradient; 72 blocks on 64 to 592 images of 8x8): a 64-wide tile is bound by the gather of 128
+// pixel rows, a 256-wide one by the MMAs.  `copies` launches of this size share the GPU.
+double im2col_ns(int bn, int n, long long rows, int num_kb, bool mn_major, int copies = 1) {
+  const long long tiles = ((rows + 127) / 128) * ((n + bn - 1) / bn) * copies, waves = (tiles + mtb_sm_count() - 1) / mtb_sm_count();
+  const double block = mn_major ? (bn == 64 ? 285 : bn == 128 ? 295 : 405) : (bn == 64 ? 232 : bn == 128 ? 262 : 376);
+  const double store = 8.0 * bn;  // a tile's epilogue: longer than the main loop of a short reduction
+  return waves * ((num_kb * block > store ? num_kb * block : store) + 900.0) + store;
+}
+
+// The tile width with the least time: one more wave costs more than a narrower or wider tile gains (256 -> 256 channels on
+// 100 images of 8x8: 200 tiles of 64 columns are two waves, 34 us; 100 tiles of 128 one, 23 us).
+int cheapest_bn(int n, long long rows, int num_kb, bool mn_major, int copies = 1) {
+  int best = pick_bn(n);
+  for (int bn = best >> 1; bn >= 64; bn >>= 1)
+    if (im2col_ns(bn, n, rows, num_kb, mn_major, copies) < im2col_ns(best, n, rows, num_kb, mn_major, copies)) best = bn;
+  return best;
+}
+
 // Tile width and reduction split for the im2col / GEMM kernel.  These kernels are bound by what one SM
 // can pull from L2 into shared memory (about 89 GB/s: 47 B per cycle), then by the MMA rate, so a launch
 // is priced as waves x reduction blocks per unit x the slower of (bytes of one block of A and B at that
@@ -597,11 +641,11 @@ int pick_bn_for(int n, long long rows) {
 // (tiles x splits <= SMs) and every unit keeps at least eight reduction blocks.
 struct GemmPlan { int bn, splits, kb_per_split; };
 
-GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, int force_bn = 0) {
+GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, bool mn_major, int force_bn = 0, int copies = 1) {
   const int sms = mtb_sm_count();
   const long long m_tiles = (rows + 127) / 128;
   static const int kSplits[] = {1, 2, 3, 4, 6, 8};
-  GemmPlan best{force_bn ? force_bn : pick_bn_for(n, rows), 1, num_kb};
+  GemmPlan best{force_bn ? force_bn : cheapest_bn(n, rows, num_kb, mn_major, copies), 1, num_kb};
   // Measured: the split only pays when even 64-wide tiles leave half the GPU idle (the 4x4 layers at 64
   // images: 41 -> 24 us for the data gradient of 512 -> 512); with more tiles than that the last unit's pass
   // over the partials costs more than the idle SMs did (256 -> 256 on 8x8 at 64 images: 20 -> 40 us).
@@ -709,15 +753,19 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                     void* stream) {
   CUtensorMap mapA, mapB;
-  int bn = pick_bn_for(n, m);
+  const int bn = cheapest_bn(n, m, (k + 31) / 32, !trans_b);
   int rc;
+  GemmParams p{};
+  p.a_blocks = trans_a && m % 32 == 0;
+  p.b_blocks = !trans_b && n % 32 == 0;
   if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, 128);
+  else if (p.a_blocks) rc = tc::encode_blocks_3d(&mapA, a, k, m, m, 32, 4);
   else rc = tc::encode_tiled_2d(&mapA, a, k, m, m, 32, 32, true);
   if (rc) return rc;
   if (trans_b) rc = tc::encode_tiled_2d(&mapB, b, n, k, k, 32, bn);
+  else if (p.b_blocks) rc = tc::encode_blocks_3d(&mapB, b, k, n, n, 32, bn / 32);
   else rc = tc::encode_tiled_2d(&mapB, b, k, n, n, 32, 32, true);
   if (rc) return rc;
-  GemmParams p{};
   p.splits = 1; p.kb_per_split = (k + 31) / 32;
   p.M = m; p.N = n; p.num_kb = (k + 31) / 32;
   p.m_tiles = (m + 127) / 128; p.n_tiles = (n + bn - 1) / bn;
@@ -750,15 +798,16 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   const long long M = (long long)n * oh * ow, K = (long long)kh * kw * cin;
   const int row_bn = pick_bn_for(cout, M);
   const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, row_bn, bn_eval ? 12u * row_bn : 0u);
-  GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), !plan.ok && workspace != nullptr);
-  if (split_partial_bytes(gp, M, cout) > workspace_bytes) gp = GemmPlan{row_bn, 1, (int)(K / 32)};
-  const int bn = plan.ok ? row_bn : gp.bn;
+  GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), !plan.ok && workspace != nullptr, false);
+  if (split_partial_bytes(gp, M, cout) > workspace_bytes) gp = GemmPlan{cheapest_bn(cout, M, (int)(K / 32), false), 1, (int)(K / 32)};
+  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), im2col_ns(gp.bn, cout, M, (int)(K / 32), false));
+  const int bn = staged ? row_bn : gp.bn;
   if (stats_rows) *stats_rows = 0;
   const bool want_stats = stats && stats_rows && !relu && cout % 32 == 0 && (!bias || al16(bias)) && !getenv("MTB_DISABLE_CONV_STATS");
   CUtensorMap mapA, mapB;
   int rc = tc::encode_tiled_2d(&mapB, wt, cout, K, K, 32, bn);
   if (rc) return rc;
-  if (plan.ok) {
+  if (staged) {
     if (want_stats) *stats_rows = row_conv_stats_rows(plan, (long long)n * plan.Hv * plan.Wp, cout, bn);
     return run_row_conv<B_KMAJOR>(plan, bn, n, h, w, cin, kh, kw, ph, pw, cout, x, mapB, nullptr, bias, residual, relu, y, (cudaStream_t)stream,
                                   want_stats ? stats : nullptr, bn_eval);
@@ -819,20 +868,24 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   // one tile width for all residue classes (the weight tensor map is shared): the one the cost model picks
   // for a class-sized problem
   const long long class_rows = (long long)n * h * w / (sh * sw);
-  const bool rows_path = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin, pick_bn_for(cin, class_rows)).ok;
   const int class_kb = ((kh + sh - 1) / sh) * ((kw + sw - 1) / sw) * (cout / 32);
-  const int bn = rows_path ? pick_bn_for(cin, class_rows) : plan_gemm(cin, class_rows, class_kb, workspace != nullptr).bn;
+  const int row_bn = pick_bn_for(cin, class_rows);
+  const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin, row_bn);
+  const int gemm_bn = plan_gemm(cin, class_rows, class_kb, workspace != nullptr, true, 0, sh * sw).bn;
+  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb, im2col_ns(gemm_bn, cin, class_rows, class_kb, true));
+  const int bn = staged ? row_bn : gemm_bn;
   cudaStream_t st = (cudaStream_t)stream;
   CUtensorMap mapB;
-  int rc = tc::encode_tiled_2d(&mapB, wt, cout, (long long)kh * kw * cin, (long long)kh * kw * cin, 32, 32, true);
+  const long long wcols = (long long)kh * kw * cin;
+  const bool b_blocks = cin % 32 == 0;  // a tap's columns then are whole blocks
+  int rc = b_blocks ? tc::encode_blocks_3d(&mapB, wt, cout, wcols, wcols, 32, bn / 32) : tc::encode_tiled_2d(&mapB, wt, cout, wcols, wcols, 32, 32, true);
   if (rc) return rc;
-  const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin, bn);
-  if (plan.ok) {
+  if (staged) {
     // stride 1: dX = dY convolved with the filter rotated by 180 degrees, same padding
     int tap_x[64];
     for (int jh = 0; jh < kh; ++jh)
       for (int jw = 0; jw < kw; ++jw) tap_x[jh * kw + jw] = ((kh - 1 - jh) * kw + (kw - 1 - jw)) * cin;
-    return run_row_conv<B_MNMAJOR>(plan, bn, n, h, w, cout, kh, kw, ph, pw, cin, dy, mapB, tap_x, nullptr, addend, 0, dx, st);
+    return run_row_conv<B_MNMAJOR>(plan, bn, n, h, w, cout, kh, kw, ph, pw, cin, dy, mapB, tap_x, nullptr, addend, 0, dx, st, nullptr, nullptr, b_blocks);
   }
   struct Axis { int taps, start, count, lower, upper; };
   auto axis = [](int a, int size, int osize, int k, int s, int pad) {
@@ -885,7 +938,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
       GemmParams p{};
       const long long M = (long long)n * ah.count * aw.count;
       p.M = (int)M; p.N = cin; p.num_kb = ah.taps * aw.taps * (cout / 32);
-      GemmPlan gp = plan_gemm(cin, M, p.num_kb, workspace != nullptr && lanes == 1, bn);
+      GemmPlan gp = plan_gemm(cin, M, p.num_kb, workspace != nullptr && lanes == 1, true, bn);
       if (split_partial_bytes(gp, M, cin) > workspace_bytes) gp = GemmPlan{bn, 1, p.num_kb};
       p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
       p.m_tiles = (int)((M + 127) / 128); p.n_tiles = (cin + bn - 1) / bn;
@@ -894,6 +947,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
       p.OW = aw.count; p.OH = ah.count; p.SW = 1; p.SH = 1; p.PW = -aw.lower; p.PH = -ah.lower; p.KW = aw.taps; p.KH = ah.taps;
       p.cchunks = cout / 32;
       p.b_per_tap = 1;
+      p.b_blocks = b_blocks;
       for (int jh = 0; jh < ah.taps; ++jh)
         for (int jw = 0; jw < aw.taps; ++jw) {
           const int fkh = a + sh * (ah.taps - 1 - jh), fkw = b + sw * (aw.taps - 1 - jw);  // dY offset j <-> filter tap
@@ -953,6 +1007,7 @@ struct WgradParams {
   int kb_total;      // ceil(pixels / PB)
   int kb_per_split;
   int OW, OH, SW, SH, PW, PH, KW;
+  int dy_blocks;     // dY through one copy per stage (Cout % 32 == 0)
   float* partial;    // [splits][Kw][Cout]
 };
 
@@ -1028,8 +1083,12 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             if (q < valid) tma_load_im2col_4d(a_dst + q * C::kChunk, &mapX, full, q_c[q], pw_, ph_, pn_, (uint16_t)q_kw[q], (uint16_t)q_kh[q]);
+          if (p.dy_blocks) {
+            tma_load_3d(b_dst, &mapDY, full, 0, m, n0 / 32);
+          } else {
 #pragma unroll
-          for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * C::kChunk, &mapDY, full, n0 + 32 * j, m);
+            for (int j = 0; j < BN / 32; ++j) tma_load_2d(b_dst + j * C::kChunk, &mapDY, full, n0 + 32 * j, m);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           ow += PB;
           while (ow >= p.OW) {
@@ -1214,7 +1273,8 @@ WgradPlan wgrad_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int s
 
 }  // namespace
 
-// Which kernel family each of forward / data gradient / weight gradient would take for a shape
+// Which kernel family each of forward / data gradient / weight gradient can take for a shape: row-staged wherever
+// its layout fits (the launch then takes that or im2col, whichever is priced lower: row_conv_pays, wgrad_rows_pay)
 // (pointers assumed 16-byte aligned), and, for the row-staged kernels, how their shared and tensor
 // memory is laid out against the furthest byte their copies write and their descriptors read.
 // Host code only: callable without a device (the SM count then defaults to 148).
@@ -1296,7 +1356,7 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
                             const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   const WgradRowsPlan rq = wgrad_rows_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
-  if (rq.ok) {
+  if (wgrad_rows_pay(rq, cin, cout)) {
     MTB_REQUIRE(workspace && workspace_bytes >= (long long)rq.splits * kh * kw * cin * cout * 4, "conv2d_wgrad: workspace too small");
     return run_wgrad_rows(rq, n, cin, h, w, kh, kw, ph, pw, cout, x, dy, dw, (float*)workspace, (cudaStream_t)stream);
   }
@@ -1305,9 +1365,10 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   CUtensorMap mapX, mapDY;
   int rc = tc::encode_im2col_4d(&mapX, x, n, h, w, cin, -pw, -ph, pw - (kw - 1), ph - (kh - 1), sw, sh, 32, q.pb, true);
   if (rc) return rc;
-  rc = tc::encode_tiled_2d(&mapDY, dy, q.pixels, cout, cout, 32, q.pb, true);
-  if (rc) return rc;
   WgradParams p{};
+  p.dy_blocks = cout % 32 == 0;
+  rc = p.dy_blocks ? tc::encode_blocks_3d(&mapDY, dy, q.pixels, cout, cout, q.pb, q.bn / 32) : tc::encode_tiled_2d(&mapDY, dy, q.pixels, cout, cout, 32, q.pb, true);
+  if (rc) return rc;
   p.Kw = (int)q.Kw; p.Cout = cout; p.chunks = (int)(q.Kw / 32); p.cchunks = cin / 32;
   p.m_tiles = q.m_tiles; p.n_tiles = q.n_tiles; p.splits = q.splits; p.kb_total = q.kb_total; p.kb_per_split = q.kb_per_split;
   p.OW = ow; p.OH = oh; p.SW = sw; p.SH = sh; p.PW = pw; p.PH = ph; p.KW = kw;
