@@ -158,6 +158,16 @@ int mtb_batch_norm2d_add_relu_backward_f32(int n, int c, int h, int w, const flo
                                            const float* residual, const float* gamma, const float* beta, double eps, float* dx,
                                            float* dresidual, float* dgamma, float* dbeta, void* workspace, long long workspace_bytes,
                                            void* stream);
+/* The same pair with the ReLU's mask handed over (n*h*w*c/4 bytes, bit i of a byte: channel i of its four was blocked), so that
+ * backward does not read the added tensor.  c % 4 == 0, tensors 16-byte aligned.  No counterpart in the reference. */
+int mtb_batch_norm2d_add_relu_forward_masked_f32(int n, int c, int h, int w, const float* x, const float* residual, const float* gamma,
+                                                 const float* beta, double eps, int training, double momentum, float* running_mean,
+                                                 float* running_var, float* y, float* mean, float* var, unsigned char* mask, const float* stats,
+                                                 int stats_rows, void* workspace, long long workspace_bytes, void* stream);
+int mtb_batch_norm2d_add_relu_backward_masked_f32(int n, int c, int h, int w, const float* dy, const float* mean, const float* var,
+                                                  const float* x, const unsigned char* mask, const float* gamma, const float* beta, double eps,
+                                                  float* dx, float* dresidual, float* dgamma, float* dbeta, void* workspace,
+                                                  long long workspace_bytes, void* stream);
 /* relu != 0 in forward fuses max(0, .) into the normalise pass; the same flag in backward masks dy where
  * gamma*xhat + beta < 0 (recomputed, so the ReLU output need not be kept).  beta may be NULL (= 0). */
 int mtb_batch_norm2d_backward_f32(int n, int c, int h, int w, const float* dy, const float* mean, const float* var, const float* x,

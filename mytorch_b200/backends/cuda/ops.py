@@ -441,9 +441,14 @@ def cuda_batch_norm2d_add_relu(x, residual, weight, bias, eps, training, momentu
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
     use_batch_stats = bool(training) or running_mean is None or running_var is None
     pre = getattr(x, "_bn_partials", None) if use_batch_stats else None
-    env.lib.batch_norm2d_add_relu_forward_f32(n, c, h, w, _ptr(x), _ptr(residual), _ptr(weight), _ptr(bias), float(eps), int(use_batch_stats),
-                                              float(momentum), _ptr(running_mean), _ptr(running_var), _ptr(y), _ptr(mean), _ptr(var),
-                                              pre[0].ptr if pre else None, pre[1] if pre else 0, ws, ws_bytes, env.stream())
+    head = (n, c, h, w, _ptr(x), _ptr(residual), _ptr(weight), _ptr(bias), float(eps), int(use_batch_stats), float(momentum), _ptr(running_mean),
+            _ptr(running_var), _ptr(y), _ptr(mean), _ptr(var))
+    tail = (pre[0] if pre else None, pre[1] if pre else 0, ws, ws_bytes, env.stream())
+    if c % 4 == 0 and not _tracker.no_grad:  # the ReLU's mask goes to backward with the statistics
+        mean._relu_mask = CudaMemory(x.device.index, n * c * h * w // 4)
+        env.lib.batch_norm2d_add_relu_forward_masked_f32(*head, mean._relu_mask, *tail)
+    else:
+        env.lib.batch_norm2d_add_relu_forward_f32(*head, *tail)
     return y, mean, var
 
 
@@ -457,8 +462,12 @@ def cuda_batch_norm2d_add_relu_backward(output_grad, mean, var, x, residual, wei
     dg = _grad_buffer(weight) if affine else None
     db = _grad_buffer(bias) if affine else None
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
-    env.lib.batch_norm2d_add_relu_backward_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), _ptr(residual), _ptr(weight), _ptr(bias),
-                                               float(eps), _ptr(dx), _ptr(dres), _ptr(dg), _ptr(db), ws, ws_bytes, env.stream())
+    tail = (_ptr(weight), _ptr(bias), float(eps), _ptr(dx), _ptr(dres), _ptr(dg), _ptr(db), ws, ws_bytes, env.stream())
+    mask = getattr(mean, "_relu_mask", None)
+    if mask is not None:
+        env.lib.batch_norm2d_add_relu_backward_masked_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), mask, *tail)
+    else:
+        env.lib.batch_norm2d_add_relu_backward_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), _ptr(residual), *tail)
     return [dx, dres, dg, db]
 
 

@@ -163,7 +163,8 @@ struct Entry<ID, K, R(A...)> {
   X(relu_backward_f32, LAUNCH) X(add_f32, LAUNCH) X(mul_f32, LAUNCH) X(add_bias_rows_f32, LAUNCH) X(binary_strided_f32, LAUNCH) \
   X(resize_channels_f32, LAUNCH) X(pack_patches_f32, LAUNCH) X(nchw_to_nhwc_f32, LAUNCH) X(nhwc_to_nchw_f32, LAUNCH) X(cast, LAUNCH) \
   X(batch_norm2d_workspace_bytes, VALUE) X(batch_norm2d_forward_f32, LAUNCH) X(batch_norm2d_backward_f32, LAUNCH) \
-  X(batch_norm2d_add_relu_forward_f32, LAUNCH) X(batch_norm2d_add_relu_backward_f32, LAUNCH) X(add_relu_f32, LAUNCH) \
+  X(batch_norm2d_add_relu_forward_f32, LAUNCH) X(batch_norm2d_add_relu_forward_masked_f32, LAUNCH) \
+  X(batch_norm2d_add_relu_backward_masked_f32, LAUNCH) X(batch_norm2d_add_relu_backward_f32, LAUNCH) X(add_relu_f32, LAUNCH) \
   X(add_relu_backward_f32, LAUNCH) X(colsum_workspace_bytes, VALUE) X(colsum_f32, LAUNCH) X(colsum_noalloc_f32, LAUNCH) \
   X(nhwc_spatial_sum_f32, LAUNCH) X(nhwc_spatial_bcast_f32, LAUNCH) X(sum_strided_f32, LAUNCH) X(max_strided_f32, LAUNCH) \
   X(max_backward_f32, LAUNCH) X(eq_strided, LAUNCH) X(max_pool2d_forward_f32, LAUNCH) X(max_pool2d_backward_f32, LAUNCH) \

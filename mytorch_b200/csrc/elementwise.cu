@@ -199,26 +199,30 @@ __global__ void __launch_bounds__(256) resize_channels_kernel(const float* __res
 struct PatchRuns {
   int N, C, H, W, KH, KW, SH, SW, PH, PW, OH, OW;
 };
-__global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restrict__ x, float4* __restrict__ out, PatchRuns d, unsigned total) {
+__global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restrict__ x, float4* __restrict__ out, PatchRuns d, unsigned pixels) {
+  // A thread always writes the same four entries of a pixel, so where they lie in the filter is worked out once; a CTA walks
+  // 32 neighbouring pixels at a time.
   const int run = d.KW * d.C, used = d.KH * run;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const unsigned pixel = i >> 3;
-    const int k0 = (int)(i & 7u) * 4;
+  const unsigned part = threadIdx.x & 7u;
+  int dh[4], dw[4], dc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = (int)part * 4 + q, kh = k / run, r = k - kh * run;
+    dh[q] = k < used ? kh - d.PH : -(1 << 28);  // far outside: reads as zero
+    dw[q] = r / d.C - d.PW;
+    dc[q] = r - r / d.C * d.C;
+  }
+  for (unsigned pixel = blockIdx.x * 32u + (threadIdx.x >> 3); pixel < pixels; pixel += gridDim.x * 32u) {
     const unsigned ow = pixel % (unsigned)d.OW, t = pixel / (unsigned)d.OW;
-    const int oh = (int)(t % (unsigned)d.OH), n = (int)(t / (unsigned)d.OH);
-    const int h0 = oh * d.SH - d.PH, w0 = (int)ow * d.SW - d.PW;
+    const int h0 = (int)(t % (unsigned)d.OH) * d.SH, w0 = (int)ow * d.SW;
+    const long long image = (long long)(t / (unsigned)d.OH) * d.H;
     float v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int k = k0 + q;
-      v[q] = 0.f;
-      if (k < used) {
-        const int kh = k / run, r = k - kh * run, kw = r / d.C;  // constant divisors per launch, small numbers
-        const int h = h0 + kh, w = w0 + kw;
-        if ((unsigned)h < (unsigned)d.H && (unsigned)w < (unsigned)d.W) v[q] = __ldg(x + (((long long)n * d.H + h) * d.W + w) * d.C + (r - kw * d.C));
-      }
+      const int h = h0 + dh[q], w = w0 + dw[q];
+      v[q] = (unsigned)h < (unsigned)d.H && (unsigned)w < (unsigned)d.W ? __ldg(x + ((image + h) * d.W + w) * d.C + dc[q]) : 0.f;
     }
-    out[i] = make_float4(v[0], v[1], v[2], v[3]);
+    out[(size_t)pixel * 8 + part] = make_float4(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -233,9 +237,9 @@ MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int
   MTB_REQUIRE((long long)kh * kw * c <= 32, "pack_patches: the filter has more than 32 entries");
   PatchRuns d{n, c, h, w, kh, kw, sh, sw, ph, pw, (h + 2 * ph - kh) / sh + 1, (w + 2 * pw - kw) / sw + 1};
   MTB_REQUIRE(d.OH > 0 && d.OW > 0 && mtb_aligned16(out), "pack_patches: empty or unaligned output");
-  const long long total = (long long)n * d.OH * d.OW * 8;
-  MTB_REQUIRE(total < (1LL << 32) - (1LL << 24), "pack_patches: too many pixels");
-  pack_patches_kernel<<<mtb_stream_grid(total, 256), 256, 0, (cudaStream_t)stream>>>(x, (float4*)out, d, (unsigned)total);
+  const long long pixels = (long long)n * d.OH * d.OW;
+  MTB_REQUIRE(pixels < (1LL << 31), "pack_patches: too many pixels");
+  pack_patches_kernel<<<mtb_stream_grid(pixels, 32), 256, 0, (cudaStream_t)stream>>>(x, (float4*)out, d, (unsigned)pixels);
   MTB_LAUNCH_CHECK("pack_patches_kernel");
   return MTB_OK;
 }

@@ -1,15 +1,17 @@
 // tcgen05 / TMEM / TMA kernels: TF32 GEMM with FP32 accumulation for Linear layers, and
 // implicit-GEMM convolution forward and (stride-1) data gradient over channels-last tensors.
 //
-// One persistent CTA per SM, 192 threads in three roles:
+// One persistent CTA per SM, 320 threads in three roles:
 //   warp 0     TMA producer: one lane fills a ring of shared-memory stages (A tile 128 x 32,
 //              B tile BN x 32 fp32, 128-byte swizzle).  The convolution's A operand is never
 //              materialised: an im2col-mode tensor map gathers 128 output pixels x 32 channels
 //              of one filter tap per load, with zero fill for the padding halo.
 //   warp 1     MMA issuer: one lane issues tcgen05.mma kind::tf32 (128 x BN x 8 per instruction),
 //              accumulating in TMEM; tcgen05.commit releases stages and publishes finished tiles.
-//   warps 2-5  epilogue: tcgen05.ld the accumulator (each warp owns a 32-lane TMEM quarter),
-//              add bias / apply ReLU, store rows to global memory.
+//   warps 2-9  epilogue: tcgen05.ld the accumulator (each warp owns a 32-lane TMEM quarter and half of the
+//              columns), add bias / apply ReLU, store rows to global memory.  A short reduction is bound by how many
+//              loads and stores these warps have in flight: eight instead of four take the 64 <- 256 channel data
+//              gradient with addition on 128 x 56x56 from 291 to 213 us.
 // Two TMEM accumulator buffers let the epilogue of tile i overlap the main loop of tile i+1.
 // All waits are bounded (tc_common.cuh); a kernel that gives up sets g_tc_status and exits.
 #include "tc_common.cuh"
@@ -173,8 +175,10 @@ struct Cfg {
 // with running statistics (then optionally add a tensor).
 enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3 };
 
+constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
+
 template <int BN, int AMODE, int BMODE, int EPI>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kGemmThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p) {
   using C = Cfg<BN>;
   constexpr int STAGES = C::kStages;
@@ -196,7 +200,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
-      mbar_init(smem_u32(&bar_tempty[b]), 4);  // one arrival per epilogue warp
+      mbar_init(smem_u32(&bar_tempty[b]), kEpilogueWarps);  // one arrival per epilogue warp
     }
     abort_flag = 0;
     fence_barrier_init();
@@ -335,15 +339,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       __syncwarp();
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quarter = warp & 3;
+    constexpr int COLS = BN / 2;                            // columns of the tile this warp handles, from c_first on
+    const int c_first = warp < 6 ? 0 : COLS;
     int t = 0;
     const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0);
     const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 31u) == 0);  // 32-byte stores
     // statistics variant: narrow tiles keep per-lane sums (cheap per tile), wide tiles merge per tile
     constexpr bool LANE_SUMS = STATS && BN == 64;
-    WarpColStats<(STATS && !LANE_SUMS) ? BN / 32 : 1> stats;
-    LaneColSums<LANE_SUMS ? BN / 32 : 1> sums;
+    WarpColStats<(STATS && !LANE_SUMS) ? COLS / 32 : 1> stats;
+    LaneColSums<LANE_SUMS ? COLS / 32 : 1> sums;
     if constexpr (LANE_SUMS) sums.reset(); else stats.reset();
     for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
       const int tile = unit / S;
@@ -371,14 +377,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       const float* arow = ADD && (!BNORM || p.addend) ? p.addend + orow_index * p.ldo : nullptr;
       const bool valid = row < p.M;
       const float cnt = STATS ? (float)__popc(__ballot_sync(0xffffffffu, valid)) : 0.f;
-      // r: this lane's row of the finished accumulator, columns c0 .. c0+31 of the tile; add: the same columns of the
+      // r: this lane's row of the finished accumulator, columns c0 .. c0+31 of the warp's half; add: the same columns of the
       // addend, fetched one chunk ahead (a memory round trip per chunk in front of the stores would make the epilogue
       // of a short reduction several times longer than its main loop)
       const bool adds = ADD && arow && valid && vec_ok && n0 + BN <= p.N;
       auto fetch_addend = [&](int c0, float4 (&add)[8]) {
         if (adds) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) add[j] = *reinterpret_cast<const float4*>(arow + n0 + c0 + 4 * j);
+          for (int j = 0; j < 8; ++j) add[j] = *reinterpret_cast<const float4*>(arow + n0 + c_first + c0 + 4 * j);
         }
       };
       float4 add[8];
@@ -387,7 +393,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         if (!wait_for_accumulator()) break;
       }
       auto finish = [&](int c0, const uint32_t (&r)[32]) {
-        const int col0 = n0 + c0;
+        const int col0 = n0 + c_first + c0;
         if constexpr (STATS) {
           // the forward convolution that feeds a BatchNorm layer: full column tiles (N % 32 == 0, checked on
           // the host), vector stores, and the per-channel statistics of what is stored
@@ -421,9 +427,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
                   if constexpr (BNORM) {
-                    const float4 mu = *reinterpret_cast<const float4*>(&bn_columns.mean[c0 + jj]);
-                    const float4 g = *reinterpret_cast<const float4*>(&bn_columns.scale[c0 + jj]);
-                    const float4 b = *reinterpret_cast<const float4*>(&bn_columns.beta[c0 + jj]);
+                    const float4 mu = *reinterpret_cast<const float4*>(&bn_columns.mean[c_first + c0 + jj]);
+                    const float4 g = *reinterpret_cast<const float4*>(&bn_columns.scale[c_first + c0 + jj]);
+                    const float4 b = *reinterpret_cast<const float4*>(&bn_columns.beta[c_first + c0 + jj]);
                     v[h].x = (v[h].x - mu.x) * g.x + b.x; v[h].y = (v[h].y - mu.y) * g.y + b.y;
                     v[h].z = (v[h].z - mu.z) * g.z + b.z; v[h].w = (v[h].w - mu.w) * g.w + b.w;
                   }
@@ -441,7 +447,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (col0 + j < p.N) {
                   float v = __uint_as_float(r[j]);
                   if (p.bias) v += p.bias[col0 + j];
-                  if constexpr (BNORM) v = (v - bn_columns.mean[c0 + j]) * bn_columns.scale[c0 + j] + bn_columns.beta[c0 + j];
+                  if constexpr (BNORM) v = (v - bn_columns.mean[c_first + c0 + j]) * bn_columns.scale[c_first + c0 + j] + bn_columns.beta[c_first + c0 + j];
                   if (ADD && arow) v += arow[col0 + j];
                   if (p.relu) v = fmaxf(v, 0.f);
                   orow[col0 + j] = v;
@@ -463,20 +469,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       if (S == 1) {
         if constexpr (STATS) {
 #pragma unroll
-          for (int c0 = 0; c0 < BN; c0 += 32) {
+          for (int c0 = 0; c0 < COLS; c0 += 32) {
             uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), r);
+            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
             tmem_ld_wait();
             finish(c0, r);
           }
         } else {
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 32) {
+          for (int c0 = 0; c0 < COLS; c0 += 32) {
             uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), r);
+            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
             if constexpr (ADD) {
               float4 next[8];
-              if (c0 + 32 < BN) fetch_addend(c0 + 32, next);
+              if (c0 + 32 < COLS) fetch_addend(c0 + 32, next);
               tmem_ld_wait();
               finish(c0, r);
 #pragma unroll
@@ -492,28 +498,28 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         continue;
       }
       // Split reduction.  partial[unit][chunk][quarter][j][lane]: a warp stores 128 contiguous bytes per column.
-      constexpr int kChunks = BN / 32;
-      float* part = p.partial + (((long long)unit * kChunks) * 4 + quarter) * 1024 + lane;
+      constexpr int kChunks = BN / 32, kMine = COLS / 32;
+      float* part = p.partial + (((long long)unit * kChunks + c_first / 32) * 4 + quarter) * 1024 + lane;
 #pragma unroll 1
-      for (int c = 0; c < kChunks; ++c) {
+      for (int c = 0; c < kMine; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c * 32), r);
+        tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c * 32), r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) part[c * 4096 + j * 32] = __uint_as_float(r[j]);
       }
       release_accumulator();
       __threadfence();
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
       if (threadIdx.x == 64) {
         const unsigned int ticket = atomicAdd(&g_gemm_tickets[tile], 1u);
         split_last = (ticket == (unsigned int)S - 1u);
         if (split_last) g_gemm_tickets[tile] = 0u;  // every unit of the tile has drawn: ready for the next launch
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
       if (!split_last) continue;
       __threadfence();
-      const float* first = p.partial + (((long long)tile * S * kChunks) * 4 + quarter) * 1024 + lane;
+      const float* first = p.partial + (((long long)tile * S * kChunks + c_first / 32) * 4 + quarter) * 1024 + lane;
       auto reduce_chunk = [&](int c, uint32_t (&r)[32]) {
         float acc[32];
 #pragma unroll
@@ -528,14 +534,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       };
       if constexpr (STATS) {
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
+        for (int c = 0; c < kMine; ++c) {
           uint32_t r[32];
           reduce_chunk(c, r);
           finish(c * 32, r);
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < kChunks; ++c) {
+        for (int c = 0; c < kMine; ++c) {
           uint32_t r[32];
           if constexpr (ADD) {
             if (c > 0) fetch_addend(c * 32, add);
@@ -549,14 +555,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         // which unit of a tile comes last differs from run to run, so the statistics of a split tile go to
         // a row chosen by the tile, not by the CTA: results stay bit-reproducible
         float* row = p.stats + ((long long)(tile / p.n_tiles) * 4 + quarter) * 3 * p.N;
-        if constexpr (LANE_SUMS) { sums.store(row, p.N, n0, p.N, p.bias, lane); sums.reset(); }
-        else { stats.store(row, p.N, n0, p.N, lane); stats.reset(); }
+        if constexpr (LANE_SUMS) { sums.store(row, p.N, n0 + c_first, p.N, p.bias, lane); sums.reset(); }
+        else { stats.store(row, p.N, n0 + c_first, p.N, lane); stats.reset(); }
       }
     }
     if (STATS && S == 1) {
       float* row = p.stats + ((long long)(blockIdx.x / p.n_tiles) * 4 + quarter) * 3 * p.N;
-      if constexpr (LANE_SUMS) sums.store(row, p.N, (blockIdx.x % p.n_tiles) * BN, p.N, p.bias, lane);
-      else if constexpr (STATS) stats.store(row, p.N, (blockIdx.x % p.n_tiles) * BN, p.N, lane);
+      if constexpr (LANE_SUMS) sums.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, p.bias, lane);
+      else if constexpr (STATS) stats.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, lane);
     }
   }
 
@@ -582,7 +588,7 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
   int tiles = p.m_tiles * p.n_tiles * p.splits;  // work units
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
   if ((EPI == EPI_STATS || EPI == EPI_BN) && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
-  kernel<<<grid, 192, C::kSmemBytes, st>>>(mapA, mapB, p);
+  kernel<<<grid, kGemmThreads, C::kSmemBytes, st>>>(mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
 }
@@ -1012,7 +1018,7 @@ struct WgradParams {
 };
 
 template <int BN, int PB>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kGemmThreads, 1)
 tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapDY, const WgradParams p) {
   using C = WCfg<BN, PB>;
   constexpr int STAGES = C::kStages;
@@ -1030,7 +1036,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
-      mbar_init(smem_u32(&bar_tempty[b]), 4);  // one arrival per epilogue warp
+      mbar_init(smem_u32(&bar_tempty[b]), kEpilogueWarps);  // one arrival per epilogue warp
     }
     abort_flag = 0;
     fence_barrier_init();
@@ -1138,7 +1144,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
       __syncwarp();
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, c_first = warp < 6 ? 0 : BN / 2;
     int t = 0;
     const bool wide_ok = (p.Cout % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.partial) & 31u) == 0);  // 32-byte stores
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++t) {
@@ -1156,7 +1162,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
       const int row = m_tile * 128 + quarter * 32 + lane;
       float* orow = p.partial + ((long long)split * p.Kw + row) * p.Cout;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = c_first; c0 < c_first + BN / 2; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), r);
         tmem_ld_wait();
@@ -1381,7 +1387,7 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
     static unsigned long long configured = 0;                                                                           \
     if (int rc_ = mtb_opt_in_smem((const void*)tc_wgrad_kernel<BN_, PB_>, (int)WCfg<BN_, PB_>::kSmemBytes, &configured)) \
       return rc_;                                                                                                       \
-    tc_wgrad_kernel<BN_, PB_><<<grid, 192, WCfg<BN_, PB_>::kSmemBytes, st>>>(mapX, mapDY, p);                           \
+    tc_wgrad_kernel<BN_, PB_><<<grid, kGemmThreads, WCfg<BN_, PB_>::kSmemBytes, st>>>(mapX, mapDY, p);                           \
   } while (0)
   if (q.bn == 64) MTB_LAUNCH_WGRAD(64, 64);
   else if (q.bn == 128) MTB_LAUNCH_WGRAD(128, 64);
