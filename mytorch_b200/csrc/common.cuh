@@ -47,6 +47,34 @@ int mtb_join_lanes(cudaStream_t main, int lanes);
   do { cudaError_t e__ = cudaGetLastError(); \
        if (e__ != cudaSuccess) return mtb_fail(MTB_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e__)); } while (0)
 
+// Programmatic dependent launch: the next kernel's CTAs are launched while this one runs, so the launch latency between the
+// two (about 1.5 us in a stream or graph) and the prologues (barriers, TMEM, tensor maps) are hidden.  Every kernel calls
+// mtb_launch_dependents() first (it says nothing about its results) and mtb_wait_prior() before it touches global memory: that
+// returns when everything before it in the stream has completed and is visible, so the order of the results is the stream's.
+// Launches without the attribute are unaffected by either call.  Measured on every kernel against on none: an 18-layer residual
+// network's step at batch 128 2400 -> 2123 us, its captured step at batch 64 1586 -> 1478 us, its inference at batch 100
+// 577 -> 540 us, a captured three-convolution step 219 -> 204 us.
+__device__ __forceinline__ void mtb_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void mtb_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// `early` false: an ordinary launch.
+template <class... P, class... A>
+static inline cudaError_t mtb_launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+#define MTB_LAUNCH(kernel, ...) MTB_CUDA(mtb_launch_after(true, kernel, __VA_ARGS__))
+
 static inline int mtb_div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Grid for a grid-stride bandwidth kernel: enough CTAs to fill the machine a few times over,

@@ -116,6 +116,8 @@ namespace {
 
 // out[i] = sum of the planes, in plane order; eight planes' loads in flight per thread.
 __global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict__ ws, float* __restrict__ out, long long n, int planes) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
 #pragma unroll 8
@@ -150,7 +152,7 @@ MTB_API int mtb_conv2d_wgrad_simt_f32(int n, int cin, int h, int w, int kh, int 
   else if (vb) rc = launch<DenseR, 1, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
   else rc = launch<DenseR, 1, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
   if (rc || c.slices == 1) return rc;
-  add_planes_kernel<<<mtb_stream_grid(total, 256), 256, 0, st>>>((const float*)workspace, dw, total, c.slices);
+  MTB_LAUNCH(add_planes_kernel, mtb_stream_grid(total, 256), 256, 0, st, (const float*)workspace, dw, total, c.slices);
   MTB_LAUNCH_CHECK("add_planes_kernel");
   return MTB_OK;
 }

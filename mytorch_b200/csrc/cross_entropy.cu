@@ -15,6 +15,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 __global__ void __launch_bounds__(128) ce_rows_kernel(const float* __restrict__ z, const long long* __restrict__ target, int B, int C,
                                                        float* __restrict__ row_loss, float* __restrict__ dz, const float* __restrict__ dy) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
   if (row >= B) return;
@@ -41,6 +43,7 @@ __global__ void __launch_bounds__(128) ce_rows_kernel(const float* __restrict__ 
 }
 
 __global__ void __launch_bounds__(256) ce_mean_kernel(const float* __restrict__ row_loss, int B, float* __restrict__ loss) {
+  mtb_wait_prior();
   __shared__ double sm[256];
   double s = 0;
   for (int i = threadIdx.x; i < B; i += 256) s += row_loss[i];
@@ -63,9 +66,9 @@ MTB_API int mtb_cross_entropy_forward_f32(int batch, int classes, const float* l
   MTB_REQUIRE(batch > 0 && classes > 0 && logits && target && loss && workspace, "cross_entropy_forward: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_cross_entropy_workspace_bytes(batch), "cross_entropy_forward: workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
-  ce_rows_kernel<<<mtb_div_up(batch, 4), 128, 0, st>>>(logits, target, batch, classes, (float*)workspace, nullptr, nullptr);
+  MTB_LAUNCH(ce_rows_kernel, mtb_div_up(batch, 4), 128, 0, st, logits, target, batch, classes, (float*)workspace, nullptr, nullptr);
   MTB_LAUNCH_CHECK("ce_rows_kernel");
-  ce_mean_kernel<<<1, 256, 0, st>>>((const float*)workspace, batch, loss);
+  MTB_LAUNCH(ce_mean_kernel, dim3(1), dim3(256), 0, st, (const float*)workspace, batch, loss);
   MTB_LAUNCH_CHECK("ce_mean_kernel");
   return MTB_OK;
 }
@@ -74,7 +77,7 @@ MTB_API int mtb_cross_entropy_forward_f32(int batch, int classes, const float* l
 MTB_API int mtb_cross_entropy_backward_f32(int batch, int classes, const float* logits, const long long* target, const float* dy,
                                            float* dlogits, void* stream) {
   MTB_REQUIRE(batch > 0 && classes > 0 && logits && target && dy && dlogits, "cross_entropy_backward: bad arguments");
-  ce_rows_kernel<<<mtb_div_up(batch, 4), 128, 0, (cudaStream_t)stream>>>(logits, target, batch, classes, nullptr, dlogits, dy);
+  MTB_LAUNCH(ce_rows_kernel, mtb_div_up(batch, 4), 128, 0, (cudaStream_t)stream, logits, target, batch, classes, nullptr, dlogits, dy);
   MTB_LAUNCH_CHECK("ce_rows_kernel");
   return MTB_OK;
 }

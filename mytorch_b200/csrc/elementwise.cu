@@ -10,6 +10,8 @@ constexpr int kThreads = 256;
 
 template <class F>
 __global__ void __launch_bounds__(kThreads) map1_kernel(float* out, const float* a, long long n4, long long n, F f) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = i; v < n4; v += stride) {
@@ -23,6 +25,8 @@ __global__ void __launch_bounds__(kThreads) map1_kernel(float* out, const float*
 template <class F>
 __global__ void __launch_bounds__(kThreads) map2_kernel(float* out, const float* a, const float* b,
                                                          long long n4, long long n, F f) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = i; v < n4; v += stride) {
@@ -44,6 +48,8 @@ struct CopyF { __device__ float operator()(float x) const { return x; } };
 // g = (x + y < 0) ? 0 : dy — backward of max(0, x + y); the sum is recomputed from the two
 // forward inputs (bit-identical to the forward's), and a sum of exactly 0 passes the gradient.
 __global__ void __launch_bounds__(kThreads) add_relu_bwd_kernel(float* g, const float* dy, const float* x, const float* y, long long n4, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = i; v < n4; v += stride) {
@@ -63,7 +69,7 @@ int launch_map1(float* out, const float* a, long long n, F f, cudaStream_t s, co
   bool vec = mtb_aligned16(out) && mtb_aligned16(a);
   long long n4 = vec ? n / 4 : 0;
   int grid = mtb_stream_grid(vec ? (n4 > 0 ? n4 : 1) : n, kThreads);
-  map1_kernel<<<grid, kThreads, 0, s>>>(out, a, n4, n, f);
+  MTB_LAUNCH(map1_kernel<F>, grid, kThreads, 0, s, out, a, n4, n, f);
   MTB_LAUNCH_CHECK(name);
   return MTB_OK;
 }
@@ -74,7 +80,7 @@ int launch_map2(float* out, const float* a, const float* b, long long n, F f, cu
   bool vec = mtb_aligned16(out) && mtb_aligned16(a) && mtb_aligned16(b);
   long long n4 = vec ? n / 4 : 0;
   int grid = mtb_stream_grid(vec ? (n4 > 0 ? n4 : 1) : n, kThreads);
-  map2_kernel<<<grid, kThreads, 0, s>>>(out, a, b, n4, n, f);
+  MTB_LAUNCH(map2_kernel<F>, grid, kThreads, 0, s, out, a, b, n4, n, f);
   MTB_LAUNCH_CHECK(name);
   return MTB_OK;
 }
@@ -82,12 +88,16 @@ int launch_map2(float* out, const float* a, const float* b, long long n, F f, cu
 // y[r, c] = x[r, c] + alpha * bias[c]; cols % 4 == 0 fast path.
 __global__ void __launch_bounds__(kThreads) bias_rows_kernel(float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ bias,
                                                               long long n, int cols, float alpha) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = i; t < n; t += stride) y[t] = x[t] + alpha * bias[t % cols];
 }
 
 __global__ void __launch_bounds__(kThreads) fill_kernel(float* out, long long n4, long long n, float v) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   float4 v4 = make_float4(v, v, v, v);
@@ -106,6 +116,8 @@ struct Strides6 {
 template <int OP>
 __global__ void __launch_bounds__(kThreads) strided_binary_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ b,
                                                                    long long n, Strides6 s, float alpha) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = i; t < n; t += stride) {
@@ -134,6 +146,8 @@ __global__ void __launch_bounds__(kThreads) strided_binary_kernel(float* __restr
 
 // NCHW -> NHWC through a shared-memory tile transpose of the [C, HW] plane of each image.
 __global__ void __launch_bounds__(256) transpose_planes_kernel(float* __restrict__ dst, const float* __restrict__ src, int rows, int cols) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   // src: [batch][rows][cols] -> dst: [batch][cols][rows]
   __shared__ float tile[32][33];
   const float* s = src + (long long)blockIdx.z * rows * cols;
@@ -151,22 +165,30 @@ __global__ void __launch_bounds__(256) transpose_planes_kernel(float* __restrict
 }
 
 __global__ void cast_i32_i64_kernel(long long* out, const int* in, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) out[i] = in[i];
 }
 __global__ void cast_i64_f32_kernel(float* out, const long long* in, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) out[i] = (float)in[i];
 }
 __global__ void cast_f32_i64_kernel(long long* out, const float* in, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) out[i] = (long long)in[i];
 }
 
 __global__ void cast_i8_f32_kernel(float* out, const signed char* in, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) out[i] = (float)in[i];
@@ -177,7 +199,7 @@ int transpose_planes(float* dst, const float* src, int batch, int rows, int cols
   MTB_REQUIRE(batch <= 65535 * 1, "layout change: batch %d exceeds grid.z", batch);
   dim3 grid(mtb_div_up(cols, 32), mtb_div_up(rows, 32), batch), block(32, 8);
   MTB_REQUIRE(grid.y <= 65535, "layout change: too many rows");
-  transpose_planes_kernel<<<grid, block, 0, s>>>(dst, src, rows, cols);
+  MTB_LAUNCH(transpose_planes_kernel, grid, block, 0, s, dst, src, rows, cols);
   MTB_LAUNCH_CHECK("transpose_planes_kernel");
   return MTB_OK;
 }
@@ -185,6 +207,8 @@ int transpose_planes(float* dst, const float* src, int batch, int rows, int cols
 // dst[r][c] = c < c_src ? src[r][c] : 0 for c < c_dst: widen a [rows, c_src] matrix with zero
 // columns (c_dst > c_src) or keep its first c_dst columns (c_dst < c_src), in one pass.
 __global__ void __launch_bounds__(256) resize_channels_kernel(const float* __restrict__ src, float* __restrict__ dst, long long rows, int c_src, int c_dst) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const long long total = rows * c_dst;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / c_dst;
@@ -200,6 +224,8 @@ struct PatchRuns {
   int N, C, H, W, KH, KW, SH, SW, PH, PW, OH, OW;
 };
 __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restrict__ x, float4* __restrict__ out, PatchRuns d, unsigned pixels) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   // A thread always writes the same four entries of a pixel, so where they lie in the filter is worked out once; a CTA walks
   // 32 neighbouring pixels at a time.
   const int run = d.KW * d.C, used = d.KH * run;
@@ -239,7 +265,7 @@ MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int
   MTB_REQUIRE(d.OH > 0 && d.OW > 0 && mtb_aligned16(out), "pack_patches: empty or unaligned output");
   const long long pixels = (long long)n * d.OH * d.OW;
   MTB_REQUIRE(pixels < (1LL << 31), "pack_patches: too many pixels");
-  pack_patches_kernel<<<mtb_stream_grid(pixels, 32), 256, 0, (cudaStream_t)stream>>>(x, (float4*)out, d, (unsigned)pixels);
+  MTB_LAUNCH(pack_patches_kernel, mtb_stream_grid(pixels, 32), 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
   MTB_LAUNCH_CHECK("pack_patches_kernel");
   return MTB_OK;
 }
@@ -249,7 +275,7 @@ MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int
 // tensor-core convolution and cuts the weight gradient back; no counterpart in the reference.
 MTB_API int mtb_resize_channels_f32(const float* src, float* dst, long long rows, int c_src, int c_dst, void* stream) {
   MTB_REQUIRE(src && dst && rows > 0 && c_src > 0 && c_dst > 0, "resize_channels: bad arguments");
-  resize_channels_kernel<<<mtb_stream_grid(rows * c_dst, kThreads), kThreads, 0, (cudaStream_t)stream>>>(src, dst, rows, c_src, c_dst);
+  MTB_LAUNCH(resize_channels_kernel, mtb_stream_grid(rows * c_dst, kThreads), kThreads, 0, (cudaStream_t)stream, src, dst, rows, c_src, c_dst);
   MTB_LAUNCH_CHECK("resize_channels_kernel");
   return MTB_OK;
 }
@@ -258,7 +284,7 @@ MTB_API int mtb_fill_f32(float* x, long long n, float value, void* stream) {
   MTB_REQUIRE(n >= 0 && (x || n == 0), "fill: bad arguments");
   if (n == 0) return MTB_OK;
   long long n4 = mtb_aligned16(x) ? n / 4 : 0;
-  fill_kernel<<<mtb_stream_grid(n4 > 0 ? n4 : n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(x, n4, n, value);
+  MTB_LAUNCH(fill_kernel, mtb_stream_grid(n4 > 0 ? n4 : n, kThreads), kThreads, 0, (cudaStream_t)stream, x, n4, n, value);
   MTB_LAUNCH_CHECK("fill_kernel");
   return MTB_OK;
 }
@@ -301,7 +327,7 @@ MTB_API int mtb_add_relu_backward_f32(const float* dy, const float* x, const flo
   if (n == 0) return MTB_OK;
   bool vec = mtb_aligned16(dy) && mtb_aligned16(x) && mtb_aligned16(y) && mtb_aligned16(g);
   long long n4 = vec ? n / 4 : 0;
-  add_relu_bwd_kernel<<<mtb_stream_grid(vec ? (n4 > 0 ? n4 : 1) : n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(g, dy, x, y, n4, n);
+  MTB_LAUNCH(add_relu_bwd_kernel, mtb_stream_grid(vec ? (n4 > 0 ? n4 : 1) : n, kThreads), kThreads, 0, (cudaStream_t)stream, g, dy, x, y, n4, n);
   MTB_LAUNCH_CHECK("add_relu_bwd_kernel");
   return MTB_OK;
 }
@@ -316,7 +342,7 @@ MTB_API int mtb_add_bias_rows_f32(const float* x, const float* bias, float* y, l
   MTB_REQUIRE(rows >= 0 && cols > 0 && x && bias && y, "add_bias_rows: bad arguments");
   long long n = rows * cols;
   if (n == 0) return MTB_OK;
-  bias_rows_kernel<<<mtb_stream_grid(n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(y, x, bias, n, cols, alpha);
+  MTB_LAUNCH(bias_rows_kernel, mtb_stream_grid(n, kThreads), kThreads, 0, (cudaStream_t)stream, y, x, bias, n, cols, alpha);
   MTB_LAUNCH_CHECK("bias_rows_kernel");
   return MTB_OK;
 }
@@ -341,14 +367,14 @@ MTB_API int mtb_binary_strided_f32(int op, int ndim, const long long* shape, con
   int grid = mtb_stream_grid(n, kThreads);
   cudaStream_t st = (cudaStream_t)stream;
   switch (op) {
-    case 0: strided_binary_kernel<0><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 1: strided_binary_kernel<1><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 2: strided_binary_kernel<2><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 3: strided_binary_kernel<3><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 4: strided_binary_kernel<4><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 6: strided_binary_kernel<6><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    case 7: strided_binary_kernel<7><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
-    default: strided_binary_kernel<5><<<grid, kThreads, 0, st>>>(z, x, y, n, s, alpha); break;
+    case 0: MTB_LAUNCH(strided_binary_kernel<0>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 1: MTB_LAUNCH(strided_binary_kernel<1>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 2: MTB_LAUNCH(strided_binary_kernel<2>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 3: MTB_LAUNCH(strided_binary_kernel<3>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 4: MTB_LAUNCH(strided_binary_kernel<4>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 6: MTB_LAUNCH(strided_binary_kernel<6>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    case 7: MTB_LAUNCH(strided_binary_kernel<7>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
+    default: MTB_LAUNCH(strided_binary_kernel<5>, grid, kThreads, 0, st, z, x, y, n, s, alpha); break;
   }
   MTB_LAUNCH_CHECK("strided_binary_kernel");
   return MTB_OK;
@@ -371,10 +397,10 @@ MTB_API int mtb_cast(int kind, const void* src, void* dst, long long n, void* st
   if (n == 0) return MTB_OK;
   int grid = mtb_stream_grid(n, kThreads);
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == 0) cast_i32_i64_kernel<<<grid, kThreads, 0, st>>>((long long*)dst, (const int*)src, n);
-  else if (kind == 1) cast_i64_f32_kernel<<<grid, kThreads, 0, st>>>((float*)dst, (const long long*)src, n);
-  else if (kind == 2) cast_f32_i64_kernel<<<grid, kThreads, 0, st>>>((long long*)dst, (const float*)src, n);
-  else if (kind == 3) cast_i8_f32_kernel<<<grid, kThreads, 0, st>>>((float*)dst, (const signed char*)src, n);
+  if (kind == 0) MTB_LAUNCH(cast_i32_i64_kernel, grid, kThreads, 0, st, (long long*)dst, (const int*)src, n);
+  else if (kind == 1) MTB_LAUNCH(cast_i64_f32_kernel, grid, kThreads, 0, st, (float*)dst, (const long long*)src, n);
+  else if (kind == 2) MTB_LAUNCH(cast_f32_i64_kernel, grid, kThreads, 0, st, (long long*)dst, (const float*)src, n);
+  else if (kind == 3) MTB_LAUNCH(cast_i8_f32_kernel, grid, kThreads, 0, st, (float*)dst, (const signed char*)src, n);
   else return mtb_fail(MTB_ERR_UNSUPPORTED, "cast kind %d", kind);
   MTB_LAUNCH_CHECK("cast kernel");
   return MTB_OK;

@@ -23,6 +23,8 @@ int dense(int m, int n, int k, const float* a, int trans_a, const float* b, int 
 // of the FMAs, and rows are spread over CTAs: K = 512, 10 x 512: 32 -> 7 us.
 __global__ void __launch_bounds__(256) gemm_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
                                                              int M, int N, int K) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   constexpr int R = 4, AHEAD = 16;
   __shared__ float part[8][R][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -65,7 +67,7 @@ MTB_API int mtb_gemm_simt_f32(int m, int n, int k, const float* a, int trans_a, 
                               float* c, void* stream) {
   MTB_REQUIRE(a && b && c && m > 0 && n > 0 && k > 0, "gemm: bad arguments");
   if (trans_a && !trans_b && m <= 16 && !bias && !relu) {
-    gemm_few_rows_kernel<<<dim3(mtb_div_up(n, 32), mtb_div_up(m, 4)), 256, 0, (cudaStream_t)stream>>>(a, b, c, m, n, k);
+    MTB_LAUNCH(gemm_few_rows_kernel, dim3(mtb_div_up(n, 32), mtb_div_up(m, 4)), 256, 0, (cudaStream_t)stream, a, b, c, m, n, k);
     MTB_LAUNCH_CHECK("gemm_few_rows_kernel");
     return MTB_OK;
   }

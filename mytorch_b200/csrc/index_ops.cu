@@ -13,6 +13,8 @@ struct MaxDims {
 // One CTA per output element.  Ties go to the lowest index (numpy.argmax).
 __global__ void __launch_bounds__(256) max_strided_kernel(const float* __restrict__ x, float* __restrict__ y, long long* __restrict__ idx, MaxDims d,
                                                           long long red_len, long long red_stride) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long o = blockIdx.x, base = 0;
   for (int k = d.nk - 1; k >= 0; --k) {
     base += (o % d.kshape[k]) * d.kstride[k];
@@ -49,6 +51,8 @@ __global__ void __launch_bounds__(256) max_strided_kernel(const float* __restric
 // dx (zero-filled beforehand) receives dy at the recorded index of every output element.
 __global__ void max_scatter_kernel(const float* __restrict__ dy, const long long* __restrict__ idx, float* __restrict__ dx, MaxDims d, long long outs,
                                    long long red_stride) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < outs; o += (long long)gridDim.x * blockDim.x) {
     long long r = o, base = 0;
     for (int k = d.nk - 1; k >= 0; --k) {
@@ -66,6 +70,8 @@ struct EqDims {
 
 template <class T>
 __global__ void eq_strided_kernel(const T* __restrict__ x, const T* __restrict__ y, signed char* __restrict__ out, EqDims d, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     long long r = t, oa = 0, ob = 0;
     for (int k = d.nd - 1; k >= 0; --k) {
@@ -97,7 +103,7 @@ MTB_API int mtb_max_strided_f32(const float* x, float* y, long long* idx, int nk
   MaxDims d;
   long long outs;
   if (int rc = fill_dims(d, nkept, kept_shape, kept_strides, &outs)) return rc;
-  max_strided_kernel<<<(unsigned)outs, 256, 0, (cudaStream_t)stream>>>(x, y, idx, d, red_len, red_stride);
+  MTB_LAUNCH(max_strided_kernel, (unsigned)outs, 256, 0, (cudaStream_t)stream, x, y, idx, d, red_len, red_stride);
   MTB_LAUNCH_CHECK("max_strided_kernel");
   return MTB_OK;
 }
@@ -112,7 +118,7 @@ MTB_API int mtb_max_backward_f32(const float* dy, const long long* idx, float* d
   if (int rc = fill_dims(d, nkept, kept_shape, kept_strides, &outs)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   MTB_CUDA(cudaMemsetAsync(dx, 0, (size_t)dx_elems * 4, st));
-  max_scatter_kernel<<<mtb_stream_grid(outs, 256), 256, 0, st>>>(dy, idx, dx, d, outs, red_stride);
+  MTB_LAUNCH(max_scatter_kernel, mtb_stream_grid(outs, 256), 256, 0, st, dy, idx, dx, d, outs, red_stride);
   MTB_LAUNCH_CHECK("max_scatter_kernel");
   return MTB_OK;
 }
@@ -127,8 +133,8 @@ MTB_API int mtb_eq_strided(int kind, int ndim, const long long* shape, const lon
   for (int i = 0; i < ndim; ++i) { d.shape[i] = shape[i]; d.a[i] = x_strides[i]; d.b[i] = y_strides[i]; n *= shape[i]; }
   if (n == 0) return MTB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == 0) eq_strided_kernel<float><<<mtb_stream_grid(n, 256), 256, 0, st>>>((const float*)x, (const float*)y, out, d, n);
-  else eq_strided_kernel<long long><<<mtb_stream_grid(n, 256), 256, 0, st>>>((const long long*)x, (const long long*)y, out, d, n);
+  if (kind == 0) MTB_LAUNCH(eq_strided_kernel<float>, mtb_stream_grid(n, 256), 256, 0, st, (const float*)x, (const float*)y, out, d, n);
+  else MTB_LAUNCH(eq_strided_kernel<long long>, mtb_stream_grid(n, 256), 256, 0, st, (const long long*)x, (const long long*)y, out, d, n);
   MTB_LAUNCH_CHECK("eq_strided_kernel");
   return MTB_OK;
 }

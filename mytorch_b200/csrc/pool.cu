@@ -17,6 +17,8 @@ struct PoolDims {
 template <int V, typename IdxT>
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, unsigned short* __restrict__ mask,
                                                            PoolDims d, long long total_ll) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const IdxT cv = (IdxT)(d.C / V), total = (IdxT)total_ll;
   IdxT i = (IdxT)blockIdx.x * blockDim.x + threadIdx.x;
   const IdxT stride = (IdxT)gridDim.x * blockDim.x;
@@ -76,6 +78,8 @@ __device__ __forceinline__ void pool2x2_one(float a, float b, float c, float e, 
 
 __global__ void __launch_bounds__(256) maxpool2x2_fwd_kernel(const float4* __restrict__ x, float4* __restrict__ y, uint2* __restrict__ mask,
                                                               unsigned C4, unsigned OW, unsigned OH, unsigned total) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const unsigned W_C4 = 2u * OW * C4;  // one input row, in float4 units
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 2u * stride) {
@@ -132,6 +136,8 @@ struct PoolDiv {
 template <int KH, int KW, int SH, int SW>
 __global__ void __launch_bounds__(256) maxpool_fwd_vec_kernel(const float4* __restrict__ x, float4* __restrict__ y, uint2* __restrict__ mask, PoolDims d,
                                                                PoolDiv cv, PoolDiv ow_, PoolDiv oh_, unsigned total) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     unsigned cg, ow, oh;
     const unsigned n = oh_.divmod(ow_.divmod(cv.divmod(i, cg), ow), oh);
@@ -166,6 +172,8 @@ __global__ void __launch_bounds__(256) maxpool_fwd_vec_kernel(const float4* __re
 template <int KH, int KW, int SH, int SW>
 __global__ void __launch_bounds__(256) maxpool_bwd_vec_kernel(const float4* __restrict__ dy, const uint2* __restrict__ mask, float4* __restrict__ dx, PoolDims d,
                                                                PoolDiv cv, PoolDiv w_, PoolDiv h_, unsigned total) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   constexpr int NH = (KH + SH - 1) / SH, NW = (KW + SW - 1) / SW;  // windows that can cover one input element
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     unsigned cg, w, h;
@@ -205,6 +213,8 @@ template <int V, int MODE>
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const float* __restrict__ dy, const unsigned short* __restrict__ mask,
                                                            const float* __restrict__ out, const float* __restrict__ x, float* __restrict__ dx,
                                                            PoolDims d, long long total) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const int cv = d.C / V;
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -252,6 +262,8 @@ __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const float* __restric
 // writes the KH*KW input gradients of its window, so nothing is read twice.
 __global__ void __launch_bounds__(256) maxpool_bwd_window_kernel(const float* __restrict__ dy, const unsigned short* __restrict__ mask,
                                                                   float* __restrict__ dx, PoolDims d, unsigned total) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const unsigned cv = d.C / 4;
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned stride = gridDim.x * blockDim.x;
@@ -274,6 +286,8 @@ __global__ void __launch_bounds__(256) maxpool_bwd_window_kernel(const float* __
 }
 
 __global__ void mask_to_argmax_kernel(const unsigned short* __restrict__ mask, unsigned char* __restrict__ argmax, long long n) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) argmax[i] = (unsigned char)(__ffs((int)mask[i]) - 1);
@@ -305,22 +319,24 @@ MTB_API int mtb_max_pool2d_forward_f32(int n, int c, int h, int w, int kh, int k
   const bool tiles2x2 = kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && h % 2 == 0 && w % 2 == 0;
   if (vec && tiles2x2 && (long long)n * h * w * (c / 4) < (1LL << 32) - (1LL << 27) && !getenv("MTB_POOL_GENERIC")) {
     const int g2 = mtb_stream_grid((total + 1) / 2, 256);
-    maxpool2x2_fwd_kernel<<<g2, 256, 0, st>>>((const float4*)x, (float4*)y, (uint2*)tiemask, (unsigned)(c / 4), (unsigned)d.OW, (unsigned)d.OH,
-                                              (unsigned)total);
+    MTB_LAUNCH(maxpool2x2_fwd_kernel, g2, 256, 0, st, (const float4*)x, (float4*)y, (uint2*)tiemask, (unsigned)(c / 4), (unsigned)d.OW,
+               (unsigned)d.OH, (unsigned)total);
     MTB_LAUNCH_CHECK("maxpool2x2_fwd_kernel");
     return MTB_OK;
   }
   if (vec && total < (1LL << 31) - (1LL << 26) && kh == 3 && kw == 3 && sh == sw && (sh == 1 || sh == 2) && (long long)n * h < (1LL << 31)) {
     const PoolDiv cv(c / 4), ow(d.OW), oh(d.OH);
-    if (sh == 2) maxpool_fwd_vec_kernel<3, 3, 2, 2><<<grid, 256, 0, st>>>((const float4*)x, (float4*)y, (uint2*)tiemask, d, cv, ow, oh, (unsigned)total);
-    else maxpool_fwd_vec_kernel<3, 3, 1, 1><<<grid, 256, 0, st>>>((const float4*)x, (float4*)y, (uint2*)tiemask, d, cv, ow, oh, (unsigned)total);
+    if (sh == 2) MTB_LAUNCH(maxpool_fwd_vec_kernel<3, 3, 2, 2>, grid, 256, 0, st, (const float4*)x, (float4*)y, (uint2*)tiemask, d, cv, ow, oh,
+                            (unsigned)total);
+    else MTB_LAUNCH(maxpool_fwd_vec_kernel<3, 3, 1, 1>, grid, 256, 0, st, (const float4*)x, (float4*)y, (uint2*)tiemask, d, cv, ow, oh,
+                    (unsigned)total);
     MTB_LAUNCH_CHECK("maxpool_fwd_vec_kernel");
     return MTB_OK;
   }
-  if (vec && small) maxpool_fwd_kernel<4, unsigned><<<grid, 256, 0, st>>>(x, y, tiemask, d, total);
-  else if (vec) maxpool_fwd_kernel<4, long long><<<grid, 256, 0, st>>>(x, y, tiemask, d, total);
-  else if (small) maxpool_fwd_kernel<1, unsigned><<<grid, 256, 0, st>>>(x, y, tiemask, d, total);
-  else maxpool_fwd_kernel<1, long long><<<grid, 256, 0, st>>>(x, y, tiemask, d, total);
+  if (vec && small) MTB_LAUNCH(maxpool_fwd_kernel<4, unsigned>, grid, 256, 0, st, x, y, tiemask, d, total);
+  else if (vec) MTB_LAUNCH(maxpool_fwd_kernel<4, long long>, grid, 256, 0, st, x, y, tiemask, d, total);
+  else if (small) MTB_LAUNCH(maxpool_fwd_kernel<1, unsigned>, grid, 256, 0, st, x, y, tiemask, d, total);
+  else MTB_LAUNCH(maxpool_fwd_kernel<1, long long>, grid, 256, 0, st, x, y, tiemask, d, total);
   MTB_LAUNCH_CHECK("maxpool_fwd_kernel");
   return MTB_OK;
 }
@@ -342,19 +358,22 @@ MTB_API int mtb_max_pool2d_backward_f32(int n, int c, int h, int w, int kh, int 
   if (tiemask && vec && tiles_exactly && (long long)n * d.OH * d.OW * (c / 4) < (1LL << 31) &&
       (reinterpret_cast<uintptr_t>(tiemask) & 7u) == 0) {
     const unsigned windows = (unsigned)((long long)n * d.OH * d.OW * (c / 4));
-    maxpool_bwd_window_kernel<<<mtb_stream_grid(windows, 256), 256, 0, st>>>(dy, tiemask, dx, d, windows);
+    MTB_LAUNCH(maxpool_bwd_window_kernel, mtb_stream_grid(windows, 256), 256, 0, st, dy, tiemask, dx, d, windows);
   } else if (tiemask && vec && (reinterpret_cast<uintptr_t>(tiemask) & 7u) == 0 && total < (1LL << 31) - (1LL << 26) &&
              ((kh == 3 && kw == 3 && sh == sw && (sh == 1 || sh == 2)) || (kh == 2 && kw == 2 && sh == 2 && sw == 2))) {
     const PoolDiv cv(c / 4), wd(w), hd(h);
-    if (kh == 2) maxpool_bwd_vec_kernel<2, 2, 2, 2><<<grid, 256, 0, st>>>((const float4*)dy, (const uint2*)tiemask, (float4*)dx, d, cv, wd, hd, (unsigned)total);
-    else if (sh == 2) maxpool_bwd_vec_kernel<3, 3, 2, 2><<<grid, 256, 0, st>>>((const float4*)dy, (const uint2*)tiemask, (float4*)dx, d, cv, wd, hd, (unsigned)total);
-    else maxpool_bwd_vec_kernel<3, 3, 1, 1><<<grid, 256, 0, st>>>((const float4*)dy, (const uint2*)tiemask, (float4*)dx, d, cv, wd, hd, (unsigned)total);
+    if (kh == 2) MTB_LAUNCH(maxpool_bwd_vec_kernel<2, 2, 2, 2>, grid, 256, 0, st, (const float4*)dy, (const uint2*)tiemask, (float4*)dx, d, cv, wd,
+                            hd, (unsigned)total);
+    else if (sh == 2) MTB_LAUNCH(maxpool_bwd_vec_kernel<3, 3, 2, 2>, grid, 256, 0, st, (const float4*)dy, (const uint2*)tiemask, (float4*)dx, d,
+                                 cv, wd, hd, (unsigned)total);
+    else MTB_LAUNCH(maxpool_bwd_vec_kernel<3, 3, 1, 1>, grid, 256, 0, st, (const float4*)dy, (const uint2*)tiemask, (float4*)dx, d, cv, wd, hd,
+                    (unsigned)total);
   } else if (tiemask) {
-    if (vec) maxpool_bwd_kernel<4, 0><<<grid, 256, 0, st>>>(dy, tiemask, out, x, dx, d, total);
-    else maxpool_bwd_kernel<1, 0><<<grid, 256, 0, st>>>(dy, tiemask, out, x, dx, d, total);
+    if (vec) MTB_LAUNCH(maxpool_bwd_kernel<4, 0>, grid, 256, 0, st, dy, tiemask, out, x, dx, d, total);
+    else MTB_LAUNCH(maxpool_bwd_kernel<1, 0>, grid, 256, 0, st, dy, tiemask, out, x, dx, d, total);
   } else {
-    if (vec) maxpool_bwd_kernel<4, 1><<<grid, 256, 0, st>>>(dy, tiemask, out, x, dx, d, total);
-    else maxpool_bwd_kernel<1, 1><<<grid, 256, 0, st>>>(dy, tiemask, out, x, dx, d, total);
+    if (vec) MTB_LAUNCH(maxpool_bwd_kernel<4, 1>, grid, 256, 0, st, dy, tiemask, out, x, dx, d, total);
+    else MTB_LAUNCH(maxpool_bwd_kernel<1, 1>, grid, 256, 0, st, dy, tiemask, out, x, dx, d, total);
   }
   MTB_LAUNCH_CHECK("maxpool_bwd_kernel");
   return MTB_OK;
@@ -364,7 +383,7 @@ MTB_API int mtb_max_pool2d_backward_f32(int n, int c, int h, int w, int kh, int 
 MTB_API int mtb_max_pool2d_argmax_u8(const unsigned short* tiemask, unsigned char* argmax, long long n, void* stream) {
   MTB_REQUIRE(tiemask && argmax && n >= 0, "max_pool2d_argmax: bad arguments");
   if (n == 0) return MTB_OK;
-  mask_to_argmax_kernel<<<mtb_stream_grid(n, 256), 256, 0, (cudaStream_t)stream>>>(tiemask, argmax, n);
+  MTB_LAUNCH(mask_to_argmax_kernel, mtb_stream_grid(n, 256), 256, 0, (cudaStream_t)stream, tiemask, argmax, n);
   MTB_LAUNCH_CHECK("mask_to_argmax_kernel");
   return MTB_OK;
 }

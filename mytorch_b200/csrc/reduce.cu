@@ -8,6 +8,8 @@ namespace {
 template <int V>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const float* __restrict__ a, long long rows, int C, int L, long long rows_per_block,
                                                               float* __restrict__ partial) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const int lane = threadIdx.x & (L - 1);
   const int rsub = threadIdx.x / L;
   const int R = 256 / L;
@@ -43,6 +45,7 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const float* __rest
 
 // Thirty-two threads per channel (consecutive threads read consecutive channels), fixed order.
 __global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restrict__ partial, int P, int C, float scale, float* __restrict__ out) {
+  mtb_wait_prior();
   const int cx = threadIdx.x & 31, py = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float s = 0.f;
@@ -60,6 +63,8 @@ __global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restr
 
 // y[n, c] = scale * sum_{hw} x[n, hw, c]; one thread per (n, c) with c fastest (coalesced).
 __global__ void __launch_bounds__(256) nhwc_spatial_sum_kernel(const float* __restrict__ x, float* __restrict__ y, long long nc, int C, int HW, float scale) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= nc) return;
   long long n = i / C;
@@ -71,6 +76,8 @@ __global__ void __launch_bounds__(256) nhwc_spatial_sum_kernel(const float* __re
 }
 
 __global__ void __launch_bounds__(256) nhwc_spatial_bcast_kernel(const float* __restrict__ dy, float* __restrict__ dx, long long total, int C, int HW, float scale) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < total; i += stride) {
@@ -88,6 +95,8 @@ struct RedDims {
 
 // One CTA per output element; threads stride over the reduced index space; fixed-order tree.
 __global__ void __launch_bounds__(256) strided_sum_kernel(const float* __restrict__ x, float* __restrict__ y, RedDims d, long long rcount, float scale) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   long long o = blockIdx.x;
   long long base = 0;
   for (int k = d.nk - 1; k >= 0; --k) {
@@ -127,10 +136,10 @@ MTB_API int mtb_colsum_f32(const float* a, long long rows, int c, float scale, f
   ColCfg cfg = mtb_col_cfg(rows, c, mtb_aligned16(a));
   dim3 grid(cfg.col_blocks, cfg.row_blocks);
   float* partial = (float*)workspace;
-  if (cfg.vec == 4) colsum_partial_kernel<4><<<grid, 256, 0, st>>>(a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
-  else colsum_partial_kernel<1><<<grid, 256, 0, st>>>(a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
+  if (cfg.vec == 4) MTB_LAUNCH(colsum_partial_kernel<4>, grid, 256, 0, st, a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
+  else MTB_LAUNCH(colsum_partial_kernel<1>, grid, 256, 0, st, a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
   MTB_LAUNCH_CHECK("colsum_partial_kernel");
-  colsum_final_kernel<<<mtb_div_up(c, 32), 1024, 0, st>>>(partial, cfg.row_blocks, c, scale, out);
+  MTB_LAUNCH(colsum_final_kernel, dim3(mtb_div_up(c, 32)), dim3(1024), 0, st, partial, cfg.row_blocks, c, scale, out);
   MTB_LAUNCH_CHECK("colsum_final_kernel");
   return MTB_OK;
 }
@@ -139,7 +148,7 @@ MTB_API int mtb_colsum_f32(const float* a, long long rows, int c, float scale, f
 MTB_API int mtb_nhwc_spatial_sum_f32(const float* x, float* y, int n, int c, int hw, float scale, void* stream) {
   MTB_REQUIRE(x && y && n > 0 && c > 0 && hw > 0, "nhwc_spatial_sum: bad arguments");
   long long nc = (long long)n * c;
-  nhwc_spatial_sum_kernel<<<mtb_div_up(nc, 256), 256, 0, (cudaStream_t)stream>>>(x, y, nc, c, hw, scale);
+  MTB_LAUNCH(nhwc_spatial_sum_kernel, mtb_div_up(nc, 256), 256, 0, (cudaStream_t)stream, x, y, nc, c, hw, scale);
   MTB_LAUNCH_CHECK("nhwc_spatial_sum_kernel");
   return MTB_OK;
 }
@@ -148,7 +157,7 @@ MTB_API int mtb_nhwc_spatial_sum_f32(const float* x, float* y, int n, int c, int
 MTB_API int mtb_nhwc_spatial_bcast_f32(const float* dy, float* dx, int n, int c, int hw, float scale, void* stream) {
   MTB_REQUIRE(dy && dx && n > 0 && c > 0 && hw > 0, "nhwc_spatial_bcast: bad arguments");
   long long total = (long long)n * c * hw;
-  nhwc_spatial_bcast_kernel<<<mtb_stream_grid(total, 256), 256, 0, (cudaStream_t)stream>>>(dy, dx, total, c, hw, scale);
+  MTB_LAUNCH(nhwc_spatial_bcast_kernel, mtb_stream_grid(total, 256), 256, 0, (cudaStream_t)stream, dy, dx, total, c, hw, scale);
   MTB_LAUNCH_CHECK("nhwc_spatial_bcast_kernel");
   return MTB_OK;
 }
@@ -165,7 +174,7 @@ MTB_API int mtb_sum_strided_f32(const float* x, float* y, int nkept, const long 
   for (int i = 0; i < nkept; ++i) { d.kshape[i] = kept_shape[i]; d.kstride[i] = kept_strides[i]; outs *= kept_shape[i]; }
   for (int i = 0; i < nred; ++i) { d.rshape[i] = red_shape[i]; d.rstride[i] = red_strides[i]; rc *= red_shape[i]; }
   MTB_REQUIRE(outs > 0 && outs < (1LL << 31), "sum_strided: output too large");
-  strided_sum_kernel<<<(unsigned)outs, 256, 0, (cudaStream_t)stream>>>(x, y, d, rc, scale);
+  MTB_LAUNCH(strided_sum_kernel, (unsigned)outs, 256, 0, (cudaStream_t)stream, x, y, d, rc, scale);
   MTB_LAUNCH_CHECK("strided_sum_kernel");
   return MTB_OK;
 }
@@ -238,10 +247,10 @@ MTB_API int mtb_colsum_noalloc_f32(const float* a, long long rows, int c, float 
   ColCfg cfg = mtb_col_cfg(rows, c, mtb_aligned16(a), kNoAllocMaxPartials);
   if (cfg.row_blocks > kNoAllocMaxPartials) return mtb_fail(MTB_ERR_UNSUPPORTED, "colsum_noalloc: internal partition exceeds the scratch");
   dim3 grid(cfg.col_blocks, cfg.row_blocks);
-  if (cfg.vec == 4) colsum_partial_kernel<4><<<grid, 256, 0, st>>>(a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
-  else colsum_partial_kernel<1><<<grid, 256, 0, st>>>(a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
+  if (cfg.vec == 4) MTB_LAUNCH(colsum_partial_kernel<4>, grid, 256, 0, st, a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
+  else MTB_LAUNCH(colsum_partial_kernel<1>, grid, 256, 0, st, a, rows, c, cfg.lanes, cfg.rows_per_block, partial);
   MTB_LAUNCH_CHECK("colsum_partial_kernel");
-  colsum_final_kernel<<<mtb_div_up(c, 32), 1024, 0, st>>>(partial, cfg.row_blocks, c, scale, out);
+  MTB_LAUNCH(colsum_final_kernel, dim3(mtb_div_up(c, 32)), dim3(1024), 0, st, partial, cfg.row_blocks, c, scale, out);
   MTB_LAUNCH_CHECK("colsum_final_kernel");
   return MTB_OK;
 }

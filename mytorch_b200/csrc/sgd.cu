@@ -38,6 +38,8 @@ __device__ __forceinline__ void sgd_span(float* p, const float* g, float* buf, l
 }
 
 __global__ void __launch_bounds__(256) sgd_kernel(float* p, const float* g, float* buf, long long n, SgdHyper h) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   sgd_span(p, g, buf, n, h, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
@@ -56,6 +58,8 @@ struct SgdTable {
 // One CTA per chunk of kSgdChunk elements of one tensor (a model has a few large tensors and dozens of
 // tiny ones: a grid of tensors x the largest tensor's chunks would be mostly empty CTAs).
 __global__ void __launch_bounds__(256) sgd_multi_kernel(const __grid_constant__ SgdTable t, SgdHyper h) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   int lo = 0, hi = t.count - 1;
   while (lo < hi) {  // last k with chunk_start[k] <= blockIdx.x
     const int mid = (lo + hi + 1) >> 1;
@@ -76,6 +80,8 @@ struct PackTable {
   int count;
 };
 __global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PackTable t, float* dst, float scale) {
+  mtb_launch_dependents();
+  mtb_wait_prior();
   int k = blockIdx.y;
   if (k >= t.count) return;
   long long n = t.n[k];
@@ -94,7 +100,7 @@ MTB_API int mtb_sgd_f32(float* param, const float* grad, float* momentum_buffer,
   MTB_REQUIRE(n >= 0 && ((param && grad && momentum_buffer) || n == 0), "sgd: bad arguments");
   if (n == 0) return MTB_OK;
   SgdHyper h{(float)lr, (float)weight_decay, (float)momentum, (float)(1.0 - dampening), (float)grad_scale, nesterov, maximize, is_first};
-  sgd_kernel<<<mtb_stream_grid((n + 3) / 4, 256), 256, 0, (cudaStream_t)stream>>>(param, grad, momentum_buffer, n, h);
+  MTB_LAUNCH(sgd_kernel, mtb_stream_grid((n + 3) / 4, 256), 256, 0, (cudaStream_t)stream, param, grad, momentum_buffer, n, h);
   MTB_LAUNCH_CHECK("sgd_kernel");
   return MTB_OK;
 }
@@ -123,7 +129,7 @@ MTB_API int mtb_sgd_multi_f32(int count, float* const* params, const float* cons
     t.chunk_start[t.count] = (int)chunks;
     if (chunks == 0) continue;
     dim3 grid((unsigned int)chunks);
-    sgd_multi_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(t, h);
+    MTB_LAUNCH(sgd_multi_kernel, grid, 256, 0, (cudaStream_t)stream, t, h);
     MTB_LAUNCH_CHECK("sgd_multi_kernel");
   }
   return MTB_OK;
@@ -147,7 +153,7 @@ MTB_API int mtb_pack_scale_f32(int count, const float* const* srcs, const long l
     int cap = mtb_sm_count() * 4;
     if (gx > cap) gx = cap;
     if (gx < 1) gx = 1;
-    pack_kernel<<<dim3(gx, t.count), 256, 0, (cudaStream_t)stream>>>(t, dst, (float)scale);
+    MTB_LAUNCH(pack_kernel, dim3(gx, t.count), 256, 0, (cudaStream_t)stream, t, dst, (float)scale);
     MTB_LAUNCH_CHECK("pack_kernel");
   }
   return MTB_OK;

@@ -386,6 +386,8 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
   constexpr int GM = TM / 4, GN = TN / 4;  // a thread's rows and columns come in groups of four, spread over the tile
   __shared__ float As[2][BK][BM + 4];
   __shared__ float Bs[2][BK][BN + 4];
+  mtb_launch_dependents();
+  mtb_wait_prior();
   const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int z = blockIdx.z / slices, slice = blockIdx.z - z * slices;
@@ -547,16 +549,18 @@ int launch_tile(const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& tab
     cfg.gridDim = grid;
     cfg.blockDim = dim3(T::THREADS);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = (unsigned)slices;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     MTB_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, SA, VA, SB, VB, true>, sa, sb, o, table, M, N, K, slices, per));
   } else {
-    gemm_kernel<T, SA, VA, SB, VB, false><<<grid, T::THREADS, 0, st>>>(sa, sb, o, table, M, N, K, slices, per);
+    MTB_LAUNCH(gemm_kernel<T, SA, VA, SB, VB, false>, grid, T::THREADS, 0, st, sa, sb, o, table, M, N, K, slices, per);
   }
   MTB_LAUNCH_CHECK(name);
   return MTB_OK;

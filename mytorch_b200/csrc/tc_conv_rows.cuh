@@ -107,6 +107,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     tmem_alloc(smem_u32(&tmem_slot), 2 * MT * BN);
     tmem_relinquish();
   }
+  mtb_wait_prior();  // everything above overlaps the end of the kernel before
   if constexpr (BNORM) load_bn_columns<BN>(bn_columns, p.bn, (int)(blockIdx.x % p.n_tiles) * BN, p.N);
   fence_proxy_async();
   tc_fence_before();
@@ -522,6 +523,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   }
 
   // ------------------------------------------------------------ teardown
+  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
   if (abort_flag) {
@@ -626,7 +628,7 @@ int launch_row_conv_kernel(const CUtensorMap& mapA, const CUtensorMap& mapB, con
   const int items = ((p.m_tiles + MT - 1) / MT) * p.n_tiles;
   int grid = items < mtb_sm_count() ? items : mtb_sm_count();
   if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one output-channel tile
-  kernel<<<grid, kRowThreads, smem_bytes, st>>>(mapA, mapB, p);
+  MTB_LAUNCH(kernel, dim3(grid), dim3(kRowThreads), smem_bytes, st, mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_conv_rows_kernel");
   return MTB_OK;
 }
@@ -754,6 +756,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_cons
     tmem_alloc(smem_u32(&tmem_slot), 512);
     tmem_relinquish();
   }
+  mtb_wait_prior();
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
@@ -898,6 +901,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_cons
     }
   }
 
+  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
   if (abort_flag) {
@@ -913,6 +917,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_cons
 // splits z, z+8, ... in order; the 8 sums are then added in index order): the same result for
 // any launch, and enough CTAs to read ~100 partial planes at full speed.
 __global__ void __launch_bounds__(1024) wgrad_reduce_many_kernel(const float* __restrict__ partial, float* __restrict__ dw, int Kw, int Cout, int splits) {
+  mtb_wait_prior();
   __shared__ float acc[8][4][33];
   const int c = blockIdx.y * 32 + threadIdx.x;
   const int r = blockIdx.x * 4 + threadIdx.y;
@@ -1002,7 +1007,7 @@ int launch_wgrad_rows(const CUtensorMap& mapX, const CUtensorMap& mapDY, const W
   auto kernel = tc_wgrad_rows_kernel<BN, FIX>;
   static unsigned long long configured = 0;
   if (int rc = mtb_opt_in_smem((const void*)kernel, 227 * 1024 - 1024, &configured)) return rc;
-  kernel<<<grid, 192, smem_bytes, st>>>(mapX, mapDY, p);
+  MTB_LAUNCH(kernel, dim3(grid), dim3(192), smem_bytes, st, mapX, mapDY, p);
   MTB_LAUNCH_CHECK("tc_wgrad_rows_kernel");
   return MTB_OK;
 }
@@ -1034,7 +1039,7 @@ int run_wgrad_rows(const WgradRowsPlan& q, int n, int cin, int h, int w, int kh,
   if (rc) return rc;
   const int Kw = kh * kw * cin;
   dim3 rgrid((unsigned)((Kw + 3) / 4), (unsigned)((cout + 31) / 32));
-  wgrad_reduce_many_kernel<<<rgrid, dim3(32, 4, 8), 0, st>>>(partial, dw, Kw, cout, q.splits);
+  MTB_LAUNCH(wgrad_reduce_many_kernel, rgrid, dim3(32, 4, 8), 0, st, partial, dw, Kw, cout, q.splits);
   MTB_LAUNCH_CHECK("wgrad_reduce_many_kernel");
   return MTB_OK;
 }

@@ -210,6 +210,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     tmem_alloc(smem_u32(&tmem_slot), C::kTmemCols);
     tmem_relinquish();
   }
+  mtb_wait_prior();  // everything above overlaps the end of the kernel before
   if constexpr (BNORM) load_bn_columns<BN>(bn_columns, p.bn, (blockIdx.x / p.splits) % p.n_tiles * BN, p.N);
   tc_fence_before();
   __syncthreads();
@@ -567,6 +568,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   }
 
   // ------------------------------------------------------------ teardown
+  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
   if (abort_flag) {
@@ -588,7 +590,7 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
   int tiles = p.m_tiles * p.n_tiles * p.splits;  // work units
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
   if ((EPI == EPI_STATS || EPI == EPI_BN) && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
-  kernel<<<grid, kGemmThreads, C::kSmemBytes, st>>>(mapA, mapB, p);
+  MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), C::kSmemBytes, st, mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
 }
@@ -1046,6 +1048,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
     tmem_alloc(smem_u32(&tmem_slot), C::kTmemCols);
     tmem_relinquish();
   }
+  mtb_wait_prior();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1189,6 +1192,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
     }
   }
 
+  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
   if (abort_flag) {
@@ -1208,6 +1212,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
 constexpr int kReduceRows = 8;
 __global__ void __launch_bounds__(32 * kReduceRows) wgrad_reduce_transpose_kernel(const float* __restrict__ partial, float* __restrict__ dw, int Kw,
                                                                                    int Cout, int splits) {
+  mtb_wait_prior();
   __shared__ float tile[128][kReduceRows + 1];
   const int r0 = blockIdx.x * kReduceRows, c0 = blockIdx.y * 128;
   const long long plane = (long long)Kw * Cout;
@@ -1387,7 +1392,7 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
     static unsigned long long configured = 0;                                                                           \
     if (int rc_ = mtb_opt_in_smem((const void*)tc_wgrad_kernel<BN_, PB_>, (int)WCfg<BN_, PB_>::kSmemBytes, &configured)) \
       return rc_;                                                                                                       \
-    tc_wgrad_kernel<BN_, PB_><<<grid, kGemmThreads, WCfg<BN_, PB_>::kSmemBytes, st>>>(mapX, mapDY, p);                           \
+    MTB_LAUNCH(tc_wgrad_kernel<BN_, PB_>, dim3(grid), dim3(kGemmThreads), WCfg<BN_, PB_>::kSmemBytes, st, mapX, mapDY, p);                           \
   } while (0)
   if (q.bn == 64) MTB_LAUNCH_WGRAD(64, 64);
   else if (q.bn == 128) MTB_LAUNCH_WGRAD(128, 64);
@@ -1395,7 +1400,7 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
 #undef MTB_LAUNCH_WGRAD
   MTB_LAUNCH_CHECK("tc_wgrad_kernel");
   dim3 rgrid((unsigned)((q.Kw + kReduceRows - 1) / kReduceRows), (unsigned)((cout + 127) / 128));
-  wgrad_reduce_transpose_kernel<<<rgrid, dim3(32, kReduceRows), 0, st>>>((const float*)workspace, dw, (int)q.Kw, cout, q.splits);
+  MTB_LAUNCH(wgrad_reduce_transpose_kernel, rgrid, dim3(32, kReduceRows), 0, st, (const float*)workspace, dw, (int)q.Kw, cout, q.splits);
   MTB_LAUNCH_CHECK("wgrad_reduce_transpose_kernel");
   return MTB_OK;
 }
