@@ -106,23 +106,31 @@ class DAGTracker:
                     if isinstance(arg, Tensor) and arg.requires_grad and arg._grad_node is None:
                         pending[id(arg)] = pending.get(id(arg), 0) + 1
 
+        funcs, fusable, deferrable = self._backward_funcs, self.fused_accumulate, self.deferrable
         for node in order:
             name, inputs = node.name, node.inputs
             fused = None  # the input whose gradient so far is handed to the operator
-            extra = {}
-            slot = self.fused_accumulate.get(name)
-            if slot is not None:
-                cand = inputs[slot]
-                if isinstance(cand, Tensor) and cand.requires_grad and cand.grad is not None:
-                    fused = cand
-                    extra["accumulate_dx"] = cand.grad
-            if join is not None and name in self.deferrable:
-                extra["defer_weight_gradient"] = True
-            grads = self._backward_funcs[name](*[t.grad for t in node.outputs], *node.helpers, *inputs, **extra)
-            for k, (arg, grad) in enumerate(zip(inputs, grads)):  # operators may return fewer gradients than they have inputs
-                if grad is None or not isinstance(arg, Tensor) or not arg.requires_grad:
+            slot = -1
+            if name in fusable or name in deferrable:
+                extra = {}
+                slot = fusable.get(name, -1)
+                if slot >= 0:
+                    cand = inputs[slot]
+                    if isinstance(cand, Tensor) and cand.requires_grad and cand.grad is not None:
+                        fused = cand
+                        extra["accumulate_dx"] = cand.grad
+                if join is not None and name in deferrable:
+                    extra["defer_weight_gradient"] = True
+                grads = funcs[name](*[t.grad for t in node.outputs], *node.helpers, *inputs, **extra)
+            else:
+                grads = funcs[name](*[t.grad for t in node.outputs], *node.helpers, *inputs)
+            for k, grad in enumerate(grads):  # operators may return fewer gradients than they have inputs
+                if grad is None:
                     continue
-                if arg.grad is None or (arg is fused and k == slot):
+                arg = inputs[k]
+                if not isinstance(arg, Tensor) or not arg.requires_grad:
+                    continue
+                if arg.grad is None or (k == slot and arg is fused):
                     arg.grad = grad
                 else:
                     if arg.grad.shape != grad.shape:

@@ -136,19 +136,25 @@ class CudaEnv:
         if count.value == 0:
             raise NativeError("no CUDA device is available; the cuda backend has no CPU fallback")
         self.lib.device_check()
-        self._streams = {}
-        self._scratch = {}
+        self._scratch = ({}, {})  # per device: of the compute stream, of the side stream
         self._retired_scratch = []
         self._capturing = False
         # weight gradients run beside the rest of backward on a second stream (see fork_side / join_side)
         self._side_streams = {}
-        self._side_scratch = {}
         self._side_keepalive = []
         self._side_busy = set()
         self._fork_events, self._join_events = {}, {}
         self.overlap_weight_gradients = not os.environ.get("MTB_SERIAL_WGRAD")
         from mytorch_b200.autograd import DAGTracker
+        from mytorch_b200.dtype import float32
+        from mytorch_b200.tensor import Tensor
 
+        # Every operator asks for these, so they are native (csrc/binding.cpp):
+        self.stream = _binding.stream  # () -> the compute stream of the current device: every operator enqueues its work there
+        # (nbytes) -> (address, bytes) of scratch for kernels that need it (split-K partials, per-CTA reduction partials): one
+        # buffer per device, shared by all operators, which run in order on one stream; the side stream has its own
+        self.workspace, self.side_workspace = _binding.workspace, _binding.side_workspace
+        _binding.set_state(Tensor, float32, CudaMemory, self, self.lib.stream_create, self._grow_scratch)
         DAGTracker.instance().join_hook = self.join_side
 
     # ---- devices, streams
@@ -158,14 +164,6 @@ class CudaEnv:
     def set_device(self, index):
         if index is not None and index != _binding.current_device():
             self.lib.set_device(int(index))
-
-    def stream(self):
-        """The compute stream of the current device: every operator enqueues its work there."""
-        dev = _binding.current_device()
-        s = self._streams.get(dev)
-        if s is None:
-            s = self._streams[dev] = self.lib.stream_create()
-        return s
 
     def new_stream(self):
         return self.lib.stream_create()
@@ -235,18 +233,9 @@ class CudaEnv:
         self._side_busy.clear()
         self._side_keepalive.clear()
 
-    def side_workspace(self, nbytes):
-        """Scratch for side-stream kernels (the compute stream's scratch may be in use at the same time)."""
-        return self._grow_scratch(self._side_scratch, nbytes)
-
     # ---- memory
-    def workspace(self, nbytes):
-        """Scratch for kernels that need it (split-K partials, per-CTA reduction partials).
-        One buffer per device, shared by all operators: they run in order on one stream."""
-        return self._grow_scratch(self._scratch, nbytes)
-
-    def _grow_scratch(self, table, nbytes):
-        dev = self.current_device()
+    def _grow_scratch(self, which, nbytes):
+        table, dev = self._scratch[which], self.current_device()
         buf = table.get(dev)
         if buf is None or buf.nbytes < nbytes:
             if buf is not None:

@@ -12,33 +12,26 @@ the logical-dimension strides of either layout to the generic strided kernels.
 from __future__ import annotations
 
 import ctypes
-import math
-from array import array
 
 import numpy as np
 
 from mytorch_b200.autograd import DAGTracker
 from mytorch_b200.backends.backend_dispatcher import BackendDispatcher
-from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory
+from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory, _binding
 from mytorch_b200.backends.utils import calculate_broadcast_shape, calculate_reduce_shape, calculate_reshaped_shape
 from mytorch_b200.dtype import float32, int32, int64
 from mytorch_b200.tensor import InvalidDataTypeError, MismatchShapesError, Tensor
 
 _tracker = DAGTracker.instance()
 _reg = BackendDispatcher.instance().register_backend_function
-_LL = ctypes.c_longlong
 _on_device = Tensor._on_device
 
 
-def _env(t):
-    env = CudaEnv._instance or CudaEnv.instance()
-    env.set_device(t.device.index)
-    return env
-
-
-def _ptr(t):
-    """A tensor as a pointer argument (the binding takes blocks as they are)."""
-    return None if t is None else t._native_array
+# Native (csrc/binding.cpp): _env(tensor) makes the tensor's device current and returns the CUDA state; _new(shape, like,
+# dtype=None) is an uninitialised result tensor.  Tensors and blocks are pointer arguments as they are, tuples and lists of
+# ints are shapes and strides.
+_env = getattr(_binding, "enter", None)
+_new = getattr(_binding, "new_like", None)
 
 
 def _numel(shape):
@@ -46,14 +39,6 @@ def _numel(shape):
     for s in shape:
         n *= s
     return n
-
-
-def _new(shape, like, dtype=None):
-    dtype = dtype or like.dtype
-    n = dtype._itemsize
-    for s in shape:
-        n *= s
-    return _on_device(shape, dtype, like.device, CudaMemory(like.device.index, n))
 
 
 def _grad_buffer(param):
@@ -90,10 +75,6 @@ def _strides(t):
     return out
 
 
-def _ll(values):
-    return (_LL * max(len(values), 1))(*values)
-
-
 # ---------------------------------------------------------------------------- host <-> device
 
 @_reg("cuda", "upload")
@@ -105,7 +86,7 @@ def cuda_upload(t, array):
         stage = CudaMemory(t.device.index, array.nbytes)
         stage.write(array)
         n, c, h, w = t.shape
-        env.lib.nchw_to_nhwc_f32(stage.ptr, _ptr(t), n, c, h, w, env.stream())
+        env.lib.nchw_to_nhwc_f32(stage.ptr, t, n, c, h, w, env.stream())
     else:
         t._native_array.write(array)
 
@@ -123,7 +104,7 @@ def upload_into(t, host):
             stage = t._stage = CudaMemory(t.device.index, t._native_array.nbytes)
         stage.write_from(src)
         n, c, h, w = t.shape
-        env.lib.nchw_to_nhwc_f32(stage.ptr, _ptr(t), n, c, h, w, env.stream())
+        env.lib.nchw_to_nhwc_f32(stage.ptr, t, n, c, h, w, env.stream())
     else:
         t._native_array.write_from(src)
         if not hasattr(host, "data_ptr") and src is not host:
@@ -136,7 +117,7 @@ def cuda_download(t):
     if _nontrivial_nhwc(t):
         tmp = CudaMemory(t.device.index, t._native_array.nbytes)
         n, c, h, w = t.shape
-        env.lib.nhwc_to_nchw_f32(_ptr(t), tmp.ptr, n, c, h, w, env.stream())
+        env.lib.nhwc_to_nchw_f32(t, tmp.ptr, n, c, h, w, env.stream())
         return tmp.read(t.shape, t.dtype.np_dtype)
     return t._native_array.read(t.shape, t.dtype.np_dtype)
 
@@ -186,7 +167,7 @@ def _stem_input(env, x, form):
         return _pad_channels(env, x, _TC_CHANNELS)
     n, c, h, w = x.shape
     out = _new((n, _TC_CHANNELS, args[2], args[3]), x)
-    env.lib.pack_patches_f32(n, c, h, w, *pack, _ptr(x), _ptr(out), env.stream())
+    env.lib.pack_patches_f32(n, c, h, w, *pack, x, out, env.stream())
     return out
 
 
@@ -202,7 +183,7 @@ def _pad_channels(env, t, channels):
     """A channels-last tensor copied into one with `channels` channels (dim 1), the new ones zero."""
     n, c, h, w = t.shape
     out = _new((n, channels, h, w), t)
-    env.lib.resize_channels_f32(_ptr(t), _ptr(out), n * h * w, c, channels, env.stream())
+    env.lib.resize_channels_f32(t, out, n * h * w, c, channels, env.stream())
     return out
 
 
@@ -210,7 +191,7 @@ def _take_channels(env, t, channels, like, out=None):
     """First `channels` channels (dim 1) of a channels-last tensor, as a new tensor (or into `out`)."""
     n, c, h, w = t.shape
     out = _new((n, channels, h, w), like) if out is None else out
-    env.lib.resize_channels_f32(_ptr(t), _ptr(out), n * h * w, c, channels, env.stream())
+    env.lib.resize_channels_f32(t, out, n * h * w, c, channels, env.stream())
     return out
 
 
@@ -228,7 +209,7 @@ def _conv_operands(env, input, weight, stride, padding):
             input._stem_held = (form, x)  # the weight gradient of this convolution reads it again
         rows, entries = _stem_filter_rows(weight.shape, form)
         block = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
-        env.lib.resize_channels_f32(_ptr(weight), block, rows, entries, _TC_CHANNELS, env.stream())
+        env.lib.resize_channels_f32(weight, block, rows, entries, _TC_CHANNELS, env.stream())
         wt = _on_device((rows, _TC_CHANNELS), float32, weight.device, block)
     return a, x, wt, _new((n, cout, oh, ow), input)
 
@@ -242,8 +223,8 @@ def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, ru
     if residual is not None and residual.shape != out.shape:
         raise MismatchShapesError([out.shape, residual.shape])
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
-    env.lib.conv2d_bn_forward_f32(*a, _ptr(x), _ptr(wt), _ptr(bias), _ptr(gamma), _ptr(beta), _ptr(running_mean), _ptr(running_var), float(eps),
-                                  _ptr(residual), int(bool(relu)), _ptr(out), ws, ws_bytes, env.stream())
+    env.lib.conv2d_bn_forward_f32(*a, x, wt, bias, gamma, beta, running_mean, running_var, float(eps),
+                                  residual, int(bool(relu)), out, ws, ws_bytes, env.stream())
     return out
 
 
@@ -259,12 +240,12 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
     if bn_stats:
         partials = CudaMemory(input.device.index, env.lib.conv2d_stats_max_rows() * 3 * a[-1] * 4)
         rows = ctypes.c_int(0)
-        env.lib.conv2d_forward_stats_f32(*a, _ptr(x), _ptr(wt), _ptr(bias), _ptr(out), 0, partials.ptr, ctypes.byref(rows), ws, ws_bytes,
+        env.lib.conv2d_forward_stats_f32(*a, x, wt, bias, out, 0, partials.ptr, ctypes.byref(rows), ws, ws_bytes,
                                          env.stream())
         if rows.value > 0:
             out._bn_partials = (partials, rows.value)
         return out
-    env.lib.conv2d_forward_f32(*a, _ptr(x), _ptr(wt), _ptr(bias), _ptr(out), 0, ws, ws_bytes, env.stream())
+    env.lib.conv2d_forward_f32(*a, x, wt, bias, out, 0, ws, ws_bytes, env.stream())
     return out
 
 
@@ -287,21 +268,22 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         wt = _pad_channels(env, weight, _TC_CHANNELS)
         a = (a[0], _TC_CHANNELS) + a[2:]
     st = env.stream()
-    ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
+    need = env.lib.conv2d_workspace_bytes(*a)
     dx = dw = db = None
     if want_dx:
+        ws, ws_bytes = env.workspace(need)
         if accumulate_dx is not None and not padded and env.lib.conv2d_dgrad_accumulates_in_place(
-                *a, _ptr(output_grad), _ptr(wt), _ptr(accumulate_dx)):
+                *a, output_grad, wt, accumulate_dx):
             # a filter smaller than its stride (the 1x1 / stride-2 shortcut) reaches only some pixels: it adds
             # to those in the gradient the input already holds, which is then the returned tensor
             dx = accumulate_dx
-            env.lib.conv2d_dgrad_add_f32(*a, _ptr(output_grad), _ptr(wt), _ptr(dx), _ptr(dx), ws, ws_bytes, st)
+            env.lib.conv2d_dgrad_add_f32(*a, output_grad, wt, dx, dx, ws, ws_bytes, st)
         elif accumulate_dx is not None and not padded:
             dx = _new(x.shape, x)
-            env.lib.conv2d_dgrad_add_f32(*a, _ptr(output_grad), _ptr(wt), _ptr(accumulate_dx), _ptr(dx), ws, ws_bytes, st)
+            env.lib.conv2d_dgrad_add_f32(*a, output_grad, wt, accumulate_dx, dx, ws, ws_bytes, st)
         else:
             dx = _new((a[0], a[1], a[2], a[3]), x)
-            env.lib.conv2d_dgrad_f32(*a, _ptr(output_grad), _ptr(wt), _ptr(dx), ws, ws_bytes, st)
+            env.lib.conv2d_dgrad_f32(*a, output_grad, wt, dx, ws, ws_bytes, st)
             if padded:
                 dx = _take_channels(env, dx, cin, dx)
             if accumulate_dx is not None:
@@ -320,22 +302,24 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
             else:
                 x = _stem_input(env, input, form)
             wa = form[1]
-            ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*wa))
-        wst, wws, wws_bytes = st, ws, ws_bytes
+            need = env.lib.conv2d_workspace_bytes(*wa)
+        wst = st
         if defer_weight_gradient and env.overlap_weight_gradients and weight.grad is None:
             wst = env.fork_side((x, output_grad))
-            wws, wws_bytes = env.side_workspace(env.lib.conv2d_workspace_bytes(*wa))
+            wws, wws_bytes = env.side_workspace(need)
+        else:
+            wws, wws_bytes = env.workspace(need)
         if form is not None:
             rows, entries = _stem_filter_rows(weight.shape, form)
             wide = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
-            env.lib.conv2d_wgrad_f32(*wa, _ptr(x), _ptr(output_grad), wide, wws, wws_bytes, wst)
+            env.lib.conv2d_wgrad_f32(*wa, x, output_grad, wide, wws, wws_bytes, wst)
             dw = _grad_buffer(weight)
-            env.lib.resize_channels_f32(wide, _ptr(dw), rows, _TC_CHANNELS, entries, wst)
+            env.lib.resize_channels_f32(wide, dw, rows, _TC_CHANNELS, entries, wst)
             if wst is not st:
                 env._side_keepalive.append(wide)
         else:
             dw = _grad_buffer(weight)
-            env.lib.conv2d_wgrad_f32(*a, _ptr(x), _ptr(output_grad), _ptr(dw), wws, wws_bytes, wst)
+            env.lib.conv2d_wgrad_f32(*a, x, output_grad, dw, wws, wws_bytes, wst)
     if bias is not None and bias.requires_grad:
         db = _colsum(env, output_grad, _numel(output_grad.shape) // a[-1], a[-1], bias, out=_grad_buffer(bias))
     return [dx, dw, db]
@@ -344,14 +328,14 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
 def _colsum(env, mat, rows, cols, like, scale=1.0, out=None):
     out = _new((cols,), like) if out is None else out
     ws, ws_bytes = env.workspace(env.lib.colsum_workspace_bytes(cols))
-    env.lib.colsum_f32(_ptr(mat), rows, cols, scale, _ptr(out), ws, ws_bytes, env.stream())
+    env.lib.colsum_f32(mat, rows, cols, scale, out, ws, ws_bytes, env.stream())
     return out
 
 
 # ---------------------------------------------------------------------------- linear / mm
 
 def _gemm(env, m, n, k, a, ta, b, tb, bias, relu, c):
-    env.lib.gemm_f32(m, n, k, _ptr(a), ta, _ptr(b), tb, _ptr(bias), relu, _ptr(c), env.stream())
+    env.lib.gemm_f32(m, n, k, a, ta, b, tb, bias, relu, c, env.stream())
 
 
 @_reg("cuda", "linear")
@@ -420,12 +404,12 @@ def cuda_batch_norm2d(x, weight, bias, eps, training, momentum, running_mean, ru
     use_batch_stats = bool(training) or running_mean is None or running_var is None
     pre = getattr(x, "_bn_partials", None)
     if use_batch_stats and pre is not None:  # the convolution that produced x already reduced its statistics
-        env.lib.batch_norm2d_forward_prestats_f32(n, c, h, w, _ptr(x), _ptr(weight), _ptr(bias), float(eps), float(momentum), _ptr(running_mean),
-                                                  _ptr(running_var), _ptr(y), _ptr(mean), _ptr(var), int(bool(relu)), pre[0].ptr, pre[1], ws, ws_bytes,
+        env.lib.batch_norm2d_forward_prestats_f32(n, c, h, w, x, weight, bias, float(eps), float(momentum), running_mean,
+                                                  running_var, y, mean, var, int(bool(relu)), pre[0].ptr, pre[1], ws, ws_bytes,
                                                   env.stream())
         return y, mean, var
-    env.lib.batch_norm2d_forward_f32(n, c, h, w, _ptr(x), _ptr(weight), _ptr(bias), float(eps), int(use_batch_stats), float(momentum),
-                                     _ptr(running_mean), _ptr(running_var), _ptr(y), _ptr(mean), _ptr(var), int(bool(relu)), ws, ws_bytes, env.stream())
+    env.lib.batch_norm2d_forward_f32(n, c, h, w, x, weight, bias, float(eps), int(use_batch_stats), float(momentum),
+                                     running_mean, running_var, y, mean, var, int(bool(relu)), ws, ws_bytes, env.stream())
     return y, mean, var
 
 
@@ -441,8 +425,8 @@ def cuda_batch_norm2d_add_relu(x, residual, weight, bias, eps, training, momentu
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
     use_batch_stats = bool(training) or running_mean is None or running_var is None
     pre = getattr(x, "_bn_partials", None) if use_batch_stats else None
-    head = (n, c, h, w, _ptr(x), _ptr(residual), _ptr(weight), _ptr(bias), float(eps), int(use_batch_stats), float(momentum), _ptr(running_mean),
-            _ptr(running_var), _ptr(y), _ptr(mean), _ptr(var))
+    head = (n, c, h, w, x, residual, weight, bias, float(eps), int(use_batch_stats), float(momentum), running_mean,
+            running_var, y, mean, var)
     tail = (pre[0] if pre else None, pre[1] if pre else 0, ws, ws_bytes, env.stream())
     if c % 4 == 0 and not _tracker.no_grad:  # the ReLU's mask goes to backward with the statistics
         mean._relu_mask = CudaMemory(x.device.index, n * c * h * w // 4)
@@ -462,12 +446,12 @@ def cuda_batch_norm2d_add_relu_backward(output_grad, mean, var, x, residual, wei
     dg = _grad_buffer(weight) if affine else None
     db = _grad_buffer(bias) if affine else None
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
-    tail = (_ptr(weight), _ptr(bias), float(eps), _ptr(dx), _ptr(dres), _ptr(dg), _ptr(db), ws, ws_bytes, env.stream())
+    tail = (weight, bias, float(eps), dx, dres, dg, db, ws, ws_bytes, env.stream())
     mask = getattr(mean, "_relu_mask", None)
     if mask is not None:
-        env.lib.batch_norm2d_add_relu_backward_masked_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), mask, *tail)
+        env.lib.batch_norm2d_add_relu_backward_masked_f32(n, c, h, w, output_grad, mean, var, x, mask, *tail)
     else:
-        env.lib.batch_norm2d_add_relu_backward_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), _ptr(residual), *tail)
+        env.lib.batch_norm2d_add_relu_backward_f32(n, c, h, w, output_grad, mean, var, x, residual, *tail)
     return [dx, dres, dg, db]
 
 
@@ -491,20 +475,20 @@ def cuda_batch_norm2d_backward(output_grad, mean, var, x, weight, bias, eps, rel
     dg = _grad_buffer(weight) if affine else None
     db = _grad_buffer(bias) if affine else None
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
-    env.lib.batch_norm2d_backward_f32(n, c, h, w, _ptr(output_grad), _ptr(mean), _ptr(var), _ptr(x), _ptr(weight), _ptr(bias), float(eps),
-                                      int(bool(relu)), _ptr(dx), _ptr(dg), _ptr(db), ws, ws_bytes, env.stream())
+    env.lib.batch_norm2d_backward_f32(n, c, h, w, output_grad, mean, var, x, weight, bias, float(eps),
+                                      int(bool(relu)), dx, dg, db, ws, ws_bytes, env.stream())
     return [dx, dg, db]
 
 
 # ---------------------------------------------------------------------------- pooling
 
 def _pool_args(x, kernel_size, stride, padding):
-    pair = lambda v: (v, v) if isinstance(v, int) else tuple(v)
-    kh, kw = pair(kernel_size)
-    sh, sw = pair(kernel_size if stride is None else stride)
-    ph, pw = pair(padding)
-    n, c, h, w = x.shape
-    return (n, c, h, w, kh, kw, sh, sw, ph, pw)
+    if stride is None:
+        stride = kernel_size
+    kh, kw = (kernel_size, kernel_size) if isinstance(kernel_size, int) else kernel_size
+    sh, sw = (stride, stride) if isinstance(stride, int) else stride
+    ph, pw = (padding, padding) if isinstance(padding, int) else padding
+    return (*x.shape, kh, kw, sh, sw, ph, pw)
 
 
 @_reg("cuda", "max_pool2d")
@@ -515,8 +499,8 @@ def cuda_max_pool2d(x, kernel_size, stride, padding):
     n, c, h, w, kh, kw, sh, sw, ph, pw = a
     oh, ow = (2 * ph + h - kh) // sh + 1, (2 * pw + w - kw) // sw + 1
     y = _new((n, c, oh, ow), x)
-    mask = CudaMemory(x.device.index, 2 * _numel(y.shape)) if kh * kw <= 16 else None
-    env.lib.max_pool2d_forward_f32(*a, _ptr(x), _ptr(y), mask.ptr if mask else None, env.stream())
+    mask = CudaMemory(x.device.index, 2 * n * c * oh * ow) if kh * kw <= 16 else None
+    env.lib.max_pool2d_forward_f32(*a, x, y, mask, env.stream())
     y._pool_tiemask = mask  # uint16 per output element, channels-last like y
     return y
 
@@ -527,7 +511,7 @@ def cuda_max_pool2d_backward(output_grad, output, x, kernel_size, stride, paddin
     a = _pool_args(x, kernel_size, stride, padding)
     dx = _new(x.shape, x)
     mask = getattr(output, "_pool_tiemask", None)
-    env.lib.max_pool2d_backward_f32(*a, _ptr(output_grad), mask.ptr if mask else None, _ptr(output), _ptr(x), _ptr(dx), env.stream())
+    env.lib.max_pool2d_backward_f32(*a, output_grad, mask, output, x, dx, env.stream())
     return [dx]
 
 
@@ -552,7 +536,7 @@ def cuda_relu(x):
     _f32(x)
     env = _env(x)
     y = _new(x.shape, x)
-    env.lib.relu_forward_f32(_ptr(x), _ptr(y), _numel(x.shape), env.stream())
+    env.lib.relu_forward_f32(x, y, _numel(x.shape), env.stream())
     return y
 
 
@@ -560,7 +544,7 @@ def cuda_relu(x):
 def cuda_relu_backward(output_grad, x):
     env = _env(x)
     dx = _new(x.shape, x)
-    env.lib.relu_backward_f32(_ptr(output_grad), _ptr(x), _ptr(dx), _numel(x.shape), env.stream())
+    env.lib.relu_backward_f32(output_grad, x, dx, _numel(x.shape), env.stream())
     return [dx]
 
 
@@ -572,7 +556,7 @@ def cuda_add_relu(x, y):
             raise MismatchShapesError([x.shape, y.shape])
     env = _env(x)
     z = _new(x.shape, x)
-    env.lib.add_relu_f32(_ptr(x), _ptr(y), _ptr(z), _numel(x.shape), env.stream())
+    env.lib.add_relu_f32(x, y, z, _numel(x.shape), env.stream())
     return z
 
 
@@ -580,7 +564,7 @@ def cuda_add_relu(x, y):
 def cuda_add_relu_backward(output_grad, x, y):
     env = _env(x)
     g = _new(x.shape, x)
-    env.lib.add_relu_backward_f32(_ptr(output_grad), _ptr(x), _ptr(y), _ptr(g), _numel(x.shape), env.stream())
+    env.lib.add_relu_backward_f32(output_grad, x, y, g, _numel(x.shape), env.stream())
     return g, g  # one tensor serves both operands: gradients are never modified in place
 
 
@@ -588,7 +572,7 @@ def cuda_add_relu_backward(output_grad, x, y):
 def cuda_fill(x, value):
     env = _env(x)
     if x.dtype is float32:
-        env.lib.fill_f32(_ptr(x), _numel(x.shape), float(value), env.stream())
+        env.lib.fill_f32(x, _numel(x.shape), float(value), env.stream())
     else:
         x._native_array.write(np.full(x.shape, value, dtype=x.dtype.np_dtype))
 
@@ -617,7 +601,7 @@ def cuda_copy(dst, src):
     if dst.shape != src.shape:
             raise MismatchShapesError([dst.shape, src.shape])
     if dst.dtype is float32:
-        env.lib.copy_f32(_ptr(dst), _ptr(src), _numel(dst.shape), env.stream())
+        env.lib.copy_f32(dst, src, _numel(dst.shape), env.stream())
     else:
         dst._native_array.copy_from(src._native_array, dst._native_array.nbytes)
 
@@ -634,7 +618,7 @@ def cuda_cast(x, dtype):
     if x._nhwc or (len(x.shape) == 4 and dtype is float32):
         raise RuntimeError("cast of 4-D tensors between float32 and integer types is not available on the cuda backend")
     out = _new(x.shape, x, dtype)
-    env.lib.cast(kind, _ptr(x), _ptr(out), _numel(x.shape), env.stream())
+    env.lib.cast(kind, x, out, _numel(x.shape), env.stream())
     return out
 
 
@@ -653,20 +637,19 @@ def _bstrides(t, out_shape):
 def _binary(name, x, y, alpha=1.0):
     _f32(x, y)
     env = _env(x)
-    shape = calculate_broadcast_shape(x.shape, y.shape)
+    shape = x.shape if x.shape == y.shape else calculate_broadcast_shape(x.shape, y.shape)
     z = _new(shape, x)
-    n = _numel(shape)
     if x.shape == y.shape and name in ("add", "sub", "mul"):
         if name == "mul":
-            env.lib.mul_f32(_ptr(x), _ptr(y), _ptr(z), n, env.stream())
+            env.lib.mul_f32(x, y, z, _numel(shape), env.stream())
         else:
-            env.lib.add_f32(_ptr(x), _ptr(y), _ptr(z), n, float(alpha) if name == "add" else -float(alpha), env.stream())
+            env.lib.add_f32(x, y, z, _numel(shape), float(alpha) if name == "add" else -float(alpha), env.stream())
         return z
     if name == "add" and len(x.shape) == 2 and y.shape == (x.shape[1],):
-        env.lib.add_bias_rows_f32(_ptr(x), _ptr(y), _ptr(z), x.shape[0], x.shape[1], float(alpha), env.stream())
+        env.lib.add_bias_rows_f32(x, y, z, x.shape[0], x.shape[1], float(alpha), env.stream())
         return z
-    env.lib.binary_strided_f32(_OPS[name], len(shape), _ll(shape), _ll(_bstrides(x, shape)), _ll(_bstrides(y, shape)),
-                               _ll(_strides(z)), _ptr(x), _ptr(y), _ptr(z), float(alpha), env.stream())
+    env.lib.binary_strided_f32(_OPS[name], len(shape), shape, _bstrides(x, shape), _bstrides(y, shape),
+                               _strides(z), x, y, z, float(alpha), env.stream())
     return z
 
 
@@ -675,7 +658,7 @@ def _scaled(t, scale):
         return t
     env = _env(t)
     out = _new(t.shape, t)
-    env.lib.scale_f32(_ptr(out), _ptr(t), _numel(t.shape), float(scale), env.stream())
+    env.lib.scale_f32(out, t, _numel(t.shape), float(scale), env.stream())
     return out
 
 
@@ -714,37 +697,46 @@ def cuda_pow(x, y):
     return _binary("pow", x, y)
 
 
+# ``needed``: which of the two gradients the caller will use (the tape has no use for one towards a constant, such as the
+# exponent of ``x ** 2``); the other is then None instead of being computed.
+_BOTH = (True, True)
+
+
 @_reg("cuda", "add_backward")
-def cuda_add_backward(output_grad, x, y, alpha):
+def cuda_add_backward(output_grad, x, y, alpha, needed=_BOTH):
     # Same-shape operands receive the upstream gradient itself (no copy): nothing mutates
     # gradients in place, accumulation always writes a fresh tensor.
-    return _reduce_to(output_grad, x.shape, x), _reduce_to(_scaled(output_grad, alpha), y.shape, y)
+    return (_reduce_to(output_grad, x.shape, x) if needed[0] else None,
+            _reduce_to(_scaled(output_grad, alpha), y.shape, y) if needed[1] else None)
 
 
 @_reg("cuda", "sub_backward")
-def cuda_sub_backward(output_grad, x, y, alpha):
-    return _reduce_to(output_grad, x.shape, x), _reduce_to(_scaled(output_grad, -alpha), y.shape, y)
+def cuda_sub_backward(output_grad, x, y, alpha, needed=_BOTH):
+    return cuda_add_backward(output_grad, x, y, -alpha, needed)
 
 
 @_reg("cuda", "mul_backward")
-def cuda_mul_backward(output_grad, x, y):
-    return _reduce_to(_binary("mul", output_grad, y), x.shape, x), _reduce_to(_binary("mul", output_grad, x), y.shape, y)
+def cuda_mul_backward(output_grad, x, y, needed=_BOTH):
+    return (_reduce_to(_binary("mul", output_grad, y), x.shape, x) if needed[0] else None,
+            _reduce_to(_binary("mul", output_grad, x), y.shape, y) if needed[1] else None)
 
 
 @_reg("cuda", "div_backward")
-def cuda_div_backward(output_grad, x, y):
+def cuda_div_backward(output_grad, x, y, needed=_BOTH):
     """dx = dy / y, dy_ = -x / y^2 * dy (``mytorch/backends/cpu/ops/broadcast_binary_ops.py:108-115``)."""
-    gx = _binary("div", output_grad, y)
-    gy = _scaled(_binary("div", _binary("mul", output_grad, x), _binary("mul", y, y)), -1.0)
-    return _reduce_to(gx, x.shape, x), _reduce_to(gy, y.shape, y)
+    gx = gy = None
+    if needed[0]:
+        gx = _reduce_to(_binary("div", output_grad, y), x.shape, x)
+    if needed[1]:
+        gy = _reduce_to(_scaled(_binary("div", _binary("mul", output_grad, x), _binary("mul", y, y)), -1.0), y.shape, y)
+    return gx, gy
 
 
 @_reg("cuda", "pow_backward")
-def cuda_pow_backward(output_grad, x, y):
+def cuda_pow_backward(output_grad, x, y, needed=_BOTH):
     """dx = y x^(y-1) dy, dy_ = x^y ln(x) dy (``mytorch/backends/cpu/ops/broadcast_binary_ops.py:130-137``)."""
-    gx = _binary("mul", _binary("pow_dx", x, y), output_grad)
-    gy = _binary("mul", _binary("pow_dy", x, y), output_grad)
-    return _reduce_to(gx, x.shape, x), _reduce_to(gy, y.shape, y)
+    return (_reduce_to(_binary("mul", _binary("pow_dx", x, y), output_grad), x.shape, x) if needed[0] else None,
+            _reduce_to(_binary("mul", _binary("pow_dy", x, y), output_grad), y.shape, y) if needed[1] else None)
 
 
 # ---------------------------------------------------------------------------- max / eq / bmm
@@ -774,7 +766,7 @@ def cuda_max(tensor, dim, keepdim):
     n_out = _numel(out_shape)
     values = Tensor(shape=(n_out,), dtype=tensor.dtype, device=tensor.device)
     indices = Tensor(shape=tuple(out_shape), dtype=int64, device=tensor.device)
-    env.lib.max_strided_f32(_ptr(src), _ptr(values), _ptr(indices), len(kept_shape), _ll(kept_shape), _ll(kept_strides), red_len, red_stride,
+    env.lib.max_strided_f32(src, values, indices, len(kept_shape), kept_shape, kept_strides, red_len, red_stride,
                             env.stream())
     return cuda_reshape(values, tuple(out_shape)), indices
 
@@ -789,13 +781,13 @@ def cuda_max_backward(output_grad, indices_tensor, tensor, dim, keepdim):
         g = cuda_reshape(g, (_numel(g.shape),))
     if dim is None:
         flat = Tensor(shape=(_numel(tensor.shape),), dtype=tensor.dtype, device=tensor.device)
-        env.lib.max_backward_f32(_ptr(g), _ptr(indices_tensor), _ptr(flat), _numel(tensor.shape), 0, _ll([]), _ll([]), 1, env.stream())
+        env.lib.max_backward_f32(g, indices_tensor, flat, _numel(tensor.shape), 0, [], [], 1, env.stream())
         return [cuda_reshape(flat, tensor.shape)]
     dim = dim + nd if dim < 0 else dim
     st = _strides(dx)
     kept = [i for i in range(nd) if i != dim]
-    env.lib.max_backward_f32(_ptr(g), _ptr(indices_tensor), _ptr(dx), _numel(tensor.shape), len(kept), _ll([tensor.shape[i] for i in kept]),
-                             _ll([st[i] for i in kept]), st[dim], env.stream())
+    env.lib.max_backward_f32(g, indices_tensor, dx, _numel(tensor.shape), len(kept), [tensor.shape[i] for i in kept],
+                             [st[i] for i in kept], st[dim], env.stream())
     return [dx]
 
 
@@ -810,7 +802,7 @@ def cuda_eq(x, y):
         raise InvalidDataTypeError(x.dtype)
     env = _env(x)
     out = Tensor(shape=x.shape, dtype=int8, device=x.device)
-    env.lib.eq_strided(kinds[x.dtype], len(x.shape), _ll(x.shape), _ll(_strides(x)), _ll(_strides(y)), _ptr(x), _ptr(y), _ptr(out), env.stream())
+    env.lib.eq_strided(kinds[x.dtype], len(x.shape), x.shape, _strides(x), _strides(y), x, y, out, env.stream())
     return out
 
 
@@ -859,22 +851,22 @@ def cuda_sum_scale(x, dim, keepdim, scale):
     st = env.stream()
     if x._nhwc and dim == (2, 3):
         n, c, h, w = x.shape
-        env.lib.nhwc_spatial_sum_f32(_ptr(x), _ptr(out), n, c, h * w, float(scale), st)
+        env.lib.nhwc_spatial_sum_f32(x, out, n, c, h * w, float(scale), st)
         return out
     if x._nhwc and dim == (0, 2, 3):
         n, c, h, w = x.shape
         ws, ws_bytes = env.workspace(env.lib.colsum_workspace_bytes(c))
-        env.lib.colsum_f32(_ptr(x), n * h * w, c, float(scale), _ptr(out), ws, ws_bytes, st)
+        env.lib.colsum_f32(x, n * h * w, c, float(scale), out, ws, ws_bytes, st)
         return out
     xs = _strides(x)
     kept = [i for i in range(len(x.shape)) if i not in dim]
     red = list(dim)
     dense = out if not _nontrivial_nhwc(out) else Tensor(shape=(_numel(out_shape),), dtype=x.dtype, device=x.device)
-    env.lib.sum_strided_f32(_ptr(x), _ptr(dense), len(kept), _ll([x.shape[i] for i in kept]), _ll([xs[i] for i in kept]),
-                            len(red), _ll([x.shape[i] for i in red]), _ll([xs[i] for i in red]), float(scale), st)
+    env.lib.sum_strided_f32(x, dense, len(kept), [x.shape[i] for i in kept], [xs[i] for i in kept],
+                            len(red), [x.shape[i] for i in red], [xs[i] for i in red], float(scale), st)
     if dense is not out:
         n, c, h, w = out_shape
-        env.lib.nchw_to_nhwc_f32(_ptr(dense), _ptr(out), n, c, h, w, st)
+        env.lib.nchw_to_nhwc_f32(dense, out, n, c, h, w, st)
     return out
 
 
@@ -886,7 +878,7 @@ def cuda_sum_scale_backward(output_grad, x, dim, keepdim, scale):
     st = env.stream()
     if x._nhwc and dim == (2, 3):
         n, c, h, w = x.shape
-        env.lib.nhwc_spatial_bcast_f32(_ptr(output_grad), _ptr(dx), n, c, h * w, float(scale), st)
+        env.lib.nhwc_spatial_bcast_f32(output_grad, dx, n, c, h * w, float(scale), st)
         return [dx]
     gs = _strides(output_grad)
     if keepdim:
@@ -894,8 +886,8 @@ def cuda_sum_scale_backward(output_grad, x, dim, keepdim, scale):
     else:
         it = iter(gs)
         src = [0 if i in dim else next(it) for i in range(len(x.shape))]
-    env.lib.binary_strided_f32(5, len(x.shape), _ll(x.shape), _ll(src), _ll(src), _ll(_strides(dx)), _ptr(output_grad), None,
-                               _ptr(dx), float(scale), st)
+    env.lib.binary_strided_f32(5, len(x.shape), x.shape, src, src, _strides(dx), output_grad, None,
+                               dx, float(scale), st)
     return [dx]
 
 
@@ -905,7 +897,7 @@ def _dense_copy(env, t):
     """Logical row-major copy of a channels-last tensor."""
     n, c, h, w = t.shape
     out = CudaMemory(t.device.index, t._native_array.nbytes)
-    env.lib.nhwc_to_nchw_f32(_ptr(t), out, n, c, h, w, env.stream())
+    env.lib.nhwc_to_nchw_f32(t, out, n, c, h, w, env.stream())
     return out
 
 
@@ -933,7 +925,7 @@ def cuda_permute(x, dims):
     out = _new(tuple(x.shape[d] for d in dims), x)
     xs = _strides(x)
     src = [xs[d] for d in dims]
-    env.lib.binary_strided_f32(5, len(dims), _ll(out.shape), _ll(src), _ll(src), _ll(_strides(out)), _ptr(x), None, _ptr(out), 1.0,
+    env.lib.binary_strided_f32(5, len(dims), out.shape, src, src, _strides(out), x, None, out, 1.0,
                                env.stream())
     return out
 
@@ -957,7 +949,7 @@ def cuda_cross_entropy(input, target):
     b, c = input.shape
     loss = _new((1,), input)
     ws, ws_bytes = env.workspace(env.lib.cross_entropy_workspace_bytes(b))
-    env.lib.cross_entropy_forward_f32(b, c, _ptr(input), _ptr(target), _ptr(loss), ws, ws_bytes, env.stream())
+    env.lib.cross_entropy_forward_f32(b, c, input, target, loss, ws, ws_bytes, env.stream())
     return loss
 
 
@@ -966,7 +958,7 @@ def cuda_cross_entropy_backward(output_grad, input, target):
     env = _env(input)
     b, c = input.shape
     dx = _new(input.shape, input)
-    env.lib.cross_entropy_backward_f32(b, c, _ptr(input), _ptr(target), _ptr(output_grad), _ptr(dx), env.stream())
+    env.lib.cross_entropy_backward_f32(b, c, input, target, output_grad, dx, env.stream())
     return [dx]
 
 
@@ -983,7 +975,7 @@ def _refuse_first_step_in_capture(env, is_first_time):
 def cuda_sgd(param, momentum_buffer, is_first_time, lr, weight_decay, momentum, dampening, nesterov, maximize):
     env = _env(param)
     _refuse_first_step_in_capture(env, is_first_time)
-    env.lib.sgd_f32(_ptr(param), _ptr(param.grad), _ptr(momentum_buffer), _numel(param.shape), int(bool(is_first_time)), float(lr),
+    env.lib.sgd_f32(param, param.grad, momentum_buffer, _numel(param.shape), int(bool(is_first_time)), float(lr),
                     float(weight_decay), float(momentum), float(dampening), int(bool(nesterov)), int(bool(maximize)), 1.0, env.stream())
 
 
@@ -994,11 +986,4 @@ def cuda_sgd_multi(entries, lr, weight_decay, momentum, dampening, nesterov, max
         return
     env = _env(entries[0][0])
     _refuse_first_step_in_capture(env, any([f for _, _, f in entries]))
-    # host tables as the C side reads them (the binding passes the arrays' storage)
-    params = array("Q", [p._native_array.ptr for p, _, _ in entries])
-    grads = array("Q", [p.grad._native_array.ptr for p, _, _ in entries])
-    bufs = array("Q", [b._native_array.ptr for _, b, _ in entries])
-    sizes = array("q", [math.prod(p.shape) for p, _, _ in entries])
-    first = array("i", [1 if f else 0 for _, _, f in entries])
-    env.lib.sgd_multi_f32(len(entries), params, grads, bufs, sizes, first, float(lr), float(weight_decay), float(momentum), float(dampening),
-                          int(bool(nesterov)), int(bool(maximize)), float(grad_scale), env.stream())
+    _binding.sgd_step(list(entries), lr, weight_decay, momentum, dampening, bool(nesterov), bool(maximize), grad_scale, env.stream())

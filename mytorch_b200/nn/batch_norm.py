@@ -81,9 +81,11 @@ def inference_conv_norm(conv, norm, x, relu=False, residual=None):
     if not tracker.no_grad and (x.requires_grad or conv.weight.requires_grad or norm.weight is not None and norm.weight.requires_grad
                                 or residual is not None and residual.requires_grad):
         return None
-    channels = (norm.num_features,)
-    tensors = [conv.weight, norm.running_mean, norm.running_var] + [t for t in (conv.bias, norm.weight, norm.bias, residual) if t is not None]
-    if (conv.weight.shape[0],) != channels or any(t.device is not x.device or t.dtype is not x.dtype for t in tensors):
+    weight, device, dtype = conv.weight, x.device, x.dtype
+    ok = weight.shape[0] == norm.num_features
+    for t in (weight, norm.running_mean, norm.running_var, conv.bias, norm.weight, norm.bias, residual):
+        ok = ok and (t is None or (t.device is device and t.dtype is dtype))
+    if not ok:
         return None  # the separate operators say what is wrong
     affine = norm.weight is not None and norm.bias is not None
     return dispatch(x.device, "conv2d_batch_norm")(x, conv.weight, conv.bias, conv.stride, conv.padding, norm.weight if affine else None,

@@ -6,8 +6,10 @@ tracker = DAGTracker.instance()
 
 
 def dispatch(device, name):
-    registry = BackendDispatcher._instance or BackendDispatcher.instance()
-    return registry.dispatch(device.type, name)
+    try:
+        return BackendDispatcher._instance._impls[device.type][name]
+    except (AttributeError, KeyError):  # not loaded yet, or not there: the registry says which
+        return BackendDispatcher.instance().dispatch(device.type, name)
 
 
 def grad_enabled(*tensors):

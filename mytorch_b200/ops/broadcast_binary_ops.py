@@ -34,27 +34,27 @@ def pow(x: Tensor, y: Tensor) -> Tensor:
 
 @tracker.register_backward_function("add")
 def add_backward(output_grad, x, y, alpha):
-    return dispatch(x.device, "add_backward")(output_grad, x, y, alpha)
+    return dispatch(x.device, "add_backward")(output_grad, x, y, alpha, needed=(x.requires_grad, y.requires_grad))
 
 
 @tracker.register_backward_function("sub")
 def sub_backward(output_grad, x, y, alpha):
-    return dispatch(x.device, "sub_backward")(output_grad, x, y, alpha)
+    return dispatch(x.device, "sub_backward")(output_grad, x, y, alpha, needed=(x.requires_grad, y.requires_grad))
 
 
 @tracker.register_backward_function("mul")
 def mul_backward(output_grad, x, y):
-    return dispatch(x.device, "mul_backward")(output_grad, x, y)
+    return dispatch(x.device, "mul_backward")(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
 
 
 @tracker.register_backward_function("div")
 def div_backward(output_grad, x, y):
-    return dispatch(x.device, "div_backward")(output_grad, x, y)
+    return dispatch(x.device, "div_backward")(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
 
 
 @tracker.register_backward_function("pow")
 def pow_backward(output_grad, x, y):
-    return dispatch(x.device, "pow_backward")(output_grad, x, y)
+    return dispatch(x.device, "pow_backward")(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
 
 
 def _copy(x: Tensor, y: Tensor):

@@ -268,7 +268,12 @@ class Tensor:
         if isinstance(other, Tensor):
             return other
         if isinstance(other, numbers.Number):
-            return Tensor(cpu_array=np.array(other, dtype=self.dtype.np_dtype), device=self.device)
+            value = np.array(other, dtype=self.dtype.np_dtype)
+            if self.device.type == "cuda" and self.dtype is float32:  # written by a kernel: an upload waits for the stream
+                scalar = Tensor(shape=(), dtype=float32, device=self.device)
+                scalar.fill_(value.item())
+                return scalar
+            return Tensor(cpu_array=value, device=self.device)
         if isinstance(other, np.ndarray):
             return Tensor(cpu_array=other.astype(self.dtype.np_dtype), device=self.device)
         raise InvalidDataTypeError(type(other))
