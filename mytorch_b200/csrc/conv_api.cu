@@ -10,8 +10,8 @@ MTB_API long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int k
   return a > b ? a : b;
 }
 
-// workspace (may be NULL): scratch of mtb_conv2d_workspace_bytes(); with it, layers whose output has too few
-// tiles to fill the GPU split their reduction across CTAs (partials in the workspace, added in a fixed order).
+// workspace (may be NULL): scratch of mtb_conv2d_workspace_bytes() for the weight gradient; forward and data gradient take it
+// for symmetry (layers whose output has too few tiles split their reduction over clusters, without scratch).
 MTB_API int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                    const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes,
                                    void* stream) {

@@ -144,17 +144,27 @@ struct GemmParams {
   // (count, mean, M2) over the output rows this CTA produced (the grid is a multiple of n_tiles, so a
   // CTA always works on the same column tile)
   float* stats;
-  // Split reduction (splits > 1): unit u = tile * splits + split works on reduction blocks
-  // [split * kb_per_split, ...); every unit writes its raw accumulator to partial[u] and draws a ticket for
-  // its tile; the unit that draws the last ticket adds the partials in split order and finishes the tile.
+  // Split reduction (splits > 1): unit u = tile * splits + split works on reduction blocks [split * kb_per_split, ...).  The
+  // units of a tile form a cluster.  When its accumulators are complete every unit hands each of the others the columns
+  // that one finishes (distributed shared memory), and adds what it received to its own in split order.
   int splits, kb_per_split;
-  float* partial;
 };
 
-// One ticket counter per output tile of a split launch; back to zero when the launch ends.  Launches that
-// split must not overlap on one GPU (they share the counters), which holds for work on one stream.
-constexpr int kMaxSplitTiles = 1024;
-static __device__ unsigned int g_gemm_tickets[kMaxSplitTiles];
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_address(uint32_t smem, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void st_cluster4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
 
 // A stage holds kKB reduction blocks of 32 (each one 128-byte swizzle span per operand row).  One
 // producer/consumer hand-over costs the issuing thread 300-400 cycles that do not overlap with MMA
@@ -177,7 +187,8 @@ enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3 };
 
 constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
 
-template <int BN, int AMODE, int BMODE, int EPI>
+// SPLIT: GemmParams::splits > 1, a kernel of its own because the exchange takes the registers that the other epilogues need.
+template <int BN, int AMODE, int BMODE, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p) {
   using C = Cfg<BN>;
@@ -187,7 +198,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  __shared__ int split_last;
   __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -216,7 +226,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
-  const int S = p.splits;
+  const int S = SPLIT ? p.splits : 1;
   const int tiles = p.m_tiles * p.n_tiles * S;  // work units: (tile, split) pairs, the splits of a tile adjacent
   volatile int* abort_ptr = &abort_flag;
 
@@ -285,6 +295,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         }
       }
     }
+    if constexpr (SPLIT) { cluster_arrive(); cluster_wait(); cluster_arrive(); cluster_wait(); }  // see the epilogue
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     // The whole warp runs the loop converged and one elected lane issues (warp-uniform control
@@ -339,11 +350,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       if (ok && elect_one()) mma_commit(smem_u32(&bar_tfull[buf]));
       __syncwarp();
     }
+    if constexpr (SPLIT) { cluster_arrive(); cluster_wait(); cluster_arrive(); cluster_wait(); }  // see the epilogue
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quarter = warp & 3;
-    constexpr int COLS = BN / 2;                            // columns of the tile this warp handles, from c_first on
-    const int c_first = warp < 6 ? 0 : COLS;
+    // columns of the tile this warp finishes: half of the tile, from c_first on, or its share of the columns of its unit
+    constexpr int COLS = BN / 2;
+    const int rank = SPLIT ? (int)(blockIdx.x % S) : 0, width = BN / S;
+    const int c_first = !SPLIT ? (warp < 6 ? 0 : COLS) : rank * width + (width >= 64 && warp >= 6 ? width / 2 : 0);
+    const int split_chunks = width >= 64 ? width / 64 : (warp < 6 ? 1 : 0);
     int t = 0;
     const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0);
     const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 31u) == 0);  // 32-byte stores
@@ -365,7 +380,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         return ok;
       };
       if constexpr (!ADD) {
-        if (!wait_for_accumulator()) break;
+        if (!SPLIT && !wait_for_accumulator()) break;
       }
       const int row = m0 + quarter * 32 + lane;
       long long orow_index = row;
@@ -391,7 +406,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       float4 add[8];
       if constexpr (ADD) {
         fetch_addend(0, add);
-        if (!wait_for_accumulator()) break;
+        if (!SPLIT && !wait_for_accumulator()) break;
       }
       auto finish = [&](int c0, const uint32_t (&r)[32]) {
         const int col0 = n0 + c_first + c0;
@@ -467,7 +482,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         if constexpr (LANE_SUMS) sums.cnt += valid ? 1.f : 0.f;
         else if constexpr (STATS) stats.n += cnt;
       };
-      if (S == 1) {
+      if constexpr (!SPLIT) {
         if constexpr (STATS) {
 #pragma unroll
           for (int c0 = 0; c0 < COLS; c0 += 32) {
@@ -496,71 +511,67 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         }
         count_rows();
         release_accumulator();
-        continue;
-      }
-      // Split reduction.  partial[unit][chunk][quarter][j][lane]: a warp stores 128 contiguous bytes per column.
-      constexpr int kChunks = BN / 32, kMine = COLS / 32;
-      float* part = p.partial + (((long long)unit * kChunks + c_first / 32) * 4 + quarter) * 1024 + lane;
-#pragma unroll 1
-      for (int c = 0; c < kMine; ++c) {
+      } else {
+      // Split reduction (one unit per CTA).  The stages are free when every unit of the cluster has its accumulator; received
+      // columns lie there as [sender][column / 4][row] float4, so that a warp writes and reads 512 contiguous bytes.  The
+      // exchange takes 1.1 to 2 us (64 to 256 columns); through bulk copies instead of stores it took the same.
+      const bool complete = wait_for_accumulator();  // a unit that gave up still takes part in the barriers
+      cluster_arrive();
+      cluster_wait();
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
+      const uint32_t row16 = (uint32_t)(quarter * 32 + lane) * 16u;
+#pragma unroll 2
+      for (int c0 = warp < 6 ? 0 : 32; c0 < BN; c0 += 64) {  // the two warps of a row quarter take turns: equal shares for every rank
+        const int owner = c0 / width;
+        if (owner == rank) continue;
         uint32_t r[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c * 32), r);
+        tmem_ld_32x32(taddr + (uint32_t)c0, r);
         tmem_ld_wait();
+        const uint32_t slot = (uint32_t)((rank < owner ? rank : rank - 1) * (width / 4) + (c0 - owner * width) / 4);
+        const uint32_t dst = cluster_address(smem_base + slot * 2048u + row16, (uint32_t)owner);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) part[c * 4096 + j * 32] = __uint_as_float(r[j]);
+        for (int j = 0; j < 32; j += 4) st_cluster4(dst + (uint32_t)(j / 4) * 2048u, r[j], r[j + 1], r[j + 2], r[j + 3]);
       }
-      release_accumulator();
-      __threadfence();
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
-      if (threadIdx.x == 64) {
-        const unsigned int ticket = atomicAdd(&g_gemm_tickets[tile], 1u);
-        split_last = (ticket == (unsigned int)S - 1u);
-        if (split_last) g_gemm_tickets[tile] = 0u;  // every unit of the tile has drawn: ready for the next launch
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
-      if (!split_last) continue;
-      __threadfence();
-      const float* first = p.partial + (((long long)tile * S * kChunks + c_first / 32) * 4 + quarter) * 1024 + lane;
+      cluster_arrive();
+      cluster_wait();
       auto reduce_chunk = [&](int c, uint32_t (&r)[32]) {
+        tmem_ld_32x32(taddr + (uint32_t)(c_first + c * 32), r);
+        tmem_ld_wait();
+        const uint32_t src = smem_base + (uint32_t)((c_first - rank * width) / 4 + c * 8) * 2048u + row16;
         float acc[32];
+        for (int sp = 0; sp < S; ++sp) {  // fixed order: split 0, 1, 2, ...
+          const uint32_t q = src + (uint32_t)((sp < rank ? sp : sp - 1) * (width / 4)) * 2048u;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = __ldcg(first + c * 4096 + j * 32);
-        for (int sp = 1; sp < S; ++sp) {  // fixed order: split 0, 1, 2, ...
-          const float* q = first + (long long)sp * kChunks * 4096 + c * 4096;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) acc[j] += __ldcg(q + j * 32);
+          for (int j = 0; j < 32; j += 4) {
+            const float4 v = sp == rank ? make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]))
+                                        : ld_shared4(q + (uint32_t)(j / 4) * 2048u);
+            if (sp == 0) { acc[j] = v.x; acc[j + 1] = v.y; acc[j + 2] = v.z; acc[j + 3] = v.w; }
+            else { acc[j] += v.x; acc[j + 1] += v.y; acc[j + 2] += v.z; acc[j + 3] += v.w; }
+          }
         }
 #pragma unroll
         for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(acc[j]);
       };
-      if constexpr (STATS) {
-#pragma unroll
-        for (int c = 0; c < kMine; ++c) {
-          uint32_t r[32];
-          reduce_chunk(c, r);
-          finish(c * 32, r);
+#pragma unroll (STATS ? COLS / 32 : 1)
+      for (int c = 0; c < COLS / 32; ++c) {
+        if (c >= split_chunks || !complete) break;
+        uint32_t r[32];
+        if constexpr (ADD) {
+          if (c > 0) fetch_addend(c * 32, add);
         }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < kMine; ++c) {
-          uint32_t r[32];
-          if constexpr (ADD) {
-            if (c > 0) fetch_addend(c * 32, add);
-          }
-          reduce_chunk(c, r);
-          finish(c * 32, r);
-        }
+        reduce_chunk(c, r);
+        finish(c * 32, r);
       }
       count_rows();
       if constexpr (STATS) {
-        // which unit of a tile comes last differs from run to run, so the statistics of a split tile go to
-        // a row chosen by the tile, not by the CTA: results stay bit-reproducible
         float* row = p.stats + ((long long)(tile / p.n_tiles) * 4 + quarter) * 3 * p.N;
-        if constexpr (LANE_SUMS) { sums.store(row, p.N, n0 + c_first, p.N, p.bias, lane); sums.reset(); }
-        else { stats.store(row, p.N, n0 + c_first, p.N, lane); stats.reset(); }
+        const int end = n0 + c_first + 32 * split_chunks < p.N ? n0 + c_first + 32 * split_chunks : p.N;
+        if constexpr (LANE_SUMS) sums.store(row, p.N, n0 + c_first, end, p.bias, lane);
+        else stats.store(row, p.N, n0 + c_first, end, lane);
+      }
       }
     }
-    if (STATS && S == 1) {
+    if constexpr (STATS && !SPLIT) {
       float* row = p.stats + ((long long)(blockIdx.x / p.n_tiles) * 4 + quarter) * 3 * p.N;
       if constexpr (LANE_SUMS) sums.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, p.bias, lane);
       else if constexpr (STATS) stats.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, lane);
@@ -584,12 +595,36 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 template <int BN, int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
   using C = Cfg<BN>;
-  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI>;
+  int tiles = p.m_tiles * p.n_tiles;
+  if (p.splits > 1) {  // one unit per CTA, the units of a tile a cluster
+    if constexpr (AMODE == A_IM2COL) {
+      auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, true>;
+      static unsigned long long configured = 0;
+      if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(tiles * p.splits);
+      cfg.blockDim = dim3(kGemmThreads);
+      cfg.dynamicSmemBytes = C::kSmemBytes;
+      cfg.stream = st;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)p.splits;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 2;
+      MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, p));
+      MTB_LAUNCH_CHECK("tc_gemm_kernel");
+      return MTB_OK;
+    }
+    return mtb_fail(MTB_ERR_INVALID, "tc_gemm: only convolutions split the reduction");
+  }
+  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, false>;
   static unsigned long long configured = 0;
   if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
-  int tiles = p.m_tiles * p.n_tiles * p.splits;  // work units
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
-  if ((EPI == EPI_STATS || EPI == EPI_BN) && p.splits == 1) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
+  if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
   MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), C::kSmemBytes, st, mapA, mapB, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
@@ -621,13 +656,16 @@ int pick_bn_for(int n, long long rows) {
   return bn;
 }
 
+// One reduction block of 32 of a tile of 128 rows, in ns (see im2col_ns).
+double kb_ns(int bn, bool mn_major) { return mn_major ? (bn == 64 ? 285 : bn == 128 ? 295 : 405) : (bn == 64 ? 232 : bn == 128 ? 262 : 376); }
+
 // What a launch of the im2col kernel without split takes, in ns: waves x (reduction blocks x the time of one block + about
 // 900 ns for filling the pipeline and the first stores).  The block times were measured (weights K-major in forward,
 // MN-major in the data gradient; 72 blocks on 64 to 592 images of 8x8): a 64-wide tile is bound by the gather of 128
 // pixel rows, a 256-wide one by the MMAs.  `copies` launches of this size share the GPU.
 double im2col_ns(int bn, int n, long long rows, int num_kb, bool mn_major, int copies = 1) {
   const long long tiles = ((rows + 127) / 128) * ((n + bn - 1) / bn) * copies, waves = (tiles + mtb_sm_count() - 1) / mtb_sm_count();
-  const double block = mn_major ? (bn == 64 ? 285 : bn == 128 ? 295 : 405) : (bn == 64 ? 232 : bn == 128 ? 262 : 376);
+  const double block = kb_ns(bn, mn_major);
   const double store = 8.0 * bn;  // a tile's epilogue: longer than the main loop of a short reduction
   return waves * ((num_kb * block > store ? num_kb * block : store) + 900.0) + store;
 }
@@ -641,46 +679,57 @@ int cheapest_bn(int n, long long rows, int num_kb, bool mn_major, int copies = 1
   return best;
 }
 
-// Tile width and reduction split for the im2col / GEMM kernel.  These kernels are bound by what one SM
-// can pull from L2 into shared memory (about 89 GB/s: 47 B per cycle), then by the MMA rate, so a launch
-// is priced as waves x reduction blocks per unit x the slower of (bytes of one block of A and B at that
-// rate, four MMAs), plus, for a split reduction, the last unit's pass over the partials.  The cheapest
-// (tile width, splits) wins; a split is only considered when all its units fit the GPU at once
-// (tiles x splits <= SMs) and every unit keeps at least eight reduction blocks.
-struct GemmPlan { int bn, splits, kb_per_split; };
-
-GemmPlan plan_gemm(int n, long long rows, int num_kb, bool may_split, bool mn_major, int force_bn = 0, int copies = 1) {
-  const int sms = mtb_sm_count();
-  const long long m_tiles = (rows + 127) / 128;
-  static const int kSplits[] = {1, 2, 3, 4, 6, 8};
-  GemmPlan best{force_bn ? force_bn : cheapest_bn(n, rows, num_kb, mn_major, copies), 1, num_kb};
-  // Measured: the split only pays when even 64-wide tiles leave half the GPU idle (the 4x4 layers at 64
-  // images: 41 -> 24 us for the data gradient of 512 -> 512); with more tiles than that the last unit's pass
-  // over the partials costs more than the idle SMs did (256 -> 256 on 8x8 at 64 images: 20 -> 40 us).
-  if (m_tiles * ((n + 63) / 64) > sms / 2 || num_kb < 64) may_split = false;  // short reductions gain nothing either
-  if (!may_split || getenv("MTB_DISABLE_SPLITK")) return best;
-  double best_ns = 1e30;
-  for (int bn = force_bn ? force_bn : pick_bn(n); bn >= (force_bn ? force_bn : 64); bn >>= 1) {
-    const long long tiles = m_tiles * ((n + bn - 1) / bn);
-    for (int want : kSplits) {
-      if (want > 1 && (tiles * want > sms || num_kb / want < 8 || tiles > kMaxSplitTiles)) continue;
-      const int per = (num_kb + want - 1) / want;
-      const int splits = (num_kb + per - 1) / per;
-      const long long waves = (tiles * splits + sms - 1) / sms;
-      const double load_ns = (16384.0 + bn * 128.0) / 89.0;
-      const double mma_ns = 4.0 * (bn == 64 ? 48.0 : bn == 128 ? 64.0 : 128.0) / 1.9;
-      double ns = (double)waves * per * (load_ns > mma_ns ? load_ns : mma_ns) + 2000.0;
-      if (splits > 1) ns += splits * 128.0 * bn * 4.0 / 150.0 + 1500.0;
-      if (ns < best_ns) { best_ns = ns; best = GemmPlan{bn, splits, per}; }
+// CTAs of the widest kernel that the GPU holds at once in clusters of `size` (clusters do not span the GPU's partitions, so
+// a few SMs stay without).
+int cluster_units(int size) {
+  static int units[9] = {};
+  if (!units[size]) {
+    const int sms = mtb_sm_count();
+    auto kernel = tc_gemm_kernel<256, A_IM2COL, B_KMAJOR, EPI_PLAIN, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sms / size * size);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = Cfg<256>::kSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<256>::kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+      (void)cudaGetLastError();  // no GPU (plans are also made without one)
+      clusters = sms * 7 / 8 / size;
     }
+    units[size] = clusters * size;
   }
-  return best;
+  return units[size];
 }
 
-long long split_partial_bytes(const GemmPlan& g, long long rows, int n) {
-  if (g.splits <= 1) return 0;
-  const long long tiles = ((rows + 127) / 128) * ((n + g.bn - 1) / g.bn);
-  return tiles * g.splits * 128LL * g.bn * 4;
+// Tile width and reduction split of the im2col kernel.  A layer with few pixels leaves most of the GPU idle on wide tiles and
+// spends its time on loading the pixels again for every narrow one (a block of 32 takes 64 columns 175 ns, 256 columns 280),
+// so its long reduction is split over a cluster of 2, 4 or 8 CTAs on wide tiles, one unit per CTA, as long as all units fit
+// the GPU at once.  Times of a split launch as measured (512 -> 512 channels on 4x4, 16 to 128 images): base (launch, pipeline
+// fill, exchange, epilogue) + blocks per unit x block time.  128 images, before -> now: forward 31 -> 22 us, data gradient
+// 38.5 -> 23.5 us; 64 images (before: partial sums through global memory) 19.0 -> 15 and 21.4 -> 16.5 us; 256 -> 256 on 8x8,
+// 64 images: 18.8 -> 14.5 and 22.6 -> 16 us.  Under 64 blocks the exchange costs what the split gains.
+// `copies` launches of this size share the GPU, of which this one may split.
+struct GemmPlan { int bn, splits, kb_per_split; double ns; };
+
+GemmPlan plan_gemm(int n, long long rows, int num_kb, bool mn_major, int force_bn = 0, int copies = 1) {
+  const long long m_tiles = (rows + 127) / 128;
+  GemmPlan best{force_bn ? force_bn : cheapest_bn(n, rows, num_kb, mn_major, copies), 1, num_kb, 0.0};
+  best.ns = im2col_ns(best.bn, n, rows, num_kb, mn_major, copies);
+  if (num_kb < 64 || getenv("MTB_DISABLE_SPLITK")) return best;
+  for (int bn = force_bn ? force_bn : pick_bn(n); bn >= (force_bn ? force_bn : 64); bn >>= 1)
+    for (int s = 2; s <= 8 && bn / s >= 32; s *= 2) {
+      if (m_tiles * ((n + bn - 1) / bn) * (s + copies - 1) > cluster_units(s)) continue;
+      const int per = (num_kb + s - 1) / s;
+      const double ns = (bn == 64 ? 6500 : bn == 128 ? 7700 : 10500) + (double)per * ((bn == 64 ? 180 : bn == 128 ? 200 : 280) + (mn_major ? 40 : 0));
+      if (ns < best.ns) best = GemmPlan{bn, s, per, ns};
+    }
+  return best;
 }
 
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -806,9 +855,8 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   const long long M = (long long)n * oh * ow, K = (long long)kh * kw * cin;
   const int row_bn = pick_bn_for(cout, M);
   const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, row_bn, bn_eval ? 12u * row_bn : 0u);
-  GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), !plan.ok && workspace != nullptr, false);
-  if (split_partial_bytes(gp, M, cout) > workspace_bytes) gp = GemmPlan{cheapest_bn(cout, M, (int)(K / 32), false), 1, (int)(K / 32)};
-  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), im2col_ns(gp.bn, cout, M, (int)(K / 32), false));
+  const GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), false);
+  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), gp.ns);
   const int bn = staged ? row_bn : gp.bn;
   if (stats_rows) *stats_rows = 0;
   const bool want_stats = stats && stats_rows && !relu && cout % 32 == 0 && (!bias || al16(bias)) && !getenv("MTB_DISABLE_CONV_STATS");
@@ -827,7 +875,7 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   p.m_tiles = (int)((M + 127) / 128); p.n_tiles = (cout + bn - 1) / bn;
   p.out = y; p.ldo = cout; p.bias = bias; p.relu = relu;
   p.OW = ow; p.OH = oh; p.SW = sw; p.SH = sh; p.PW = pw; p.PH = ph; p.KW = kw; p.KH = kh; p.cchunks = cin / 32;
-  p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
+  p.splits = gp.splits; p.kb_per_split = gp.kb_per_split;
   // short reductions (1x1 shortcuts) leave the epilogue no main loop to hide the statistics behind
   // ... unless the output is small: then BatchNorm's own pass is all launch latency, and the epilogue is cheaper
   // (measured on the three 1x1 shortcuts of ResNet-18: 1.782 -> 1.770 ms per step at 64 images, but
@@ -879,9 +927,9 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   const int class_kb = ((kh + sh - 1) / sh) * ((kw + sw - 1) / sw) * (cout / 32);
   const int row_bn = pick_bn_for(cin, class_rows);
   const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin, row_bn);
-  const int gemm_bn = plan_gemm(cin, class_rows, class_kb, workspace != nullptr, true, 0, sh * sw).bn;
-  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb, im2col_ns(gemm_bn, cin, class_rows, class_kb, true));
-  const int bn = staged ? row_bn : gemm_bn;
+  const GemmPlan class_plan = plan_gemm(cin, class_rows, class_kb, true, 0, sh * sw);
+  const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb, class_plan.ns);
+  const int bn = staged ? row_bn : class_plan.bn;
   cudaStream_t st = (cudaStream_t)stream;
   CUtensorMap mapB;
   const long long wcols = (long long)kh * kw * cin;
@@ -921,7 +969,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   const bool fused_add = addend != nullptr && !in_place && al16(addend) && kh * kw == 1 && sh * sw == 1;
   if (need_zero && !in_place) MTB_CUDA(cudaMemsetAsync(dx, 0, (size_t)n * h * w * cin * 4, st));
   // The classes write disjoint pixels.  When one class fills only part of the GPU they run side by side on
-  // separate lanes (then without split reductions, whose tickets and partials one launch at a time owns).
+  // separate lanes.
   int live = 0;
   for (int a = 0; a < sh; ++a)
     for (int b = 0; b < sw; ++b) {
@@ -946,9 +994,8 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
       GemmParams p{};
       const long long M = (long long)n * ah.count * aw.count;
       p.M = (int)M; p.N = cin; p.num_kb = ah.taps * aw.taps * (cout / 32);
-      GemmPlan gp = plan_gemm(cin, M, p.num_kb, workspace != nullptr && lanes == 1, true, bn);
-      if (split_partial_bytes(gp, M, cin) > workspace_bytes) gp = GemmPlan{bn, 1, p.num_kb};
-      p.splits = gp.splits; p.kb_per_split = gp.kb_per_split; p.partial = (float*)workspace;
+      const GemmPlan gp = plan_gemm(cin, M, p.num_kb, true, bn, lanes);
+      p.splits = gp.splits; p.kb_per_split = gp.kb_per_split;
       p.m_tiles = (int)((M + 127) / 128); p.n_tiles = (cin + bn - 1) / bn;
       p.out = dx; p.ldo = cin; p.bias = nullptr; p.relu = 0;
       p.addend = in_place || fused_add ? addend : nullptr;
@@ -1342,9 +1389,6 @@ long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, in
   if (cin % 32) return 0;
   WgradPlan q = wgrad_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   long long bytes = (long long)q.splits * q.Kw * cout * 4 + 256;
-  // forward / data gradient with a split reduction: at most one unit per SM, each a 128 x 256 fp32 partial
-  const long long split_bytes = (long long)mtb_sm_count() * 128 * 256 * 4;
-  if (split_bytes > bytes) bytes = split_bytes;
   const WgradRowsPlan rq = wgrad_rows_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (rq.ok) {
     const long long b2 = (long long)rq.splits * q.Kw * cout * 4 + 256;
