@@ -195,6 +195,9 @@ def _take_channels(env, t, channels, like, out=None):
     return out
 
 
+_BIAS_BESIDE_BYTES = 16 << 20
+
+
 def _conv_operands(env, input, weight, stride, padding):
     """(arguments, input, filter, output tensor) of a forward convolution, the operands in the form its kernel reads."""
     x, wt = input, weight
@@ -270,6 +273,13 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
     st = env.stream()
     need = env.lib.conv2d_workspace_bytes(*a)
     dx = dw = db = None
+    # The bias gradient reads all of dY and needs little else of an SM, so it goes beside the tensor-core kernels of this call on
+    # the side stream, if dY is large enough for the two events to pay (64 channels, 128 images of 56x56, forward and
+    # backward: 277 -> 261 us).  A deferred weight gradient has the side stream already, and the longer of the two queues.
+    want_db = bias is not None and bias.requires_grad
+    beside = want_db and want_dx and not defer_weight_gradient and output_grad._native_array.nbytes >= _BIAS_BESIDE_BYTES
+    if beside:
+        side = env.fork_side((output_grad,))
     if want_dx:
         ws, ws_bytes = env.workspace(need)
         if accumulate_dx is not None and not padded and env.lib.conv2d_dgrad_accumulates_in_place(
@@ -288,6 +298,8 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
                 dx = _take_channels(env, dx, cin, dx)
             if accumulate_dx is not None:
                 dx = BackendDispatcher.instance().dispatch("cuda", "add")(dx, accumulate_dx, 1)
+    if beside:
+        db = _bias_gradient(env, output_grad, a[-1], bias, side, env.side_workspace)
     if want_dw:
         # Nothing in the rest of backward reads this layer's weight gradient, so it runs on the side
         # stream, beside the data-gradient / BatchNorm chain that the next layer waits for, and is
@@ -320,9 +332,18 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         else:
             dw = _grad_buffer(weight)
             env.lib.conv2d_wgrad_f32(*a, x, output_grad, dw, wws, wws_bytes, wst)
-    if bias is not None and bias.requires_grad:
-        db = _colsum(env, output_grad, _numel(output_grad.shape) // a[-1], a[-1], bias, out=_grad_buffer(bias))
+    if want_db and db is None:
+        db = _bias_gradient(env, output_grad, a[-1], bias, st, env.workspace)
+    if beside:
+        env.join_side()
     return [dx, dw, db]
+
+
+def _bias_gradient(env, output_grad, channels, bias, stream, workspace):
+    out = _grad_buffer(bias)
+    ws, ws_bytes = workspace(env.lib.colsum_workspace_bytes(channels))
+    env.lib.colsum_f32(output_grad, _numel(output_grad.shape) // channels, channels, 1.0, out, ws, ws_bytes, stream)
+    return out
 
 
 def _colsum(env, mat, rows, cols, like, scale=1.0, out=None):
