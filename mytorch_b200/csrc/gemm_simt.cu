@@ -18,18 +18,19 @@ int dense(int m, int n, int k, const float* a, int trans_a, const float* b, int 
 }
 
 // C[M,N] = A^T B for A stored [K][M] with M <= 16 and B [K][N]: the weight gradient of a Linear layer with few outputs
-// (dW[10][512] = dY^T X).  A CTA owns 32 columns and four rows; its 8 warps take every eighth k, in order, and the 8 partial
-// sums are added in warp order.  Bound by the latency of the loads along k, so sixteen steps of them are issued ahead
-// of the FMAs, and rows are spread over CTAs: K = 512, 10 x 512: 32 -> 7 us.
+// (dW[10][512] = dY^T X).  A CTA owns 32 columns and two rows; its 8 warps take every eighth k, in order, and the 8 partial
+// sums are added in warp order.  Bound by the latency of the loads along k, so 32 steps of them are issued ahead of the
+// FMAs, and rows are spread over CTAs (one row alone took 27 us, the compiler then issues no loads ahead): with two rows and
+// 32 steps instead of four and 16, 10 x 512, K = 512: 10.2 -> 4.1 us; 1 x 500, K = 1000: 18.7 -> 6.1; 1 x 500, K = 8000: 137 -> 35.
 __global__ void __launch_bounds__(256) gemm_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c,
                                                              int M, int N, int K) {
   mtb_launch_dependents();
   mtb_wait_prior();
-  constexpr int R = 4, AHEAD = 16;
+  constexpr int R = 2, AHEAD = 32;
   __shared__ float part[8][R][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 32 + lane, m0 = blockIdx.y * R;
-  float acc[R] = {0.f, 0.f, 0.f, 0.f};
+  float acc[R] = {};
   if (col < N) {
     for (int k0 = warp; k0 < K; k0 += 8 * AHEAD) {
       float bv[AHEAD], av[AHEAD][R];
@@ -67,7 +68,7 @@ MTB_API int mtb_gemm_simt_f32(int m, int n, int k, const float* a, int trans_a, 
                               float* c, void* stream) {
   MTB_REQUIRE(a && b && c && m > 0 && n > 0 && k > 0, "gemm: bad arguments");
   if (trans_a && !trans_b && m <= 16 && !bias && !relu) {
-    MTB_LAUNCH(gemm_few_rows_kernel, dim3(mtb_div_up(n, 32), mtb_div_up(m, 4)), 256, 0, (cudaStream_t)stream, a, b, c, m, n, k);
+    MTB_LAUNCH(gemm_few_rows_kernel, dim3(mtb_div_up(n, 32), mtb_div_up(m, 2)), 256, 0, (cudaStream_t)stream, a, b, c, m, n, k);
     MTB_LAUNCH_CHECK("gemm_few_rows_kernel");
     return MTB_OK;
   }
