@@ -170,11 +170,16 @@ __device__ __forceinline__ float4 ld_shared4(uint32_t a) {
 // producer/consumer hand-over costs the issuing thread 300-400 cycles that do not overlap with MMA
 // work, and four MMAs of a narrow tile are only 192-256 cycles of work, so tiles up to 128 wide
 // take two blocks (8 MMAs) per stage.
+//
+// 32-wide tiles are for matrices of at most 64 rows and a long reduction (the classifier of a small network): their time is what
+// one SM loads, so A comes in boxes of 64 rows (the MMA's rows 64 to 127 read what lies behind them and are never stored) and a
+// stage takes four blocks.  64 x 128, K = 9216: 53 -> 40 us, the same bits.
 template <int BN>
 struct Cfg {
-  static constexpr int kKB = BN <= 128 ? 2 : 1;
+  static constexpr int kKB = BN == 32 ? 4 : BN <= 128 ? 2 : 1;
   static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 3 : 4);
-  static constexpr uint32_t kABytes = 128 * 32 * 4;   // one reduction block of A
+  static constexpr int kRowsA = BN == 32 ? 64 : 128;
+  static constexpr uint32_t kABytes = kRowsA * 32 * 4;   // one reduction block of A
   static constexpr uint32_t kBBytes = BN * 32 * 4;    // one reduction block of B
   static constexpr uint32_t kStageBytes = kKB * (kABytes + kBBytes);  // [A blocks][B blocks]
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 1024;  // + alignment slack
@@ -328,18 +333,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_lo = a_lo0 + stage * (C::kStageBytes >> 4), b_lo = b_lo0 + stage * (C::kStageBytes >> 4);
-        const bool second = C::kKB == 2 && kb + 1 < kb1;
         if (elect_one()) {
-          mma_tf32_words(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, acc);
-          mma_tf32_words(d_tmem, a_lo + a_step, a_hi, b_lo + b_step, b_hi, idesc, 1u);
-          mma_tf32_words(d_tmem, a_lo + 2 * a_step, a_hi, b_lo + 2 * b_step, b_hi, idesc, 1u);
-          mma_tf32_words(d_tmem, a_lo + 3 * a_step, a_hi, b_lo + 3 * b_step, b_hi, idesc, 1u);
-          if (second) {
-            constexpr uint32_t a2 = C::kABytes >> 4, b2 = C::kBBytes >> 4;
-            mma_tf32_words(d_tmem, a_lo + a2, a_hi, b_lo + b2, b_hi, idesc, 1u);
-            mma_tf32_words(d_tmem, a_lo + a2 + a_step, a_hi, b_lo + b2 + b_step, b_hi, idesc, 1u);
-            mma_tf32_words(d_tmem, a_lo + a2 + 2 * a_step, a_hi, b_lo + b2 + 2 * b_step, b_hi, idesc, 1u);
-            mma_tf32_words(d_tmem, a_lo + a2 + 3 * a_step, a_hi, b_lo + b2 + 3 * b_step, b_hi, idesc, 1u);
+#pragma unroll
+          for (int h = 0; h < C::kKB; ++h) {
+            if (h > 0 && kb + h >= kb1) break;
+            const uint32_t a = a_lo + h * (C::kABytes >> 4), b = b_lo + h * (C::kBBytes >> 4);
+            mma_tf32_words(d_tmem, a, a_hi, b, b_hi, idesc, h == 0 ? acc : 1u);
+            mma_tf32_words(d_tmem, a + a_step, a_hi, b + b_step, b_hi, idesc, 1u);
+            mma_tf32_words(d_tmem, a + 2 * a_step, a_hi, b + 2 * b_step, b_hi, idesc, 1u);
+            mma_tf32_words(d_tmem, a + 3 * a_step, a_hi, b + 3 * b_step, b_hi, idesc, 1u);
           }
           mma_commit(smem_u32(&bar_empty[stage]));
         }
@@ -355,7 +357,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quarter = warp & 3;
     // columns of the tile this warp finishes: half of the tile, from c_first on, or its share of the columns of its unit
-    constexpr int COLS = BN / 2;
+    constexpr int COLS = BN >= 64 ? BN / 2 : BN;
+    const int cols_here = BN < 64 && warp >= 6 ? 0 : COLS;  // a tile of 32 columns has work for four of the warps
     const int rank = SPLIT ? (int)(blockIdx.x % S) : 0, width = BN / S;
     const int c_first = !SPLIT ? (warp < 6 ? 0 : COLS) : rank * width + (width >= 64 && warp >= 6 ? width / 2 : 0);
     const int split_chunks = width >= 64 ? width / 64 : (warp < 6 ? 1 : 0);
@@ -493,7 +496,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
           }
         } else {
 #pragma unroll 1
-          for (int c0 = 0; c0 < COLS; c0 += 32) {
+          for (int c0 = 0; c0 < cols_here; c0 += 32) {
             uint32_t r[32];
             tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
             if constexpr (ADD) {
@@ -638,6 +641,8 @@ int stats_rows_for(int tiles, int n_tiles) {
 
 template <int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc_bn(int bn, const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
+  if constexpr (AMODE == A_KMAJOR && BMODE == B_KMAJOR && EPI == EPI_PLAIN)
+    if (bn == 32) return launch_tc<32, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   if (bn == 64) return launch_tc<64, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   if (bn == 128) return launch_tc<128, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   return launch_tc<256, AMODE, BMODE, EPI>(mapA, mapB, p, st);
@@ -810,12 +815,13 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                     void* stream) {
   CUtensorMap mapA, mapB;
-  const int bn = cheapest_bn(n, m, (k + 31) / 32, !trans_b);
+  const bool narrow = m <= 64 && !trans_a && trans_b && n <= 32 * mtb_sm_count();  // see Cfg
+  const int bn = narrow ? 32 : cheapest_bn(n, m, (k + 31) / 32, !trans_b);
   int rc;
   GemmParams p{};
   p.a_blocks = trans_a && m % 32 == 0;
   p.b_blocks = !trans_b && n % 32 == 0;
-  if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, 128);
+  if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, narrow ? 64 : 128);
   else if (p.a_blocks) rc = tc::encode_blocks_3d(&mapA, a, k, m, m, 32, 4);
   else rc = tc::encode_tiled_2d(&mapA, a, k, m, m, 32, 32, true);
   if (rc) return rc;
