@@ -114,6 +114,11 @@ __global__ void __launch_bounds__(1024) bn_stats_final_kernel(const float* __res
   const int cx = threadIdx.x & 7, g = threadIdx.x >> 3;
   const int c = blockIdx.x * 8 + cx;
   float n = 0.f, mean = 0.f, m2 = 0.f;
+  // what the last step needs is on its way beside the partials: one round trip less in a kernel that is
+  // all round trips (and in the backward's; ResNet-18 step captured at 64 images 1379 -> 1344 us, at batch 128 2026 -> 1994)
+  const bool last = g == 0 && c < C;
+  const float gam = last && gamma ? gamma[c] : 1.f;
+  const float rm = last && running_mean ? running_mean[c] : 0.f, rv = last && running_var ? running_var[c] : 0.f;
   if (c < C) {
     for (int p0 = g; p0 < P; p0 += G * B) {
       float v[B][3];
@@ -146,9 +151,9 @@ __global__ void __launch_bounds__(1024) bn_stats_final_kernel(const float* __res
   mean_out[c] = mu;
   var_out[c] = var;
   float rstd = 1.0f / sqrtf(var + eps);
-  scale_out[c] = gamma ? gamma[c] * rstd : rstd;
-  if (running_mean) running_mean[c] = __fadd_rn(__fmul_rn(one_minus_m, running_mean[c]), __fmul_rn(m, mu));
-  if (running_var) running_var[c] = __fadd_rn(__fmul_rn(one_minus_m, running_var[c]), __fmul_rn(m, var));
+  scale_out[c] = gamma ? gam * rstd : rstd;
+  if (running_mean) running_mean[c] = __fadd_rn(__fmul_rn(one_minus_m, rm), __fmul_rn(m, mu));
+  if (running_var) running_var[c] = __fadd_rn(__fmul_rn(one_minus_m, rv), __fmul_rn(m, var));
 }
 
 // Inference mode: statistics are the running ones.
@@ -308,6 +313,8 @@ __global__ void __launch_bounds__(1024) bn_bwd_final_kernel(const float* __restr
   const int cx = threadIdx.x & 7, g = threadIdx.x >> 3;
   const int c = blockIdx.x * 8 + cx;
   float s0 = 0.f, s1 = 0.f;
+  const bool last = g == 0 && c < C;
+  const float gm = last && gamma ? gamma[c] : 1.f, variance = last ? var[c] : 1.f;
   if (c < C) {
     for (int p0 = g; p0 < P; p0 += G * B) {
       float v[B][2];
@@ -336,8 +343,7 @@ __global__ void __launch_bounds__(1024) bn_bwd_final_kernel(const float* __restr
   float db = s0, dg = s1;
   if (dbeta) dbeta[c] = db;
   if (dgamma) dgamma[c] = dg;
-  float rstd = 1.0f / sqrtf(var[c] + eps);
-  float gm = gamma ? gamma[c] : 1.f;
+  float rstd = 1.0f / sqrtf(variance + eps);
   coef[c] = gm * rstd;               // k1
   coef[C + c] = db * inv_m;          // k2
   coef[2 * C + c] = rstd * dg * inv_m;  // k3: (x - mean) * k3 = xhat * dgamma / m
