@@ -5,7 +5,7 @@ from mytorch_b200.dtype import float32
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d, _batch_norm2d_add_relu, _batch_norm2d_relu
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.parameter import Parameter
-from mytorch_b200.ops._common import dispatch, tracker
+from mytorch_b200.ops._common import dispatch, grad_enabled
 from mytorch_b200.tensor import Tensor
 
 
@@ -78,8 +78,7 @@ def inference_conv_norm(conv, norm, x, relu=False, residual=None):
     None elsewhere.  Same bits as the separate layers."""
     if norm.training or norm.running_mean is None or x.device.type != "cuda":
         return None
-    if not tracker.no_grad and (x.requires_grad or conv.weight.requires_grad or norm.weight is not None and norm.weight.requires_grad
-                                or residual is not None and residual.requires_grad):
+    if grad_enabled(x, conv.weight, conv.bias, norm.weight, norm.bias, residual):
         return None
     weight, device, dtype = conv.weight, x.device, x.dtype
     ok = weight.shape[0] == norm.num_features
