@@ -59,6 +59,10 @@ class DAGTracker:
         # backward can add itself (keyword ``accumulate_dx``); the tape then stores the returned
         # gradient instead of launching an add
         self.fused_accumulate = {}
+        # those of them that may return the handed-in tensor itself, with their share added in place.  They return
+        # dx in memory of its own otherwise, and are told ``accumulate_shared=True`` where the gradient so far may
+        # also be another tensor's (an addition passes one tensor to both operands) or was there before the pass
+        self.accumulates_in_place = set()
 
     def register_backward_function(self, op_name):
         def decorator(func):
@@ -106,7 +110,8 @@ class DAGTracker:
                     if isinstance(arg, Tensor) and arg.requires_grad and arg._grad_node is None:
                         pending[id(arg)] = pending.get(id(arg), 0) + 1
 
-        funcs, fusable, deferrable = self._backward_funcs, self.fused_accumulate, self.deferrable
+        funcs, fusable, deferrable, in_place = self._backward_funcs, self.fused_accumulate, self.deferrable, self.accumulates_in_place
+        owned = set()  # ids of the tensors whose gradient was made in this pass, for them alone
         for node in order:
             name, inputs = node.name, node.inputs
             fused = None  # the input whose gradient so far is handed to the operator
@@ -119,6 +124,8 @@ class DAGTracker:
                     if isinstance(cand, Tensor) and cand.requires_grad and cand.grad is not None:
                         fused = cand
                         extra["accumulate_dx"] = cand.grad
+                        if name in in_place and id(cand) not in owned:
+                            extra["accumulate_shared"] = True
                 if join is not None and name in deferrable:
                     extra["defer_weight_gradient"] = True
                 grads = funcs[name](*[t.grad for t in node.outputs], *node.helpers, *inputs, **extra)
@@ -132,12 +139,15 @@ class DAGTracker:
                     continue
                 if arg.grad is None or (k == slot and arg is fused):
                     arg.grad = grad
+                    if k == slot and name in in_place:
+                        owned.add(id(arg))
                 else:
                     if arg.grad.shape != grad.shape:
                         raise MismatchShapesError([arg.grad.shape, grad.shape])
                     if join is not None and arg._grad_node is None:  # a leaf: its gradient may come from there
                         join()
                     arg.grad = arg.grad + grad
+                    owned.add(id(arg))
             if hook is not None:
                 for arg in inputs:
                     if isinstance(arg, Tensor) and arg.requires_grad and id(arg) in pending:

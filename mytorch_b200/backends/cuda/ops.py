@@ -253,10 +253,12 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
 
 
 @_reg("cuda", "conv2d_backward")
-def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accumulate_dx=None, defer_weight_gradient=False):
+def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accumulate_dx=None, defer_weight_gradient=False,
+                         accumulate_shared=False):
     """``accumulate_dx``: a gradient the input has already received from another consumer; when given,
     the returned dx is the data gradient PLUS that tensor (added in the convolution's epilogue where
-    the kernel allows), and the caller stores it instead of adding the two itself.
+    the kernel allows), and the caller stores it instead of adding the two itself.  The returned tensor may be that
+    tensor, changed in place, unless ``accumulate_shared`` says that others hold it too.
     ``defer_weight_gradient``: the caller (the tape) does not need dw until it calls ``CudaEnv.join_side``;
     the weight gradient then runs on the device's side stream, beside whatever the caller enqueues next."""
     _f32(output_grad, input, weight)
@@ -282,7 +284,7 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         side = env.fork_side((output_grad,))
     if want_dx:
         ws, ws_bytes = env.workspace(need)
-        if accumulate_dx is not None and not padded and env.lib.conv2d_dgrad_accumulates_in_place(
+        if accumulate_dx is not None and not padded and not accumulate_shared and env.lib.conv2d_dgrad_accumulates_in_place(
                 *a, output_grad, wt, accumulate_dx):
             # a filter smaller than its stride (the 1x1 / stride-2 shortcut) reaches only some pixels: it adds
             # to those in the gradient the input already holds, which is then the returned tensor
