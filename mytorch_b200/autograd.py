@@ -19,7 +19,7 @@ import operator
 
 
 class _Node:
-    __slots__ = ("name", "inputs", "outputs", "helpers", "seq")
+    __slots__ = ("name", "inputs", "outputs", "helpers", "seq", "keywords")
 
     def __init__(self, name, inputs, outputs, helpers, seq):
         self.name = name
@@ -27,6 +27,7 @@ class _Node:
         self.outputs = outputs
         self.helpers = helpers
         self.seq = seq
+        self.keywords = None  # more for the backward function, by name: what forward made and backward can use again
 
 
 _creation = operator.attrgetter("seq")
@@ -116,8 +117,8 @@ class DAGTracker:
             name, inputs = node.name, node.inputs
             fused = None  # the input whose gradient so far is handed to the operator
             slot = -1
-            if name in fusable or name in deferrable:
-                extra = {}
+            if name in fusable or name in deferrable or node.keywords:
+                extra = dict(node.keywords) if node.keywords else {}
                 slot = fusable.get(name, -1)
                 if slot >= 0:
                     cand = inputs[slot]
@@ -162,6 +163,7 @@ class DAGTracker:
             for t in node.outputs:
                 t._grad_node = None
             node.inputs = node.outputs = node.helpers = ()
+            node.keywords = None
 
 
 class NoGrad:

@@ -198,8 +198,9 @@ def _take_channels(env, t, channels, like, out=None):
 _BIAS_BESIDE_BYTES = 16 << 20
 
 
-def _conv_operands(env, input, weight, stride, padding):
-    """(arguments, input, filter, output tensor) of a forward convolution, the operands in the form its kernel reads."""
+def _conv_operands(env, input, weight, stride, padding, packed=None):
+    """(arguments, input, filter, output tensor) of a forward convolution, the operands in the form its kernel reads.
+    ``packed``: a list that takes the input as it was packed, if it was."""
     x, wt = input, weight
     a = _conv_args(x, wt, stride, padding)
     n, cin, h, w, kh, kw, sh, sw, ph, pw, cout = a
@@ -208,8 +209,8 @@ def _conv_operands(env, input, weight, stride, padding):
     if form is not None:
         a = form[1]
         x = _stem_input(env, input, form)
-        if weight.requires_grad and not _tracker.no_grad:
-            input._stem_held = (form, x)  # the weight gradient of this convolution reads it again
+        if packed is not None:
+            packed.append(x)
         rows, entries = _stem_filter_rows(weight.shape, form)
         block = CudaMemory(weight.device.index, rows * _TC_CHANNELS * 4)
         env.lib.resize_channels_f32(weight, block, rows, entries, _TC_CHANNELS, env.stream())
@@ -232,13 +233,15 @@ def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, ru
 
 
 @_reg("cuda", "conv2d")
-def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
+def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False, packed=None):
     """``bn_stats``: the output feeds a BatchNorm layer in training mode; where the kernel allows, the
     convolution's epilogue also reduces the per-channel batch statistics of the output and leaves them
-    on the result (``_bn_partials``) for ``batch_norm2d``, which then skips its own pass over the tensor."""
+    on the result (``_bn_partials``) for ``batch_norm2d``, which then skips its own pass over the tensor.
+    ``packed`` (a list): takes the input in the form the kernel read, where few channels had to be packed; the weight
+    gradient of the same values can read it again (``packed_input`` of the backward)."""
     _f32(input, weight, bias)
     env = _env(input)
-    a, x, wt, out = _conv_operands(env, input, weight, stride, padding)
+    a, x, wt, out = _conv_operands(env, input, weight, stride, padding, packed)
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     if bn_stats:
         partials = CudaMemory(input.device.index, env.lib.conv2d_stats_max_rows() * 3 * a[-1] * 4)
@@ -254,7 +257,7 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False):
 
 @_reg("cuda", "conv2d_backward")
 def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accumulate_dx=None, defer_weight_gradient=False,
-                         accumulate_shared=False):
+                         accumulate_shared=False, packed_input=None):
     """``accumulate_dx``: a gradient the input has already received from another consumer; when given,
     the returned dx is the data gradient PLUS that tensor (added in the convolution's epilogue where
     the kernel allows), and the caller stores it instead of adding the two itself.  The returned tensor may be that
@@ -309,12 +312,7 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         # A weight that already holds a gradient (shared weights) accumulates on the compute stream.
         wa = a
         if form is not None:
-            held = getattr(input, "_stem_held", None)
-            if held is not None and held[0] == form:
-                x = held[1]
-                del input._stem_held
-            else:
-                x = _stem_input(env, input, form)
+            x = _stem_input(env, input, form) if packed_input is None else packed_input
             wa = form[1]
             need = env.lib.conv2d_workspace_bytes(*wa)
         wst = st
