@@ -109,10 +109,10 @@ inline bool from_py(PyObject* o, T*& v) {
     if (!memory) return false;
     const bool block = PyObject_TypeCheck(memory, &BlockType);
     v = block ? (T*)((Block*)memory)->ptr : nullptr;
-    const bool none = memory == Py_None;
     Py_DECREF(memory);  // the tensor holds it
-    if (!block && !none) PyErr_SetString(PyExc_TypeError, "a tensor without device memory");
-    return block || none;
+    // not NULL: an optional operand (a bias, running statistics) would be taken as absent
+    if (!block) PyErr_SetString(PyExc_TypeError, "a tensor without device memory");
+    return block;
   }
   if constexpr (std::is_same_v<T, const long long>) {
     if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
