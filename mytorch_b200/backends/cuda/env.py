@@ -51,7 +51,8 @@ _SIGNATURES = _binding.entry_points if _binding is not None else ()
 class NativeLibrary:
     """The entry points of ``libmytorch_b200.so`` as attributes, without their ``mtb_`` prefix; a call raises on a
     non-zero status (or a NULL pointer from the entry points that return one).  Pointer arguments are None,
-    addresses, ``CudaMemory`` blocks or ctypes objects (host arrays, ``byref``)."""
+    addresses, ``CudaMemory`` blocks or tensors; those that the header calls HOST are None, addresses or ctypes storage
+    (arrays, ``byref``), shapes and strides also tuples or lists."""
 
     def __init__(self, path=LIBRARY_PATH):
         if not os.path.exists(path) or _binding is None:

@@ -245,11 +245,11 @@ def cuda_conv2d(input, weight, bias, stride, padding, bn_stats=False, packed=Non
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     if bn_stats:
         partials = CudaMemory(input.device.index, env.lib.conv2d_stats_max_rows() * 3 * a[-1] * 4)
-        rows = ctypes.c_int(0)
-        env.lib.conv2d_forward_stats_f32(*a, x, wt, bias, out, 0, partials.ptr, ctypes.byref(rows), ws, ws_bytes,
+        rows = (ctypes.c_int * 1)()
+        env.lib.conv2d_forward_stats_f32(*a, x, wt, bias, out, 0, partials.ptr, rows, ws, ws_bytes,
                                          env.stream())
-        if rows.value > 0:
-            out._bn_partials = (partials, rows.value)
+        if rows[0] > 0:
+            out._bn_partials = (partials, rows[0])
         return out
     env.lib.conv2d_forward_f32(*a, x, wt, bias, out, 0, ws, ws_bytes, env.stream())
     return out

@@ -74,47 +74,78 @@ inline bool from_py(PyObject* o, float& v) {
   return true;
 }
 
-// An address that is neither None, an integer nor a block: a ctypes byref(), array or scalar (its storage), or a
-// ctypes pointer value.
-bool address_of(PyObject* o, void*& v) {
-  PyObject* target = PyObject_GetAttrString(o, "_obj");  // byref(x)
-  const bool by_reference = target != nullptr;
-  if (!target) { PyErr_Clear(); Py_INCREF(o); target = o; }
-  if (!by_reference && !strcmp(Py_TYPE(o)->tp_name, "c_void_p")) {
-    PyObject* value = PyObject_GetAttrString(o, "value");
-    Py_DECREF(target);
-    if (!value) return false;
-    v = value == Py_None ? nullptr : PyLong_AsVoidPtr(value);
-    Py_DECREF(value);
-    return !PyErr_Occurred();
+// ctypes, for the objects that hold or describe an address (imported on the first of them).
+struct CTypes {
+  PyObject *cast, *c_void_p, *pointer, *array;
+};
+const CTypes* ctypes() {
+  static CTypes c{};
+  if (!c.array) {
+    PyObject* m = PyImport_ImportModule("ctypes");
+    if (!m) return nullptr;
+    c.cast = PyObject_GetAttrString(m, "cast");
+    c.c_void_p = PyObject_GetAttrString(m, "c_void_p");
+    c.pointer = PyObject_GetAttrString(m, "_Pointer");
+    c.array = PyObject_GetAttrString(m, "Array");
+    Py_DECREF(m);
+    if (!c.cast || !c.c_void_p || !c.pointer || !c.array) { c.array = nullptr; return nullptr; }
   }
+  return &c;
+}
+bool ctypes_address(const CTypes& c, PyObject* o, void*& v) {  // refuses what a c_void_p argument refuses
+  PyObject* p = PyObject_CallFunctionObjArgs(c.cast, o, c.c_void_p, nullptr);
+  PyObject* value = p ? PyObject_GetAttrString(p, "value") : nullptr;
+  Py_XDECREF(p);
+  if (!value) return false;
+  v = value == Py_None ? nullptr : PyLong_AsVoidPtr(value);
+  Py_DECREF(value);
+  return !PyErr_Occurred();
+}
+
+// Where the header says HOST: None, an integer, or ctypes storage (an array, byref(x), a pointer); for shapes and strides
+// also a tuple or list.
+bool host_address(PyObject* o, void*& v) {
+  const CTypes* c = ctypes();
+  if (!c) return false;
+  const int array = PyObject_IsInstance(o, c->array);
+  if (array <= 0) return array == 0 && ctypes_address(*c, o, v);
   Py_buffer view;
-  const int rc = PyObject_GetBuffer(target, &view, PyBUF_SIMPLE);
-  Py_DECREF(target);  // the caller's argument keeps the storage alive during the call
-  if (rc) return false;
+  if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE)) return false;
   v = view.buf;
-  PyBuffer_Release(&view);
+  PyBuffer_Release(&view);  // the caller's argument keeps the storage alive during the call
   return true;
 }
-template <class T>
-inline bool from_py(PyObject* o, T*& v) {
-  if (o == Py_None) { v = nullptr; return true; }
-  if (PyLong_CheckExact(o)) {
-    v = (T*)PyLong_AsVoidPtr(o);
-    return !(v == nullptr && PyErr_Occurred());
-  }
-  if (PyObject_TypeCheck(o, &BlockType)) { v = (T*)((Block*)o)->ptr; return true; }
+// Everywhere else (device memory, streams, events, graphs): None, an integer, a block, a tensor, or a ctypes pointer's value.
+// Anything that merely has storage is host memory, which a kernel must not be given.
+bool device_address(PyObject* o, void*& v) {
+  if (PyObject_TypeCheck(o, &BlockType)) { v = (void*)((Block*)o)->ptr; return true; }
   if (g_tensor_type && PyObject_TypeCheck(o, g_tensor_type)) {
     PyObject* memory = PyObject_GetAttr(o, N__native_array);
     if (!memory) return false;
     const bool block = PyObject_TypeCheck(memory, &BlockType);
-    v = block ? (T*)((Block*)memory)->ptr : nullptr;
+    v = block ? (void*)((Block*)memory)->ptr : nullptr;
     Py_DECREF(memory);  // the tensor holds it
     // not NULL: an optional operand (a bias, running statistics) would be taken as absent
     if (!block) PyErr_SetString(PyExc_TypeError, "a tensor without device memory");
     return block;
   }
-  if constexpr (std::is_same_v<T, const long long>) {
+  const CTypes* c = ctypes();
+  if (!c) return false;
+  int value = PyObject_IsInstance(o, c->c_void_p);
+  if (!value) value = PyObject_IsInstance(o, c->pointer);
+  if (value > 0) return ctypes_address(*c, o, v);
+  if (value == 0) PyErr_Format(PyExc_TypeError, "device memory, a tensor, an address or None expected, not %.80s", Py_TYPE(o)->tp_name);
+  return false;
+}
+
+template <bool HOST, class T>
+inline bool pointer(PyObject* o, T*& v) {
+  if (o == Py_None) { v = nullptr; return true; }
+  if (PyLong_Check(o)) {
+    v = (T*)PyLong_AsVoidPtr(o);
+    return !(v == nullptr && PyErr_Occurred());
+  }
+  if constexpr (HOST && std::is_same_v<T, const long long>) {
     if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
       // shapes and strides: read by the entry point before it returns, so a few slots per thread taken in turn are enough
       constexpr int kSlots = 16, kLength = 64;
@@ -130,9 +161,15 @@ inline bool from_py(PyObject* o, T*& v) {
     }
   }
   void* p = nullptr;
-  if (!address_of(o, p)) return false;
+  if (!(HOST ? host_address(o, p) : device_address(o, p))) return false;
   v = (T*)p;
   return true;
+}
+// One argument of an entry point; HOST: it is a pointer to host memory.
+template <bool HOST, class T>
+inline bool argument(PyObject* o, T& v) {
+  if constexpr (std::is_pointer_v<T>) return pointer<HOST>(o, v);
+  else return from_py(o, v);
 }
 
 inline PyObject* to_py(int v) { return PyLong_FromLong(v); }
@@ -154,17 +191,17 @@ PyObject* raise_native(const char* name, int rc) {
   return nullptr;
 }
 
-template <int ID, Kind K, class Sig>
+template <int ID, Kind K, unsigned HOST, class Sig>
 struct Entry;
-template <int ID, Kind K, class R, class... A>
-struct Entry<ID, K, R(A...)> {
+template <int ID, Kind K, unsigned HOST, class R, class... A>
+struct Entry<ID, K, HOST, R(A...)> {
   static inline R (*fn)(A...) = nullptr;
   static inline const char* name = nullptr;
 
   template <size_t... I>
   static PyObject* invoke(PyObject* const* args, std::index_sequence<I...>) {
     std::tuple<A...> a;
-    if (!(from_py(args[I], std::get<I>(a)) && ... && true)) return nullptr;
+    if (!(argument<(HOST >> I & 1u) != 0>(args[I], std::get<I>(a)) && ... && true)) return nullptr;
     if constexpr (K == VALUE) {
       return to_py(fn(std::get<I>(a)...));
     } else {
@@ -192,33 +229,40 @@ struct Entry<ID, K, R(A...)> {
   }
 };
 
+// name, kind, and which arguments (counted from 0) the public header calls HOST memory
+template <class... I>
+constexpr unsigned HOST(I... i) { return (0u | ... | (1u << i)); }
 #define MTB_ENTRIES(X) \
-  X(version, VALUE) X(device_check, STATUS) X(fill_f32, LAUNCH) X(copy_f32, LAUNCH) X(scale_f32, LAUNCH) X(relu_forward_f32, LAUNCH) \
-  X(relu_backward_f32, LAUNCH) X(add_f32, LAUNCH) X(mul_f32, LAUNCH) X(add_bias_rows_f32, LAUNCH) X(binary_strided_f32, LAUNCH) \
-  X(resize_channels_f32, LAUNCH) X(pack_patches_f32, LAUNCH) X(nchw_to_nhwc_f32, LAUNCH) X(nhwc_to_nchw_f32, LAUNCH) X(cast, LAUNCH) \
-  X(batch_norm2d_workspace_bytes, VALUE) X(batch_norm2d_forward_f32, LAUNCH) X(batch_norm2d_backward_f32, LAUNCH) \
-  X(batch_norm2d_add_relu_forward_f32, LAUNCH) X(batch_norm2d_add_relu_forward_masked_f32, LAUNCH) \
-  X(batch_norm2d_add_relu_backward_masked_f32, LAUNCH) X(batch_norm2d_add_relu_backward_f32, LAUNCH) X(add_relu_f32, LAUNCH) \
-  X(add_relu_backward_f32, LAUNCH) X(colsum_workspace_bytes, VALUE) X(colsum_f32, LAUNCH) X(colsum_noalloc_f32, LAUNCH) \
-  X(nhwc_spatial_sum_f32, LAUNCH) X(nhwc_spatial_bcast_f32, LAUNCH) X(sum_strided_f32, LAUNCH) X(max_strided_f32, LAUNCH) \
-  X(max_backward_f32, LAUNCH) X(eq_strided, LAUNCH) X(max_pool2d_forward_f32, LAUNCH) X(max_pool2d_backward_f32, LAUNCH) \
-  X(max_pool2d_argmax_u8, LAUNCH) X(cross_entropy_workspace_bytes, VALUE) X(cross_entropy_forward_f32, LAUNCH) \
-  X(cross_entropy_backward_f32, LAUNCH) X(sgd_f32, LAUNCH) X(sgd_multi_f32, LAUNCH) X(pack_scale_f32, LAUNCH) \
-  X(conv2d_workspace_bytes, VALUE) X(conv2d_plan_f32, STATUS) X(conv2d_forward_f32, LAUNCH) X(conv2d_stats_max_rows, VALUE) \
-  X(conv2d_forward_stats_f32, LAUNCH) X(conv2d_bn_forward_f32, LAUNCH) X(batch_norm2d_forward_prestats_f32, LAUNCH) X(conv2d_dgrad_f32, LAUNCH) \
-  X(conv2d_dgrad_add_f32, LAUNCH) X(conv2d_dgrad_accumulates_in_place, VALUE) X(conv2d_wgrad_f32, LAUNCH) X(gemm_f32, LAUNCH) \
-  X(tc_status, STATUS) X(tc_wait_selftest, LAUNCH) \
-  X(malloc, POINTER) X(free, STATUS) X(pool_reserved_bytes, VALUE) X(pool_in_use_bytes, VALUE) X(pool_trim, STATUS) X(set_device, STATUS) \
-  X(get_device, STATUS) X(device_count, STATUS) X(device_synchronize, STATUS) X(mem_get_info, STATUS) X(memcpy_h2d_async, STATUS) \
-  X(memcpy_d2h_async, STATUS) X(memcpy_d2d_async, STATUS) X(memset_async, STATUS) X(host_alloc_pinned, POINTER) X(host_free_pinned, STATUS) \
-  X(stream_create, POINTER) X(stream_destroy, STATUS) X(stream_synchronize, STATUS) X(stream_wait_event, STATUS) X(event_create, POINTER) \
-  X(event_destroy, STATUS) X(event_record, STATUS) X(event_synchronize, STATUS) X(event_elapsed_ms, STATUS) X(graph_begin_capture, STATUS) \
-  X(graph_end_capture, STATUS) X(graph_launch, STATUS) X(graph_destroy, STATUS)
+  X(version, VALUE, 0) X(device_check, STATUS, 0) X(fill_f32, LAUNCH, 0) X(copy_f32, LAUNCH, 0) X(scale_f32, LAUNCH, 0) \
+  X(relu_forward_f32, LAUNCH, 0) X(relu_backward_f32, LAUNCH, 0) X(add_f32, LAUNCH, 0) X(mul_f32, LAUNCH, 0) \
+  X(add_bias_rows_f32, LAUNCH, 0) X(binary_strided_f32, LAUNCH, HOST(2, 3, 4, 5)) X(resize_channels_f32, LAUNCH, 0) \
+  X(pack_patches_f32, LAUNCH, 0) X(nchw_to_nhwc_f32, LAUNCH, 0) X(nhwc_to_nchw_f32, LAUNCH, 0) X(cast, LAUNCH, 0) \
+  X(batch_norm2d_workspace_bytes, VALUE, 0) X(batch_norm2d_forward_f32, LAUNCH, 0) X(batch_norm2d_backward_f32, LAUNCH, 0) \
+  X(batch_norm2d_add_relu_forward_f32, LAUNCH, 0) X(batch_norm2d_add_relu_forward_masked_f32, LAUNCH, 0) \
+  X(batch_norm2d_add_relu_backward_masked_f32, LAUNCH, 0) X(batch_norm2d_add_relu_backward_f32, LAUNCH, 0) X(add_relu_f32, LAUNCH, 0) \
+  X(add_relu_backward_f32, LAUNCH, 0) X(colsum_workspace_bytes, VALUE, 0) X(colsum_f32, LAUNCH, 0) X(colsum_noalloc_f32, LAUNCH, 0) \
+  X(nhwc_spatial_sum_f32, LAUNCH, 0) X(nhwc_spatial_bcast_f32, LAUNCH, 0) X(sum_strided_f32, LAUNCH, HOST(3, 4, 6, 7)) \
+  X(max_strided_f32, LAUNCH, HOST(4, 5)) X(max_backward_f32, LAUNCH, HOST(5, 6)) X(eq_strided, LAUNCH, HOST(2, 3, 4)) \
+  X(max_pool2d_forward_f32, LAUNCH, 0) X(max_pool2d_backward_f32, LAUNCH, 0) X(max_pool2d_argmax_u8, LAUNCH, 0) \
+  X(cross_entropy_workspace_bytes, VALUE, 0) X(cross_entropy_forward_f32, LAUNCH, 0) X(cross_entropy_backward_f32, LAUNCH, 0) \
+  X(sgd_f32, LAUNCH, 0) X(sgd_multi_f32, LAUNCH, HOST(1, 2, 3, 4, 5)) X(pack_scale_f32, LAUNCH, HOST(1, 2, 3)) \
+  X(conv2d_workspace_bytes, VALUE, 0) X(conv2d_plan_f32, STATUS, HOST(11)) X(conv2d_forward_f32, LAUNCH, 0) \
+  X(conv2d_stats_max_rows, VALUE, 0) X(conv2d_forward_stats_f32, LAUNCH, HOST(17)) X(conv2d_bn_forward_f32, LAUNCH, 0) \
+  X(batch_norm2d_forward_prestats_f32, LAUNCH, 0) X(conv2d_dgrad_f32, LAUNCH, 0) X(conv2d_dgrad_add_f32, LAUNCH, 0) \
+  X(conv2d_dgrad_accumulates_in_place, VALUE, 0) X(conv2d_wgrad_f32, LAUNCH, 0) X(gemm_f32, LAUNCH, 0) X(tc_status, STATUS, HOST(0)) \
+  X(tc_wait_selftest, LAUNCH, 0) X(malloc, POINTER, 0) X(free, STATUS, 0) X(pool_reserved_bytes, VALUE, 0) X(pool_in_use_bytes, VALUE, 0) \
+  X(pool_trim, STATUS, 0) X(set_device, STATUS, 0) X(get_device, STATUS, HOST(0)) X(device_count, STATUS, HOST(0)) \
+  X(device_synchronize, STATUS, 0) X(mem_get_info, STATUS, HOST(0, 1)) X(memcpy_h2d_async, STATUS, HOST(1)) \
+  X(memcpy_d2h_async, STATUS, HOST(0)) X(memcpy_d2d_async, STATUS, 0) X(memset_async, STATUS, 0) X(host_alloc_pinned, POINTER, 0) \
+  X(host_free_pinned, STATUS, HOST(0)) X(stream_create, POINTER, 0) X(stream_destroy, STATUS, 0) X(stream_synchronize, STATUS, 0) \
+  X(stream_wait_event, STATUS, 0) X(event_create, POINTER, 0) X(event_destroy, STATUS, 0) X(event_record, STATUS, 0) \
+  X(event_synchronize, STATUS, 0) X(event_elapsed_ms, STATUS, HOST(2)) X(graph_begin_capture, STATUS, 0) \
+  X(graph_end_capture, STATUS, HOST(1)) X(graph_launch, STATUS, 0) X(graph_destroy, STATUS, 0)
 
-#define X(n, k) ID_##n,
+#define X(n, k, h) ID_##n,
 enum EntryId { MTB_ENTRIES(X) kEntries };
 #undef X
-#define X(n, k) using E_##n = Entry<ID_##n, k, std::remove_pointer_t<decltype(&mtb_##n)>>;
+#define X(n, k, h) using E_##n = Entry<ID_##n, k, h, std::remove_pointer_t<decltype(&mtb_##n)>>;
 MTB_ENTRIES(X)
 #undef X
 
@@ -407,13 +451,15 @@ PyObject* sgd_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
   void* st;
   for (int i = 0; i < 4; ++i)
     if (!from_py(args[1 + i], h[i])) return nullptr;
-  if (!from_py(args[5], nesterov) || !from_py(args[6], maximize) || !from_py(args[7], scale) || !from_py(args[8], st)) return nullptr;
+  if (!from_py(args[5], nesterov) || !from_py(args[6], maximize) || !from_py(args[7], scale) || !pointer<false>(args[8], st)) return nullptr;
   for (Py_ssize_t i = 0; i < count; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (!PyTuple_CheckExact(e) || PyTuple_GET_SIZE(e) != 3) { PyErr_SetString(PyExc_TypeError, "(parameter, buffer, first) expected"); return nullptr; }
     PyObject* param = PyTuple_GET_ITEM(e, 0);
     Ref grad(PyObject_GetAttr(param, N_grad)), shape(PyObject_GetAttr(param, N_shape));
-    if (!grad || !shape || !from_py(param, params[i]) || !from_py((PyObject*)grad, grads[i]) || !from_py(PyTuple_GET_ITEM(e, 1), bufs[i])) return nullptr;
+    if (!grad || !shape || !pointer<false>(param, params[i]) || !pointer<false>((PyObject*)grad, grads[i]) ||
+        !pointer<false>(PyTuple_GET_ITEM(e, 1), bufs[i]))
+      return nullptr;
     const int is_first = PyObject_IsTrue(PyTuple_GET_ITEM(e, 2));
     if (is_first < 0 || !params[i] || !grads[i] || !bufs[i] || !PyTuple_Check(shape)) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "sgd_step: a parameter without device memory, gradient or buffer"); return nullptr; }
     first[i] = is_first;
@@ -467,7 +513,7 @@ PyObject* load(PyObject*, PyObject* args) {
     return p;
   };
   if (!(g_last_error = (decltype(g_last_error))find("mtb_last_error"))) return nullptr;
-#define X(n, k) \
+#define X(n, k, h) \
   E_##n::name = "mtb_" #n; \
   if (!(E_##n::fn = (decltype(E_##n::fn))find("mtb_" #n))) return nullptr;
   MTB_ENTRIES(X)
@@ -503,7 +549,7 @@ PyMethodDef methods[] = {
     {"sgd_step", (PyCFunction)(void (*)())sgd_step, METH_FASTCALL, "One SGD update of a list of (parameter, buffer, first)."},
     {"workspace", workspace<0>, METH_O, "(address, bytes) of scratch for compute-stream kernels."},
     {"side_workspace", workspace<1>, METH_O, "(address, bytes) of scratch for side-stream kernels."},
-#define X(n, k) {#n, (PyCFunction)(void (*)())E_##n::call, METH_FASTCALL, nullptr},
+#define X(n, k, h) {#n, (PyCFunction)(void (*)())E_##n::call, METH_FASTCALL, nullptr},
     MTB_ENTRIES(X)
 #undef X
     {nullptr, nullptr, 0, nullptr}};
@@ -529,7 +575,7 @@ PyMODINIT_FUNC PyInit__mtb_binding() {
   MTB_NAMES(X)
 #undef X
   PyObject* names = PyTuple_New(kEntries);
-#define X(n, k) PyTuple_SET_ITEM(names, ID_##n, PyUnicode_FromString("mtb_" #n));
+#define X(n, k, h) PyTuple_SET_ITEM(names, ID_##n, PyUnicode_FromString("mtb_" #n));
   MTB_ENTRIES(X)
 #undef X
   Py_INCREF(&BlockType);
