@@ -51,6 +51,9 @@ int mtb_tc_wait_selftest(long long limit_cycles, int code, void* stream);
  * mtb_graph_destroy: it can be reused inside the capture but never by anything outside it. */
 void* mtb_malloc(long long nbytes);
 int mtb_free(void* ptr);
+/* the same where neither the driver nor a wait for another thread is needed; NULL / 0: not done, and no error */
+void* mtb_malloc_if_ready(long long nbytes);
+int mtb_free_if_ready(void* ptr);
 long long mtb_pool_reserved_bytes(void);
 long long mtb_pool_in_use_bytes(void);
 int mtb_pool_trim(void);

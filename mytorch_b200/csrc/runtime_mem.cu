@@ -78,6 +78,43 @@ int trim_locked(DevicePool& pool) {
 
 }  // namespace
 
+// A block for `want` bytes out of the free lists, or nullptr.
+static void* take_free(Runtime& r, DevicePool& pool, size_t want) {
+  size_t got = 0;
+  void* p = nullptr;
+  if (r.capturing) p = take_fit(pool.graph_free[r.capturing], want, &got);
+  if (!p) p = take_fit(pool.free_blocks, want, &got);
+  if (!p) return nullptr;
+  r.blocks[p].graph = r.capturing;
+  pool.in_use += got;
+  return p;
+}
+static void put_back(Runtime& r, const Block& b, void* ptr) {
+  DevicePool& pool = r.pools[b.device];
+  pool.in_use -= b.size;
+  if (b.graph) pool.graph_free[b.graph].emplace(b.size, ptr);
+  else pool.free_blocks.emplace(b.size, ptr);
+}
+
+// What needs neither the driver nor a wait: a caller that holds a lock of its own (an interpreter's) tries these first and lets
+// go of it for mtb_malloc / mtb_free, which may wait for a thread that is growing the pool.  NULL / 0: not done, no error.
+MTB_API void* mtb_malloc_if_ready(long long nbytes) {
+  int dev = 0;
+  if (nbytes < 0 || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  Runtime& r = rt();
+  std::unique_lock<std::mutex> lock(r.mu, std::try_to_lock);
+  return lock ? take_free(r, r.pools[dev], round_size((size_t)nbytes)) : nullptr;
+}
+MTB_API int mtb_free_if_ready(void* ptr) {
+  Runtime& r = rt();
+  std::unique_lock<std::mutex> lock(r.mu, std::try_to_lock);
+  if (!lock) return 0;
+  auto it = r.blocks.find(ptr);
+  if (it == r.blocks.end()) return 0;
+  put_back(r, it->second, ptr);
+  return 1;
+}
+
 // Device memory from the pool of the current device (NULL on failure, see mtb_last_error).
 MTB_API void* mtb_malloc(long long nbytes) {
   if (nbytes < 0) { mtb_fail(MTB_ERR_INVALID, "mtb_malloc: negative size"); return nullptr; }
@@ -87,28 +124,22 @@ MTB_API void* mtb_malloc(long long nbytes) {
   Runtime& r = rt();
   std::lock_guard<std::mutex> lock(r.mu);
   DevicePool& pool = r.pools[dev];
-  size_t got = 0;
-  void* p = nullptr;
-  if (r.capturing) p = take_fit(pool.graph_free[r.capturing], want, &got);
-  if (!p) p = take_fit(pool.free_blocks, want, &got);
-  if (!p) {
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) {  // give back what is cached and try once more
-      cudaGetLastError();
-      trim_locked(pool);
-      e = cudaMalloc(&p, want);
-    }
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      mtb_fail(MTB_ERR_CUDA, "mtb_malloc: cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
-      return nullptr;
-    }
-    got = want;
-    pool.reserved += want;
-    r.blocks[p] = Block{want, dev, 0};
+  void* p = take_free(r, pool, want);
+  if (p) return p;
+  cudaError_t e = cudaMalloc(&p, want);
+  if (e != cudaSuccess) {  // give back what is cached and try once more
+    cudaGetLastError();
+    trim_locked(pool);
+    e = cudaMalloc(&p, want);
   }
-  r.blocks[p].graph = r.capturing;
-  pool.in_use += got;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    mtb_fail(MTB_ERR_CUDA, "mtb_malloc: cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
+    return nullptr;
+  }
+  pool.reserved += want;
+  r.blocks[p] = Block{want, dev, r.capturing};
+  pool.in_use += want;
   return p;
 }
 
@@ -118,11 +149,7 @@ MTB_API int mtb_free(void* ptr) {
   std::lock_guard<std::mutex> lock(r.mu);
   auto it = r.blocks.find(ptr);
   if (it == r.blocks.end()) return mtb_fail(MTB_ERR_INVALID, "mtb_free: %p was not allocated by mtb_malloc", ptr);
-  Block& b = it->second;
-  DevicePool& pool = r.pools[b.device];
-  pool.in_use -= b.size;
-  if (b.graph) pool.graph_free[b.graph].emplace(b.size, ptr);
-  else pool.free_blocks.emplace(b.size, ptr);
+  put_back(r, it->second, ptr);
   return MTB_OK;
 }
 
