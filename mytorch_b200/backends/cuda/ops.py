@@ -284,7 +284,10 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
     want_db = bias is not None and bias.requires_grad
     beside = want_db and want_dx and not defer_weight_gradient and output_grad._native_array.nbytes >= _BIAS_BESIDE_BYTES
     if beside:
-        side = env.fork_side((output_grad,))
+        # Memory before the fork: a block that is free now was last used by work the side stream waits for, one that the calls
+        # below give back is still used by theirs.
+        db, scratch = _grad_buffer(bias), env.side_workspace(env.lib.colsum_workspace_bytes(a[-1]))
+        side = env.fork_side((output_grad, db))
     if want_dx:
         ws, ws_bytes = env.workspace(need)
         if accumulate_dx is not None and not padded and not accumulate_shared and env.lib.conv2d_dgrad_accumulates_in_place(
@@ -304,7 +307,7 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
             if accumulate_dx is not None:
                 dx = BackendDispatcher.instance().dispatch("cuda", "add")(dx, accumulate_dx, 1)
     if beside:
-        db = _bias_gradient(env, output_grad, a[-1], bias, side, env.side_workspace)
+        _bias_gradient(env, output_grad, a[-1], db, scratch, side)
     if want_dw:
         # Nothing in the rest of backward reads this layer's weight gradient, so it runs on the side
         # stream, beside the data-gradient / BatchNorm chain that the next layer waits for, and is
@@ -332,18 +335,16 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
         else:
             dw = _grad_buffer(weight)
             env.lib.conv2d_wgrad_f32(*a, x, output_grad, dw, wws, wws_bytes, wst)
-    if want_db and db is None:
-        db = _bias_gradient(env, output_grad, a[-1], bias, st, env.workspace)
     if beside:
         env.join_side()
+    elif want_db:
+        db = _grad_buffer(bias)
+        _bias_gradient(env, output_grad, a[-1], db, env.workspace(env.lib.colsum_workspace_bytes(a[-1])), st)
     return [dx, dw, db]
 
 
-def _bias_gradient(env, output_grad, channels, bias, stream, workspace):
-    out = _grad_buffer(bias)
-    ws, ws_bytes = workspace(env.lib.colsum_workspace_bytes(channels))
-    env.lib.colsum_f32(output_grad, _numel(output_grad.shape) // channels, channels, 1.0, out, ws, ws_bytes, stream)
-    return out
+def _bias_gradient(env, output_grad, channels, out, scratch, stream):
+    env.lib.colsum_f32(output_grad, _numel(output_grad.shape) // channels, channels, 1.0, out, *scratch, stream)
 
 
 def _colsum(env, mat, rows, cols, like, scale=1.0, out=None):
