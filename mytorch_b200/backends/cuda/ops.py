@@ -282,7 +282,8 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
     # the side stream, if dY is large enough for the two events to pay (64 channels, 128 images of 56x56, forward and
     # backward: 277 -> 261 us).  A deferred weight gradient has the side stream already, and the longer of the two queues.
     want_db = bias is not None and bias.requires_grad
-    beside = want_db and want_dx and not defer_weight_gradient and output_grad._native_array.nbytes >= _BIAS_BESIDE_BYTES
+    beside = (want_db and want_dx and not defer_weight_gradient and env.overlap_weight_gradients
+              and output_grad._native_array.nbytes >= _BIAS_BESIDE_BYTES)
     if beside:
         # Memory before the fork: a block that is free now was last used by work the side stream waits for, one that the calls
         # below give back is still used by theirs.

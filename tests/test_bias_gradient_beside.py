@@ -79,6 +79,13 @@ def test_memory_comes_before_the_fork(monkeypatch, cin, accumulate):
     assert events.index(("memory", (96,))) < fork and names.index("scratch") < fork
 
 
+@pytest.mark.parametrize("more", [{"overlap": False}, {"defer_weight_gradient": True}])
+def test_compute_stream_when_the_side_stream_is_off_or_taken(monkeypatch, more):
+    events, (_, _, db), _ = _backward(monkeypatch, **more)
+    assert [e for e in events if e[0] == "colsum_f32"] == [("colsum_f32", "main")] and db.shape == (96,)
+    assert ("fork" in [e[0] for e in events]) == ("overlap" not in more)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,cin,cout,hw,k", [(2, 64, 64, 16, 3), (3, 48, 82, 13, 3), (2, 3, 64, 32, 3), (2, 3, 64, 32, 7), (1, 20, 7, 9, 1)])
 @pytest.mark.parametrize("accumulate", [False, True])
