@@ -444,6 +444,7 @@ int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, c
   MTB_REQUIRE(mode != 2 || res, "batch_norm2d_add_relu_forward: the tensor to add is missing");
   long long rows = (long long)n * h * w;
   bool aligned = mtb_aligned16(x) && mtb_aligned16(y) && (mode != 2 || mtb_aligned16(res));
+  MTB_REQUIRE(!mask || (aligned && c % 4 == 0), "batch_norm2d_add_relu_forward: a mask needs four channels a byte and 16-byte alignment");
   float* partial = (float*)workspace;
   float* scale = partial + (long long)mtb_col_max_partials() * 3 * c;
   if (training) {
@@ -464,7 +465,6 @@ int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, c
     MTB_LAUNCH(bn_eval_prep_kernel, mtb_div_up(c, 128), 128, 0, st, c, gamma, (float)eps, running_mean, running_var, mean, var, scale);
     MTB_LAUNCH_CHECK("bn_eval_prep_kernel");
   }
-  MTB_REQUIRE(!mask || (aligned && c % 4 == 0), "batch_norm2d_add_relu_forward: a mask needs four channels a byte and 16-byte alignment");
   return launch_normalize(x, y, rows, c, aligned, mean, scale, beta, mode, res, st, nullptr, 0.f, mask);
 }
 
