@@ -75,6 +75,14 @@ def _strides(t):
     return out
 
 
+def _aligned(*tensors):
+    """All on 16-byte boundaries: windows of larger blocks may start at any float."""
+    for t in tensors:
+        if t._native_array.ptr % 16:
+            return False
+    return True
+
+
 # ---------------------------------------------------------------------------- host <-> device
 
 @_reg("cuda", "upload")
@@ -451,7 +459,7 @@ def cuda_batch_norm2d_add_relu(x, residual, weight, bias, eps, training, momentu
     head = (n, c, h, w, x, residual, weight, bias, float(eps), int(use_batch_stats), float(momentum), running_mean,
             running_var, y, mean, var)
     tail = (pre[0] if pre else None, pre[1] if pre else 0, ws, ws_bytes, env.stream())
-    if c % 4 == 0 and not _tracker.no_grad:  # the ReLU's mask goes to backward with the statistics
+    if c % 4 == 0 and not _tracker.no_grad and _aligned(x, residual):  # the ReLU's mask goes to backward with the statistics
         mean._relu_mask = CudaMemory(x.device.index, n * c * h * w // 4)
         env.lib.batch_norm2d_add_relu_forward_masked_f32(*head, mean._relu_mask, *tail)
     else:
@@ -471,7 +479,7 @@ def cuda_batch_norm2d_add_relu_backward(output_grad, mean, var, x, residual, wei
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
     tail = (weight, bias, float(eps), dx, dres, dg, db, ws, ws_bytes, env.stream())
     mask = getattr(mean, "_relu_mask", None)
-    if mask is not None:
+    if mask is not None and _aligned(x, output_grad):
         env.lib.batch_norm2d_add_relu_backward_masked_f32(n, c, h, w, output_grad, mean, var, x, mask, *tail)
     else:
         env.lib.batch_norm2d_add_relu_backward_f32(n, c, h, w, output_grad, mean, var, x, residual, *tail)
