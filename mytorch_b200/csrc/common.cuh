@@ -75,6 +75,10 @@ static inline cudaError_t mtb_launch_after(bool early, void (*kernel)(P...), dim
 
 #define MTB_LAUNCH(kernel, ...) MTB_CUDA(mtb_launch_after(true, kernel, __VA_ARGS__))
 
+// Whether a window of `window` elements lies in `extent` of them with `pad` more on either side: where it does not, an output
+// extent computed as (extent + 2 * pad - window) / stride + 1 may still be 1, as C divides towards zero.
+static inline bool mtb_window_fits(int extent, int pad, int window) { return (long long)extent + 2LL * pad >= window; }
+
 static inline int mtb_div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Grid for a grid-stride bandwidth kernel: enough CTAs to fill the machine a few times over,

@@ -5,6 +5,8 @@
 #include "kernels.h"
 
 MTB_API long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
+  // no such convolution: the call that the scratch is for says so
+  if (n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return 0;
   long long a = mtb_conv2d_wgrad_simt_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   long long b = mtb_tc_conv2d_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   return a > b ? a : b;

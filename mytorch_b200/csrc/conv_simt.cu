@@ -9,6 +9,7 @@ using namespace simt;
 
 int conv_dims(ConvDims& d, int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   MTB_REQUIRE(n > 0 && cin > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0 && ph >= 0 && pw >= 0 && cout > 0, "conv2d: bad shape");
+  MTB_REQUIRE(mtb_window_fits(h, ph, kh) && mtb_window_fits(w, pw, kw), "conv2d: a %dx%d filter is larger than the padded %dx%d input", kh, kw, h, w);
   d = ConvDims{n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, (h + 2 * ph - kh) / sh + 1, (w + 2 * pw - kw) / sw + 1};
   MTB_REQUIRE(d.OH > 0 && d.OW > 0, "conv2d: empty output");
   constexpr long long limit = (1LL << 31) - 256;  // rows and reduction positions are 31-bit numbers, tiles overshoot

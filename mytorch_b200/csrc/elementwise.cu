@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restri
 MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, const float* x, float* out, void* stream) {
   MTB_REQUIRE(x && out && n > 0 && c > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0 && ph >= 0 && pw >= 0, "pack_patches: bad arguments");
   MTB_REQUIRE((long long)kh * kw * c <= 32, "pack_patches: the filter has more than 32 entries");
+  MTB_REQUIRE(mtb_window_fits(h, ph, kh) && mtb_window_fits(w, pw, kw), "pack_patches: a %dx%d window is larger than the padded %dx%d input", kh, kw, h, w);
   PatchRuns d{n, c, h, w, kh, kw, sh, sw, ph, pw, (h + 2 * ph - kh) / sh + 1, (w + 2 * pw - kw) / sw + 1};
   MTB_REQUIRE(d.OH > 0 && d.OW > 0 && mtb_aligned16(out), "pack_patches: empty or unaligned output");
   const long long pixels = (long long)n * d.OH * d.OW;

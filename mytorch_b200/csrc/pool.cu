@@ -295,6 +295,7 @@ __global__ void mask_to_argmax_kernel(const unsigned short* __restrict__ mask, u
 
 int pool_dims(PoolDims& d, int n, int c, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw) {
   MTB_REQUIRE(n > 0 && c > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0 && ph >= 0 && pw >= 0, "max_pool2d: bad shape");
+  MTB_REQUIRE(mtb_window_fits(h, ph, kh) && mtb_window_fits(w, pw, kw), "max_pool2d: a %dx%d window is larger than the padded %dx%d input", kh, kw, h, w);
   d = PoolDims{n, c, h, w, kh, kw, sh, sw, ph, pw, (2 * ph + h - kh) / sh + 1, (2 * pw + w - kw) / sw + 1};
   MTB_REQUIRE(d.OH > 0 && d.OW > 0, "max_pool2d: empty output");
   return MTB_OK;

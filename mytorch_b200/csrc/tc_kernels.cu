@@ -844,6 +844,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
 bool mtb_tc_conv2d_forward_supported(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                      const float* wt, const float* y) {
   if (getenv("MTB_DISABLE_TC")) return false;
+  if (!mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return false;  // the other kernels say so
   if (!al16(x) || !al16(wt) || !al16(y)) return false;
   if (cin % 32 || cout % 4) return false;
   if (sh > 8 || sw > 8 || ph > 100 || pw > 100 || kh > 32 || kw > 32) return false;
@@ -905,6 +906,7 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
 bool mtb_tc_conv2d_dgrad_supported(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                                    const float* wt, const float* dx) {
   if (getenv("MTB_DISABLE_TC")) return false;
+  if (!mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return false;  // the other kernels say so
   if (!al16(dy) || !al16(wt) || !al16(dx)) return false;
   if (cout % 32 || cin % 4) return false;
   if (kh * kw > 64 || sh > 8 || sw > 8 || ph > 64 || pw > 64) return false;
@@ -1406,6 +1408,7 @@ long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, in
 bool mtb_tc_conv2d_wgrad_supported(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                    const float* dy, const float* dw) {
   if (getenv("MTB_DISABLE_TC")) return false;
+  if (!mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return false;  // the other kernels say so
   if (!al16(x) || !al16(dy) || !al16(dw)) return false;
   if (cin % 32 || cout % 4) return false;
   if (sh > 8 || sw > 8 || ph > 100 || pw > 100 || kh > 32 || kw > 32) return false;
