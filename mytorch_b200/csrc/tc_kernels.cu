@@ -866,7 +866,13 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), gp.ns);
   const int bn = staged ? row_bn : gp.bn;
   if (stats_rows) *stats_rows = 0;
-  const bool want_stats = stats && stats_rows && !relu && cout % 32 == 0 && (!bias || al16(bias)) && !getenv("MTB_DISABLE_CONV_STATS");
+  // the statistics and BatchNorm epilogues keep a CTA on one column tile: there must be a CTA for each
+  const bool a_cta_per_column = (cout + bn - 1) / bn <= mtb_sm_count();
+  if (bn_eval && !a_cta_per_column) {
+    const int rc = mtb_tc_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, 0, workspace, workspace_bytes, stream);
+    return rc ? rc : mtb_bn_eval_apply(y, y, M, cout, *bn_eval, residual, relu, (cudaStream_t)stream);
+  }
+  const bool want_stats = stats && stats_rows && a_cta_per_column && !relu && cout % 32 == 0 && (!bias || al16(bias)) && !getenv("MTB_DISABLE_CONV_STATS");
   CUtensorMap mapA, mapB;
   int rc = tc::encode_tiled_2d(&mapB, wt, cout, K, K, 32, bn);
   if (rc) return rc;
