@@ -7,7 +7,7 @@ initialisation consumes one random draw per weight / bias tensor in creation ord
 """
 import mytorch_b200.nn as nn
 import mytorch_b200.nn.functional as F
-from mytorch_b200.nn.batch_norm import inference_conv_norm
+from mytorch_b200.nn.batch_norm import inference_conv_norm, runs_as_written
 
 
 class Flatten(nn.Module):
@@ -35,9 +35,9 @@ def _feed_batch_norm(*convs):
 
 def _conv_norm(conv, norm, x, *residual):
     """norm(conv(x), *residual), in the convolution's launch where nothing is differentiated."""
-    kind = type(norm)
-    if not norm.training and (kind is not nn.BatchNorm2d or not residual):
-        y = inference_conv_norm(conv, norm, x, kind is not nn.BatchNorm2d, *residual)
+    kinds = (nn.BatchNormAddReLU2d,) if residual else (nn.BatchNorm2d, nn.BatchNormReLU2d)
+    if not norm.training and runs_as_written(norm, *kinds) and runs_as_written(conv, nn.Conv2d):
+        y = inference_conv_norm(conv, norm, x, type(norm) is not nn.BatchNorm2d, *residual)
         if y is not None:
             return y
     return norm(conv(x), *residual)

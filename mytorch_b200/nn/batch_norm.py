@@ -72,6 +72,12 @@ class BatchNorm1d(BatchNorm2d):
         return y.reshape(x.shape)
 
 
+def runs_as_written(layer, *kinds):
+    """Whether a layer is one of these classes itself and runs its class's forward: what may be replaced by an operator that does
+    the same.  A subclass, or a forward put on the instance (to wrap or trace it), is called."""
+    return type(layer) in kinds and "forward" not in layer.__dict__
+
+
 def inference_conv_norm(conv, norm, x, relu=False, residual=None):
     """``norm(conv(x))``, then optionally ``+ residual``, then optionally ReLU, as one operator where that is possible: a
     convolution and a BatchNorm layer that normalises with its running statistics, on CUDA, with no gradient to record.
