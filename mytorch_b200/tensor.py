@@ -55,14 +55,15 @@ class Device:
     """``"cpu"``, ``"cuda"`` or ``"cuda:<index>"`` (mytorch/tensor.py:52-81).  One object per device: equality is
     identity, so the checks every operator makes cost nothing."""
 
-    _known = {}
+    _known, _named = {}, {}  # by (type, index), by the text asked for
+    _unpickled = object()
 
-    def __new__(cls, device=None):
-        if device is None:  # unpickling: the state follows, and Device(that object) is the known one
+    def __new__(cls, device=_unpickled):
+        if device is Device._unpickled:  # a pickle without __reduce__: the state follows, and Device(that object) is the known one
             return object.__new__(cls)
         if isinstance(device, Device):
             return cls._known.setdefault((device.type, device.index), device)
-        found = cls._known.get(device)
+        found = cls._named.get(device) if isinstance(device, str) else None
         if found is None:
             head, sep, tail = device.strip().partition(":")
             key = (head.strip(), int(tail) if sep else None)
@@ -71,7 +72,7 @@ class Device:
                 found = object.__new__(cls)
                 found.type, found.index = key
                 found = cls._known.setdefault(key, found)
-            cls._known[device] = found
+            cls._named[device] = found
         return found
 
     def __reduce__(self):
