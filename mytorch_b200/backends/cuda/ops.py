@@ -729,14 +729,15 @@ def cuda_pow(x, y):
 
 
 # ``needed``: which of the two gradients the caller will use (the tape has no use for one towards a constant, such as the
-# exponent of ``x ** 2``); the other is then None instead of being computed.
+# exponent of ``x ** 2``); the other is then None instead of being computed.  The front-end hands it to functions that are
+# marked for it (``skips_gradients``).
 _BOTH = (True, True)
 
 
 @_reg("cuda", "add_backward")
 def cuda_add_backward(output_grad, x, y, alpha, needed=_BOTH):
-    # Same-shape operands receive the upstream gradient itself (no copy): nothing mutates
-    # gradients in place, accumulation always writes a fresh tensor.
+    # Same-shape operands receive the upstream gradient itself (no copy): the tape lets no operator change a
+    # gradient in place that is not its tensor's alone.
     return (_reduce_to(output_grad, x.shape, x) if needed[0] else None,
             _reduce_to(_scaled(output_grad, alpha), y.shape, y) if needed[1] else None)
 
@@ -768,6 +769,10 @@ def cuda_pow_backward(output_grad, x, y, needed=_BOTH):
     """dx = y x^(y-1) dy, dy_ = x^y ln(x) dy (``mytorch/backends/cpu/ops/broadcast_binary_ops.py:130-137``)."""
     return (_reduce_to(_binary("mul", _binary("pow_dx", x, y), output_grad), x.shape, x) if needed[0] else None,
             _reduce_to(_binary("mul", _binary("pow_dy", x, y), output_grad), y.shape, y) if needed[1] else None)
+
+
+for _f in (cuda_add_backward, cuda_sub_backward, cuda_mul_backward, cuda_div_backward, cuda_pow_backward):
+    _f.skips_gradients = True
 
 
 # ---------------------------------------------------------------------------- max / eq / bmm
