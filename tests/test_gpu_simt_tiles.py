@@ -48,5 +48,5 @@ def test_convolution(n, cin, cout, h, w, kh, kw, stride, pad, monkeypatch):
     y = g.op("conv2d")(xt, wtt, bt, stride, pad)
     dx, dw, db = g.op("conv2d_backward")(g.dev(dy), xt, wtt, bt, stride, pad)
     rdx, rdw, rdb = O.conv2d_backward(dy, x, wt, True, stride, pad)
-    for got, ref in ((y, want), (dx, rdx), (dw, rdw)):
+    for got, ref in ((y, want), (dx, rdx), (dw, rdw), (db, rdb)):
         assert rel_err(g.host(got), ref) < 1e-5
