@@ -87,8 +87,9 @@ int mtb_graph_destroy(void* graph_exec);
  *      mytorch/backends/cuda/ops/conv.py:9-90) ---- */
 long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
 /* y[N,OH,OW,Cout] = conv(x[N,H,W,Cin], wt[Cout,KH,KW,Cin]) + bias (bias may be NULL); relu != 0 clamps at 0.
- * workspace (mtb_conv2d_workspace_bytes(); may be NULL): lets a layer with too few output tiles to fill the
- * GPU split its reduction across CTAs; the partials are added in a fixed order, results are reproducible. */
+ * workspace: not used, may be NULL (only the weight gradient needs mtb_conv2d_workspace_bytes()).  A layer with too few output
+ * tiles to fill the GPU splits its reduction over a cluster of CTAs, which add in a fixed order: results are reproducible.
+ * A filter larger than the padded input is refused by every entry point. */
 int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                            const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes, void* stream);
 /* The same forward pass for a convolution whose output feeds a BatchNorm layer: where the kernel family
@@ -104,7 +105,7 @@ int mtb_conv2d_forward_stats_f32(int n, int cin, int h, int w, int kh, int kw, i
                                  long long workspace_bytes, void* stream);
 /* Inference: y = batch_norm(conv(x) + bias) (+ residual) (ReLU) with running statistics, in one launch (the reference runs
  * conv2d, batch_norm2d, add and relu: mytorch/nn/conv.py:71, mytorch/nn/batch_norm.py:123-135, mytorch/nn/relu.py:5-10).
- * gamma, beta, bias and residual (shape of y) may be NULL; the bits are those of the separate operators. */
+ * gamma, beta, bias and residual (shape of y; given only with relu != 0) may be NULL; the bits are those of the separate operators. */
 int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                               const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
                               const float* running_var, double eps, const float* residual, int relu, float* y, void* workspace,

@@ -159,7 +159,7 @@ def _stem_form(x_shape, w_shape, stride, padding):
     if c >= _TC_CHANNELS or cout % 4 or n * h * w * _TC_CHANNELS * 4 < (1 << 17):
         return None
     oh, ow = (h + 2 * ph - kh) // sh + 1, (w + 2 * pw - kw) // sw + 1
-    if c == 1:  # 28x28 digits: no gain was measured from fewer blocks (the step is all launches), so the form stays
+    if c == 1:  # measured on 28x28 digits only, where a step is all launches and fewer blocks gain nothing; larger images were not
         return None, (n, _TC_CHANNELS, h, w, kh, kw, sh, sw, ph, pw, cout)
     if kh * kw * c <= _TC_CHANNELS:
         return (kh, kw, sh, sw, ph, pw), (n, _TC_CHANNELS, oh, ow, 1, 1, 1, 1, 0, 0, cout)
@@ -288,7 +288,9 @@ def cuda_conv2d_backward(output_grad, input, weight, bias, stride, padding, accu
     dx = dw = db = None
     # The bias gradient reads all of dY and needs little else of an SM, so it goes beside the tensor-core kernels of this call on
     # the side stream, if dY is large enough for the two events to pay (64 channels, 128 images of 56x56, forward and
-    # backward: 277 -> 261 us).  A deferred weight gradient has the side stream already, and the longer of the two queues.
+    # backward, cold L2: 287 -> 266 us; 48 -> 82 channels, 32 images of 37x37, under the limit: 442 us with and without; no
+    # sizes in between were measured).  For direct calls of the operator: the tape defers weight gradients, and a deferred one
+    # has the side stream already, and the longer of the two queues.
     want_db = bias is not None and bias.requires_grad
     beside = (want_db and want_dx and not defer_weight_gradient and env.overlap_weight_gradients
               and output_grad._native_array.nbytes >= _BIAS_BESIDE_BYTES)
@@ -376,7 +378,7 @@ def cuda_linear(x, weight, bias):
     b, fin = x.shape
     fout = weight.shape[0]
     if weight.shape[1] != fin:
-            raise MismatchShapesError([x.shape, weight.shape])
+        raise MismatchShapesError([x.shape, weight.shape])
     y = _new((b, fout), x)
     _gemm(env, b, fout, fin, x, 0, weight, 1, bias, 0, y)
     return y
@@ -405,7 +407,7 @@ def cuda_mm(x, y):
     env = _env(x)
     (m, k), (k2, n) = x.shape, y.shape
     if k != k2:
-            raise MismatchShapesError([x.shape, y.shape])
+        raise MismatchShapesError([x.shape, y.shape])
     z = _new((m, n), x)
     _gemm(env, m, n, k, x, 0, y, 0, None, 0, z)
     return z
@@ -449,7 +451,7 @@ def cuda_batch_norm2d_add_relu(x, residual, weight, bias, eps, training, momentu
     """max(0, batch_norm2d(x) + residual) in one normalise pass; returns (y, mean, var)."""
     _f32(x, residual, weight, bias, running_mean, running_var)
     if x.shape != residual.shape:
-            raise MismatchShapesError([x.shape, residual.shape])
+        raise MismatchShapesError([x.shape, residual.shape])
     env = _env(x)
     n, c, h, w = x.shape
     y, mean, var = _new(x.shape, x), _new((c,), x), _new((c,), x)
@@ -584,7 +586,7 @@ def cuda_add_relu(x, y):
     """max(0, x + y) for same-shape operands (residual connection followed by ReLU)."""
     _f32(x, y)
     if x.shape != y.shape:
-            raise MismatchShapesError([x.shape, y.shape])
+        raise MismatchShapesError([x.shape, y.shape])
     env = _env(x)
     z = _new(x.shape, x)
     env.lib.add_relu_f32(x, y, z, _numel(x.shape), env.stream())
@@ -630,7 +632,7 @@ def cuda_normal(x, seed, mean, stddev):
 def cuda_copy(dst, src):
     env = _env(dst)
     if dst.shape != src.shape:
-            raise MismatchShapesError([dst.shape, src.shape])
+        raise MismatchShapesError([dst.shape, src.shape])
     if dst.dtype is float32:
         env.lib.copy_f32(dst, src, _numel(dst.shape), env.stream())
     else:

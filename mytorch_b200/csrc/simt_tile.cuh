@@ -16,7 +16,7 @@
 //   * small problems split the reduction over the CTAs of a cluster, which add their tiles through distributed
 //     shared memory in rank order: one launch, no scratch, the same bits every time.
 // 48 -> 82 channels, 3x3, 32 images of 37x37, 3.1 GFLOP each: forward 383 -> 110 us, data gradient 585 -> 154 us, weight
-// gradient 606 -> 142 us; 4095 x 4095 x 1023: 47 TFLOP/s; one output of a single image (128 -> 32 channels on 7x7):
+// gradient 606 -> 171 us; 4095 x 4095 x 1023: 47 TFLOP/s; one output of a single image (128 -> 32 channels on 7x7):
 // 224 -> 10 us.
 #pragma once
 #include "common.cuh"

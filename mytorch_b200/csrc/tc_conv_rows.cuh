@@ -176,7 +176,7 @@ tc_conv_rows_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
               if (BMODE == B_KMAJOR) {
                 tma_load_2d(b_dst, &mapB, bfull, tap * p.kc_total + cc * 32, n0);
               } else {
-              if (p.b_blocks) {
+                if (p.b_blocks) {
                   tma_load_3d(b_dst, &mapB, bfull, 0, cc * 32, (p.b_tap_x[tap] + n0) / 32);
                 } else {
 #pragma unroll

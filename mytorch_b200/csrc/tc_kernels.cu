@@ -171,9 +171,10 @@ __device__ __forceinline__ float4 ld_shared4(uint32_t a) {
 // work, and four MMAs of a narrow tile are only 192-256 cycles of work, so tiles up to 128 wide
 // take two blocks (8 MMAs) per stage.
 //
-// 32-wide tiles are for matrices of at most 64 rows and a long reduction (the classifier of a small network): their time is what
-// one SM loads, so A comes in boxes of 64 rows (the MMA's rows 64 to 127 read what lies behind them and are never stored) and a
-// stage takes four blocks.  64 x 128, K = 9216: 53 -> 40 us, the same bits.
+// 32-wide tiles are for matrices of at most 64 rows (the classifier of a small network), whatever the reduction: their time is
+// what one SM loads, so A comes in boxes of 64 rows (the MMA's rows 64 to 127 read what lies behind them and are never stored)
+// and a stage takes four blocks.  64 x 128, K = 9216: 53 -> 40 us, the same bits.  Against 64 columns and more, 32 and 64 rows,
+// 32 to 4736 columns, K = 32 to 9216, cold: up to K = 512 within 1 us either way, from there on faster (K = 2048 by 15 %).
 template <int BN>
 struct Cfg {
   static constexpr int kKB = BN == 32 ? 4 : BN <= 128 ? 2 : 1;
@@ -650,9 +651,10 @@ int launch_tc_bn(int bn, const CUtensorMap& mapA, const CUtensorMap& mapB, const
 
 int pick_bn(int n) { return n <= 64 ? 64 : (n <= 128 ? 128 : 256); }
 
-// Tile width for a GEMM with `rows` output rows: the widest tile (best MMA efficiency) that still
+// Tile width of the row-staged kernels for `rows` output rows: the widest tile (best MMA efficiency) that still
 // yields enough tiles to occupy most SMs; small problems (late layers at small batch) fall back
-// to narrower tiles so that more CTAs take part.
+// to narrower tiles so that more CTAs take part.  A rule, not a price (the im2col kernel's width is priced: cheapest_bn);
+// row_conv_pays then compares the price of the width it gives.
 int pick_bn_for(int n, long long rows) {
   const long long m_tiles = (rows + 127) / 128;
   const int want = mtb_sm_count() * 3 / 4;
@@ -713,12 +715,14 @@ int cluster_units(int size) {
 }
 
 // Tile width and reduction split of the im2col kernel.  A layer with few pixels leaves most of the GPU idle on wide tiles and
-// spends its time on loading the pixels again for every narrow one (a block of 32 takes 64 columns 175 ns, 256 columns 280),
+// spends its time on loading the pixels again for every narrow one (kb_ns: a block of 32 takes 64 columns 232 ns, 256 columns 376),
 // so its long reduction is split over a cluster of 2, 4 or 8 CTAs on wide tiles, one unit per CTA, as long as all units fit
 // the GPU at once.  Times of a split launch as measured (512 -> 512 channels on 4x4, 16 to 128 images): base (launch, pipeline
 // fill, exchange, epilogue) + blocks per unit x block time.  128 images, before -> now: forward 31 -> 22 us, data gradient
 // 38.5 -> 23.5 us; 64 images (before: partial sums through global memory) 19.0 -> 15 and 21.4 -> 16.5 us; 256 -> 256 on 8x8,
-// 64 images: 18.8 -> 14.5 and 22.6 -> 16 us.  Under 64 blocks the exchange costs what the split gains.
+// 64 images: 18.8 -> 14.5 and 22.6 -> 16 us.  Under 64 blocks the exchange costs what the split gains.  The block times fitted
+// to these launches (180 / 200 / 280 ns) are a quarter below kb_ns, which was fitted to launches over larger images; what
+// makes the difference was not looked into, so neither set should be used for the other kind of launch.
 // `copies` launches of this size share the GPU, of which this one may split.
 struct GemmPlan { int bn, splits, kb_per_split; double ns; };
 
