@@ -88,6 +88,8 @@ def inference_conv_norm(conv, norm, x, relu=False, residual=None):
         return None
     weight, device, dtype = conv.weight, x.device, x.dtype
     ok = weight.shape[0] == norm.num_features
+    for t in (norm.weight, norm.bias, norm.running_mean, norm.running_var):  # layers' tensors may have been replaced
+        ok = ok and (t is None or t.shape == weight.shape[:1])
     for t in (weight, norm.running_mean, norm.running_var, conv.bias, norm.weight, norm.bias, residual):
         ok = ok and (t is None or (t.device is device and t.dtype is dtype))
     if not ok:

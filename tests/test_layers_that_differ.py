@@ -79,6 +79,21 @@ def test_forward_on_an_instance_is_called(operators):
         seen.clear()
 
 
+@pytest.mark.parametrize("name", ["weight", "bias", "running_mean", "running_var"])
+def test_vectors_of_another_length_go_to_the_layer_that_checks_them(operators, name):
+    conv, norm = nn.Conv2d(4, 4, 1), nn.BatchNorm2d(4)
+    other = nn.BatchNorm2d(3)
+    x = _on_device(conv, norm, other)
+    setattr(norm, name, getattr(other, name))
+    with mt.no_grad():
+        if name in ("weight", "bias"):
+            with pytest.raises(RuntimeError, match="shape"):
+                _conv_norm(conv, norm, x)
+        else:
+            _conv_norm(conv, norm, x)
+    assert "conv2d_batch_norm" not in [o[0] for o in operators]
+
+
 def test_residual_goes_to_the_layer_that_adds_it(operators):
     conv, norm = nn.Conv2d(4, 4, 1), nn.BatchNormAddReLU2d(4)
     x = _on_device(conv, norm)
