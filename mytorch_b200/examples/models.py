@@ -7,7 +7,7 @@ initialisation consumes one random draw per weight / bias tensor in creation ord
 """
 import mytorch_b200.nn as nn
 import mytorch_b200.nn.functional as F
-from mytorch_b200.nn.batch_norm import inference_conv_norm, runs_as_written
+from mytorch_b200.nn.batch_norm import inference_conv_norm
 
 
 class Flatten(nn.Module):
@@ -35,9 +35,10 @@ def _feed_batch_norm(*convs):
 
 def _conv_norm(conv, norm, x, *residual):
     """norm(conv(x), *residual), in the convolution's launch where nothing is differentiated."""
-    kinds = (nn.BatchNormAddReLU2d,) if residual else (nn.BatchNorm2d, nn.BatchNormReLU2d)
-    if not norm.training and runs_as_written(norm, *kinds) and runs_as_written(conv, nn.Conv2d):
-        y = inference_conv_norm(conv, norm, x, type(norm) is not nn.BatchNorm2d, *residual)
+    kind = type(norm)
+    expected = kind is nn.BatchNormAddReLU2d if residual else kind is nn.BatchNorm2d or kind is nn.BatchNormReLU2d
+    if expected and type(conv) is nn.Conv2d and not (norm.training or conv._forward_replaced or norm._forward_replaced):
+        y = inference_conv_norm(conv, norm, x, kind is not nn.BatchNorm2d, *residual)
         if y is not None:
             return y
     return norm(conv(x), *residual)

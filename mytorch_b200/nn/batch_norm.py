@@ -5,7 +5,7 @@ from mytorch_b200.dtype import float32
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d, _batch_norm2d_add_relu, _batch_norm2d_relu
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.parameter import Parameter
-from mytorch_b200.ops._common import dispatch, grad_enabled
+from mytorch_b200.ops._common import dispatch, grad_enabled, tracker
 from mytorch_b200.tensor import Tensor
 
 
@@ -72,28 +72,24 @@ class BatchNorm1d(BatchNorm2d):
         return y.reshape(x.shape)
 
 
-def runs_as_written(layer, *kinds):
-    """Whether a layer is one of these classes itself and runs its class's forward: what may be replaced by an operator that does
-    the same.  A subclass, or a forward put on the instance (to wrap or trace it), is called."""
-    return type(layer) in kinds and "forward" not in layer.__dict__
-
-
 def inference_conv_norm(conv, norm, x, relu=False, residual=None):
     """``norm(conv(x))``, then optionally ``+ residual``, then optionally ReLU, as one operator where that is possible: a
     convolution and a BatchNorm layer that normalises with its running statistics, on CUDA, with no gradient to record.
     None elsewhere.  Same bits as the separate layers."""
-    if norm.training or norm.running_mean is None or x.device.type != "cuda":
+    mean, device = norm.running_mean, x.device
+    if norm.training or mean is None or device.type != "cuda":
         return None
-    if grad_enabled(x, conv.weight, conv.bias, norm.weight, norm.bias, residual):
+    weight, bias, gamma, beta, var = conv.weight, conv.bias, norm.weight, norm.bias, norm.running_var
+    if not tracker.no_grad and grad_enabled(x, weight, bias, gamma, beta, residual):
         return None
-    weight, device, dtype = conv.weight, x.device, x.dtype
-    ok = weight.shape[0] == norm.num_features
-    for t in (norm.weight, norm.bias, norm.running_mean, norm.running_var):  # layers' tensors may have been replaced
-        ok = ok and (t is None or t.shape == weight.shape[:1])
-    for t in (weight, norm.running_mean, norm.running_var, conv.bias, norm.weight, norm.bias, residual):
-        ok = ok and (t is None or (t.device is device and t.dtype is dtype))
-    if not ok:
-        return None  # the separate operators say what is wrong
-    affine = norm.weight is not None and norm.bias is not None
-    return dispatch(x.device, "conv2d_batch_norm")(x, conv.weight, conv.bias, conv.stride, conv.padding, norm.weight if affine else None,
-                                                   norm.bias if affine else None, norm.running_mean, norm.running_var, norm.eps, relu, residual)
+    dtype, channels = x.dtype, weight.shape[:1]
+    # layers' tensors may have been replaced: the separate operators say what is wrong
+    for t in (mean, var, gamma, beta):
+        if t is not None and (t.shape != channels or t.device is not device or t.dtype is not dtype):
+            return None
+    for t in (weight, bias, residual):
+        if t is not None and (t.device is not device or t.dtype is not dtype):
+            return None
+    if gamma is None or beta is None:
+        gamma = beta = None
+    return dispatch(device, "conv2d_batch_norm")(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, relu, residual)

@@ -13,13 +13,11 @@ def conv2d(input: Tensor, weight: Tensor, bias=None, stride=1, padding=0, bn_sta
         raise MismatchDataTypesError([t.dtype for t in (input, weight, bias) if t is not None])
     stride = (stride, stride) if isinstance(stride, int) else tuple(stride)
     padding = (padding, padding) if isinstance(padding, int) else tuple(padding)
-    extra, packed = {}, []
-    if input.device.type == "cuda":
-        if bn_stats:
-            extra["bn_stats"] = True
-        if grad_enabled(weight):
-            extra["packed"] = packed
-    out = dispatch(input.device, "conv2d")(input, weight, bias, stride, padding, **extra)
+    packed = [] if weight.requires_grad and not tracker.no_grad else None
+    if input.device.type == "cuda" and (bn_stats or packed is not None):
+        out = dispatch(input.device, "conv2d")(input, weight, bias, stride, padding, bn_stats, packed)
+    else:
+        out = dispatch(input.device, "conv2d")(input, weight, bias, stride, padding)
     out.requires_grad = grad_enabled(input, weight, bias)
     record("conv2d", [input, weight, bias, stride, padding], out)
     if packed:  # kept by this node alone: it lives as long as the graph and belongs to the values forward saw

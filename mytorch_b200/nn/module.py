@@ -10,6 +10,9 @@ _log = logging.getLogger("mytorch_b200")
 
 
 class Module:
+    # a forward was put on the instance (to wrap or trace it): it has to be called, no operator may stand in for the layer
+    _forward_replaced = False
+
     def __init__(self):
         object.__setattr__(self, "_parameters", {})
         object.__setattr__(self, "_buffers", {})
@@ -33,6 +36,8 @@ class Module:
         object.__setattr__(self, name, module)
 
     def __setattr__(self, name, value):
+        if name == "forward":
+            object.__setattr__(self, "_forward_replaced", True)
         if isinstance(value, Module):
             self.register_module(name, value)
         elif isinstance(value, Parameter):

@@ -1,8 +1,10 @@
-from mytorch_b200.nn.batch_norm import BatchNorm2d, BatchNormReLU2d, inference_conv_norm, runs_as_written
+from mytorch_b200.nn.batch_norm import BatchNorm2d, BatchNormReLU2d, inference_conv_norm
 from mytorch_b200.nn.conv import Conv2d
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.relu import ReLU
+
+_NORMS = (BatchNorm2d, BatchNormReLU2d)
 
 
 class Sequential(Module):
@@ -20,14 +22,16 @@ class Sequential(Module):
         i = 0
         while layers[i] is not None:
             layer, after = layers[i], layers[i + 1]
-            if runs_as_written(layer, Conv2d) and runs_as_written(after, BatchNorm2d, BatchNormReLU2d) and not after.training:
-                relu = type(after) is BatchNorm2d and runs_as_written(layers[i + 2], ReLU)
-                y = inference_conv_norm(layer, after, input, relu or type(after) is BatchNormReLU2d)
+            kind, kind_after = type(layer), type(after)
+            if kind is Conv2d and kind_after in _NORMS and not (after.training or layer._forward_replaced or after._forward_replaced):
+                behind = layers[i + 2]
+                relu = kind_after is BatchNorm2d and type(behind) is ReLU and not behind._forward_replaced
+                y = inference_conv_norm(layer, after, input, relu or kind_after is BatchNormReLU2d)
                 if y is not None:
                     input = y
                     i += 3 if relu else 2
                     continue
-            if runs_as_written(layer, BatchNorm2d) and runs_as_written(after, ReLU) and input.device.type == "cuda":
+            if kind is BatchNorm2d and kind_after is ReLU and input.device.type == "cuda" and not (layer._forward_replaced or after._forward_replaced):
                 input = _batch_norm2d_relu(input, layer.weight, layer.bias, layer.eps, layer.training, layer.momentum, layer.running_mean,
                                            layer.running_var)
                 i += 2
