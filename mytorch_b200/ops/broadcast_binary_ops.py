@@ -32,37 +32,47 @@ def pow(x: Tensor, y: Tensor) -> Tensor:
     return _binary("pow", x, y)
 
 
-def _gradients(name, output_grad, x, y, *extra):
-    """Both gradients, or, from a backend function that can leave one out (``skips_gradients``), those the tape will use."""
-    backend = dispatch(x.device, name)
-    if getattr(backend, "skips_gradients", False):
-        return backend(output_grad, x, y, *extra, needed=(x.requires_grad, y.requires_grad))
-    return backend(output_grad, x, y, *extra)
-
+# Backend functions that can leave a gradient out are marked ``skips_gradients`` and told which ones the tape will use; others are
+# called with their documented arguments and compute both.
 
 @tracker.register_backward_function("add")
 def add_backward(output_grad, x, y, alpha):
-    return _gradients("add_backward", output_grad, x, y, alpha)
+    backend = dispatch(x.device, "add_backward")
+    if hasattr(backend, "skips_gradients"):
+        return backend(output_grad, x, y, alpha, needed=(x.requires_grad, y.requires_grad))
+    return backend(output_grad, x, y, alpha)
 
 
 @tracker.register_backward_function("sub")
 def sub_backward(output_grad, x, y, alpha):
-    return _gradients("sub_backward", output_grad, x, y, alpha)
+    backend = dispatch(x.device, "sub_backward")
+    if hasattr(backend, "skips_gradients"):
+        return backend(output_grad, x, y, alpha, needed=(x.requires_grad, y.requires_grad))
+    return backend(output_grad, x, y, alpha)
 
 
 @tracker.register_backward_function("mul")
 def mul_backward(output_grad, x, y):
-    return _gradients("mul_backward", output_grad, x, y)
+    backend = dispatch(x.device, "mul_backward")
+    if hasattr(backend, "skips_gradients"):
+        return backend(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
+    return backend(output_grad, x, y)
 
 
 @tracker.register_backward_function("div")
 def div_backward(output_grad, x, y):
-    return _gradients("div_backward", output_grad, x, y)
+    backend = dispatch(x.device, "div_backward")
+    if hasattr(backend, "skips_gradients"):
+        return backend(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
+    return backend(output_grad, x, y)
 
 
 @tracker.register_backward_function("pow")
 def pow_backward(output_grad, x, y):
-    return _gradients("pow_backward", output_grad, x, y)
+    backend = dispatch(x.device, "pow_backward")
+    if hasattr(backend, "skips_gradients"):
+        return backend(output_grad, x, y, needed=(x.requires_grad, y.requires_grad))
+    return backend(output_grad, x, y)
 
 
 def _copy(x: Tensor, y: Tensor):
