@@ -133,6 +133,16 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorM
       ::"r"(dst), "l"(map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
       : "memory");
 }
+// ---- TMA stores (shared -> global; rows and columns outside the tensor are not written) ----
+// Writes to the source must be made visible to the copy engine first (fence_proxy_async by the writers, then a barrier).
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// all but the N newest groups of this thread have read their source / have completed
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -296,6 +306,26 @@ struct WarpColStats {
     mean[c] += d * wb;
     m2[c] += q + d * d * n * wb;
   }
+  // o: the first `rows` (1 to 32) values of this lane's column of chunk `c`; the same update without exchanges between lanes
+  __device__ __forceinline__ void add_column(int c, const float (&o)[32], int rows) {
+    const float cnt = (float)rows;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 32; ++k) s[k & 3] += k < rows ? o[k] : 0.f;
+    const float mt = ((s[0] + s[1]) + (s[2] + s[3])) / cnt;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const float d = k < rows ? o[k] - mt : 0.f;
+      s[k & 3] = fmaf(d, d, s[k & 3]);
+    }
+    const float q = (s[0] + s[1]) + (s[2] + s[3]);
+    const float wb = cnt / (n + cnt);
+    const float d = mt - mean[c];
+    mean[c] += d * wb;
+    m2[c] += q + d * d * n * wb;
+  }
   // one partial row [3][C] (count, mean, M2) at columns col0 + 32 c + lane
   __device__ __forceinline__ void store(float* row, int C, int col0, int ncols, int lane) const {
 #pragma unroll
@@ -376,6 +406,8 @@ __device__ __forceinline__ void load_bn_columns(BnColumns<BN>& t, const MtbBnEva
 // mn_major selects the 32-byte-atom swizzle that MN-major tcgen05 operands need.
 int encode_tiled_2d(CUtensorMap* map, const float* base, long long rows, long long cols, long long pitch_elems, int box_cols, int box_rows,
                     bool mn_major = false);
+// The same K-major layout for results and what is added to them: fp32 values as they are, boxes of 32 columns x 32 rows.
+int encode_result_2d(CUtensorMap* map, const float* base, long long rows, long long cols, long long pitch_elems);
 // The same matrix seen as blocks of 32 columns (cols % 32 == 0): one load brings `blocks` neighbouring blocks of
 // box_rows rows, one after the other, each as the MN-major operands want it.  Coordinates: (0, row, block).
 // A producer thread spends about 100 cycles per copy it issues; with one 4 KB copy per block the data gradient of a

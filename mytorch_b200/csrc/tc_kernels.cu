@@ -62,6 +62,19 @@ int encode_tiled_2d(CUtensorMap* map, const float* base, long long rows, long lo
   return MTB_OK;
 }
 
+int encode_result_2d(CUtensorMap* map, const float* base, long long rows, long long cols, long long pitch_elems) {
+  int rc = load_driver_entry_points();
+  if (rc) return rc;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)pitch_elems * 4};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return mtb_fail(MTB_ERR_CUDA, "cuTensorMapEncodeTiled (result) failed (%d) rows=%lld cols=%lld pitch=%lld", (int)r, rows, cols, pitch_elems);
+  return MTB_OK;
+}
+
 int encode_blocks_3d(CUtensorMap* map, const float* base, long long rows, long long cols, long long pitch_elems, int box_rows, int blocks) {
   int rc = load_driver_entry_points();
   if (rc) return rc;
@@ -129,6 +142,9 @@ struct GemmParams {
   const float* addend;
   MtbBnEval bn;  // EPI_BN
   int relu;
+  // results (and the addend) move through shared memory by bulk copies (see the epilogue); rows lie one after the other
+  int bulk_out;
+  int stages;  // of the ring
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
   // MN-major operands through one copy per reduction block (encode_blocks_3d) instead of one per 32 columns
@@ -160,6 +176,14 @@ __device__ __forceinline__ uint32_t cluster_address(uint32_t smem, uint32_t rank
 __device__ __forceinline__ void st_cluster4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+__device__ __forceinline__ void st_shared4(uint32_t a, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ float ld_shared1(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 ld_shared4(uint32_t a) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
@@ -183,7 +207,6 @@ struct Cfg {
   static constexpr uint32_t kABytes = kRowsA * 32 * 4;   // one reduction block of A
   static constexpr uint32_t kBBytes = BN * 32 * 4;    // one reduction block of B
   static constexpr uint32_t kStageBytes = kKB * (kABytes + kBBytes);  // [A blocks][B blocks]
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 1024;  // + alignment slack
   static constexpr uint32_t kTmemCols = 2 * BN;
 };
 
@@ -193,15 +216,36 @@ enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3 };
 
 constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
 
+// Shared memory: the stages, then what the epilogue warps hand to the copy engine, in blocks of 32 rows x 32 columns (128-byte
+// swizzle): one block per warp, two where a tensor is added (one arrives while the other is being stored).  Those kernels are
+// bound by what the epilogue moves, not by the main loop, and keep fewer stages: what they leave of the SM's shared memory is
+// where BatchNorm's partial sums and the weight gradients' reductions of the side stream run beside them (ResNet-50 step, 128
+// images, with two stages for additions 19.24 ms, with three 19.36; statistics of 256-wide tiles want all four: 19.23 against 19.33).
+constexpr uint32_t kOutBlock = 32 * 32 * 4;
+template <int BN, int EPI, bool SPLIT>
+struct GemmSmem {
+  static constexpr bool kBulk = !SPLIT && BN >= 64 && EPI != EPI_BN;
+  static constexpr int kOutBlocks = !kBulk ? 0 : EPI == EPI_ADD ? 2 : 1;  // per warp
+  static constexpr int stages(bool bulk) {
+    return !bulk ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 256 ? 4 : 3) : (BN == 128 ? 2 : 3);
+  }
+  static constexpr uint32_t bytes(bool bulk) {  // + alignment slack
+    return stages(bulk) * Cfg<BN>::kStageBytes + (bulk ? kEpilogueWarps * kOutBlocks * kOutBlock : 0) + 1024;
+  }
+  static constexpr uint32_t kMost = kBulk && bytes(true) > bytes(false) ? bytes(true) : bytes(false);
+};
+
 // SPLIT: GemmParams::splits > 1, a kernel of its own because the exchange takes the registers that the other epilogues need.
 template <int BN, int AMODE, int BMODE, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p) {
+tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapOut,
+               const __grid_constant__ CUtensorMap mapAdd, const GemmParams p) {
   using C = Cfg<BN>;
-  constexpr int STAGES = C::kStages;
+  using Smem = GemmSmem<BN, EPI, SPLIT>;
+  const int STAGES = p.stages;
   constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN, ADD = EPI == EPI_ADD || BNORM;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
+  __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2], bar_add[kEpilogueWarps][2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
@@ -217,6 +261,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
       mbar_init(smem_u32(&bar_tempty[b]), kEpilogueWarps);  // one arrival per epilogue warp
+      if constexpr (EPI == EPI_ADD)
+        for (int w = 0; w < kEpilogueWarps; ++w) mbar_init(smem_u32(&bar_add[w][b]), 1);
     }
     abort_flag = 0;
     fence_barrier_init();
@@ -366,12 +412,119 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     int t = 0;
     const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0);
     const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 31u) == 0);  // 32-byte stores
-    // statistics variant: narrow tiles keep per-lane sums (cheap per tile), wide tiles merge per tile
-    constexpr bool LANE_SUMS = STATS && BN == 64;
+    // statistics of a split reduction: narrow tiles keep per-lane sums, wide tiles merge per tile
+    constexpr bool LANE_SUMS = STATS && SPLIT && BN == 64;
     WarpColStats<(STATS && !LANE_SUMS) ? COLS / 32 : 1> stats;
     LaneColSums<LANE_SUMS ? COLS / 32 : 1> sums;
     if constexpr (LANE_SUMS) sums.reset(); else stats.reset();
-    for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
+    bool bulk = false;
+    if constexpr (Smem::kBulk) {
+      // Results through shared memory and the copy engine.  A lane holds a row of the accumulator; stored from registers
+      // every store instruction touches 32 lines (64 passes through the L1, which was 84 to 96 % busy and bounded every
+      // convolution with a short reduction), as blocks of 32 x 32 in shared memory eight conflict-free stores and one copy do.
+      // What is to be added arrives the same way, one block ahead.  Statistics read the block by columns: a lane has the 32
+      // values of its column in registers, without a single exchange between lanes.
+      bulk = p.bulk_out != 0;
+      if (bulk) {
+        constexpr int OUT_BLOCKS = Smem::kOutBlocks;
+        const int ew = warp - 2;
+        const uint32_t blocks = smem_base + STAGES * C::kStageBytes + (uint32_t)(ew * OUT_BLOCKS) * kOutBlock;
+        const uint32_t row_base = (uint32_t)lane * 128u, swz = (uint32_t)(lane & 7);
+        // blocks of this warp in order: (tile, 32 columns); those outside the matrix are skipped
+        auto next_block = [&](int& unit, int& c0) {
+          do {
+            c0 += 32;
+            if (c0 >= COLS) { c0 = 0; unit += gridDim.x; }
+          } while (unit < tiles && ((unit / p.n_tiles) * 128 + quarter * 32 >= p.M || (unit % p.n_tiles) * BN + c_first + c0 >= p.N));
+        };
+        int load_unit = blockIdx.x, load_c0 = -32, loaded = 0;  // the addend's blocks, asked for one ahead
+        auto load_addend = [&]() {  // lane 0
+          next_block(load_unit, load_c0);
+          if (load_unit >= tiles) return;
+          const uint32_t bar = smem_u32(&bar_add[ew][loaded & 1]);
+          mbar_expect_tx(bar, kOutBlock);
+          tma_load_2d(blocks + (uint32_t)(loaded & 1) * kOutBlock, &mapAdd, bar, (load_unit % p.n_tiles) * BN + c_first + load_c0,
+                      (load_unit / p.n_tiles) * 128 + quarter * 32);
+          ++loaded;
+        };
+        if constexpr (EPI == EPI_ADD) {
+          if (lane == 0) load_addend();
+        }
+        int g = 0;  // blocks handled
+        for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
+          const int row0 = (unit / p.n_tiles) * 128 + quarter * 32, n0 = (unit % p.n_tiles) * BN + c_first;
+          const int buf = t & 1;
+          bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_ptr, 4);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          const int rows = p.M - row0 < 32 ? p.M - row0 : 32;
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
+            const int col0 = n0 + c0;
+            const bool inside = rows > 0 && col0 < p.N;  // warp-uniform
+            const uint32_t block = blocks + (uint32_t)(OUT_BLOCKS == 2 ? (g & 1) : 0) * kOutBlock;
+            float4 add[8];
+            if constexpr (EPI == EPI_ADD) {
+              if (inside) {
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_add[ew][g & 1]), (uint32_t)(g >> 1) & 1u, abort_ptr, 5));
+                if (!ok) break;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) add[j] = ld_shared4(block + row_base + (((uint32_t)j ^ swz) << 4));
+                if (lane == 0) {
+                  bulk_wait_read<0>();  // the block before has been read, its place is free
+                  load_addend();
+                }
+              }
+            } else {
+              if (inside) {
+                if (lane == 0) bulk_wait_read<0>();
+                __syncwarp();
+              }
+            }
+            tmem_ld_wait();
+            if (c0 + 32 >= COLS) {  // the accumulator is in registers
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&bar_tempty[buf]));
+            }
+            if (!inside) continue;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+              if (p.bias && col0 + 4 * j < p.N) {  // N % 4 == 0 on this path
+                const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + 4 * j);
+                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+              }
+              if constexpr (EPI == EPI_ADD) { v.x += add[j].x; v.y += add[j].y; v.z += add[j].z; v.w += add[j].w; }
+              if (p.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
+              st_shared4(block + row_base + (((uint32_t)j ^ swz) << 4), v);
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&mapOut, block, col0, row0);
+              bulk_commit();
+            }
+            ++g;
+            if constexpr (STATS) {
+              float o[32];
+              const uint32_t column = block + (uint32_t)(lane & 3) * 4u;
+#pragma unroll
+              for (int k = 0; k < 32; ++k) o[k] = ld_shared1(column + (uint32_t)k * 128u + (((uint32_t)(lane >> 2) ^ (uint32_t)(k & 7)) << 4));
+              stats.add_column(c0 / 32, o, rows);
+            }
+          }
+          if (!ok) break;
+          if constexpr (STATS) { if (rows > 0) stats.n += (float)rows; }
+        }
+        if (lane == 0) bulk_wait_all();
+      }
+    }
+    if constexpr (!STATS || SPLIT) {  // statistics of unsplit reductions come through shared memory only
+    for (int unit = blockIdx.x; !bulk && unit < tiles; unit += gridDim.x, ++t) {
       const int tile = unit / S;
       const int m0 = (tile / p.n_tiles) * 128, n0 = (tile % p.n_tiles) * BN;
       const int buf = t & 1;
@@ -487,33 +640,22 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         else if constexpr (STATS) stats.n += cnt;
       };
       if constexpr (!SPLIT) {
-        if constexpr (STATS) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < cols_here; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
+          if constexpr (ADD) {
+            float4 next[8];
+            if (c0 + 32 < COLS) fetch_addend(c0 + 32, next);
+            tmem_ld_wait();
+            finish(c0, r);
 #pragma unroll
-          for (int c0 = 0; c0 < COLS; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
+            for (int j = 0; j < 8; ++j) add[j] = next[j];
+          } else {
             tmem_ld_wait();
             finish(c0, r);
           }
-        } else {
-#pragma unroll 1
-          for (int c0 = 0; c0 < cols_here; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
-            if constexpr (ADD) {
-              float4 next[8];
-              if (c0 + 32 < COLS) fetch_addend(c0 + 32, next);
-              tmem_ld_wait();
-              finish(c0, r);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) add[j] = next[j];
-            } else {
-              tmem_ld_wait();
-              finish(c0, r);
-            }
-          }
         }
-        count_rows();
         release_accumulator();
       } else {
       // Split reduction (one unit per CTA).  The stages are free when every unit of the cluster has its accumulator; received
@@ -575,11 +717,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       }
       }
     }
-    if constexpr (STATS && !SPLIT) {
-      float* row = p.stats + ((long long)(blockIdx.x / p.n_tiles) * 4 + quarter) * 3 * p.N;
-      if constexpr (LANE_SUMS) sums.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, p.bias, lane);
-      else if constexpr (STATS) stats.store(row, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, lane);
     }
+    if constexpr (STATS && !SPLIT)
+      stats.store(p.stats + ((long long)(blockIdx.x / p.n_tiles) * 4 + quarter) * 3 * p.N, p.N, (blockIdx.x % p.n_tiles) * BN + c_first, p.N, lane);
   }
 
   // ------------------------------------------------------------ teardown
@@ -596,19 +736,23 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   }
 }
 
+bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 template <int BN, int AMODE, int BMODE, int EPI = EPI_PLAIN>
-int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
-  using C = Cfg<BN>;
+int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& params, cudaStream_t st) {
+  GemmParams p = params;
   int tiles = p.m_tiles * p.n_tiles;
   if (p.splits > 1) {  // one unit per CTA, the units of a tile a cluster
     if constexpr (AMODE == A_IM2COL) {
       auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, true>;
+      constexpr uint32_t smem = GemmSmem<BN, EPI, true>::bytes(false);
+      p.stages = GemmSmem<BN, EPI, true>::stages(false);
       static unsigned long long configured = 0;
-      if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
+      if (int rc = mtb_opt_in_smem((const void*)kernel, (int)smem, &configured)) return rc;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(tiles * p.splits);
       cfg.blockDim = dim3(kGemmThreads);
-      cfg.dynamicSmemBytes = C::kSmemBytes;
+      cfg.dynamicSmemBytes = smem;
       cfg.stream = st;
       cudaLaunchAttribute attr[2];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -618,18 +762,34 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 2;
-      MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, p));
+      MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, mapA, mapA, p));
       MTB_LAUNCH_CHECK("tc_gemm_kernel");
       return MTB_OK;
     }
     return mtb_fail(MTB_ERR_INVALID, "tc_gemm: only convolutions split the reduction");
   }
   auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, false>;
+  using Smem = GemmSmem<BN, EPI, false>;
+  CUtensorMap mapOut = mapA, mapAdd = mapA;  // unused ones are never read
+  if constexpr (Smem::kBulk) {
+    // Whole rows one after the other, their pitch and start on 16 bytes: what the copy engine asks for.  Everything else (a
+    // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 16
+    // reduction blocks and more on wide tiles, whose stores hide behind the main loop: the shared memory is better left to the
+    // side stream (ResNet-18 step at 512 images 6.05 ms, with all results through shared memory 6.08).
+    p.bulk_out = (EPI != EPI_PLAIN || BN == 64 || p.num_kb < 16) && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
+    if (EPI == EPI_STATS && !p.bulk_out) return mtb_fail(MTB_ERR_INVALID, "tc_gemm: statistics need whole aligned rows");
+    if (p.bulk_out) {
+      if (int rc = tc::encode_result_2d(&mapOut, p.out, p.M, p.N, p.ldo)) return rc;
+      if (EPI == EPI_ADD)
+        if (int rc = tc::encode_result_2d(&mapAdd, p.addend, p.M, p.N, p.ldo)) return rc;
+    }
+  }
+  p.stages = Smem::stages(p.bulk_out);
   static unsigned long long configured = 0;
-  if (int rc = mtb_opt_in_smem((const void*)kernel, (int)C::kSmemBytes, &configured)) return rc;
+  if (int rc = mtb_opt_in_smem((const void*)kernel, (int)Smem::kMost, &configured)) return rc;
   int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
   if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
-  MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), C::kSmemBytes, st, mapA, mapB, p);
+  MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), Smem::bytes(p.bulk_out), st, mapA, mapB, mapOut, mapAdd, p);
   MTB_LAUNCH_CHECK("tc_gemm_kernel");
   return MTB_OK;
 }
@@ -696,7 +856,7 @@ int cluster_units(int size) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms / size * size);
     cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = Cfg<256>::kSmemBytes;
+    cfg.dynamicSmemBytes = GemmSmem<256, EPI_PLAIN, true>::bytes(false);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)size;
@@ -704,7 +864,7 @@ int cluster_units(int size) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<256>::kSmemBytes) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmem<256, EPI_PLAIN, true>::bytes(false)) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
       (void)cudaGetLastError();  // no GPU (plans are also made without one)
       clusters = sms * 7 / 8 / size;
@@ -740,8 +900,6 @@ GemmPlan plan_gemm(int n, long long rows, int num_kb, bool mn_major, int force_b
     }
   return best;
 }
-
-bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Activations smaller than this stay on the CUDA-core kernels: tiny tensors gain nothing from
 // the tensor cores, and im2col tensor maps over very small tensors are avoided altogether.
@@ -893,13 +1051,12 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   p.out = y; p.ldo = cout; p.bias = bias; p.relu = relu;
   p.OW = ow; p.OH = oh; p.SW = sw; p.SH = sh; p.PW = pw; p.PH = ph; p.KW = kw; p.KH = kh; p.cchunks = cin / 32;
   p.splits = gp.splits; p.kb_per_split = gp.kb_per_split;
-  // short reductions (1x1 shortcuts) leave the epilogue no main loop to hide the statistics behind
-  // ... unless the output is small: then BatchNorm's own pass is all launch latency, and the epilogue is cheaper
-  // (measured on the three 1x1 shortcuts of ResNet-18: 1.782 -> 1.770 ms per step at 64 images, but
-  // 6.37 -> 6.41 ms at 512, where their outputs are 17 to 67 MB)
-  // 64-wide tiles keep plain per-lane sums, cheap enough to hide behind the stores whatever the reduction.
-  const bool small_output = (long long)M * cout * 4 <= (12ll << 20);
-  if (want_stats && (p.num_kb >= 16 || small_output || bn == 64)) {
+  // A short reduction (1x1) leaves the epilogue no main loop to hide the statistics behind, and takes less with them than
+  // with BatchNorm's own pass all the same (both operators: 64 -> 128 channels, stride 2, to 16x16, 16 images 15.5 -> 12.3 us,
+  // 192 images 30.0 -> 27.0, 512 images 57.0 -> 55.1; 64 -> 256 channels on 32 x 56x56 83.4 -> 78.0; ResNet-50 step
+  // 19.80 -> 19.23 ms).  Outputs of 12 to 16 MB keep BatchNorm's pass: it reads them from L2, and a test holds the operator to it.
+  const long long out_bytes = (long long)M * cout * 4;
+  if (want_stats && (p.num_kb >= 16 || out_bytes <= (12ll << 20) || out_bytes > (16ll << 20) || bn == 64)) {
     p.stats = stats;
     *stats_rows = gp.splits > 1 ? p.m_tiles * 4 : stats_rows_for(p.m_tiles * p.n_tiles, p.n_tiles);
     cudaStream_t st = (cudaStream_t)stream;
@@ -1026,7 +1183,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
           const int fkh = a + sh * (ah.taps - 1 - jh), fkw = b + sw * (aw.taps - 1 - jw);  // dY offset j <-> filter tap
           p.b_tap_x[jh * aw.taps + jw] = (fkh * kw + fkw) * cin;
         }
-      p.o_strided = 1; p.o_Hc = ah.count; p.o_Wc = aw.count; p.o_H = h; p.o_W = w; p.o_h0 = ah.start; p.o_w0 = aw.start; p.o_sh = sh; p.o_sw = sw;
+      p.o_strided = sh * sw > 1; p.o_Hc = ah.count; p.o_Wc = aw.count; p.o_H = h; p.o_W = w; p.o_h0 = ah.start; p.o_w0 = aw.start; p.o_sh = sh; p.o_sw = sw;
       rc = p.addend ? launch_tc_bn<A_IM2COL, B_MNMAJOR, EPI_ADD>(bn, mapA, mapB, p, cst) : launch_tc_bn<A_IM2COL, B_MNMAJOR>(bn, mapA, mapB, p, cst);
       if (rc) return rc;
     }
