@@ -9,8 +9,47 @@ MTB_API long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int k
   if (n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return 0;
   long long a = mtb_conv2d_wgrad_simt_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   long long b = mtb_tc_conv2d_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
+  for (int direction = 0; direction < 3; ++direction) {  // those that the TF32 kernels leave (unaligned tensors aside, which then take the CUDA cores)
+    if (direction == 1 ? cout % 32 == 0 && cin % 4 == 0 : cin % 32 == 0 && cout % 4 == 0) continue;
+    const long long c = mtb_split_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
+    if (c > b) b = c;
+  }
   return a > b ? a : b;
 }
+
+namespace {
+
+// Whether the two-term products take this convolution: they need the scratch (a caller without it gets the CUDA-core kernels).
+bool split_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction, const void* workspace,
+                 long long workspace_bytes) {
+  if (!workspace || !mtb_aligned16(workspace) || n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0 ||
+      !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw))
+    return false;
+  const long long need = mtb_split_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
+  return need > 0 && workspace_bytes >= need;
+}
+
+// Forward of the shapes that the TF32 kernels do not take.
+int forward_fp32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt, const float* bias,
+                 float* y, int relu, void* workspace, long long workspace_bytes, void* stream) {
+  const int* guard = nullptr;
+  int guards = 0;
+  if (x && wt && y && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0, workspace, workspace_bytes))
+    if (int rc = mtb_split_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, (cudaStream_t)stream, &guard, &guards))
+      return rc;
+  return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream, guard, guards);
+}
+
+int dgrad_fp32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy, const float* wt, float* dx,
+               void* workspace, long long workspace_bytes, void* stream) {
+  const int* guard = nullptr;
+  int guards = 0;
+  if (dy && wt && dx && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 1, workspace, workspace_bytes))
+    if (int rc = mtb_split_conv2d_dgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, workspace, (cudaStream_t)stream, &guard, &guards)) return rc;
+  return mtb_conv2d_dgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream, guard, guards);
+}
+
+}  // namespace
 
 // workspace (may be NULL): scratch of mtb_conv2d_workspace_bytes() for the weight gradient; forward and data gradient take it
 // for symmetry (layers whose output has too few tiles split their reduction over clusters, without scratch).
@@ -19,7 +58,7 @@ MTB_API int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw,
                                    void* stream) {
   if (mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, y))
     return mtb_tc_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream);
-  return mtb_conv2d_forward_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, stream);
+  return forward_fp32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream);
 }
 
 // Forward convolution that also prepares the batch statistics of its output for a BatchNorm layer
@@ -38,7 +77,7 @@ MTB_API int mtb_conv2d_forward_stats_f32(int n, int cin, int h, int w, int kh, i
   if (mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, y))
     return mtb_tc_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream, stats,
                                      stats_rows);
-  return mtb_conv2d_forward_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, stream);
+  return forward_fp32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream);
 }
 
 // Inference: y = relu?(batch_norm(conv(x)) + residual), BatchNorm with running statistics, in one launch.  The epilogue applies
@@ -54,6 +93,11 @@ MTB_API int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int 
   if (mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, y) && (!residual || mtb_aligned16(residual)))
     return mtb_tc_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, workspace_bytes, stream, nullptr,
                                      nullptr, &bn, residual);
+  if (split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0, workspace, workspace_bytes)) {
+    if (int rc = forward_fp32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, 0, workspace, workspace_bytes, stream)) return rc;
+    const long long rows = (long long)n * ((h + 2 * ph - kh) / sh + 1) * ((w + 2 * pw - kw) / sw + 1);
+    return mtb_bn_eval_apply(y, y, rows, cout, bn, residual, relu, (cudaStream_t)stream);
+  }
   return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, &bn, residual, stream);
 }
 
@@ -61,7 +105,7 @@ MTB_API int mtb_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, i
                                  const float* wt, float* dx, void* workspace, long long workspace_bytes, void* stream) {
   if (mtb_tc_conv2d_dgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx))
     return mtb_tc_conv2d_dgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, nullptr, dx, workspace, workspace_bytes, stream);
-  return mtb_conv2d_dgrad_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream);
+  return dgrad_fp32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, workspace, workspace_bytes, stream);
 }
 
 // dx = dgrad(dy, wt) + addend: the data gradient added to a gradient the same tensor already received
@@ -79,7 +123,7 @@ MTB_API int mtb_conv2d_dgrad_add_f32(int n, int cin, int h, int w, int kh, int k
   }
   if (mtb_tc_conv2d_dgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx))
     return mtb_tc_conv2d_dgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, addend, dx, workspace, workspace_bytes, stream);
-  int rc = mtb_conv2d_dgrad_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream);
+  int rc = dgrad_fp32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, workspace, workspace_bytes, stream);
   if (rc) return rc;
   return mtb_add_f32(dx, addend, dx, (long long)n * h * w * cin, 1.0f, stream);
 }
@@ -95,7 +139,11 @@ MTB_API int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, i
                                  const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
   if (mtb_tc_conv2d_wgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw))
     return mtb_tc_conv2d_wgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream);
-  return mtb_conv2d_wgrad_simt_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream);
+  const int* guard = nullptr;
+  int guards = 0;
+  if (x && dy && dw && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 2, workspace, workspace_bytes))
+    if (int rc = mtb_split_conv2d_wgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, (cudaStream_t)stream, &guard, &guards)) return rc;
+  return mtb_conv2d_wgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream, guard, guards);
 }
 
 MTB_API int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,

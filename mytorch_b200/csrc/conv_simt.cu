@@ -37,22 +37,41 @@ Choice wgrad_choice(const ConvDims& d) {
 
 }  // namespace
 
+// What the kernels below are priced at, in us (direction: 0 forward, 1 data gradient, 2 weight gradient).
+double mtb_conv2d_simt_us(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction) {
+  ConvDims d;
+  if (conv_dims(d, n, cin, h, w, kh, kw, sh, sw, ph, pw, cout)) return 0.0;
+  Choice c;
+  if (direction == 0) {
+    c = choose((long long)n * d.OH * d.OW, cout, (long long)kh * kw * cin, 1, 1);
+  } else if (direction == 1) {
+    const int classes = sh * sw < kMaxClasses ? sh * sw : kMaxClasses;
+    c = choose(((long long)n * h * w + sh * sw - 1) / (sh * sw), cin, (long long)((kh + sh - 1) / sh) * ((kw + sw - 1) / sw) * cout, classes, 1);
+    c.cycles *= (double)sh * sw / classes;
+  } else {
+    c = wgrad_choice(d);
+  }
+  // the prices are those of float4 loads; single floats cost about 1.4 times as much (16 images of 40x40, 129 -> 130 channels)
+  const bool four = direction == 0 ? cin % 4 == 0 : direction == 1 ? cout % 4 == 0 : cin % 4 == 0 && cout % 4 == 0;
+  return c.cycles / 1850.0 * (four ? 1.0 : 1.4);
+}
+
 int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
-                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream) {
+                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream, const int* guard, int guards) {
   ConvDims d;
   int rc = conv_dims(d, n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (rc) return rc;
   MTB_REQUIRE(x && wt && y, "conv2d_forward: null pointer");
   const int K = kh * kw * cin, M = n * d.OH * d.OW;
   Out o{};
-  o.out = y; o.ld = cout; o.bias = bias; o.relu = relu;
+  o.out = y; o.ld = cout; o.bias = bias; o.relu = relu; o.guard = guard; o.guards = guards;
   const Choice c = choose(M, cout, K, 1, 1);
   if (bn_eval) {
     if (tile_info(c.tile).cluster) {  // small tiles: BatchNorm in the store
       o.bn = *bn_eval;
       o.residual = residual;
     } else {
-      const int rc2 = mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, 0, nullptr, nullptr, stream);
+      const int rc2 = mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, 0, nullptr, nullptr, stream, nullptr, 0);
       return rc2 ? rc2 : mtb_bn_eval_apply(y, y, M, cout, *bn_eval, residual, relu, (cudaStream_t)stream);
     }
   }
@@ -64,17 +83,22 @@ int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh
 
 MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                         const float* wt, const float* bias, float* y, int relu, void* stream) {
-  return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream);
+  return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream, nullptr, 0);
 }
 
 MTB_API int mtb_conv2d_dgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                                       const float* wt, float* dx, void* stream) {
+  return mtb_conv2d_dgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream, nullptr, 0);
+}
+
+int mtb_conv2d_dgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy, const float* wt, float* dx,
+                          void* stream, const int* guard, int guards) {
   ConvDims d;
   int rc = conv_dims(d, n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (rc) return rc;
   MTB_REQUIRE(dy && wt && dx, "conv2d_dgrad: null pointer");
   Out o{};
-  o.out = dx; o.ld = cin; o.H = h; o.W = w; o.SH = sh; o.SW = sw;
+  o.out = dx; o.ld = cin; o.H = h; o.W = w; o.SH = sh; o.SW = sw; o.guard = guard; o.guards = guards;
   const DgradK a{dy, d, FastDiv(cout), nullptr};
   const DgradR b{wt, d, FastDiv(cout), nullptr};
   const bool va = cout % 4 == 0 && mtb_aligned16(dy), vb = cin % 4 == 0 && mtb_aligned16(wt);
@@ -131,17 +155,23 @@ __global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict
 
 MTB_API int mtb_conv2d_wgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                       const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
+  return mtb_conv2d_wgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream, nullptr, 0);
+}
+
+int mtb_conv2d_wgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* dy, float* dw,
+                          void* workspace, long long workspace_bytes, void* stream, const int* guard, int guards) {
   ConvDims d;
   int rc = conv_dims(d, n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (rc) return rc;
   MTB_REQUIRE(x && dy && dw, "conv2d_wgrad: null pointer");
   const int K = kh * kw * cin, pixels = n * d.OH * d.OW;
-  const Choice c = wgrad_choice(d);
+  // guarded: one launch that usually does nothing, so its slices add up in clusters
+  const Choice c = guard ? choose(cout, K, pixels, 1, 1) : wgrad_choice(d);
   const long long total = (long long)cout * K;
   cudaStream_t st = (cudaStream_t)stream;
   Out o{};
-  o.out = dw; o.ld = K;
-  if (c.slices > 1) {
+  o.out = dw; o.ld = K; o.guard = guard; o.guards = guards;
+  if (c.slices > 1 && !guard) {
     MTB_REQUIRE(workspace && workspace_bytes >= c.slices * total * 4, "conv2d_wgrad: workspace too small");
     o.out = (float*)workspace;
     o.split_plane = total;
@@ -152,7 +182,7 @@ MTB_API int mtb_conv2d_wgrad_simt_f32(int n, int cin, int h, int w, int kh, int 
   else if (va) rc = launch<DenseR, 4, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
   else if (vb) rc = launch<DenseR, 1, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
   else rc = launch<DenseR, 1, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
-  if (rc || c.slices == 1) return rc;
+  if (rc || c.slices == 1 || guard) return rc;
   MTB_LAUNCH(add_planes_kernel, mtb_stream_grid(total, 256), 256, 0, st, (const float*)workspace, dw, total, c.slices);
   MTB_LAUNCH_CHECK("add_planes_kernel");
   return MTB_OK;

@@ -7,7 +7,13 @@ MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, in
                                         const float* wt, const float* bias, float* y, int relu, void* stream);
 // the same, followed by BatchNorm with running statistics and an optional addition before the ReLU
 int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
-                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream);
+                            const float* bias, float* y, int relu, const MtbBnEval* bn_eval, const float* residual, void* stream,
+                            const int* guard = nullptr, int guards = 0);
+// guard: device words (guards of them); unless one is set nothing is done
+int mtb_conv2d_dgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy, const float* wt, float* dx,
+                          void* stream, const int* guard, int guards);
+int mtb_conv2d_wgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* dy, float* dw,
+                          void* workspace, long long workspace_bytes, void* stream, const int* guard, int guards);
 // y = relu?(batch_norm(x) + residual) over [rows, c] with running statistics; x == y is allowed (batch_norm.cu)
 int mtb_bn_eval_apply(const float* x, float* y, long long rows, int c, const MtbBnEval& bn, const float* residual, int relu, cudaStream_t st);
 MTB_API int mtb_conv2d_dgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
@@ -41,3 +47,14 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                     void* stream);
 
+double mtb_conv2d_simt_us(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction);
+
+// FP32 accuracy on the tensor cores for channel counts of any size: operands as sums of two TF32 numbers (tc_split.cuh).
+// direction: 0 forward, 1 data gradient, 2 weight gradient.  0 bytes: not taken.
+long long mtb_split_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction);
+int mtb_split_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
+                                 const float* bias, float* y, int relu, void* workspace, cudaStream_t st, const int** guard, int* guards);
+int mtb_split_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy, const float* wt,
+                               float* dx, void* workspace, cudaStream_t st, const int** guard, int* guards);
+int mtb_split_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* dy,
+                               float* dw, void* workspace, cudaStream_t st, const int** guard, int* guards);

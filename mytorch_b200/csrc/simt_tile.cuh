@@ -310,6 +310,8 @@ struct Out {
   long long split_plane;     // > 0: every slice of the reduction writes its own plane of partials
   const DgradClass* cls;     // data gradient: row -> pixel of the residue class
   int H, W, SH, SW;
+  const int* guard;          // not NULL: nothing is done unless one of these words is set
+  int guards;
 };
 
 __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
@@ -388,6 +390,11 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
   __shared__ float Bs[2][BK][BN + 4];
   mtb_launch_dependents();
   mtb_wait_prior();
+  if (o.guard) {
+    int any = 0;
+    for (int i = 0; i < o.guards; ++i) any |= o.guard[i];
+    if (!any) return;
+  }
   const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int z = blockIdx.z / slices, slice = blockIdx.z - z * slices;
@@ -492,7 +499,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
 // A block of BK = 16 of one CTA costs its multiplications plus about 500 cycles of load latency when nothing else on
 // the SM hides it; with other CTAs beside it the FFMA pipe bounds, at `eff` of its rate.  A launch is priced as CTAs per
 // SM x blocks x the slower of the two (plus the cluster's exchange, or the pass over the planes) and the cheapest is taken.
-struct Choice { int tile, slices; };
+struct Choice { int tile, slices; double cycles; };
 enum { XL = 0, L = 1, MD = 2, SM = 3, XS = 4, kTiles = 5 };
 struct TileInfo { int bm, bn, occ; double eff; bool cluster; };
 inline const TileInfo& tile_info(int t) {
@@ -506,8 +513,7 @@ inline const TileInfo& tile_info(int t) {
 inline Choice choose(long long rows, long long cols, long long k, int classes, int max_planes) {
   static const int kSlices[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512};
   const double sms = mtb_sm_count();
-  Choice best{SM, 1};
-  double best_cycles = 1e300;
+  Choice best{SM, 1, 1e300};
   for (int t = 0; t < kTiles; ++t) {
     const TileInfo& info = tile_info(t);
     const double tiles = (double)((rows + info.bm - 1) / info.bm) * (double)((cols + info.bn - 1) / info.bn) * classes;
@@ -524,7 +530,7 @@ inline Choice choose(long long rows, long long cols, long long k, int classes, i
       const double alone = (500 + mul) / beside, piped = mul / info.eff;
       double cycles = queue * blocks * (alone > piped ? alone : piped) + 2000;
       if (s > 1) cycles += max_planes > 1 ? 4000 + s * (double)rows * cols * 8 / 2500 : 2500;
-      if (cycles < best_cycles) { best_cycles = cycles; best = Choice{t, s}; }
+      if (cycles < best.cycles) best = Choice{t, s, cycles};
     }
   }
   return best;

@@ -1082,6 +1082,21 @@ bool mtb_tc_conv2d_dgrad_supported(int n, int cin, int h, int w, int kh, int kw,
   return true;
 }
 
+namespace {
+// One axis of residue class a: its taps, its pixels (start + s * i, i < count) and the corners of the window its outputs see.
+struct ClassAxis { int taps, start, count, lower, upper; };
+ClassAxis class_axis(int a, int size, int osize, int k, int s, int pad) {
+  ClassAxis r{};
+  r.taps = a < k ? (k - a + s - 1) / s : 0;
+  r.start = (((a - pad) % s) + s) % s;
+  r.count = r.start < size ? (size - r.start + s - 1) / s : 0;
+  const int c0 = (r.start + pad - a) / s;
+  r.lower = c0 - (r.taps - 1);
+  r.upper = r.count - osize + r.lower;
+  return r;
+}
+}  // namespace
+
 // Data gradient.  For stride 1 this is a convolution of dY with the filter rotated by 180
 // degrees.  For stride s the input pixels fall into s*s residue classes; pixels of class (a, b)
 // only see the taps kh = a (mod s), kw = b (mod s), and over the class's own (coarser) grid
@@ -1118,21 +1133,10 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
       for (int jw = 0; jw < kw; ++jw) tap_x[jh * kw + jw] = ((kh - 1 - jh) * kw + (kw - 1 - jw)) * cin;
     return run_row_conv<B_MNMAJOR>(plan, bn, n, h, w, cout, kh, kw, ph, pw, cin, dy, mapB, tap_x, nullptr, addend, 0, dx, st, nullptr, nullptr, b_blocks);
   }
-  struct Axis { int taps, start, count, lower, upper; };
-  auto axis = [](int a, int size, int osize, int k, int s, int pad) {
-    Axis r{};
-    r.taps = a < k ? (k - a + s - 1) / s : 0;
-    r.start = (((a - pad) % s) + s) % s;
-    r.count = r.start < size ? (size - r.start + s - 1) / s : 0;
-    const int c0 = (r.start + pad - a) / s;
-    r.lower = c0 - (r.taps - 1);
-    r.upper = r.count - osize + r.lower;
-    return r;
-  };
   bool need_zero = false;
   for (int a = 0; a < sh; ++a)
     for (int b = 0; b < sw; ++b) {
-      Axis ah = axis(a, h, oh, kh, sh, ph), aw = axis(b, w, ow, kw, sw, pw);
+      const ClassAxis ah = class_axis(a, h, oh, kh, sh, ph), aw = class_axis(b, w, ow, kw, sw, pw);
       if (ah.count > 0 && aw.count > 0 && (ah.taps == 0 || aw.taps == 0)) need_zero = true;
     }
   // addend == dx: dx already holds the gradient to add to; every class adds its own pixels in its epilogue
@@ -1148,7 +1152,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   int live = 0;
   for (int a = 0; a < sh; ++a)
     for (int b = 0; b < sw; ++b) {
-      Axis ah = axis(a, h, oh, kh, sh, ph), aw = axis(b, w, ow, kw, sw, pw);
+      const ClassAxis ah = class_axis(a, h, oh, kh, sh, ph), aw = class_axis(b, w, ow, kw, sw, pw);
       if (ah.count > 0 && aw.count > 0 && ah.taps > 0 && aw.taps > 0) ++live;
     }
   const long long class_units = ((class_rows + 127) / 128) * ((cin + bn - 1) / bn);
@@ -1160,7 +1164,7 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   int launched = 0;
   for (int a = 0; a < sh; ++a) {
     for (int b = 0; b < sw; ++b) {
-      Axis ah = axis(a, h, oh, kh, sh, ph), aw = axis(b, w, ow, kw, sw, pw);
+      const ClassAxis ah = class_axis(a, h, oh, kh, sh, ph), aw = class_axis(b, w, ow, kw, sw, pw);
       if (ah.count == 0 || aw.count == 0 || ah.taps == 0 || aw.taps == 0) continue;
       cudaStream_t cst = lane_stream[launched++ % lanes];
       CUtensorMap mapA;
@@ -1624,3 +1628,5 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   MTB_LAUNCH_CHECK("wgrad_reduce_transpose_kernel");
   return MTB_OK;
 }
+
+#include "tc_split.cuh"

@@ -1,0 +1,91 @@
+"""Convolutions over channel counts of any size on the tensor cores, operands as sums of two TF32 numbers: tiles, blocks of
+channels and pixels that are not full, strides, several groups of images, against 64 bits and against the CUDA-core kernels."""
+import numpy as np
+import pytest
+
+from oracle import ops as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(n, cin, cout, h, w, k, stride, pad, seed=0):
+    rng = np.random.default_rng(seed + cin + cout)
+    x, wt = rng.standard_normal((n, cin, h, w)).astype(np.float32), (rng.standard_normal((cout, cin, k, k)) / (cin * k * k) ** 0.5).astype(np.float32)
+    dy = rng.standard_normal((n, cout, (h + 2 * pad - k) // stride + 1, (w + 2 * pad - k) // stride + 1)).astype(np.float32)
+    return x, wt, dy
+
+
+def _run(x, wt, b, dy, stride, pad):
+    import gpu_util as g
+
+    s, p = (stride, stride), (pad, pad)
+    xt, wtt, bt = g.dev(x, True), g.dev(wt, True), g.dev(b)
+    y = g.op("conv2d")(xt, wtt, bt, s, p)
+    dx, dw, _ = g.op("conv2d_backward")(g.dev(dy), xt, wtt, None, s, p)
+    return [g.host(t) for t in (y, dx, dw)]
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w,k,stride,pad", [
+    (8, 33, 31, 12, 13, 3, 1, 1), (5, 48, 82, 19, 17, 3, 1, 1), (9, 70, 129, 21, 15, 3, 2, 1), (40, 36, 100, 9, 11, 1, 1, 0), (3, 130, 66, 23, 20, 5, 1, 0),
+    (33, 41, 161, 10, 10, 3, 3, 0), (20, 37, 35, 16, 16, 1, 2, 0), (2, 64, 70, 41, 39, 3, 1, 2)])
+def test_against_64_bits_and_the_other_kernels(n, cin, cout, h, w, k, stride, pad, monkeypatch):
+    x, wt, dy = _operands(n, cin, cout, h, w, k, stride, pad)
+    b = np.random.default_rng(1).standard_normal(cout).astype(np.float32)
+    monkeypatch.setenv("MTB_TC_SPLIT_ALWAYS", "1")
+    got = _run(x, wt, b, dy, stride, pad)
+    assert all(np.array_equal(u, v) for u, v in zip(got, _run(x, wt, b, dy, stride, pad)))
+    monkeypatch.delenv("MTB_TC_SPLIT_ALWAYS")
+    monkeypatch.setenv("MTB_DISABLE_TC", "1")
+    other = _run(x, wt, b, dy, stride, pad)
+    d = [t.astype(np.float64) for t in (x, wt, b, dy)]
+    s, p = (stride, stride), (pad, pad)
+    exact = lambda x, wt, b, dy: [O.conv2d_forward(x, wt, b, s, p), *O.conv2d_backward(dy, x, wt, False, s, p)[:2]]
+    terms = (cin * k * k, cout * k * k, dy[:, 0].size)
+    for a, o, want, size, count in zip(got, other, exact(*d), exact(*(np.abs(t) for t in d)), terms):
+        # an operand is off by 2^-22 at most, the term left out is 2^-22, a chain truncates 12 times, chains are added in FP32
+        assert (np.abs(a - want) <= (18 + count / 32) * 2.0 ** -23 * size).all()
+        err = lambda t: np.linalg.norm(t - want) / np.linalg.norm(want)
+        assert err(a) <= max(err(o), 2.0e-7)  # 2e-7: what sums of some hundred terms, which these kernels are taken for, have in FP32
+
+
+def test_several_groups_of_images(monkeypatch):
+    x, wt, dy = _operands(70, 33, 40, 64, 64, 3, 1, 1)  # packed, 2 MB an image: three groups
+    b = np.zeros(40, np.float32)
+    monkeypatch.setenv("MTB_TC_SPLIT_ALWAYS", "1")
+    got = _run(x, wt, b, dy, 1, 1)
+    monkeypatch.delenv("MTB_TC_SPLIT_ALWAYS")
+    monkeypatch.setenv("MTB_DISABLE_TC", "1")
+    want, size = _run(x, wt, b, dy, 1, 1), _run(*(np.abs(t) for t in (x, wt, b, dy)), 1, 1)
+    for a, o, m, count in zip(got, want, size, (33 * 9, 40 * 9, 70 * 64 * 64)):
+        terms = 18 + count / 32 + count  # both sides' rounding
+        assert (np.abs(a - o) <= terms * 2.0 ** -23 * m).all()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.3e38])
+def test_values_that_cannot_be_split(value, monkeypatch):
+    x, wt, dy = _operands(70, 33, 40, 64, 64, 3, 1, 1)
+    x[69, 5, 7, 9] = dy[1, 2, 3, 4] = value  # x in the last group of images, dy in the first
+    b = np.zeros(40, np.float32)
+    monkeypatch.setenv("MTB_TC_SPLIT_ALWAYS", "1")
+    got = _run(x, wt, b, dy, 1, 1)
+    monkeypatch.delenv("MTB_TC_SPLIT_ALWAYS")
+    monkeypatch.setenv("MTB_DISABLE_TC", "1")
+    want = _run(x, wt, b, dy, 1, 1)
+    assert np.array_equal(got[0], want[0], equal_nan=True) and np.array_equal(got[1], want[1], equal_nan=True)
+    a, o = got[2], want[2]  # the sum over pixels is split otherwise: a partial sum may overflow on one side only
+    clean = np.isfinite(a) & np.isfinite(o) & (np.abs(o) < 1e30)
+    assert np.array_equal(np.isnan(a), np.isnan(o)) if not np.isfinite(value) else True
+    assert np.allclose(a[clean], o[clean], rtol=0, atol=1e-5 * 70 * 64 * 64 ** 0.5) and clean.any()
+
+
+def test_without_scratch_the_other_kernels_run():
+    import gpu_util as g
+    from mytorch_b200.backends.cuda.env import CudaEnv
+
+    env = CudaEnv.instance()
+    x, wt, _ = _operands(32, 48, 82, 37, 37, 3, 1, 1)
+    xt, wtt = g.dev(x), g.dev(wt)
+    y, args = g.dev(np.zeros((32, 82, 37, 37), np.float32)), (32, 48, 37, 37, 3, 3, 1, 1, 1, 1, 82)
+    env.lib.conv2d_forward_f32(*args, xt, wtt, None, y, 0, None, 0, env.stream())
+    want = g.host(g.op("conv2d")(xt, wtt, None, (1, 1), (1, 1)))
+    assert np.abs(g.host(y) - want).max() <= 432 * 2.0 ** -23 * np.abs(x).max() * np.abs(wt).sum((1, 2, 3)).max()
