@@ -121,16 +121,22 @@ __global__ void __launch_bounds__(256) nhwc_spatial_sum_kernel(const float* __re
   y[i] = s * scale;
 }
 
-__global__ void __launch_bounds__(256) nhwc_spatial_bcast_kernel(const float* __restrict__ dy, float* __restrict__ dx, long long total, int C, int HW, float scale) {
+// A thread keeps its V channels of one image and writes them to the pixels of its share: no index arithmetic and no load per
+// element (one division of a 64-bit index per float before: 128 x 2048 x 7x7 42 -> 14 us).
+template <int V>
+__global__ void __launch_bounds__(256) nhwc_spatial_bcast_kernel(const float* __restrict__ dy, float* __restrict__ dx, long long groups, int C, int HW, int per, float scale) {
   mtb_launch_dependents();
   mtb_wait_prior();
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (; i < total; i += stride) {
-    int c = (int)(i % C);
-    long long n = i / ((long long)C * HW);
-    dx[i] = dy[n * C + c] * scale;
-  }
+  const long long g = blockIdx.x * 256LL + threadIdx.x;  // (image, group of V channels)
+  if (g >= groups) return;
+  const long long n = g / (C / V);
+  const int c = (int)(g - n * (C / V)) * V;
+  VecF<V> v = vload<V>(dy + g * V);
+#pragma unroll
+  for (int j = 0; j < V; ++j) v.v[j] *= scale;
+  const int p0 = blockIdx.y * per, p1 = p0 + per < HW ? p0 + per : HW;
+  float* out = dx + n * HW * C + c;
+  for (int p = p0; p < p1; ++p) vstore<V>(out + (long long)p * C, v);
 }
 
 struct RedDims {
@@ -207,8 +213,16 @@ MTB_API int mtb_nhwc_spatial_sum_f32(const float* x, float* y, int n, int c, int
 // Backward of the above: dx[n,hw,c] = scale * dy[n,c].
 MTB_API int mtb_nhwc_spatial_bcast_f32(const float* dy, float* dx, int n, int c, int hw, float scale, void* stream) {
   MTB_REQUIRE(dy && dx && n > 0 && c > 0 && hw > 0, "nhwc_spatial_bcast: bad arguments");
-  long long total = (long long)n * c * hw;
-  MTB_LAUNCH(nhwc_spatial_bcast_kernel, mtb_stream_grid(total, 256), 256, 0, (cudaStream_t)stream, dy, dx, total, c, hw, scale);
+  const bool four = c % 4 == 0 && mtb_aligned16(dy) && mtb_aligned16(dx);
+  const long long groups = (long long)n * c / (four ? 4 : 1), blocks = (groups + 255) / 256;
+  // enough CTAs to fill the GPU a few times over, at least four pixels each
+  long long shares = (8LL * mtb_sm_count() + blocks - 1) / blocks;
+  if (shares > (hw + 3) / 4) shares = (hw + 3) / 4;
+  if (shares > 65535) shares = 65535;
+  const int per = (int)((hw + shares - 1) / shares);
+  const dim3 grid((unsigned)blocks, (unsigned)((hw + per - 1) / per));
+  if (four) MTB_LAUNCH(nhwc_spatial_bcast_kernel<4>, grid, 256, 0, (cudaStream_t)stream, dy, dx, groups, c, hw, per, scale);
+  else MTB_LAUNCH(nhwc_spatial_bcast_kernel<1>, grid, 256, 0, (cudaStream_t)stream, dy, dx, groups, c, hw, per, scale);
   MTB_LAUNCH_CHECK("nhwc_spatial_bcast_kernel");
   return MTB_OK;
 }
