@@ -195,19 +195,22 @@ __device__ __forceinline__ float4 ld_shared4(uint32_t a) {
 // work, and four MMAs of a narrow tile are only 192-256 cycles of work, so tiles up to 128 wide
 // take two blocks (8 MMAs) per stage.
 //
-// 32-wide tiles are for matrices of at most 64 rows (the classifier of a small network), whatever the reduction: their time is
-// what one SM loads, so A comes in boxes of 64 rows (the MMA's rows 64 to 127 read what lies behind them and are never stored)
-// and a stage takes four blocks.  64 x 128, K = 9216: 53 -> 40 us, the same bits.  Against 64 columns and more, 32 and 64 rows,
-// 32 to 4736 columns, K = 32 to 9216, cold: up to K = 512 within 1 us either way, from there on faster (K = 2048 by 15 %).
+// Tiles of 64 x 32 and 32 x 16 are for products with few outputs and a long reduction (the classifier of a small network),
+// which have nothing but the rate at which an SM loads its operands (84 GB/s) to go by: A comes in boxes of as many rows as the
+// tile has (the MMA's rows behind them read what lies there and are never stored) and a stage takes four blocks or eight.  The sum of an
+// output is the same whatever the tile.  64 x 128, K = 9216: 53 us in tiles
+// of 128 x 64, 40 in 64 x 32, 35 in 32 x 16 with eight blocks a stage (40 with four: a hand-over costs 350 cycles, a block of four
+// MMAs 170); 512 x 512, K = 4000: 26.6 -> 20.5 us in 64 x 32.
 template <int BN>
 struct Cfg {
-  static constexpr int kKB = BN == 32 ? 4 : BN <= 128 ? 2 : 1;
+  static constexpr int kKB = BN == 16 ? 8 : BN == 32 ? 4 : BN <= 128 ? 2 : 1;
   static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 3 : 4);
-  static constexpr int kRowsA = BN == 32 ? 64 : 128;
+  static constexpr int kRowsA = BN == 16 ? 32 : BN == 32 ? 64 : 128;  // rows of the tile
+  static constexpr int kAccCols = BN < 32 ? 32 : BN;                  // of one accumulator (read in 32 columns)
   static constexpr uint32_t kABytes = kRowsA * 32 * 4;   // one reduction block of A
   static constexpr uint32_t kBBytes = BN * 32 * 4;    // one reduction block of B
   static constexpr uint32_t kStageBytes = kKB * (kABytes + kBBytes);  // [A blocks][B blocks]
-  static constexpr uint32_t kTmemCols = 2 * BN;
+  static constexpr uint32_t kTmemCols = 2 * kAccCols;
 };
 
 // What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, add a tensor, or BatchNorm
@@ -220,17 +223,18 @@ constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
 // swizzle): one block per warp, two where a tensor is added (one arrives while the other is being stored).  Those kernels are
 // bound by what the epilogue moves, not by the main loop, and keep fewer stages: what they leave of the SM's shared memory is
 // where BatchNorm's partial sums and the weight gradients' reductions of the side stream run beside them (ResNet-50 step, 128
-// images, with two stages for additions 19.24 ms, with three 19.36; statistics of 256-wide tiles want all four: 19.23 against 19.33).
+// images, with two stages for additions 19.24 ms, with three 19.36).  Statistics want the depth: 256-wide tiles with four stages
+// 19.23 ms, with three 19.33; the 7x7 stem's 64-wide ones 198 us and 204, and 212 with three and a second block per warp.
 constexpr uint32_t kOutBlock = 32 * 32 * 4;
 template <int BN, int EPI, bool SPLIT>
 struct GemmSmem {
   static constexpr bool kBulk = !SPLIT && BN >= 64 && EPI != EPI_BN;
   static constexpr int kOutBlocks = !kBulk ? 0 : EPI == EPI_ADD ? 2 : 1;  // per warp
   static constexpr int stages(bool bulk) {
-    return !bulk ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 256 ? 4 : 3) : (BN == 128 ? 2 : 3);
+    return !bulk ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 128 ? 3 : 4) : (BN == 128 ? 2 : 3);
   }
-  static constexpr uint32_t bytes(bool bulk) {  // + alignment slack
-    return stages(bulk) * Cfg<BN>::kStageBytes + (bulk ? kEpilogueWarps * kOutBlocks * kOutBlock : 0) + 1024;
+  static constexpr uint32_t bytes(bool bulk) {  // + alignment slack, + rows that the MMA reads behind the last box of few rows
+    return stages(bulk) * Cfg<BN>::kStageBytes + (bulk ? kEpilogueWarps * kOutBlocks * kOutBlock : 0) + 1024 + (BN < 64 ? 128 * 128 : 0);
   }
   static constexpr uint32_t kMost = kBulk && bytes(true) > bytes(false) ? bytes(true) : bytes(false);
 };
@@ -294,7 +298,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int tile = unit / S, split = unit - tile * S;
         const int kb0 = split * p.kb_per_split;
         const int kb1 = kb0 + p.kb_per_split < p.num_kb ? kb0 + p.kb_per_split : p.num_kb;
-        const int m0 = (tile / p.n_tiles) * 128, n0 = (tile % p.n_tiles) * BN;
+        const int m0 = (tile / p.n_tiles) * C::kRowsA, n0 = (tile % p.n_tiles) * BN;
         int pix_w = 0, pix_h = 0, pix_n = 0;
         if (AMODE == A_IM2COL) {
           int ow = m0 % p.OW, t = m0 / p.OW;
@@ -373,7 +377,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_tempty[buf]), (use & 1u) ^ 1u, abort_ptr, 2));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t d_tmem = tmem_base + buf * BN;
+      const uint32_t d_tmem = tmem_base + buf * C::kAccCols;
       uint32_t acc = 0;
       for (int kb = kb0; kb < kb1; kb += C::kKB) {
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[stage]), phase, abort_ptr, 3));
@@ -404,8 +408,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quarter = warp & 3;
     // columns of the tile this warp finishes: half of the tile, from c_first on, or its share of the columns of its unit
-    constexpr int COLS = BN >= 64 ? BN / 2 : BN;
-    const int cols_here = BN < 64 && warp >= 6 ? 0 : COLS;  // a tile of 32 columns has work for four of the warps
+    constexpr int COLS = BN >= 64 ? BN / 2 : 32;
+    const int cols_here = BN < 64 && (warp >= 6 || (warp & 3) * 32 >= C::kRowsA) ? 0 : COLS;  // a narrow tile has work for one or two of the warps
     const int rank = SPLIT ? (int)(blockIdx.x % S) : 0, width = BN / S;
     const int c_first = !SPLIT ? (warp < 6 ? 0 : COLS) : rank * width + (width >= 64 && warp >= 6 ? width / 2 : 0);
     const int split_chunks = width >= 64 ? width / 64 : (warp < 6 ? 1 : 0);
@@ -480,7 +484,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
               }
             } else {
               if (inside) {
-                if (lane == 0) bulk_wait_read<0>();
+                if (lane == 0) bulk_wait_read<0>();  // the block before has been read
                 __syncwarp();
               }
             }
@@ -526,7 +530,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     if constexpr (!STATS || SPLIT) {  // statistics of unsplit reductions come through shared memory only
     for (int unit = blockIdx.x; !bulk && unit < tiles; unit += gridDim.x, ++t) {
       const int tile = unit / S;
-      const int m0 = (tile / p.n_tiles) * 128, n0 = (tile % p.n_tiles) * BN;
+      const int m0 = (tile / p.n_tiles) * C::kRowsA, n0 = (tile % p.n_tiles) * BN;
+      const int col_end = BN >= 32 || n0 + BN > p.N ? p.N : n0 + BN;
       const int buf = t & 1;
       const uint32_t use = (uint32_t)(t >> 1);
       // one lane polls (128 threads spinning on the barrier slow the other roles' barrier traffic down)
@@ -586,8 +591,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             }
           }
         } else {
-          if (valid && col0 < p.N) {
-            if (vec_ok && col0 + 32 <= p.N) {
+          if (valid && col0 < col_end) {
+            if (vec_ok && col0 + 32 <= col_end) {
 #pragma unroll
               for (int j = 0; j < 32; j += 8) {
                 float4 v[2];
@@ -617,7 +622,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             } else {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
-                if (col0 + j < p.N) {
+                if (col0 + j < col_end) {
                   float v = __uint_as_float(r[j]);
                   if (p.bias) v += p.bias[col0 + j];
                   if constexpr (BNORM) v = (v - bn_columns.mean[c_first + c0 + j]) * bn_columns.scale[c_first + c0 + j] + bn_columns.beta[c_first + c0 + j];
@@ -643,7 +648,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 #pragma unroll 1
         for (int c0 = 0; c0 < cols_here; c0 += 32) {
           uint32_t r[32];
-          tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
+          tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * C::kAccCols + c_first + c0), r);
           if constexpr (ADD) {
             float4 next[8];
             if (c0 + 32 < COLS) fetch_addend(c0 + 32, next);
@@ -773,10 +778,10 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
   CUtensorMap mapOut = mapA, mapAdd = mapA;  // unused ones are never read
   if constexpr (Smem::kBulk) {
     // Whole rows one after the other, their pitch and start on 16 bytes: what the copy engine asks for.  Everything else (a
-    // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 16
-    // reduction blocks and more on wide tiles, whose stores hide behind the main loop: the shared memory is better left to the
-    // side stream (ResNet-18 step at 512 images 6.05 ms, with all results through shared memory 6.08).
-    p.bulk_out = (EPI != EPI_PLAIN || BN == 64 || p.num_kb < 16) && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
+    // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 8
+    // reduction blocks and more: their stores hide behind the main loop, which wants the stages (8192 x 2000, K = 64:
+    // 18.8 -> 15.5 us, K = 480: 33.9 from registers, 37.2 through shared memory).
+    p.bulk_out = (EPI != EPI_PLAIN || p.num_kb < 8) && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
     if (EPI == EPI_STATS && !p.bulk_out) return mtb_fail(MTB_ERR_INVALID, "tc_gemm: statistics need whole aligned rows");
     if (p.bulk_out) {
       if (int rc = tc::encode_result_2d(&mapOut, p.out, p.M, p.N, p.ldo)) return rc;
@@ -802,8 +807,10 @@ int stats_rows_for(int tiles, int n_tiles) {
 
 template <int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc_bn(int bn, const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
-  if constexpr (AMODE == A_KMAJOR && BMODE == B_KMAJOR && EPI == EPI_PLAIN)
+  if constexpr (AMODE == A_KMAJOR && BMODE == B_KMAJOR && EPI == EPI_PLAIN) {
+    if (bn == 16) return launch_tc<16, AMODE, BMODE, EPI>(mapA, mapB, p, st);
     if (bn == 32) return launch_tc<32, AMODE, BMODE, EPI>(mapA, mapB, p, st);
+  }
   if (bn == 64) return launch_tc<64, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   if (bn == 128) return launch_tc<128, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   return launch_tc<256, AMODE, BMODE, EPI>(mapA, mapB, p, st);
@@ -977,13 +984,22 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                     void* stream) {
   CUtensorMap mapA, mapB;
-  const bool narrow = m <= 64 && !trans_a && trans_b && n <= 32 * mtb_sm_count();  // see Cfg
-  const int bn = narrow ? 32 : cheapest_bn(n, m, (k + 31) / 32, !trans_b);
+  int bn = cheapest_bn(n, m, (k + 31) / 32, !trans_b), rows = 128;
+  if (!trans_a && trans_b) {  // see Cfg
+    auto narrow_ns = [&](int r, int c, double block) {
+      const long long tiles = (long long)((m + r - 1) / r) * ((n + c - 1) / c);
+      return (tiles + mtb_sm_count() - 1) / mtb_sm_count() * (((k + 31) / 32) * block + 900.0);
+    };
+    double best = im2col_ns(bn, n, m, (k + 31) / 32, false);
+    if (m <= 64 && narrow_ns(64, 32, 146) <= 900 + ((k + 31) / 32) * 146.0) { bn = 32; rows = 64; best = narrow_ns(64, 32, 146); }
+    else if (narrow_ns(64, 32, 146) < 0.9 * best) { bn = 32; rows = 64; best = narrow_ns(64, 32, 146); }
+    if (narrow_ns(32, 16, 92) < 0.9 * best) { bn = 16; rows = 32; }
+  }
   int rc;
   GemmParams p{};
   p.a_blocks = trans_a && m % 32 == 0;
   p.b_blocks = !trans_b && n % 32 == 0;
-  if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, narrow ? 64 : 128);
+  if (!trans_a) rc = tc::encode_tiled_2d(&mapA, a, m, k, k, 32, rows);
   else if (p.a_blocks) rc = tc::encode_blocks_3d(&mapA, a, k, m, m, 32, 4);
   else rc = tc::encode_tiled_2d(&mapA, a, k, m, m, 32, 32, true);
   if (rc) return rc;
@@ -993,7 +1009,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   if (rc) return rc;
   p.splits = 1; p.kb_per_split = (k + 31) / 32;
   p.M = m; p.N = n; p.num_kb = (k + 31) / 32;
-  p.m_tiles = (m + 127) / 128; p.n_tiles = (n + bn - 1) / bn;
+  p.m_tiles = (m + rows - 1) / rows; p.n_tiles = (n + bn - 1) / bn;
   p.out = c; p.ldo = n; p.bias = bias; p.relu = relu;
   p.KH = 1; p.KW = 1; p.cchunks = p.num_kb;
   cudaStream_t st = (cudaStream_t)stream;
