@@ -87,7 +87,8 @@ int mtb_graph_destroy(void* graph_exec);
  *      mytorch/backends/cuda/ops/conv.py:9-90) ---- */
 long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
 /* y[N,OH,OW,Cout] = conv(x[N,H,W,Cin], wt[Cout,KH,KW,Cin]) + bias (bias may be NULL); relu != 0 clamps at 0.
- * workspace: not used, may be NULL (only the weight gradient needs mtb_conv2d_workspace_bytes()).  A layer with too few output
+ * workspace: may be NULL (only the weight gradient needs mtb_conv2d_workspace_bytes()); with that many bytes, channel counts
+ * that fit no block of 32 run on the tensor cores too, in FP32 accuracy.  A layer with too few output
  * tiles to fill the GPU splits its reduction over a cluster of CTAs, which add in a fixed order: results are reproducible.
  * A filter larger than the padded input is refused by every entry point. */
 int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
@@ -138,6 +139,8 @@ int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, i
  * C[M,N] = op(A) op(B) (+ bias[N]) (relu). A is [M,K] (trans_a 0) or [K,M]; B is [K,N] (trans_b 0) or [N,K]. */
 int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
                  void* stream);
+/* y = max(0, x w^T + bias) for x [m,k], w [n,k]; pre (may be NULL) takes x w^T + bias, which the ReLU's backward masks by. */
+int mtb_linear_relu_f32(int m, int n, int k, const float* x, const float* w, const float* bias, float* pre, float* y, void* stream);
 
 /* ---- BatchNorm2d (replaces batch_norm2d_reference_<dt> and its backward,
  *      mytorch/native/cuda/batch_norm.cu/source.cu:134-166 and :269-289) ---- */

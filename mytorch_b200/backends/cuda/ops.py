@@ -384,6 +384,29 @@ def cuda_linear(x, weight, bias):
     return y
 
 
+@_reg("cuda", "linear_relu")
+def cuda_linear_relu(x, weight, bias, keep):
+    """(relu(x Wᵀ + b), x Wᵀ + b or None): a Linear layer and the ReLU behind it in one launch.  ``keep``: a backward pass will
+    ask for the second, whose sign masks the gradient."""
+    _f32(x, weight, bias)
+    env = _env(x)
+    b, fin = x.shape
+    fout = weight.shape[0]
+    if weight.shape[1] != fin:
+        raise MismatchShapesError([x.shape, weight.shape])
+    y, pre = _new((b, fout), x), _new((b, fout), x) if keep else None
+    env.lib.linear_relu_f32(b, fout, fin, x, weight, bias, pre, y, env.stream())
+    return y, pre
+
+
+@_reg("cuda", "linear_relu_backward")
+def cuda_linear_relu_backward(output_grad, pre, x, weight, bias):
+    env = _env(x)
+    masked = _new(pre.shape, pre)
+    env.lib.relu_backward_f32(output_grad, pre, masked, _numel(pre.shape), env.stream())
+    return cuda_linear_backward(masked, x, weight, bias)
+
+
 @_reg("cuda", "linear_backward")
 def cuda_linear_backward(output_grad, x, weight, bias):
     env = _env(x)

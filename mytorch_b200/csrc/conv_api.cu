@@ -51,8 +51,8 @@ int dgrad_fp32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int
 
 }  // namespace
 
-// workspace (may be NULL): scratch of mtb_conv2d_workspace_bytes() for the weight gradient; forward and data gradient take it
-// for symmetry (layers whose output has too few tiles split their reduction over clusters, without scratch).
+// workspace (may be NULL): scratch of mtb_conv2d_workspace_bytes() for the weight gradient, and for the operands of channel counts
+// that fit no block of 32 (tc_split.cuh); without it forward and data gradient of those run on the CUDA cores.
 MTB_API int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                    const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes,
                                    void* stream) {
@@ -151,4 +151,11 @@ MTB_API int mtb_gemm_f32(int m, int n, int k, const float* a, int trans_a, const
   if (mtb_tc_gemm_supported(m, n, k, a, trans_a, b, trans_b, c))
     return mtb_tc_gemm_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream);
   return mtb_gemm_simt_f32(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream);
+}
+
+// y = max(0, x w^T + bias) for x [m,k], w [n,k], and, with pre != NULL, pre = x w^T + bias: a Linear layer and the ReLU behind it
+// in one launch, with what the ReLU's backward masks by.
+MTB_API int mtb_linear_relu_f32(int m, int n, int k, const float* x, const float* w, const float* bias, float* pre, float* y, void* stream) {
+  if (mtb_tc_gemm_supported(m, n, k, x, 0, w, 1, y)) return mtb_tc_gemm_f32(m, n, k, x, 0, w, 1, bias, 1, y, stream, pre);
+  return mtb_gemm_simt(m, n, k, x, 0, w, 1, bias, 1, y, stream, pre);
 }

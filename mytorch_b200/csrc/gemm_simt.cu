@@ -1,5 +1,6 @@
 // Dense matrix products on the CUDA cores (FP32): `mm` / Linear shapes whose pitches or sizes the tensor-core GEMM does
 // not take.  See simt_tile.cuh for the kernel.
+#include "kernels.h"
 #include "simt_tile.cuh"
 
 namespace {
@@ -66,6 +67,11 @@ __global__ void __launch_bounds__(256) gemm_few_rows_kernel(const float* __restr
 // (trans_b == 0) or [N,K]; all row-major and dense.
 MTB_API int mtb_gemm_simt_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu,
                               float* c, void* stream) {
+  return mtb_gemm_simt(m, n, k, a, trans_a, b, trans_b, bias, relu, c, stream, nullptr);
+}
+
+int mtb_gemm_simt(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c, void* stream,
+                  float* pre) {
   MTB_REQUIRE(a && b && c && m > 0 && n > 0 && k > 0, "gemm: bad arguments");
   if (trans_a && !trans_b && m <= 16 && !bias && !relu) {
     MTB_LAUNCH(gemm_few_rows_kernel, dim3(mtb_div_up(n, 32), mtb_div_up(m, 2)), 256, 0, (cudaStream_t)stream, a, b, c, m, n, k);
@@ -73,7 +79,7 @@ MTB_API int mtb_gemm_simt_f32(int m, int n, int k, const float* a, int trans_a, 
     return MTB_OK;
   }
   Out o{};
-  o.out = c; o.ld = n; o.bias = bias; o.relu = relu;
+  o.out = c; o.ld = n; o.bias = bias; o.relu = relu; o.pre = pre;
   // four neighbours of each operand in one load: along k for [rows][K] operands, along the row for [K][rows] ones
   const bool vec = mtb_aligned16(a) && mtb_aligned16(b) && (trans_a ? m : k) % 4 == 0 && (trans_b ? k : n) % 4 == 0;
   return vec ? dense<4>(m, n, k, a, trans_a, b, trans_b, o, (cudaStream_t)stream)

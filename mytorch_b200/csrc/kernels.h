@@ -23,6 +23,9 @@ MTB_API int mtb_conv2d_wgrad_simt_f32(int n, int cin, int h, int w, int kh, int 
                                       const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream);
 MTB_API int mtb_gemm_simt_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu,
                               float* c, void* stream);
+// pre (may be NULL; neither operand transposed in memory): the result before the ReLU
+int mtb_gemm_simt(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c, void* stream,
+                  float* pre);
 
 // tcgen05 tensor-core family (tc_*.cu)
 long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
@@ -45,7 +48,7 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
                             const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream);
 bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* c);
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* stream);
+                    void* stream, float* pre = nullptr);
 
 double mtb_conv2d_simt_us(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction);
 

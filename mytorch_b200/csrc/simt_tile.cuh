@@ -307,6 +307,7 @@ struct Out {
   MtbBnEval bn;              // mean != NULL: BatchNorm with running statistics after the bias (cluster kernels only)
   const float* residual;     // laid out like out: added before the ReLU (cluster kernels only)
   int relu;
+  float* pre;                // laid out like out, takes the value before the ReLU (dense products of two operands along k only)
   long long split_plane;     // > 0: every slice of the reduction writes its own plane of partials
   const DgradClass* cls;     // data gradient: row -> pixel of the residue class
   int H, W, SH, SW;
@@ -325,7 +326,7 @@ __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
 }
 
 // TAIL: with BatchNorm and the residual of Out (the cluster kernels, whose store is one loop)
-template <bool TAIL>
+template <bool TAIL, bool PRE>
 __device__ __forceinline__ void store4(const Out& o, float* row, int j, int N, bool vec, float4 v) {
   float t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -338,6 +339,9 @@ __device__ __forceinline__ void store4(const Out& o, float* row, int j, int N, b
         t[q] = (t[q] - o.bn.mean[j + q]) * scale + beta;
       }
       if (o.residual && j + q < N) t[q] += o.residual[row - o.out + j + q];
+    }
+    if constexpr (PRE) {
+      if (o.pre && j + q < N) o.pre[row - o.out + j + q] = t[q];
     }
     if (o.relu) t[q] = fmaxf(t[q], 0.f);
   }
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
         const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], q));
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
       }
-      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>>(o, out_row(o, m0 + r, z), n0 + c, N, vec, s);
+      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>, std::is_same_v<SA, DenseK> && std::is_same_v<SB, DenseK>>(o, out_row(o, m0 + r, z), n0 + c, N, vec, s);
     }
     cluster.sync();  // nobody leaves while its tile is being read
   } else {
@@ -489,7 +493,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
       float* row = out_row(o, i, z) + slice * o.split_plane;
 #pragma unroll
       for (int g = 0; g < GN; ++g)
-        store4<false>(o, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
+        store4<false, std::is_same_v<SA, DenseK> && std::is_same_v<SB, DenseK>>(o, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
     }
   }
 }

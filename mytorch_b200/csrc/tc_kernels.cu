@@ -142,6 +142,7 @@ struct GemmParams {
   const float* addend;
   MtbBnEval bn;  // EPI_BN
   int relu;
+  float* pre;  // dense K-major products only: laid out like `out`, takes the result before the ReLU (may be NULL)
   // results (and the addend) move through shared memory by bulk copies (see the epilogue); rows lie one after the other
   int bulk_out;
   int stages;  // of the ring
@@ -248,6 +249,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   using Smem = GemmSmem<BN, EPI, SPLIT>;
   const int STAGES = p.stages;
   constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN, ADD = EPI == EPI_ADD || BNORM;
+  constexpr bool PRE = EPI == EPI_PLAIN && AMODE == A_KMAJOR && BMODE == B_KMAJOR;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2], bar_add[kEpilogueWarps][2];
   __shared__ uint32_t tmem_slot;
@@ -414,8 +416,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int c_first = !SPLIT ? (warp < 6 ? 0 : COLS) : rank * width + (width >= 64 && warp >= 6 ? width / 2 : 0);
     const int split_chunks = width >= 64 ? width / 64 : (warp < 6 ? 1 : 0);
     int t = 0;
-    const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0);
-    const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 31u) == 0);  // 32-byte stores
+    const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.pre)) & 15u) == 0);
+    const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pre)) & 31u) == 0);  // 32-byte stores
     // statistics of a split reduction: narrow tiles keep per-lane sums, wide tiles merge per tile
     constexpr bool LANE_SUMS = STATS && SPLIT && BN == 64;
     WarpColStats<(STATS && !LANE_SUMS) ? COLS / 32 : 1> stats;
@@ -615,7 +617,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     const float4 b = adds ? add[jj / 4] : *reinterpret_cast<const float4*>(arow + col0 + jj);
                     v[h].x += b.x; v[h].y += b.y; v[h].z += b.z; v[h].w += b.w;
                   }
-                  if (p.relu) { v[h].x = fmaxf(v[h].x, 0.f); v[h].y = fmaxf(v[h].y, 0.f); v[h].z = fmaxf(v[h].z, 0.f); v[h].w = fmaxf(v[h].w, 0.f); }
+                  if constexpr (!PRE) {
+                    if (p.relu) { v[h].x = fmaxf(v[h].x, 0.f); v[h].y = fmaxf(v[h].y, 0.f); v[h].z = fmaxf(v[h].z, 0.f); v[h].w = fmaxf(v[h].w, 0.f); }
+                  }
+                }
+                if constexpr (PRE) {
+                  if (p.pre) st_row8(p.pre + orow_index * p.ldo + col0 + j, v[0], v[1], wide_ok);
+                  if (p.relu) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) { v[h].x = fmaxf(v[h].x, 0.f); v[h].y = fmaxf(v[h].y, 0.f); v[h].z = fmaxf(v[h].z, 0.f); v[h].w = fmaxf(v[h].w, 0.f); }
+                  }
                 }
                 st_row8(orow + col0 + j, v[0], v[1], wide_ok);
               }
@@ -627,6 +638,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                   if (p.bias) v += p.bias[col0 + j];
                   if constexpr (BNORM) v = (v - bn_columns.mean[c_first + c0 + j]) * bn_columns.scale[c_first + c0 + j] + bn_columns.beta[c_first + c0 + j];
                   if (ADD && arow) v += arow[col0 + j];
+                  if constexpr (PRE) { if (p.pre) p.pre[orow_index * p.ldo + col0 + j] = v; }
                   if (p.relu) v = fmaxf(v, 0.f);
                   orow[col0 + j] = v;
                 }
@@ -781,7 +793,7 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
     // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 8
     // reduction blocks and more: their stores hide behind the main loop, which wants the stages (8192 x 2000, K = 64:
     // 18.8 -> 15.5 us, K = 480: 33.9 from registers, 37.2 through shared memory).
-    p.bulk_out = (EPI != EPI_PLAIN || p.num_kb < 8) && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
+    p.bulk_out = (EPI != EPI_PLAIN || p.num_kb < 8) && !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
     if (EPI == EPI_STATS && !p.bulk_out) return mtb_fail(MTB_ERR_INVALID, "tc_gemm: statistics need whole aligned rows");
     if (p.bulk_out) {
       if (int rc = tc::encode_result_2d(&mapOut, p.out, p.M, p.N, p.ldo)) return rc;
@@ -982,7 +994,7 @@ bool mtb_tc_gemm_supported(int m, int n, int k, const float* a, int trans_a, con
 }
 
 int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const float* bias, int relu, float* c,
-                    void* stream) {
+                    void* stream, float* pre) {
   CUtensorMap mapA, mapB;
   int bn = cheapest_bn(n, m, (k + 31) / 32, !trans_b), rows = 128;
   if (!trans_a && trans_b) {  // see Cfg
@@ -1010,7 +1022,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   p.splits = 1; p.kb_per_split = (k + 31) / 32;
   p.M = m; p.N = n; p.num_kb = (k + 31) / 32;
   p.m_tiles = (m + rows - 1) / rows; p.n_tiles = (n + bn - 1) / bn;
-  p.out = c; p.ldo = n; p.bias = bias; p.relu = relu;
+  p.out = c; p.ldo = n; p.bias = bias; p.relu = relu; p.pre = pre;
   p.KH = 1; p.KW = 1; p.cchunks = p.num_kb;
   cudaStream_t st = (cudaStream_t)stream;
   if (!trans_a && trans_b) return launch_tc_bn<A_KMAJOR, B_KMAJOR>(bn, mapA, mapB, p, st);

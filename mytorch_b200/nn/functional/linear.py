@@ -19,3 +19,18 @@ def linear(x: Tensor, weight: Tensor, bias=None) -> Tensor:
 @tracker.register_backward_function("linear")
 def linear_backward(output_grad, x, weight, bias):
     return dispatch(x.device, "linear_backward")(output_grad, x, weight, bias)
+
+
+def _linear_relu(x: Tensor, weight: Tensor, bias=None) -> Tensor:
+    """relu(linear(x, weight, bias)) as one operator on CUDA, the same bits (``nn.Sequential`` runs such neighbours this way)."""
+    if x.device != weight.device or (bias is not None and bias.device != x.device):
+        raise MismatchDevicesError([x.device, weight.device])
+    wanted = grad_enabled(x, weight, bias)
+    out, pre = dispatch(x.device, "linear_relu")(x, weight, bias, wanted)
+    out.requires_grad = wanted
+    return record("linear_relu", [x, weight, bias], out, [pre])
+
+
+@tracker.register_backward_function("linear_relu")
+def _linear_relu_backward(output_grad, pre, x, weight, bias):
+    return dispatch(x.device, "linear_relu_backward")(output_grad, pre, x, weight, bias)

@@ -1,6 +1,8 @@
 from mytorch_b200.nn.batch_norm import BatchNorm2d, BatchNormReLU2d, inference_conv_norm
 from mytorch_b200.nn.conv import Conv2d
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu
+from mytorch_b200.nn.functional.linear import _linear_relu
+from mytorch_b200.nn.linear import Linear
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.relu import ReLU
 
@@ -9,7 +11,7 @@ _NORMS = (BatchNorm2d, BatchNormReLU2d)
 
 class Sequential(Module):
     """Layers one after the other.  Neighbours that exist as one operator with the same bits run as one on CUDA: BatchNorm2d +
-    ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU) with running statistics.  A step of the
+    ReLU, Linear + ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU) with running statistics.  A step of the
     MNIST example is 300 library calls of a few microseconds each, so every operator left out shows."""
 
     def __init__(self, *args):
@@ -34,6 +36,11 @@ class Sequential(Module):
             if kind is BatchNorm2d and kind_after is ReLU and input.device.type == "cuda" and not (layer._forward_replaced or after._forward_replaced):
                 input = _batch_norm2d_relu(input, layer.weight, layer.bias, layer.eps, layer.training, layer.momentum, layer.running_mean,
                                            layer.running_var)
+                i += 2
+                continue
+            if (kind is Linear and kind_after is ReLU and input.device.type == "cuda" and len(input.shape) == 2
+                    and not (layer._forward_replaced or after._forward_replaced)):
+                input = _linear_relu(input, layer.weight, layer.bias)
                 i += 2
                 continue
             input = layer(input)
