@@ -441,6 +441,7 @@ int split_bn(int n) {
 }
 
 constexpr long long kSplitPacked = 64LL << 20;      // packed activations of one operand at a time, which the L2 holds
+constexpr long long kSplitImage = 256LL << 20;      // most that one packed image may take: scratch is kept, and is not to grow with the image
 constexpr long long kSplitHeader = 4 * (2 * 1024 + 1024);  // words of the packing pass, then one per group of images
 
 // images per pass
@@ -497,8 +498,9 @@ double split_us(const SplitGeometry& q, int direction) {
 // Whether the two-term products take a direction: within the copy engine's limits, cheaper than the CUDA-core kernels, and a
 // reduction of at least 96.  A sum of fewer terms rounds less in FP32 than the operands do here (relative errors against 64
 // bits: 20 terms 8.2e-8 on the CUDA cores, 1.15e-7 here; 27 terms 9.4e-8 and 1.07e-7; 96 terms 1.76e-7 and 1.33e-7; 432 terms
-// 3.7e-7 and 1.5e-7; 3600 terms 1.06e-6 and 2.3e-7; weight gradients over 43,808 pixels 6.6e-7 and 2.1e-7).  Prices against
-// measurements on 30 shapes from 8 to 512 channels: within 40 %, and the faster side taken where they differ by a quarter.
+// 3.7e-7 and 1.5e-7; 3600 terms 1.06e-6 and 2.3e-7; weight gradients over 43,808 pixels 6.6e-7 and 2.1e-7).  Of 30 shapes
+// of 3 to 512 channels the price took the slower side for none; it left the faster one for seven directions, by 1.8 times at
+// most (strided data gradients, few pixels under a wide filter).
 bool split_takes(const SplitGeometry& q, int direction) {
   const bool always = getenv("MTB_TC_SPLIT_ALWAYS") != nullptr;  // for tests of small shapes
   // 4e7 products take the CUDA cores about 15 us, less than the launches here; a small network's calls end at this test
@@ -506,6 +508,7 @@ bool split_takes(const SplitGeometry& q, int direction) {
   if (getenv("MTB_DISABLE_TC") || getenv("MTB_DISABLE_TC_SPLIT")) return false;
   if (q.sh > 8 || q.sw > 8 || q.ph > 64 || q.pw > 64 || q.kh > 32 || q.kw > 32 || q.kh * q.kw > 64) return false;
   if (split_x_bytes(q, q.n) < kMinIm2colBytes || split_dy_bytes(q, q.n) < kMinIm2colBytes) return false;
+  if (split_x_bytes(q, 1) > kSplitImage || split_dy_bytes(q, 1) > kSplitImage) return false;
   const int terms = direction == 0 ? q.kh * q.kw * q.cin : direction == 1 ? (q.kh / q.sh > 0 ? q.kh / q.sh : 1) * (q.kw / q.sw > 0 ? q.kw / q.sw : 1) * q.cout : 96;
   if (terms < 96 && !always) return false;
   // items of the packing pass are numbered with 32 bits
