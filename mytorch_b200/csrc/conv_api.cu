@@ -4,14 +4,26 @@
 #include "common.cuh"
 #include "kernels.h"
 
+namespace {
+
+// Scratch of the two-term products for one direction, 0 where they do not take it.  Their channel counts are those that fit no
+// block of 32, whatever else keeps the TF32 kernels from a call (a small or an unaligned tensor: CUDA cores).  The size that a
+// caller is told and the choice of the kernel both rest on this number, so that the choice never depends on how much
+// scratch more than that the caller happens to pass.
+long long split_scratch_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction) {
+  if (direction == 1 ? cout % 32 == 0 && cin % 4 == 0 : cin % 32 == 0 && cout % 4 == 0) return 0;
+  return mtb_split_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
+}
+
+}  // namespace
+
 MTB_API long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   // no such convolution: the call that the scratch is for says so
   if (n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return 0;
   long long a = mtb_conv2d_wgrad_simt_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   long long b = mtb_tc_conv2d_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
-  for (int direction = 0; direction < 3; ++direction) {  // those that the TF32 kernels leave (unaligned tensors aside, which then take the CUDA cores)
-    if (direction == 1 ? cout % 32 == 0 && cin % 4 == 0 : cin % 32 == 0 && cout % 4 == 0) continue;
-    const long long c = mtb_split_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
+  for (int direction = 0; direction < 3; ++direction) {
+    const long long c = split_scratch_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
     if (c > b) b = c;
   }
   return a > b ? a : b;
@@ -25,7 +37,7 @@ bool split_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, i
   if (!workspace || !mtb_aligned16(workspace) || n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0 ||
       !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw))
     return false;
-  const long long need = mtb_split_workspace_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
+  const long long need = split_scratch_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, direction);
   return need > 0 && workspace_bytes >= need;
 }
 
