@@ -495,6 +495,16 @@ double split_us(const SplitGeometry& q, int direction) {
   return 8 + (forward ? x : dy) / 4.5e6 + passes * classes * ((products > store ? products : store) + 4);
 }
 
+// Most terms of a sum that are not padding: of an output's window at most h x w taps lie on the image, of an input's window (the
+// residue class with the fewest taps) at most oh x ow; a filter entry meets every image at most ceil(h / sh) x ceil(w / sw) times.
+long long split_terms(const SplitGeometry& q, int direction) {
+  auto least = [](int a, int b) { return a < b ? a : b; };
+  auto class_taps = [&](int k, int s, int size) { return least(k / s > 0 ? k / s : 1, size); };
+  if (direction == 0) return (long long)least(q.kh, q.h) * least(q.kw, q.w) * q.cin;
+  if (direction == 1) return (long long)class_taps(q.kh, q.sh, q.oh) * class_taps(q.kw, q.sw, q.ow) * q.cout;
+  return (long long)q.n * least(q.oh, (q.h + q.sh - 1) / q.sh) * least(q.ow, (q.w + q.sw - 1) / q.sw);
+}
+
 // Whether the two-term products take a direction: within the copy engine's limits, cheaper than the CUDA-core kernels, and a
 // reduction of at least 96.  A sum of fewer terms rounds less in FP32 than the operands do here (relative errors against 64
 // bits: 20 terms 8.2e-8 on the CUDA cores, 1.15e-7 here; 27 terms 9.4e-8 and 1.07e-7; 96 terms 1.76e-7 and 1.33e-7; 432 terms
@@ -509,8 +519,7 @@ bool split_takes(const SplitGeometry& q, int direction) {
   if (q.sh > 8 || q.sw > 8 || q.ph > 64 || q.pw > 64 || q.kh > 32 || q.kw > 32 || q.kh * q.kw > 64) return false;
   if (split_x_bytes(q, q.n) < kMinIm2colBytes || split_dy_bytes(q, q.n) < kMinIm2colBytes) return false;
   if (split_x_bytes(q, 1) > kSplitImage || split_dy_bytes(q, 1) > kSplitImage) return false;
-  const int terms = direction == 0 ? q.kh * q.kw * q.cin : direction == 1 ? (q.kh / q.sh > 0 ? q.kh / q.sh : 1) * (q.kw / q.sw > 0 ? q.kw / q.sw : 1) * q.cout : 96;
-  if (terms < 96 && !always) return false;
+  if (split_terms(q, direction) < 96 && !always) return false;
   // items of the packing pass are numbered with 32 bits
   const int images = split_images(q, true, true);
   const long long most = (split_x_bytes(q, images) + split_dy_bytes(q, images)) / 32 + (long long)q.kh * q.kw * (q.cin + 32LL) * (q.cout + 32LL);

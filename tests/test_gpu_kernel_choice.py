@@ -36,3 +36,25 @@ def test_more_scratch_than_asked_for_changes_no_bit(n, cin, h, cout, k, pad, off
 
     for got, want, what in zip(run(LARGE), run(need), ("forward", "data gradient", "weight gradient")):
         assert np.array_equal(got, want), what
+
+
+@pytest.mark.parametrize("n,cin,h,cout,k,pad,which", [
+    (40000, 24, 1, 130, 3, 1, 0),   # 9 x 24 terms, of which 24 are not padding
+    (20000, 100, 2, 12, 5, 2, 1),   # 25 x 12 and 48
+    (1, 1500, 6, 470, 7, 3, 2)])    # sums over 36 pixels
+def test_short_sums_stay_in_fp32(n, cin, h, cout, k, pad, which, monkeypatch):
+    """Sums of fewer than 96 terms round less in FP32 than the operands of the two-term products do."""
+    import gpu_util as g
+
+    rng = np.random.default_rng(which)
+    x, wt, dy = (rng.standard_normal(shape).astype(np.float32) for shape in ((n, cin, h, h), (cout, cin, k, k), (n, cout, h, h)))
+
+    def run():
+        xt, wtt = g.dev(x, True), g.dev(wt, True)
+        if which == 0:
+            return g.host(g.op("conv2d")(xt, wtt, None, (1, 1), (pad, pad)))
+        return g.host(g.op("conv2d_backward")(g.dev(dy), xt, wtt, None, (1, 1), (pad, pad))[which - 1])
+
+    got = run()
+    monkeypatch.setenv("MTB_DISABLE_TC_SPLIT", "1")
+    assert np.array_equal(got, run())
