@@ -441,7 +441,7 @@ int split_bn(int n) {
 }
 
 constexpr long long kSplitPacked = 64LL << 20;      // packed activations of one operand at a time, which the L2 holds
-constexpr long long kSplitImage = 256LL << 20;      // most that one packed image may take: scratch is kept, and is not to grow with the image
+constexpr long long kSplitMost = 256LL << 20;       // most that one packed image, or the packed filter, may take: scratch is kept, and is not to grow with them
 constexpr long long kSplitHeader = 4 * (2 * 1024 + 1024);  // words of the packing pass, then one per group of images
 
 // images per pass
@@ -456,7 +456,18 @@ int split_images(const SplitGeometry& q, bool with_x, bool with_dy) {
 long long split_x_bytes(const SplitGeometry& q, int images) { return (long long)images * q.h * q.w * split_blocks(q.cin) * 256; }
 long long split_dy_bytes(const SplitGeometry& q, int images) { return (long long)images * q.oh * q.ow * split_blocks(q.cout) * 256; }
 
-struct SplitWgradPlan { int images, bn, chunks, m_tiles, n_tiles, splits; };
+// The filter as forward and data gradient read it; for the weight gradient one plane of sums.
+long long split_filter_bytes(const SplitGeometry& q, int direction) {
+  const long long taps = (long long)q.kh * q.kw;
+  if (direction == 0) return q.cout * taps * split_blocks(q.cin) * 256;
+  if (direction == 1) return q.cin * taps * split_blocks(q.cout) * 256;
+  return q.cout * taps * q.cin * 4;
+}
+
+struct SplitWgradPlan {
+  int images, bn, chunks, m_tiles, n_tiles, splits;
+  bool whole;  // one group of images in one piece: sums go to dw, not to planes
+};
 SplitWgradPlan split_wgrad_plan(const SplitGeometry& q) {
   SplitWgradPlan r;
   r.images = split_images(q, true, true);
@@ -468,6 +479,7 @@ SplitWgradPlan split_wgrad_plan(const SplitGeometry& q) {
   int s = mtb_sm_count() / (r.m_tiles * r.n_tiles);
   if (s > kb / 8) s = kb / 8;
   r.splits = s < 1 ? 1 : s;
+  r.whole = r.splits == 1 && r.images >= q.n;
   return r;
 }
 
@@ -518,7 +530,7 @@ bool split_takes(const SplitGeometry& q, int direction) {
   if (getenv("MTB_DISABLE_TC") || getenv("MTB_DISABLE_TC_SPLIT")) return false;
   if (q.sh > 8 || q.sw > 8 || q.ph > 64 || q.pw > 64 || q.kh > 32 || q.kw > 32 || q.kh * q.kw > 64) return false;
   if (split_x_bytes(q, q.n) < kMinIm2colBytes || split_dy_bytes(q, q.n) < kMinIm2colBytes) return false;
-  if (split_x_bytes(q, 1) > kSplitImage || split_dy_bytes(q, 1) > kSplitImage) return false;
+  if (split_x_bytes(q, 1) > kSplitMost || split_dy_bytes(q, 1) > kSplitMost || split_filter_bytes(q, direction) > kSplitMost) return false;
   if (split_terms(q, direction) < 96 && !always) return false;
   // items of the packing pass are numbered with 32 bits
   const int images = split_images(q, true, true);
@@ -576,11 +588,11 @@ SplitGeometry split_geometry(int n, int cin, int h, int w, int kh, int kw, int s
 long long mtb_split_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction) {
   const SplitGeometry q = split_geometry(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (!split_takes(q, direction)) return 0;
-  const long long taps = (long long)kh * kw;
-  if (direction == 0) return kSplitHeader + split_x_bytes(q, split_images(q, true, false)) + cout * taps * split_blocks(cin) * 256;
-  if (direction == 1) return kSplitHeader + split_dy_bytes(q, split_images(q, false, true)) + cin * taps * split_blocks(cout) * 256;
+  const long long filter = split_filter_bytes(q, direction);
+  if (direction == 0) return kSplitHeader + split_x_bytes(q, split_images(q, true, false)) + filter;
+  if (direction == 1) return kSplitHeader + split_dy_bytes(q, split_images(q, false, true)) + filter;
   const SplitWgradPlan r = split_wgrad_plan(q);
-  return kSplitHeader + split_x_bytes(q, r.images) + split_dy_bytes(q, r.images) + (long long)r.splits * cout * taps * cin * 4;
+  return kSplitHeader + split_x_bytes(q, r.images) + split_dy_bytes(q, r.images) + (r.whole ? 0 : r.splits * filter);
 }
 
 // *guard: the words that say whether the operands could not be split (*guards of them; the CUDA-core kernel then does the work).
@@ -709,8 +721,7 @@ int mtb_split_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int
     p.kb_per_split = (p.kb_total + r.splits - 1) / r.splits;
     p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;
     p.OW = q.ow; p.OH = q.oh; p.SW = sw; p.SH = sh; p.PW = pw; p.PH = ph; p.KW = kw;
-    const bool whole = p.splits == 1 && r.images >= n;
-    p.partial = whole ? dw : planes;
+    p.partial = r.whole ? dw : planes;
     p.Kw = (long long)kh * kw * cin;
     p.bad = bad; p.n_bad = count; p.any_bad = any + pass;
     if (r.bn == 32) rc = launch_split_wgrad<32>(mapX, mapDY, p, st);
@@ -718,7 +729,7 @@ int mtb_split_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int
     else if (r.bn == 96) rc = launch_split_wgrad<96>(mapX, mapDY, p, st);
     else rc = launch_split_wgrad<128>(mapX, mapDY, p, st);
     if (rc) return rc;
-    if (!whole) {
+    if (!r.whole) {
       MTB_LAUNCH(split_add_planes_kernel, dim3(mtb_stream_grid(total, 256)), dim3(256), 0, st, planes, dw, total, p.splits, pass > 0, any + pass);
       MTB_LAUNCH_CHECK("split_add_planes_kernel");
     }

@@ -30,3 +30,12 @@ def test_taken_where_they_pay(scratch):
 def test_weight_gradients_over_few_pixels_are_not_taken(scratch):
     asked, without = scratch(1, 1500, 6, 6, 7, 7, 1, 1, 3, 3, 470)  # no other direction of it is taken either
     assert asked == without
+
+
+def test_scratch_is_bounded(scratch):
+    """64 MB of packed activations an operand or one image of at most 256 MB, a packed filter of at most 256 MB, and planes of
+    sums only where a weight gradient is added up from several."""
+    header = 4 * 3 * 1024
+    # forward and data gradient of 2000 -> 470, 7x7 would pack 370 MB of filter; its weight gradient over one image is written in one piece
+    asked, without = scratch(1, 2000, 11, 11, 7, 7, 1, 1, 3, 3, 470)
+    assert without < asked == header + 121 * (63 + 15) * 256
