@@ -10,8 +10,10 @@
 // is one reduction block (the two small products first, then four steps of hi * hi'); the epilogue warps add the chains up in
 // registers with FP32 rounding while the next ones run (four accumulators in tensor memory).
 //
-// Infinities, NaN and magnitudes above 3e38 do not survive the split (inf - inf): the packing pass reports them, the products
-// then do nothing, and the CUDA-core kernel, which is enqueued behind and otherwise returns at once, computes the result.
+// Infinities, NaN and magnitudes above 3e38 do not survive the split (inf - inf), and where a whole operand is tiny lo falls
+// under the smallest normal number, which the tensor core takes for zero (values of 1e-37: error 3.3e-5 instead of 2.6e-7 on the
+// CUDA cores).  The packing pass reports both, the products then do nothing, and the CUDA-core kernel, which is
+// enqueued behind and otherwise returns at once, computes the result.
 //
 // What bounds it: copies into shared memory (a block of 128 x 96 outputs takes 56 KB, 0.63 us at the measured 89 GB/s per SM,
 // for 576 cycles of MMAs).
@@ -33,7 +35,23 @@ struct SplitSide {
 
 constexpr int kSplitPackBlocks = 1024;  // most CTAs of the packing pass, each with its word in `bad`
 
+// A word: what a CTA has seen of the first operand, and three bits higher of the second.  Below 2^-114 lo may be lost, an error
+// of 2^-126 at most, which is nothing beside an operand with any value from 2^-96 on.
+enum { kSplitRefused = 1, kSplitTiny = 2, kSplitOrdinary = 4 };
+__device__ __forceinline__ bool split_refused(int word) {
+  return (word & (kSplitRefused | kSplitRefused << 3)) || (word & (kSplitTiny | kSplitOrdinary)) == kSplitTiny ||
+         (word >> 3 & (kSplitTiny | kSplitOrdinary)) == kSplitTiny;
+}
+// The words of all threads of the CTA in *all (shared, zero before; a barrier must follow).
+__device__ __forceinline__ void split_gather(int* all, int word) {
+  word = __reduce_or_sync(0xffffffffu, word);
+  if ((threadIdx.x & 31) == 0 && word) atomicOr(all, word);
+}
+
 __global__ void __launch_bounds__(256) split_pack_kernel(const SplitSide a, const SplitSide b, int* __restrict__ bad) {
+  __shared__ int all;
+  if (threadIdx.x == 0) all = 0;
+  __syncthreads();
   mtb_launch_dependents();
   mtb_wait_prior();
   int found = 0;
@@ -55,20 +73,26 @@ __global__ void __launch_bounds__(256) split_pack_kernel(const SplitSide a, cons
       for (int j = 0; j < 4; ++j) v[j] = c + j < s.C ? src[(c + j) * s.s_c] : 0.f;
     }
     float hi[4], lo[4];
+    unsigned most = 0, least = ~0u;  // magnitudes as integers, which order like the numbers; least: of those that are not zero, less one
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      found |= !(fabsf(v[j]) <= 3.0e38f);
+      const unsigned u = __float_as_uint(v[j]) & 0x7fffffffu;
+      most = most > u ? most : u;
+      least = least < u - 1 ? least : u - 1;
       uint32_t r;
       asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v[j]));
       hi[j] = __uint_as_float(r);
       lo[j] = v[j] - hi[j];
     }
+    const int seen = (__uint_as_float(most) <= 3.0e38f ? 0 : kSplitRefused) | (least < (13u << 23) - 1 ? kSplitTiny : 0) | (most >= (31u << 23) ? kSplitOrdinary : 0);
+    found |= first ? seen : seen << 3;
     float* d = s.dst + ((long long)row * s.blocks + g / 8) * 64 + (g % 8) * 4;
     st4(d, make_float4(hi[0], hi[1], hi[2], hi[3]));
     st4(d + 32, make_float4(lo[0], lo[1], lo[2], lo[3]));
   }
-  found = __syncthreads_or(found);
-  if (threadIdx.x == 0) bad[blockIdx.x] = found;
+  split_gather(&all, found);
+  __syncthreads();
+  if (threadIdx.x == 0) bad[blockIdx.x] = all;
 }
 
 // ------------------------------------------------------------------------------ products
@@ -117,6 +141,7 @@ struct SplitShared {
   uint64_t full[4], empty[4], tfull[kSplitAcc], tempty[kSplitAcc];
   uint32_t tmem_slot;
   int abort_flag;
+  int words;  // of the packing pass
 };
 
 template <int BN>
@@ -131,6 +156,7 @@ __device__ __forceinline__ void split_setup(SplitShared& s, int warp) {
       mbar_init(smem_u32(&s.tempty[b]), kEpilogueWarps);
     }
     s.abort_flag = 0;
+    s.words = 0;
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -223,12 +249,15 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   split_setup<BN>(s, warp);
+  __syncthreads();
   mtb_wait_prior();
-  int bad = 0;
-  for (int i = threadIdx.x; i < p.n_bad; i += kGemmThreads) bad |= p.bad[i];
+  int word = 0;
+  for (int i = threadIdx.x; i < p.n_bad; i += kGemmThreads) word |= p.bad[i];
+  split_gather(&s.words, word);
   tc_fence_before();
-  bad = __syncthreads_or(bad);
+  __syncthreads();
   tc_fence_after();
+  const bool bad = split_refused(s.words);
   if (blockIdx.x == 0 && threadIdx.x == 0) *p.any_bad = bad;
   const uint32_t tmem_base = s.tmem_slot;
   const int tiles = bad ? 0 : p.m_tiles * p.n_tiles;
@@ -324,12 +353,15 @@ split_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   split_setup<BN>(s, warp);
+  __syncthreads();
   mtb_wait_prior();
-  int bad = 0;
-  for (int i = threadIdx.x; i < p.n_bad; i += kGemmThreads) bad |= p.bad[i];
+  int word = 0;
+  for (int i = threadIdx.x; i < p.n_bad; i += kGemmThreads) word |= p.bad[i];
+  split_gather(&s.words, word);
   tc_fence_before();
-  bad = __syncthreads_or(bad);
+  __syncthreads();
   tc_fence_after();
+  const bool bad = split_refused(s.words);
   if (blockIdx.x == 0 && threadIdx.x == 0) *p.any_bad = bad;
   const uint32_t tmem_base = s.tmem_slot;
   const int units = bad ? 0 : p.m_tiles * p.n_tiles * p.splits;

@@ -78,6 +78,31 @@ def test_values_that_cannot_be_split(value, monkeypatch):
     assert np.allclose(a[clean], o[clean], rtol=0, atol=1e-5 * 70 * 64 * 64 ** 0.5) and clean.any()
 
 
+@pytest.mark.parametrize("x_scale,w_scale", [(1e-37, 1.0), (1.0, 1e-37), (1e-35, 1e10), (0.0, 1.0)])
+def test_tiny_operands(x_scale, w_scale, monkeypatch):
+    """Where a whole operand is so small that its remainders are no normal numbers, the other kernels do the work."""
+    x, wt, dy = _operands(5, 48, 82, 19, 17, 3, 1, 1)
+    x, wt, dy = x * np.float32(x_scale), wt * np.float32(w_scale), dy * np.float32(x_scale)
+    b = np.zeros(82, np.float32)
+    monkeypatch.setenv("MTB_TC_SPLIT_ALWAYS", "1")
+    got = _run(x, wt, b, dy, 1, 1)[:2]  # weight gradients of such operands are zero, or do not see the filter
+    monkeypatch.delenv("MTB_TC_SPLIT_ALWAYS")
+    monkeypatch.setenv("MTB_DISABLE_TC", "1")
+    assert all(np.array_equal(a, o) for a, o in zip(got, _run(x, wt, b, dy, 1, 1)))
+
+
+def test_a_tiny_value_among_others_refuses_nothing(monkeypatch):
+    x, wt, dy = _operands(5, 48, 82, 19, 17, 3, 1, 1)
+    x[1, 2, 3, 4] = wt[5, 6, 1, 1] = 1e-39
+    b = np.zeros(82, np.float32)
+    monkeypatch.setenv("MTB_TC_SPLIT_ALWAYS", "1")
+    got = _run(x, wt, b, dy, 1, 1)
+    monkeypatch.delenv("MTB_TC_SPLIT_ALWAYS")
+    monkeypatch.setenv("MTB_DISABLE_TC", "1")
+    for a, o in zip(got, _run(x, wt, b, dy, 1, 1)):
+        assert not np.array_equal(a, o) and np.linalg.norm(a - o) <= 2e-6 * np.linalg.norm(o)
+
+
 def test_without_scratch_the_other_kernels_run():
     import gpu_util as g
     from mytorch_b200.backends.cuda.env import CudaEnv
