@@ -143,9 +143,6 @@ struct GemmParams {
   MtbBnEval bn;  // EPI_BN
   int relu;
   float* pre;  // dense K-major products only: laid out like `out`, takes the result before the ReLU (may be NULL)
-  // results (and the addend) move through shared memory by bulk copies (see the epilogue); rows lie one after the other
-  int bulk_out;
-  int stages;  // of the ring
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
   // MN-major operands through one copy per reduction block (encode_blocks_3d) instead of one per 32 columns
@@ -227,31 +224,42 @@ constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
 // images, with two stages for additions 19.24 ms, with three 19.36).  Statistics want the depth: 256-wide tiles with four stages
 // 19.23 ms, with three 19.33; the 7x7 stem's 64-wide ones 198 us and 204, and 212 with three and a second block per warp.
 constexpr uint32_t kOutBlock = 32 * 32 * 4;
-template <int BN, int EPI, bool SPLIT>
+template <int BN, int EPI, bool BULK>
 struct GemmSmem {
-  static constexpr bool kBulk = !SPLIT && BN >= 64 && EPI != EPI_BN;
-  static constexpr int kOutBlocks = !kBulk ? 0 : EPI == EPI_ADD ? 2 : 1;  // per warp
-  static constexpr int stages(bool bulk) {
-    return !bulk ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 128 ? 3 : 4) : (BN == 128 ? 2 : 3);
-  }
-  static constexpr uint32_t bytes(bool bulk) {  // + alignment slack, + rows that the MMA reads behind the last box of few rows
-    return stages(bulk) * Cfg<BN>::kStageBytes + (bulk ? kEpilogueWarps * kOutBlocks * kOutBlock : 0) + 1024 + (BN < 64 ? 128 * 128 : 0);
-  }
-  static constexpr uint32_t kMost = kBulk && bytes(true) > bytes(false) ? bytes(true) : bytes(false);
+  static constexpr int kOutBlocks = !BULK ? 0 : EPI == EPI_ADD ? 2 : 1;  // per warp
+  static constexpr int kStages = !BULK ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 128 ? 3 : 4) : (BN == 128 ? 2 : 3);
+  static constexpr uint32_t kBytes =  // + alignment slack, + rows that the MMA reads behind the last box of few rows
+      kStages * Cfg<BN>::kStageBytes + kEpilogueWarps * kOutBlocks * kOutBlock + 1024 + (BN < 64 ? 128 * 128 : 0);
 };
 
+// Tensor maps of what the epilogue moves by bulk copies: the result, and what is added to it.
+template <int N>
+struct BulkMaps {
+  CUtensorMap map[N];
+};
+template <>
+struct BulkMaps<0> {};
+template <int EPI, bool BULK>
+using BulkMapsOf = BulkMaps<!BULK ? 0 : EPI == EPI_ADD ? 2 : 1>;
+
 // SPLIT: GemmParams::splits > 1, a kernel of its own because the exchange takes the registers that the other epilogues need.
-template <int BN, int AMODE, int BMODE, int EPI, bool SPLIT>
+// BULK: results (and the addend) move through shared memory by bulk copies, for rows that lie one after the other.  Kernels of
+// their own, too: with the depth of the ring a parameter of the launch and two more maps in every launch, those that
+// move nothing in bulk took 0.3 to 0.45 us longer (256 -> 256 data gradient on 128 x 8x8 21.85 -> 22.20 us, 512 -> 512
+// on 4x4 22.82 -> 23.19, a weight product of 8192 x 2000 x 480 87.4 -> 88.7).
+template <int BN, int AMODE, int BMODE, int EPI, bool SPLIT, bool BULK>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapOut,
-               const __grid_constant__ CUtensorMap mapAdd, const GemmParams p) {
+tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p,
+               const __grid_constant__ BulkMapsOf<EPI, BULK> bulk) {
+  static_assert(!BULK || (!SPLIT && BN >= 64 && EPI != EPI_BN));
   using C = Cfg<BN>;
-  using Smem = GemmSmem<BN, EPI, SPLIT>;
-  const int STAGES = p.stages;
+  using Smem = GemmSmem<BN, EPI, BULK>;
+  constexpr int STAGES = Smem::kStages;
   constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN, ADD = EPI == EPI_ADD || BNORM;
   constexpr bool PRE = EPI == EPI_PLAIN && AMODE == A_KMAJOR && BMODE == B_KMAJOR;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2], bar_add[kEpilogueWarps][2];
+  __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
+  __shared__ uint64_t bar_add[BULK && EPI == EPI_ADD ? kEpilogueWarps : 1][2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
@@ -267,7 +275,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_tfull[b]), 1);
       mbar_init(smem_u32(&bar_tempty[b]), kEpilogueWarps);  // one arrival per epilogue warp
-      if constexpr (EPI == EPI_ADD)
+      if constexpr (BULK && EPI == EPI_ADD)
         for (int w = 0; w < kEpilogueWarps; ++w) mbar_init(smem_u32(&bar_add[w][b]), 1);
     }
     abort_flag = 0;
@@ -423,114 +431,110 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     WarpColStats<(STATS && !LANE_SUMS) ? COLS / 32 : 1> stats;
     LaneColSums<LANE_SUMS ? COLS / 32 : 1> sums;
     if constexpr (LANE_SUMS) sums.reset(); else stats.reset();
-    bool bulk = false;
-    if constexpr (Smem::kBulk) {
+    if constexpr (BULK) {
       // Results through shared memory and the copy engine.  A lane holds a row of the accumulator; stored from registers
       // every store instruction touches 32 lines (64 passes through the L1, which was 84 to 96 % busy and bounded every
       // convolution with a short reduction), as blocks of 32 x 32 in shared memory eight conflict-free stores and one copy do.
       // What is to be added arrives the same way, one block ahead.  Statistics read the block by columns: a lane has the 32
       // values of its column in registers, without a single exchange between lanes.
-      bulk = p.bulk_out != 0;
-      if (bulk) {
-        constexpr int OUT_BLOCKS = Smem::kOutBlocks;
-        const int ew = warp - 2;
-        const uint32_t blocks = smem_base + STAGES * C::kStageBytes + (uint32_t)(ew * OUT_BLOCKS) * kOutBlock;
-        const uint32_t row_base = (uint32_t)lane * 128u, swz = (uint32_t)(lane & 7);
-        // blocks of this warp in order: (tile, 32 columns); those outside the matrix are skipped
-        auto next_block = [&](int& unit, int& c0) {
-          do {
-            c0 += 32;
-            if (c0 >= COLS) { c0 = 0; unit += gridDim.x; }
-          } while (unit < tiles && ((unit / p.n_tiles) * 128 + quarter * 32 >= p.M || (unit % p.n_tiles) * BN + c_first + c0 >= p.N));
-        };
-        int load_unit = blockIdx.x, load_c0 = -32, loaded = 0;  // the addend's blocks, asked for one ahead
-        auto load_addend = [&]() {  // lane 0
-          next_block(load_unit, load_c0);
-          if (load_unit >= tiles) return;
-          const uint32_t bar = smem_u32(&bar_add[ew][loaded & 1]);
-          mbar_expect_tx(bar, kOutBlock);
-          tma_load_2d(blocks + (uint32_t)(loaded & 1) * kOutBlock, &mapAdd, bar, (load_unit % p.n_tiles) * BN + c_first + load_c0,
-                      (load_unit / p.n_tiles) * 128 + quarter * 32);
-          ++loaded;
-        };
-        if constexpr (EPI == EPI_ADD) {
-          if (lane == 0) load_addend();
-        }
-        int g = 0;  // blocks handled
-        for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
-          const int row0 = (unit / p.n_tiles) * 128 + quarter * 32, n0 = (unit % p.n_tiles) * BN + c_first;
-          const int buf = t & 1;
-          bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_ptr, 4);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-          const int rows = p.M - row0 < 32 ? p.M - row0 : 32;
+      constexpr int OUT_BLOCKS = Smem::kOutBlocks;
+      const int ew = warp - 2;
+      const uint32_t blocks = smem_base + STAGES * C::kStageBytes + (uint32_t)(ew * OUT_BLOCKS) * kOutBlock;
+      const uint32_t row_base = (uint32_t)lane * 128u, swz = (uint32_t)(lane & 7);
+      // blocks of this warp in order: (tile, 32 columns); those outside the matrix are skipped
+      auto next_block = [&](int& unit, int& c0) {
+        do {
+          c0 += 32;
+          if (c0 >= COLS) { c0 = 0; unit += gridDim.x; }
+        } while (unit < tiles && ((unit / p.n_tiles) * 128 + quarter * 32 >= p.M || (unit % p.n_tiles) * BN + c_first + c0 >= p.N));
+      };
+      int load_unit = blockIdx.x, load_c0 = -32, loaded = 0;  // the addend's blocks, asked for one ahead
+      auto load_addend = [&]() {  // lane 0
+        next_block(load_unit, load_c0);
+        if (load_unit >= tiles) return;
+        const uint32_t bar = smem_u32(&bar_add[ew][loaded & 1]);
+        mbar_expect_tx(bar, kOutBlock);
+        tma_load_2d(blocks + (uint32_t)(loaded & 1) * kOutBlock, &bulk.map[EPI == EPI_ADD ? 1 : 0], bar, (load_unit % p.n_tiles) * BN + c_first + load_c0,
+                    (load_unit / p.n_tiles) * 128 + quarter * 32);
+        ++loaded;
+      };
+      if constexpr (EPI == EPI_ADD) {
+        if (lane == 0) load_addend();
+      }
+      int g = 0;  // blocks handled
+      for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
+        const int row0 = (unit / p.n_tiles) * 128 + quarter * 32, n0 = (unit % p.n_tiles) * BN + c_first;
+        const int buf = t & 1;
+        bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_ptr, 4);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const int rows = p.M - row0 < 32 ? p.M - row0 : 32;
 #pragma unroll
-          for (int c0 = 0; c0 < COLS; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
-            const int col0 = n0 + c0;
-            const bool inside = rows > 0 && col0 < p.N;  // warp-uniform
-            const uint32_t block = blocks + (uint32_t)(OUT_BLOCKS == 2 ? (g & 1) : 0) * kOutBlock;
-            float4 add[8];
-            if constexpr (EPI == EPI_ADD) {
-              if (inside) {
-                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_add[ew][g & 1]), (uint32_t)(g >> 1) & 1u, abort_ptr, 5));
-                if (!ok) break;
+        for (int c0 = 0; c0 < COLS; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_first + c0), r);
+          const int col0 = n0 + c0;
+          const bool inside = rows > 0 && col0 < p.N;  // warp-uniform
+          const uint32_t block = blocks + (uint32_t)(OUT_BLOCKS == 2 ? (g & 1) : 0) * kOutBlock;
+          float4 add[8];
+          if constexpr (EPI == EPI_ADD) {
+            if (inside) {
+              ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_add[ew][g & 1]), (uint32_t)(g >> 1) & 1u, abort_ptr, 5));
+              if (!ok) break;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) add[j] = ld_shared4(block + row_base + (((uint32_t)j ^ swz) << 4));
-                if (lane == 0) {
-                  bulk_wait_read<0>();  // the block before has been read, its place is free
-                  load_addend();
-                }
-              }
-            } else {
-              if (inside) {
-                if (lane == 0) bulk_wait_read<0>();  // the block before has been read
-                __syncwarp();
+              for (int j = 0; j < 8; ++j) add[j] = ld_shared4(block + row_base + (((uint32_t)j ^ swz) << 4));
+              if (lane == 0) {
+                bulk_wait_read<0>();  // the block before has been read, its place is free
+                load_addend();
               }
             }
-            tmem_ld_wait();
-            if (c0 + 32 >= COLS) {  // the accumulator is in registers
-              tc_fence_before();
+          } else {
+            if (inside) {
+              if (lane == 0) bulk_wait_read<0>();  // the block before has been read
               __syncwarp();
-              if (lane == 0) mbar_arrive(smem_u32(&bar_tempty[buf]));
-            }
-            if (!inside) continue;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-              if (p.bias && col0 + 4 * j < p.N) {  // N % 4 == 0 on this path
-                const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + 4 * j);
-                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-              }
-              if constexpr (EPI == EPI_ADD) { v.x += add[j].x; v.y += add[j].y; v.z += add[j].z; v.w += add[j].w; }
-              if (p.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
-              st_shared4(block + row_base + (((uint32_t)j ^ swz) << 4), v);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&mapOut, block, col0, row0);
-              bulk_commit();
-            }
-            ++g;
-            if constexpr (STATS) {
-              float o[32];
-              const uint32_t column = block + (uint32_t)(lane & 3) * 4u;
-#pragma unroll
-              for (int k = 0; k < 32; ++k) o[k] = ld_shared1(column + (uint32_t)k * 128u + (((uint32_t)(lane >> 2) ^ (uint32_t)(k & 7)) << 4));
-              stats.add_column(c0 / 32, o, rows);
             }
           }
-          if (!ok) break;
-          if constexpr (STATS) { if (rows > 0) stats.n += (float)rows; }
+          tmem_ld_wait();
+          if (c0 + 32 >= COLS) {  // the accumulator is in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bar_tempty[buf]));
+          }
+          if (!inside) continue;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+            if (p.bias && col0 + 4 * j < p.N) {  // N % 4 == 0 on this path
+              const float4 b = *reinterpret_cast<const float4*>(p.bias + col0 + 4 * j);
+              v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+            }
+            if constexpr (EPI == EPI_ADD) { v.x += add[j].x; v.y += add[j].y; v.z += add[j].z; v.w += add[j].w; }
+            if (p.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
+            st_shared4(block + row_base + (((uint32_t)j ^ swz) << 4), v);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&bulk.map[0], block, col0, row0);
+            bulk_commit();
+          }
+          ++g;
+          if constexpr (STATS) {
+            float o[32];
+            const uint32_t column = block + (uint32_t)(lane & 3) * 4u;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) o[k] = ld_shared1(column + (uint32_t)k * 128u + (((uint32_t)(lane >> 2) ^ (uint32_t)(k & 7)) << 4));
+            stats.add_column(c0 / 32, o, rows);
+          }
         }
-        if (lane == 0) bulk_wait_all();
+        if (!ok) break;
+        if constexpr (STATS) { if (rows > 0) stats.n += (float)rows; }
       }
+      if (lane == 0) bulk_wait_all();
     }
-    if constexpr (!STATS || SPLIT) {  // statistics of unsplit reductions come through shared memory only
-    for (int unit = blockIdx.x; !bulk && unit < tiles; unit += gridDim.x, ++t) {
+    if constexpr (!BULK) {
+    for (int unit = blockIdx.x; unit < tiles; unit += gridDim.x, ++t) {
       const int tile = unit / S;
       const int m0 = (tile / p.n_tiles) * C::kRowsA, n0 = (tile % p.n_tiles) * BN;
       const int col_end = BN >= 32 || n0 + BN > p.N ? p.N : n0 + BN;
@@ -755,19 +759,30 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+template <int BN, int AMODE, int BMODE, int EPI, bool BULK>
+int launch_tc_whole(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, const BulkMapsOf<EPI, BULK>& bulk, cudaStream_t st) {
+  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, false, BULK>;
+  constexpr uint32_t smem = GemmSmem<BN, EPI, BULK>::kBytes;
+  static unsigned long long configured = 0;
+  if (int rc = mtb_opt_in_smem((const void*)kernel, (int)smem, &configured)) return rc;
+  const int tiles = p.m_tiles * p.n_tiles;
+  int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
+  if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
+  MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), smem, st, mapA, mapB, p, bulk);
+  MTB_LAUNCH_CHECK("tc_gemm_kernel");
+  return MTB_OK;
+}
+
 template <int BN, int AMODE, int BMODE, int EPI = EPI_PLAIN>
-int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& params, cudaStream_t st) {
-  GemmParams p = params;
-  int tiles = p.m_tiles * p.n_tiles;
+int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
   if (p.splits > 1) {  // one unit per CTA, the units of a tile a cluster
     if constexpr (AMODE == A_IM2COL) {
-      auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, true>;
-      constexpr uint32_t smem = GemmSmem<BN, EPI, true>::bytes(false);
-      p.stages = GemmSmem<BN, EPI, true>::stages(false);
+      auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, true, false>;
+      constexpr uint32_t smem = GemmSmem<BN, EPI, false>::kBytes;
       static unsigned long long configured = 0;
       if (int rc = mtb_opt_in_smem((const void*)kernel, (int)smem, &configured)) return rc;
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(tiles * p.splits);
+      cfg.gridDim = dim3(p.m_tiles * p.n_tiles * p.splits);
       cfg.blockDim = dim3(kGemmThreads);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = st;
@@ -779,36 +794,27 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 2;
-      MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, mapA, mapA, p));
+      MTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapA, mapB, p, BulkMaps<0>{}));
       MTB_LAUNCH_CHECK("tc_gemm_kernel");
       return MTB_OK;
     }
     return mtb_fail(MTB_ERR_INVALID, "tc_gemm: only convolutions split the reduction");
   }
-  auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, false>;
-  using Smem = GemmSmem<BN, EPI, false>;
-  CUtensorMap mapOut = mapA, mapAdd = mapA;  // unused ones are never read
-  if constexpr (Smem::kBulk) {
+  if constexpr (BN >= 64 && EPI != EPI_BN) {
     // Whole rows one after the other, their pitch and start on 16 bytes: what the copy engine asks for.  Everything else (a
     // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 8
     // reduction blocks and more: their stores hide behind the main loop, which wants the stages (8192 x 2000, K = 64:
     // 18.8 -> 15.5 us, K = 480: 33.9 from registers, 37.2 through shared memory).
-    p.bulk_out = (EPI != EPI_PLAIN || p.num_kb < 8) && !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
-    if (EPI == EPI_STATS && !p.bulk_out) return mtb_fail(MTB_ERR_INVALID, "tc_gemm: statistics need whole aligned rows");
-    if (p.bulk_out) {
-      if (int rc = tc::encode_result_2d(&mapOut, p.out, p.M, p.N, p.ldo)) return rc;
-      if (EPI == EPI_ADD)
-        if (int rc = tc::encode_result_2d(&mapAdd, p.addend, p.M, p.N, p.ldo)) return rc;
+    if ((EPI != EPI_PLAIN || p.num_kb < 8) && !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend)) {
+      BulkMapsOf<EPI, true> bulk;
+      if (int rc = tc::encode_result_2d(&bulk.map[0], p.out, p.M, p.N, p.ldo)) return rc;
+      if constexpr (EPI == EPI_ADD)
+        if (int rc = tc::encode_result_2d(&bulk.map[1], p.addend, p.M, p.N, p.ldo)) return rc;
+      return launch_tc_whole<BN, AMODE, BMODE, EPI, true>(mapA, mapB, p, bulk, st);
     }
   }
-  p.stages = Smem::stages(p.bulk_out);
-  static unsigned long long configured = 0;
-  if (int rc = mtb_opt_in_smem((const void*)kernel, (int)Smem::kMost, &configured)) return rc;
-  int grid = tiles < mtb_sm_count() ? tiles : mtb_sm_count();
-  if (EPI == EPI_STATS || EPI == EPI_BN) grid = grid / p.n_tiles * p.n_tiles;  // every CTA stays on one column tile (see GemmParams::stats)
-  MTB_LAUNCH(kernel, dim3(grid), dim3(kGemmThreads), Smem::bytes(p.bulk_out), st, mapA, mapB, mapOut, mapAdd, p);
-  MTB_LAUNCH_CHECK("tc_gemm_kernel");
-  return MTB_OK;
+  if constexpr (EPI == EPI_STATS) return mtb_fail(MTB_ERR_INVALID, "tc_gemm: statistics need whole aligned rows");
+  else return launch_tc_whole<BN, AMODE, BMODE, EPI, false>(mapA, mapB, p, {}, st);
 }
 
 // Partial-statistics rows the STATS variant writes for a problem of `tiles` tiles in `n_tiles` column tiles.
@@ -871,11 +877,11 @@ int cluster_units(int size) {
   static int units[9] = {};
   if (!units[size]) {
     const int sms = mtb_sm_count();
-    auto kernel = tc_gemm_kernel<256, A_IM2COL, B_KMAJOR, EPI_PLAIN, true>;
+    auto kernel = tc_gemm_kernel<256, A_IM2COL, B_KMAJOR, EPI_PLAIN, true, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms / size * size);
     cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = GemmSmem<256, EPI_PLAIN, true>::bytes(false);
+    cfg.dynamicSmemBytes = GemmSmem<256, EPI_PLAIN, false>::kBytes;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)size;
@@ -883,7 +889,7 @@ int cluster_units(int size) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmem<256, EPI_PLAIN, true>::bytes(false)) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmem<256, EPI_PLAIN, false>::kBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
       (void)cudaGetLastError();  // no GPU (plans are also made without one)
       clusters = sms * 7 / 8 / size;
