@@ -759,6 +759,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// From how many reduction blocks on results are stored from registers.  Times through shared memory over times from registers,
+// means over 1279 products of 1,000 to 200,000 rows and 32 to 9,216 columns (tiles of 64 / 128 / 256 columns):
+//   with addition, one wave of tiles    4 blocks 1.02 / 0.83 / 0.72   8: 1.04 / 0.85 / 0.78   16: 1.00 / 0.87 / 0.88   32: 1.00 / 0.92 / 1.06
+//   with addition, more                 4 blocks 0.82 / 0.65 / 0.67   8: 1.00 / 0.78 / 0.77   16: 1.08 / 0.96 / 1.06   32: 1.17 / 1.11 / 1.42
+//   plain, one wave                     2 blocks 1.00 / 0.98 / 0.9    4: 1.01 / 0.98 / 0.88    7: 1.03 / 0.99 / 0.88
+//   plain, more                         2 blocks 0.95 / 0.86 / 0.79   4: 0.97 / 0.88 / 0.83    7: 1.06 / 1.07 / 0.90
+// 512 <- 1024 channels with addition on 32 x 28x28: 54.8 us from registers, 78.2 through shared memory with two stages.  Rows that
+// are no whole sectors of 32 bytes are stored 16 bytes at a time from registers (1000 x 500, 4 blocks: 5.8 us, 4.8).
+int bulk_limit(int bn, bool adds, bool one_wave, bool whole_sectors) {
+  if (bn == 64) return !whole_sectors ? 8 : one_wave ? 0 : adds ? 8 : 5;
+  if (adds) return !one_wave ? 16 : bn == 128 ? 40 : 32;
+  return bn == 128 && whole_sectors ? 6 : 8;
+}
+
 template <int BN, int AMODE, int BMODE, int EPI, bool BULK>
 int launch_tc_whole(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, const BulkMapsOf<EPI, BULK>& bulk, cudaStream_t st) {
   auto kernel = tc_gemm_kernel<BN, AMODE, BMODE, EPI, false, BULK>;
@@ -802,10 +816,11 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
   }
   if constexpr (BN >= 64 && EPI != EPI_BN) {
     // Whole rows one after the other, their pitch and start on 16 bytes: what the copy engine asks for.  Everything else (a
-    // residue class of a strided data gradient, odd widths) is stored from registers, and so are plain results of 8
-    // reduction blocks and more: their stores hide behind the main loop, which wants the stages (8192 x 2000, K = 64:
-    // 18.8 -> 15.5 us, K = 480: 33.9 from registers, 37.2 through shared memory).
-    if ((EPI != EPI_PLAIN || p.num_kb < 8) && !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend)) {
+    // residue class of a strided data gradient, odd widths) is stored from registers, and so are the results of long reductions,
+    // whose stores hide behind the main loop, which wants the stages.
+    const bool whole_sectors = p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0;
+    const bool fits = !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
+    if (fits && (EPI == EPI_STATS || p.num_kb < bulk_limit(BN, EPI == EPI_ADD, p.m_tiles * p.n_tiles <= mtb_sm_count(), whole_sectors))) {
       BulkMapsOf<EPI, true> bulk;
       if (int rc = tc::encode_result_2d(&bulk.map[0], p.out, p.M, p.N, p.ldo)) return rc;
       if constexpr (EPI == EPI_ADD)

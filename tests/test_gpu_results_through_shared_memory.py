@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,cin,cout,h,w", [
-    (1, 32, 64, 32, 33), (3, 64, 96, 19, 23), (1, 32, 36, 45, 31), (2, 256, 260, 17, 9), (5, 96, 320, 41, 37), (9, 64, 132, 64, 61), (40, 64, 256, 33, 31)])
+    (1, 32, 64, 32, 33), (3, 64, 96, 19, 23), (1, 32, 36, 45, 31), (2, 256, 260, 17, 9), (5, 96, 320, 41, 37), (9, 64, 132, 64, 61), (40, 64, 256, 33, 31),
+    # either side of where results are stored from registers: few and many reduction blocks, a wave of tiles and more
+    (40, 96, 64, 33, 31), (40, 64, 512, 33, 31), (20, 256, 480, 31, 33), (20, 256, 512, 31, 33), (2, 512, 992, 17, 15), (2, 512, 1024, 17, 15)])
 def test_pointwise_convolution(n, cin, cout, h, w):
     import gpu_util as g
 
