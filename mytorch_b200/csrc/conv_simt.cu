@@ -64,7 +64,7 @@ int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh
   MTB_REQUIRE(x && wt && y, "conv2d_forward: null pointer");
   const int K = kh * kw * cin, M = n * d.OH * d.OW;
   Out o{};
-  o.out = y; o.ld = cout; o.bias = bias; o.relu = relu; o.guard = guard; o.guards = guards;
+  o.out = y; o.ld = cout; o.bias = bias; o.relu = relu;
   const Choice c = choose(M, cout, K, 1, 1);
   if (bn_eval) {
     if (tile_info(c.tile).cluster) {  // small tiles: BatchNorm in the store
@@ -75,10 +75,11 @@ int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh
       return rc2 ? rc2 : mtb_bn_eval_apply(y, y, M, cout, *bn_eval, residual, relu, (cudaStream_t)stream);
     }
   }
+  const Extra extra{guard, guards, nullptr};
   const DenseK filter{wt, K};
   if (cin % 4 == 0 && mtb_aligned16(x) && mtb_aligned16(wt))
-    return launch<PatchK, 4, DenseK, 4>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt");
-  return launch<PatchK, 1, DenseK, 1>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt");
+    return launch<PatchK, 4, DenseK, 4>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt", extra);
+  return launch<PatchK, 1, DenseK, 1>(c, patch_k(x, d), filter, o, NoTable{}, 1, M, cout, K, (cudaStream_t)stream, "conv2d_forward_simt", extra);
 }
 
 MTB_API int mtb_conv2d_forward_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
@@ -98,7 +99,8 @@ int mtb_conv2d_dgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, 
   if (rc) return rc;
   MTB_REQUIRE(dy && wt && dx, "conv2d_dgrad: null pointer");
   Out o{};
-  o.out = dx; o.ld = cin; o.H = h; o.W = w; o.SH = sh; o.SW = sw; o.guard = guard; o.guards = guards;
+  o.out = dx; o.ld = cin; o.H = h; o.W = w; o.SH = sh; o.SW = sw;
+  const Extra extra{guard, guards, nullptr};
   const DgradK a{dy, d, FastDiv(cout), nullptr};
   const DgradR b{wt, d, FastDiv(cout), nullptr};
   const bool va = cout % 4 == 0 && mtb_aligned16(dy), vb = cin % 4 == 0 && mtb_aligned16(wt);
@@ -121,10 +123,10 @@ int mtb_conv2d_dgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, 
     if (rows == 0) continue;
     const Choice c = choose(rows, cin, K, classes, 1);
     cudaStream_t st = (cudaStream_t)stream;
-    if (va && vb) rc = launch<DgradK, 4, DgradR, 4>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt");
-    else if (va) rc = launch<DgradK, 4, DgradR, 1>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt");
-    else if (vb) rc = launch<DgradK, 1, DgradR, 4>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt");
-    else rc = launch<DgradK, 1, DgradR, 1>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt");
+    if (va && vb) rc = launch<DgradK, 4, DgradR, 4>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt", extra);
+    else if (va) rc = launch<DgradK, 4, DgradR, 1>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt", extra);
+    else if (vb) rc = launch<DgradK, 1, DgradR, 4>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt", extra);
+    else rc = launch<DgradK, 1, DgradR, 1>(c, a, b, o, table, classes, rows, cin, K, st, "conv2d_dgrad_simt", extra);
     if (rc) return rc;
   }
   return MTB_OK;
@@ -170,7 +172,8 @@ int mtb_conv2d_wgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, 
   const long long total = (long long)cout * K;
   cudaStream_t st = (cudaStream_t)stream;
   Out o{};
-  o.out = dw; o.ld = K; o.guard = guard; o.guards = guards;
+  o.out = dw; o.ld = K;
+  const Extra extra{guard, guards, nullptr};
   if (c.slices > 1 && !guard) {
     MTB_REQUIRE(workspace && workspace_bytes >= c.slices * total * 4, "conv2d_wgrad: workspace too small");
     o.out = (float*)workspace;
@@ -178,10 +181,10 @@ int mtb_conv2d_wgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, 
   }
   const DenseR a{dy, cout};
   const bool va = cout % 4 == 0 && mtb_aligned16(dy), vb = cin % 4 == 0 && mtb_aligned16(x);
-  if (va && vb) rc = launch<DenseR, 4, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
-  else if (va) rc = launch<DenseR, 4, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
-  else if (vb) rc = launch<DenseR, 1, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
-  else rc = launch<DenseR, 1, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt");
+  if (va && vb) rc = launch<DenseR, 4, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt", extra);
+  else if (va) rc = launch<DenseR, 4, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt", extra);
+  else if (vb) rc = launch<DenseR, 1, PatchR, 4>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt", extra);
+  else rc = launch<DenseR, 1, PatchR, 1>(c, a, patch_r(x, d), o, NoTable{}, 1, cout, K, pixels, st, "conv2d_wgrad_simt", extra);
   if (rc || c.slices == 1 || guard) return rc;
   MTB_LAUNCH(add_planes_kernel, mtb_stream_grid(total, 256), 256, 0, st, (const float*)workspace, dw, total, c.slices);
   MTB_LAUNCH_CHECK("add_planes_kernel");

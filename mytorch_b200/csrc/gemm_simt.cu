@@ -7,12 +7,12 @@ namespace {
 using namespace simt;
 
 template <int VEC>
-int dense(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const Out& o, cudaStream_t st) {
+int dense(int m, int n, int k, const float* a, int trans_a, const float* b, int trans_b, const Out& o, float* pre, cudaStream_t st) {
   const Choice c = choose(m, n, k, 1, 1);
   const NoTable none;
   const DenseK ak{a, k}, bk{b, k};
   const DenseR ar{a, m}, br{b, n};
-  if (!trans_a && trans_b) return launch<DenseK, VEC, DenseK, VEC>(c, ak, bk, o, none, 1, m, n, k, st, "gemm_simt");
+  if (!trans_a && trans_b) return launch<DenseK, VEC, DenseK, VEC>(c, ak, bk, o, none, 1, m, n, k, st, "gemm_simt", Extra{nullptr, 0, pre});
   if (!trans_a) return launch<DenseK, VEC, DenseR, VEC>(c, ak, br, o, none, 1, m, n, k, st, "gemm_simt");
   if (trans_b) return launch<DenseR, VEC, DenseK, VEC>(c, ar, bk, o, none, 1, m, n, k, st, "gemm_simt");
   return launch<DenseR, VEC, DenseR, VEC>(c, ar, br, o, none, 1, m, n, k, st, "gemm_simt");
@@ -79,9 +79,9 @@ int mtb_gemm_simt(int m, int n, int k, const float* a, int trans_a, const float*
     return MTB_OK;
   }
   Out o{};
-  o.out = c; o.ld = n; o.bias = bias; o.relu = relu; o.pre = pre;
+  o.out = c; o.ld = n; o.bias = bias; o.relu = relu;
   // four neighbours of each operand in one load: along k for [rows][K] operands, along the row for [K][rows] ones
   const bool vec = mtb_aligned16(a) && mtb_aligned16(b) && (trans_a ? m : k) % 4 == 0 && (trans_b ? k : n) % 4 == 0;
-  return vec ? dense<4>(m, n, k, a, trans_a, b, trans_b, o, (cudaStream_t)stream)
-             : dense<1>(m, n, k, a, trans_a, b, trans_b, o, (cudaStream_t)stream);
+  return vec ? dense<4>(m, n, k, a, trans_a, b, trans_b, o, pre, (cudaStream_t)stream)
+             : dense<1>(m, n, k, a, trans_a, b, trans_b, o, pre, (cudaStream_t)stream);
 }

@@ -307,13 +307,22 @@ struct Out {
   MtbBnEval bn;              // mean != NULL: BatchNorm with running statistics after the bias (cluster kernels only)
   const float* residual;     // laid out like out: added before the ReLU (cluster kernels only)
   int relu;
-  float* pre;                // laid out like out, takes the value before the ReLU (dense products of two operands along k only)
   long long split_plane;     // > 0: every slice of the reduction writes its own plane of partials
   const DgradClass* cls;     // data gradient: row -> pixel of the residue class
   int H, W, SH, SW;
-  const int* guard;          // not NULL: nothing is done unless one of these words is set
-  int guards;
 };
+
+// What few launches need beside the product, in instantiations of their own and as their last parameter: as members of Out, tested
+// in every kernel, the two took small convolutions and products 2 to 10 % (128 -> 32 channels 3x3 on one 7x7 image 8.75 -> 9.6 us).
+enum { EXTRA_NONE, EXTRA_GUARD, EXTRA_PRE };
+struct Extra {
+  const int* guard;  // convolutions only; not NULL: nothing is done unless one of these words is set
+  int guards;
+  float* pre;        // dense products of two operands along k only; not NULL: laid out like out, takes the value before the ReLU
+};
+struct NoExtra {};
+template <int EXTRA>
+using ExtraOf = std::conditional_t<EXTRA == EXTRA_NONE, NoExtra, Extra>;
 
 __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
   long long r = i;
@@ -326,8 +335,8 @@ __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
 }
 
 // TAIL: with BatchNorm and the residual of Out (the cluster kernels, whose store is one loop)
-template <bool TAIL, bool PRE>
-__device__ __forceinline__ void store4(const Out& o, float* row, int j, int N, bool vec, float4 v) {
+template <bool TAIL, int EXTRA>
+__device__ __forceinline__ void store4(const Out& o, const ExtraOf<EXTRA>& extra, float* row, int j, int N, bool vec, float4 v) {
   float t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -340,8 +349,8 @@ __device__ __forceinline__ void store4(const Out& o, float* row, int j, int N, b
       }
       if (o.residual && j + q < N) t[q] += o.residual[row - o.out + j + q];
     }
-    if constexpr (PRE) {
-      if (o.pre && j + q < N) o.pre[row - o.out + j + q] = t[q];
+    if constexpr (EXTRA == EXTRA_PRE) {
+      if (j + q < N) extra.pre[row - o.out + j + q] = t[q];
     }
     if (o.relu) t[q] = fmaxf(t[q], 0.f);
   }
@@ -385,18 +394,18 @@ using TableOf = std::conditional_t<std::is_same_v<SA, DgradK>, ClassTable, NoTab
 
 // blockIdx.z = class * slices + slice.  CLUSTER: the slices of a tile form a cluster and add up at the end;
 // otherwise slices > 1 only with planes of partials (Out::split_plane).
-template <class T, class SA, int VA, class SB, int VB, bool CLUSTER>
+template <class T, class SA, int VA, class SB, int VB, bool CLUSTER, int EXTRA>
 __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB sb, Out o, const __grid_constant__ TableOf<SA> table, int M, int N, int K,
-                                                          int slices, int k_per_slice) {
+                                                          int slices, int k_per_slice, const ExtraOf<EXTRA> extra) {
   constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, THREADS = T::THREADS;
   constexpr int GM = TM / 4, GN = TN / 4;  // a thread's rows and columns come in groups of four, spread over the tile
   __shared__ float As[2][BK][BM + 4];
   __shared__ float Bs[2][BK][BN + 4];
   mtb_launch_dependents();
   mtb_wait_prior();
-  if (o.guard) {
+  if constexpr (EXTRA == EXTRA_GUARD) {
     int any = 0;
-    for (int i = 0; i < o.guards; ++i) any |= o.guard[i];
+    for (int i = 0; i < extra.guards; ++i) any |= extra.guard[i];
     if (!any) return;
   }
   const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
@@ -482,7 +491,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
         const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], q));
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
       }
-      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>, std::is_same_v<SA, DenseK> && std::is_same_v<SB, DenseK>>(o, out_row(o, m0 + r, z), n0 + c, N, vec, s);
+      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>, EXTRA>(o, extra, out_row(o, m0 + r, z), n0 + c, N, vec, s);
     }
     cluster.sync();  // nobody leaves while its tile is being read
   } else {
@@ -493,7 +502,7 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
       float* row = out_row(o, i, z) + slice * o.split_plane;
 #pragma unroll
       for (int g = 0; g < GN; ++g)
-        store4<false, std::is_same_v<SA, DenseK> && std::is_same_v<SB, DenseK>>(o, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
+        store4<false, EXTRA>(o, extra, row, n0 + g * (BN / GN) + tx * 4, N, vec, four(p, g));
     }
   }
 }
@@ -546,12 +555,14 @@ using TileM = Tile<128, 64, 8, 8, 3>;
 using TileS = Tile<64, 64, 8, 4, 4>;
 using TileXS = Tile<64, 32, 4, 4, 6>;
 
-template <class T, class SA, int VA, class SB, int VB, bool CLUSTER>
+template <int EXTRA, class T, class SA, int VA, class SB, int VB, bool CLUSTER>
 int launch_tile(const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, int slices, cudaStream_t st,
-                const char* name) {
+                const char* name, const Extra& extra) {
   int per = (K + slices - 1) / slices;
   per = (per + BK - 1) / BK * BK;
   if (per < BK) per = BK;
+  ExtraOf<EXTRA> with{};
+  if constexpr (EXTRA != EXTRA_NONE) with = extra;
   dim3 grid(mtb_div_up(M, T::BM), mtb_div_up(N, T::BN), classes * slices);
   MTB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "%s: grid too large", name);
   if constexpr (CLUSTER) {
@@ -568,29 +579,41 @@ int launch_tile(const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& tab
     attr[0].val.clusterDim.z = (unsigned)slices;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    MTB_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, SA, VA, SB, VB, true>, sa, sb, o, table, M, N, K, slices, per));
+    MTB_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, SA, VA, SB, VB, true, EXTRA>, sa, sb, o, table, M, N, K, slices, per, with));
   } else {
-    MTB_LAUNCH(gemm_kernel<T, SA, VA, SB, VB, false>, grid, T::THREADS, 0, st, sa, sb, o, table, M, N, K, slices, per);
+    MTB_LAUNCH(gemm_kernel<T, SA, VA, SB, VB, false, EXTRA>, grid, T::THREADS, 0, st, sa, sb, o, table, M, N, K, slices, per, with);
   }
   MTB_LAUNCH_CHECK(name);
   return MTB_OK;
 }
 
-template <class SA, int VA, class SB, int VB>
-int launch(const Choice& c, const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, cudaStream_t st,
-           const char* name) {
+template <int EXTRA, class SA, int VA, class SB, int VB>
+int launch_extra(const Choice& c, const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, cudaStream_t st,
+                 const char* name, const Extra& extra) {
   const bool cluster = (c.slices > 1 && o.split_plane == 0) || o.bn.mean;
   switch (c.tile) {
-    case XL: return launch_tile<TileXL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
-    case L: return launch_tile<TileL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
-    case MD: return launch_tile<TileM, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
+    case XL: return launch_tile<EXTRA, TileXL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
+    case L: return launch_tile<EXTRA, TileL, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
+    case MD: return launch_tile<EXTRA, TileM, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
     case SM:
-      if (cluster) return launch_tile<TileS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
-      return launch_tile<TileS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
+      if (cluster) return launch_tile<EXTRA, TileS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
+      return launch_tile<EXTRA, TileS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
     default:
-      if (cluster) return launch_tile<TileXS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
-      return launch_tile<TileXS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name);
+      if (cluster) return launch_tile<EXTRA, TileXS, SA, VA, SB, VB, true>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
+      return launch_tile<EXTRA, TileXS, SA, VA, SB, VB, false>(sa, sb, o, table, classes, M, N, K, c.slices, st, name, extra);
   }
+}
+
+template <class SA, int VA, class SB, int VB>
+int launch(const Choice& c, const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, cudaStream_t st,
+           const char* name, const Extra& extra = {}) {
+  constexpr bool dense = (std::is_same_v<SA, DenseK> || std::is_same_v<SA, DenseR>) && (std::is_same_v<SB, DenseK> || std::is_same_v<SB, DenseR>);
+  if constexpr (!dense) {
+    if (extra.guard) return launch_extra<EXTRA_GUARD, SA, VA, SB, VB>(c, sa, sb, o, table, classes, M, N, K, st, name, extra);
+  } else if constexpr (std::is_same_v<SA, DenseK> && std::is_same_v<SB, DenseK>) {
+    if (extra.pre) return launch_extra<EXTRA_PRE, SA, VA, SB, VB>(c, sa, sb, o, table, classes, M, N, K, st, name, extra);
+  }
+  return launch_extra<EXTRA_NONE, SA, VA, SB, VB>(c, sa, sb, o, table, classes, M, N, K, st, name, extra);
 }
 
 }  // namespace simt
