@@ -223,16 +223,16 @@ __global__ void __launch_bounds__(256) resize_channels_kernel(const float* __res
 struct PatchRuns {
   int N, C, H, W, KH, KW, SH, SW, PH, PW, OH, OW;
 };
-// ROW: the window is a single filter row (KH = 1), whose entries are neighbours in memory: one address and a range say all, and a
-// thread has four pixels' loads in flight before it writes the first (7x7 over 3 channels of 128 x 224x224: 155 -> 98 us, of
-// which the 411 MB written take 63).  The others did not gain from loads ahead (3x3 over 3 channels of 512 x 32x32: 32 us, 34).
-template <bool ROW>
+// ROW: the window is a single filter row (KH = 1), whose entries are neighbours in memory: one address and a range say all.
+// AHEAD: pixels of a thread whose loads are in flight before it writes the first, four where it has as many (7x7 over 3
+// channels of 128 x 224x224: 155 -> 98 us, of which the 411 MB written take 63; one image, a pixel a thread: 3.7 us, 4.6 with
+// three that are not there).  Whole windows did not gain from loads ahead (3x3 over 3 channels of 512 x 32x32: 32 us, 34).
+template <bool ROW, int AHEAD>
 __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restrict__ x, float4* __restrict__ out, PatchRuns d, unsigned pixels) {
   mtb_launch_dependents();
   mtb_wait_prior();
   // A thread always writes the same four entries of a pixel, so where they lie in the filter is worked out once; a CTA walks
   // 32 neighbouring pixels at a time.
-  constexpr int AHEAD = ROW ? 4 : 1;
   const int run = d.KW * d.C, used = d.KH * run;
   const unsigned part = threadIdx.x & 7u;
   int dh[4], dw[4], dc[4];
@@ -291,8 +291,10 @@ MTB_API int mtb_pack_patches_f32(int n, int c, int h, int w, int kh, int kw, int
   const long long pixels = (long long)n * d.OH * d.OW;
   MTB_REQUIRE(pixels < (1LL << 31), "pack_patches: too many pixels");
   const int grid = mtb_stream_grid(pixels, 32);
-  if (kh == 1 && (long long)w * c + 64 < (1LL << 31)) MTB_LAUNCH(pack_patches_kernel<true>, grid, 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
-  else MTB_LAUNCH(pack_patches_kernel<false>, grid, 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
+  const bool row = kh == 1 && (long long)w * c + 64 < (1LL << 31);
+  if (row && pixels >= 4LL * 32 * grid) MTB_LAUNCH(pack_patches_kernel<true, 4>, grid, 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
+  else if (row) MTB_LAUNCH(pack_patches_kernel<true, 1>, grid, 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
+  else MTB_LAUNCH(pack_patches_kernel<false, 1>, grid, 256, 0, (cudaStream_t)stream, x, (float4*)out, d, (unsigned)pixels);
   MTB_LAUNCH_CHECK("pack_patches_kernel");
   return MTB_OK;
 }

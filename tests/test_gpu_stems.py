@@ -36,6 +36,23 @@ def test_few_input_channels(n, cin, cout, h, w, kh, kw, stride, pad):
     assert rel_err(g.host(g.op("conv2d")(xt, wtt, bt, stride, pad)), O.conv2d_forward(x2, wt, b, stride, pad)) < TF32_TOL
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 5, 9), (2, 33, 40), (7, 224, 224)])  # a pixel a thread, and several
+def test_packed_filter_rows(n, h, w):
+    import gpu_util as g
+    from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory
+
+    env = CudaEnv.instance()
+    x = np.random.default_rng(w).standard_normal((n, 3, h, w)).astype(np.float32)
+    ow = (w + 6 - 7) // 2 + 1
+    out = CudaMemory(0, n * h * ow * 32 * 4)
+    env.lib.pack_patches_f32(n, 3, h, w, 1, 7, 1, 2, 0, 3, g.dev(x), out.ptr, env.stream())
+    padded = np.pad(x.transpose(0, 2, 3, 1), ((0, 0), (0, 0), (3, 3), (0, 0)))
+    want = np.zeros((n, h, ow, 32), np.float32)
+    for dw in range(7):
+        want[..., 3 * dw:3 * dw + 3] = padded[:, :, dw:dw + 2 * ow - 1:2]
+    assert np.array_equal(out.read(want.shape, np.float32), want)
+
+
 @pytest.mark.parametrize("n,cin,cout,hw", [(3, 256, 64, 28), (2, 64, 32, 33), (5, 68, 64, 17), (2, 132, 96, 29)])
 def test_pointwise_data_gradient_adds_in_its_epilogue(n, cin, cout, hw):
     import gpu_util as g
