@@ -122,21 +122,24 @@ __global__ void __launch_bounds__(256) nhwc_spatial_sum_kernel(const float* __re
 }
 
 // A thread keeps its V channels of one image and writes them to the pixels of its share: no index arithmetic and no load per
-// element (one division of a 64-bit index per float before: 128 x 2048 x 7x7 42 -> 14 us).
-template <int V>
-__global__ void __launch_bounds__(256) nhwc_spatial_bcast_kernel(const float* __restrict__ dy, float* __restrict__ dx, long long groups, int C, int HW, int per, float scale) {
+// element (one division of a 64-bit index per float before: 128 x 2048 x 7x7 42 -> 14 us).  FEW channels: a CTA has
+// one image and its threads `rows` neighbouring pixels at a time, which lie one after the other in memory.
+template <int V, bool FEW>
+__global__ void __launch_bounds__(256) nhwc_spatial_bcast_kernel(const float* __restrict__ dy, float* __restrict__ dx, long long groups, int C, int HW, int per, int rows,
+                                                                 float scale) {
   mtb_launch_dependents();
   mtb_wait_prior();
-  const long long g = blockIdx.x * 256LL + threadIdx.x;  // (image, group of V channels)
-  if (g >= groups) return;
-  const long long n = g / (C / V);
-  const int c = (int)(g - n * (C / V)) * V;
+  const int G = C / V, r = FEW ? (int)threadIdx.x / G : 0;
+  const long long g = FEW ? (long long)blockIdx.x * G + (int)threadIdx.x % G : blockIdx.x * 256LL + threadIdx.x;  // (image, group of V channels)
+  if (g >= groups || (FEW && r >= rows)) return;
+  const long long n = g / G;
+  const int c = (int)(g - n * G) * V;
   VecF<V> v = vload<V>(dy + g * V);
 #pragma unroll
   for (int j = 0; j < V; ++j) v.v[j] *= scale;
   const int p0 = blockIdx.y * per, p1 = p0 + per < HW ? p0 + per : HW;
   float* out = dx + n * HW * C + c;
-  for (int p = p0; p < p1; ++p) vstore<V>(out + (long long)p * C, v);
+  for (int p = p0 + r; p < p1; p += FEW ? rows : 1) vstore<V>(out + (long long)p * C, v);
 }
 
 struct RedDims {
@@ -214,15 +217,22 @@ MTB_API int mtb_nhwc_spatial_sum_f32(const float* x, float* y, int n, int c, int
 MTB_API int mtb_nhwc_spatial_bcast_f32(const float* dy, float* dx, int n, int c, int hw, float scale, void* stream) {
   MTB_REQUIRE(dy && dx && n > 0 && c > 0 && hw > 0, "nhwc_spatial_bcast: bad arguments");
   const bool four = c % 4 == 0 && mtb_aligned16(dy) && mtb_aligned16(dx);
-  const long long groups = (long long)n * c / (four ? 4 : 1), blocks = (groups + 255) / 256;
-  // enough CTAs to fill the GPU a few times over, at least four pixels each
+  const int G = four ? c / 4 : c;
+  const long long groups = (long long)n * G;
+  // few channels of large images: CTAs of one image each (see the kernel); four pixels a thread at least
+  const int rows = G < 64 && hw / (256 / G) >= 4 ? 256 / G : 1;
+  const long long blocks = rows > 1 ? n : (groups + 255) / 256;
+  // enough CTAs to fill the GPU a few times over, at least four pixels a thread
   long long shares = (8LL * mtb_sm_count() + blocks - 1) / blocks;
-  if (shares > (hw + 3) / 4) shares = (hw + 3) / 4;
+  const long long most = (hw + 4LL * rows - 1) / (4LL * rows);
+  if (shares > most) shares = most;
   if (shares > 65535) shares = 65535;
   const int per = (int)((hw + shares - 1) / shares);
   const dim3 grid((unsigned)blocks, (unsigned)((hw + per - 1) / per));
-  if (four) MTB_LAUNCH(nhwc_spatial_bcast_kernel<4>, grid, 256, 0, (cudaStream_t)stream, dy, dx, groups, c, hw, per, scale);
-  else MTB_LAUNCH(nhwc_spatial_bcast_kernel<1>, grid, 256, 0, (cudaStream_t)stream, dy, dx, groups, c, hw, per, scale);
+#define MTB_BCAST(V_, FEW_) MTB_LAUNCH(nhwc_spatial_bcast_kernel<V_, FEW_>, grid, 256, 0, (cudaStream_t)stream, dy, dx, groups, c, hw, per, rows, scale)
+  if (rows > 1) { if (four) MTB_BCAST(4, true); else MTB_BCAST(1, true); }
+  else { if (four) MTB_BCAST(4, false); else MTB_BCAST(1, false); }
+#undef MTB_BCAST
   MTB_LAUNCH_CHECK("nhwc_spatial_bcast_kernel");
   return MTB_OK;
 }

@@ -26,7 +26,8 @@ def test_max_pool_3x3_stride_2(n, c, h, w, pad):
     assert np.array_equal(g.host(dx), want[:, :, pad:pad + h, pad:pad + w])  # at most four terms, added in the order of the windows
 
 
-@pytest.mark.parametrize("n,c,hw,offset", [(1, 1, 1, 0), (3, 5, 7, 0), (2, 8, 49, 0), (128, 512, 16, 0), (5, 260, 1000, 0), (2, 8, 49, 1), (300, 4, 3, 0)])
+@pytest.mark.parametrize("n,c,hw,offset", [(1, 1, 1, 0), (3, 5, 7, 0), (2, 8, 49, 0), (128, 512, 16, 0), (5, 260, 1000, 0), (2, 8, 49, 1), (300, 4, 3, 0),
+                                           (2, 3, 1000, 0), (1, 4, 5000, 0), (3, 63, 17, 0), (2, 8, 2049, 1), (2, 1, 200000, 0)])
 def test_spatial_broadcast(n, c, hw, offset):
     import gpu_util as g
     from mytorch_b200.backends.cuda.env import CudaEnv, CudaMemory
