@@ -1019,14 +1019,24 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   CUtensorMap mapA, mapB;
   int bn = cheapest_bn(n, m, (k + 31) / 32, !trans_b), rows = 128;
   if (!trans_a && trans_b) {  // see Cfg
-    auto narrow_ns = [&](int r, int c, double block) {
+    auto narrow_ns = [&](int r, int c, double block, double fixed) {
       const long long tiles = (long long)((m + r - 1) / r) * ((n + c - 1) / c);
-      return (tiles + mtb_sm_count() - 1) / mtb_sm_count() * (((k + 31) / 32) * block + 900.0);
+      return (tiles + mtb_sm_count() - 1) / mtb_sm_count() * (((k + 31) / 32) * block + fixed);
     };
     double best = im2col_ns(bn, n, m, (k + 31) / 32, false);
-    if (m <= 64 && narrow_ns(64, 32, 146) <= 900 + ((k + 31) / 32) * 146.0) { bn = 32; rows = 64; best = narrow_ns(64, 32, 146); }
-    else if (narrow_ns(64, 32, 146) < 0.9 * best) { bn = 32; rows = 64; best = narrow_ns(64, 32, 146); }
-    if (narrow_ns(32, 16, 92) < 0.9 * best) { bn = 16; rows = 32; }
+    const double wide_32 = narrow_ns(64, 32, 146, 900);  // as calibrated against the tiles of 128 rows
+    if ((m <= 64 && wide_32 <= 900 + ((k + 31) / 32) * 146.0) || wide_32 < 0.9 * best) {
+      // against 32 x 16: the time of a block is what both take from K = 1024 on; rows that are no whole sectors of 32 bytes cost
+      // the 32 columns of this tile 600 ns more
+      bn = 32; rows = 64;
+      best = narrow_ns(64, 32, 125, n % 8 ? 1500 : 900);
+    } else {
+      best *= 0.9;
+    }
+    // Eight blocks a stage fill late: 500 ns more than 64 x 32 before the first MMA, 20 ns a block less from there on.  64 x 128 in one
+    // wave, 64 x 32 and 32 x 16: K = 288 4.3 and 5.0 us, 768 6.2 and 6.5, 1024 7.6 and 7.4, 4096 19.5 and 17.4.  Over 1053 products of
+    // 32 to 2000 rows, 10 to 2048 columns and K = 32 to 9216 the tile taken is 0.3 % off the fastest of the three, 10 % at most.
+    if (narrow_ns(32, 16, 104, 1400) < best) { bn = 16; rows = 32; }
   }
   int rc;
   GemmParams p{};

@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m,n,k,bias", [(64, 128, 9216, True), (33, 40, 2052, True), (32, 16, 4096, False), (100, 70, 3000, True), (300, 128, 1184, True),
-                                        (65, 8, 900, False), (97, 17, 132, True)])
+                                        (65, 8, 900, False), (97, 17, 132, True),
+                                        (64, 128, 288, True), (64, 96, 1024, False), (40, 10, 92, True)])
 def test_linear(m, n, k, bias):
     import gpu_util as g
 
