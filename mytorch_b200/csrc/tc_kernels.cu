@@ -228,8 +228,9 @@ template <int BN, int EPI, bool BULK>
 struct GemmSmem {
   static constexpr int kOutBlocks = !BULK ? 0 : EPI == EPI_ADD ? 2 : 1;  // per warp
   static constexpr int kStages = !BULK ? Cfg<BN>::kStages : EPI == EPI_ADD ? 2 : EPI == EPI_STATS ? (BN == 128 ? 3 : 4) : (BN == 128 ? 2 : 3);
-  static constexpr uint32_t kBytes =  // + alignment slack, + rows that the MMA reads behind the last box of few rows
-      kStages * Cfg<BN>::kStageBytes + kEpilogueWarps * kOutBlocks * kOutBlock + 1024 + (BN < 64 ? 128 * 128 : 0);
+  static constexpr uint32_t kBytes = kStages * Cfg<BN>::kStageBytes + kEpilogueWarps * kOutBlocks * kOutBlock + 1024;  // + alignment slack
+  static_assert(kBytes <= 227 * 1024);
+  static_assert((Cfg<BN>::kKB - 1) * Cfg<BN>::kABytes + 128 * 128 <= Cfg<BN>::kStageBytes);  // the MMA reads 128 rows of A, behind the last box of few rows blocks of B
 };
 
 // Tensor maps of what the epilogue moves by bulk copies: the result, and what is added to it.
