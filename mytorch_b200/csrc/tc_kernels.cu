@@ -1113,10 +1113,9 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   p.splits = gp.splits; p.kb_per_split = gp.kb_per_split;
   // A short reduction (1x1) leaves the epilogue no main loop to hide the statistics behind, and takes less with them than
   // with BatchNorm's own pass all the same (both operators: 64 -> 128 channels, stride 2, to 16x16, 16 images 15.5 -> 12.3 us,
-  // 192 images 30.0 -> 27.0, 512 images 57.0 -> 55.1; 64 -> 256 channels on 32 x 56x56 83.4 -> 78.0; ResNet-50 step
-  // 19.80 -> 19.23 ms).  Outputs of 12 to 16 MB keep BatchNorm's pass: it reads them from L2, and a test holds the operator to it.
-  const long long out_bytes = (long long)M * cout * 4;
-  if (want_stats && (p.num_kb >= 16 || out_bytes <= (12ll << 20) || out_bytes > (16ll << 20) || bn == 64)) {
+  // 128 images 22.9 -> 20.1, 192 images 30.0 -> 27.0, 512 images 57.0 -> 55.1; 256 -> 512 on 8 x 28x28 26.2 -> 19.0;
+  // 64 -> 256 channels on 32 x 56x56 83.4 -> 78.0; ResNet-50 step 19.80 -> 19.23 ms).
+  if (want_stats) {
     p.stats = stats;
     *stats_rows = gp.splits > 1 ? p.m_tiles * 4 : stats_rows_for(p.m_tiles * p.n_tiles, p.n_tiles);
     cudaStream_t st = (cudaStream_t)stream;

@@ -450,8 +450,9 @@ def test_bounded_wait_runs_out_reports_once_and_leaves_the_context_usable(g):
     (8, 64, 32, 32, 128, 3, 2, 1, None),     # im2col kernel, stride 2
     (32, 512, 4, 4, 512, 3, 1, 1, None),     # im2col kernel, several column tiles per row tile
     (8, 3, 32, 32, 64, 3, 1, 1, None),       # image stem (channels padded to one block)
-    (8, 64, 32, 32, 128, 1, 2, 0, None),     # 1x1 shortcut, small output: statistics although the reduction is short
-    (128, 64, 32, 32, 128, 1, 2, 0, None),   # 1x1 shortcut, 17 MB of output: too short a reduction, no statistics expected
+    (8, 64, 32, 32, 128, 1, 2, 0, None),     # 1x1 shortcut, small output
+    (128, 64, 32, 32, 128, 1, 2, 0, None),   # 1x1 shortcut, 17 MB of output
+    (192, 64, 32, 32, 128, 1, 2, 0, None),   # 1x1 shortcut, 25 MB of output
 ])
 def test_conv_epilogue_hands_batch_norm_its_statistics(g, cfg, monkeypatch):
     """A convolution asked for BatchNorm statistics leaves partial (count, mean, M2) rows on its output;
@@ -471,9 +472,7 @@ def test_conv_epilogue_hands_batch_norm_its_statistics(g, cfg, monkeypatch):
     fused = g.op("conv2d")(xt, wtt, bt, (s, s), (p, p), bn_stats=True)
     yh = g.host(fused)
     assert np.array_equal(yh, g.host(plain))
-    oh, ow = O.conv_out_hw(h, w, k, k, s, p)
-    expect_stats = k > 1 or n * oh * ow * co * 4 <= (12 << 20)
-    assert (getattr(fused, "_bn_partials", None) is not None) == expect_stats
+    assert getattr(fused, "_bn_partials", None) is not None
     outs = []
     for src in (fused, plain):
         rm, rv = g.dev(np.zeros(co, np.float32)), g.dev(np.ones(co, np.float32))
