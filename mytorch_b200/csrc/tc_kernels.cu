@@ -142,7 +142,6 @@ struct GemmParams {
   const float* addend;
   MtbBnEval bn;  // EPI_BN
   int relu;
-  float* pre;  // dense K-major products only: laid out like `out`, takes the result before the ReLU (may be NULL)
   // geometry of the im2col'ed tensor (A operand of a convolution)
   int OW, OH, SW, SH, PW, PH, KW, KH, cchunks;
   // MN-major operands through one copy per reduction block (encode_blocks_3d) instead of one per 32 columns
@@ -162,6 +161,7 @@ struct GemmParams {
   // units of a tile form a cluster.  When its accumulators are complete every unit hands each of the others the columns
   // that one finishes (distributed shared memory), and adds what it received to its own in split order.
   int splits, kb_per_split;
+  float* pre;  // EPI_PRE: laid out like `out`, takes the result before the ReLU
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -211,9 +211,9 @@ struct Cfg {
   static constexpr uint32_t kTmemCols = 2 * kAccCols;
 };
 
-// What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, add a tensor, or BatchNorm
-// with running statistics (then optionally add a tensor).
-enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3 };
+// What the epilogue does beside bias / ReLU / store: nothing, BatchNorm statistics of the output, add a tensor, BatchNorm
+// with running statistics (then optionally add a tensor), or store the result before the ReLU too (dense products).
+enum { EPI_PLAIN = 0, EPI_STATS = 1, EPI_ADD = 2, EPI_BN = 3, EPI_PRE = 4 };
 
 constexpr int kEpilogueWarps = 8, kGemmThreads = 64 + 32 * kEpilogueWarps;
 
@@ -252,12 +252,12 @@ template <int BN, int AMODE, int BMODE, int EPI, bool SPLIT, bool BULK>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const GemmParams p,
                const __grid_constant__ BulkMapsOf<EPI, BULK> bulk) {
-  static_assert(!BULK || (!SPLIT && BN >= 64 && EPI != EPI_BN));
+  static_assert(!BULK || (!SPLIT && BN >= 64 && EPI != EPI_BN && EPI != EPI_PRE));
   using C = Cfg<BN>;
   using Smem = GemmSmem<BN, EPI, BULK>;
   constexpr int STAGES = Smem::kStages;
   constexpr bool STATS = EPI == EPI_STATS, BNORM = EPI == EPI_BN, ADD = EPI == EPI_ADD || BNORM;
-  constexpr bool PRE = EPI == EPI_PLAIN && AMODE == A_KMAJOR && BMODE == B_KMAJOR;
+  constexpr bool PRE = EPI == EPI_PRE;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[8], bar_empty[8], bar_tfull[2], bar_tempty[2];
   __shared__ uint64_t bar_add[BULK && EPI == EPI_ADD ? kEpilogueWarps : 1][2];
@@ -425,8 +425,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int c_first = !SPLIT ? (warp < 6 ? 0 : COLS) : rank * width + (width >= 64 && warp >= 6 ? width / 2 : 0);
     const int split_chunks = width >= 64 ? width / 64 : (warp < 6 ? 1 : 0);
     int t = 0;
-    const bool vec_ok = (p.ldo % 4 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.pre)) & 15u) == 0);
-    const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pre)) & 31u) == 0);  // 32-byte stores
+    const uintptr_t results = reinterpret_cast<uintptr_t>(p.out) | (PRE ? reinterpret_cast<uintptr_t>(p.pre) : 0);
+    const bool vec_ok = (p.ldo % 4 == 0) && (((results | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0);
+    const bool wide_ok = vec_ok && (p.ldo % 8 == 0) && ((results & 31u) == 0);  // 32-byte stores
     // statistics of a split reduction: narrow tiles keep per-lane sums, wide tiles merge per tile
     constexpr bool LANE_SUMS = STATS && SPLIT && BN == 64;
     WarpColStats<(STATS && !LANE_SUMS) ? COLS / 32 : 1> stats;
@@ -627,7 +628,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                   }
                 }
                 if constexpr (PRE) {
-                  if (p.pre) st_row8(p.pre + orow_index * p.ldo + col0 + j, v[0], v[1], wide_ok);
+                  st_row8(p.pre + orow_index * p.ldo + col0 + j, v[0], v[1], wide_ok);
                   if (p.relu) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) { v[h].x = fmaxf(v[h].x, 0.f); v[h].y = fmaxf(v[h].y, 0.f); v[h].z = fmaxf(v[h].z, 0.f); v[h].w = fmaxf(v[h].w, 0.f); }
@@ -643,7 +644,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                   if (p.bias) v += p.bias[col0 + j];
                   if constexpr (BNORM) v = (v - bn_columns.mean[c_first + c0 + j]) * bn_columns.scale[c_first + c0 + j] + bn_columns.beta[c_first + c0 + j];
                   if (ADD && arow) v += arow[col0 + j];
-                  if constexpr (PRE) { if (p.pre) p.pre[orow_index * p.ldo + col0 + j] = v; }
+                  if constexpr (PRE) p.pre[orow_index * p.ldo + col0 + j] = v;
                   if (p.relu) v = fmaxf(v, 0.f);
                   orow[col0 + j] = v;
                 }
@@ -815,12 +816,12 @@ int launch_tc(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams
     }
     return mtb_fail(MTB_ERR_INVALID, "tc_gemm: only convolutions split the reduction");
   }
-  if constexpr (BN >= 64 && EPI != EPI_BN) {
+  if constexpr (BN >= 64 && EPI != EPI_BN && EPI != EPI_PRE) {
     // Whole rows one after the other, their pitch and start on 16 bytes: what the copy engine asks for.  Everything else (a
     // residue class of a strided data gradient, odd widths) is stored from registers, and so are the results of long reductions,
     // whose stores hide behind the main loop, which wants the stages.
     const bool whole_sectors = p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0;
-    const bool fits = !p.pre && !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
+    const bool fits = !p.o_strided && p.ldo % 4 == 0 && p.N % 4 == 0 && al16(p.out) && al16(p.bias) && al16(p.addend);
     if (fits && (EPI == EPI_STATS || p.num_kb < bulk_limit(BN, EPI == EPI_ADD, p.m_tiles * p.n_tiles <= mtb_sm_count(), whole_sectors))) {
       BulkMapsOf<EPI, true> bulk;
       if (int rc = tc::encode_result_2d(&bulk.map[0], p.out, p.M, p.N, p.ldo)) return rc;
@@ -841,7 +842,7 @@ int stats_rows_for(int tiles, int n_tiles) {
 
 template <int AMODE, int BMODE, int EPI = EPI_PLAIN>
 int launch_tc_bn(int bn, const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmParams& p, cudaStream_t st) {
-  if constexpr (AMODE == A_KMAJOR && BMODE == B_KMAJOR && EPI == EPI_PLAIN) {
+  if constexpr (AMODE == A_KMAJOR && BMODE == B_KMAJOR && (EPI == EPI_PLAIN || EPI == EPI_PRE)) {
     if (bn == 16) return launch_tc<16, AMODE, BMODE, EPI>(mapA, mapB, p, st);
     if (bn == 32) return launch_tc<32, AMODE, BMODE, EPI>(mapA, mapB, p, st);
   }
@@ -1057,6 +1058,7 @@ int mtb_tc_gemm_f32(int m, int n, int k, const float* a, int trans_a, const floa
   p.out = c; p.ldo = n; p.bias = bias; p.relu = relu; p.pre = pre;
   p.KH = 1; p.KW = 1; p.cchunks = p.num_kb;
   cudaStream_t st = (cudaStream_t)stream;
+  if (!trans_a && trans_b && pre) return launch_tc_bn<A_KMAJOR, B_KMAJOR, EPI_PRE>(bn, mapA, mapB, p, st);
   if (!trans_a && trans_b) return launch_tc_bn<A_KMAJOR, B_KMAJOR>(bn, mapA, mapB, p, st);
   if (!trans_a && !trans_b) return launch_tc_bn<A_KMAJOR, B_MNMAJOR>(bn, mapA, mapB, p, st);
   if (trans_a && trans_b) return launch_tc_bn<A_MNMAJOR, B_KMAJOR>(bn, mapA, mapB, p, st);
