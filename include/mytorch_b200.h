@@ -87,8 +87,11 @@ int mtb_graph_destroy(void* graph_exec);
  *      mytorch/backends/cuda/ops/conv.py:9-90) ---- */
 long long mtb_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
 /* y[N,OH,OW,Cout] = conv(x[N,H,W,Cin], wt[Cout,KH,KW,Cin]) + bias (bias may be NULL); relu != 0 clamps at 0.
- * workspace: may be NULL (only the weight gradient needs mtb_conv2d_workspace_bytes()); with that many bytes, channel counts
- * that fit no block of 32 run on the tensor cores too, in FP32 accuracy.  A layer with too few output
+ * workspace (this and the two data gradients): may be NULL.  With mtb_conv2d_workspace_bytes() of it, channel counts that fit no
+ * block of 32 run on the tensor cores, operands as sums of two TF32 numbers (23 of their 24 bits; a sum of 96 terms and more rounds
+ * less than FP32 FMAs do); without, on the CUDA cores in FP32.  More scratch than that changes nothing.  Such a call
+ * leaves its operands in the scratch from one launch to the next, as the weight gradient leaves its partial sums: a block belongs
+ * to one stream.  A layer with too few output
  * tiles to fill the GPU splits its reduction over a cluster of CTAs, which add in a fixed order: results are reproducible.
  * A filter larger than the padded input is refused by every entry point. */
 int mtb_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
@@ -129,7 +132,7 @@ int mtb_conv2d_dgrad_accumulates_in_place(int n, int cin, int h, int w, int kh, 
  * would take for this shape and how the row-staged kernels lay out shared and tensor memory.
  * out: 25 ints, see the definition in csrc/tc_kernels.cu.  No counterpart in the reference. */
 int mtb_conv2d_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out);
-/* dw[Cout,KH,KW,Cin]; split-K partials go to workspace and are summed in a fixed order */
+/* dw[Cout,KH,KW,Cin]; needs mtb_conv2d_workspace_bytes() of workspace: split-K partials go there and are summed in a fixed order */
 int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                          const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream);
 

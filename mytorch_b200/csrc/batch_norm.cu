@@ -438,6 +438,7 @@ int launch_normalize(const float* x, float* y, long long rows, int c, bool align
 int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps, int training, double momentum,
                float* running_mean, float* running_var, float* y, float* mean, float* var, int mode, const float* res, unsigned char* mask,
                const float* stats, int stats_rows, void* workspace, long long workspace_bytes, cudaStream_t st) {
+  const MtbScratchTurn turn;
   MTB_REQUIRE(n > 0 && c > 0 && h > 0 && w > 0 && x && y && mean && var && workspace, "batch_norm2d_forward: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_batch_norm2d_workspace_bytes(n, c, h, w), "batch_norm2d_forward: workspace too small");
   MTB_REQUIRE(training || (running_mean && running_var), "batch_norm2d_forward: inference needs running statistics");
@@ -473,6 +474,7 @@ int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, c
 int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, const float* var, const float* x, const float* gamma,
                 const float* beta, double eps, int mode, const float* res, const unsigned char* mask, float* dx, float* dres, float* dgamma, float* dbeta, void* workspace,
                 long long workspace_bytes, cudaStream_t st) {
+  const MtbScratchTurn turn;
   MTB_REQUIRE(n > 0 && c > 0 && h > 0 && w > 0 && dy && mean && var && x && dx && workspace, "batch_norm2d_backward: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_batch_norm2d_workspace_bytes(n, c, h, w), "batch_norm2d_backward: workspace too small");
   MTB_REQUIRE(mode != 2 || ((res || mask) && dres), "batch_norm2d_add_relu_backward: the added tensor (or forward's mask) and its gradient buffer are required");

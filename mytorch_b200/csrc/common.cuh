@@ -36,6 +36,17 @@ constexpr int kMaxLanes = 4;
 int mtb_fork_lanes(cudaStream_t main, int lanes, cudaStream_t* out);
 int mtb_join_lanes(cudaStream_t main, int lanes);
 
+// Held by every entry point that leaves something in the caller's scratch in one launch and reads it in a later one: two host
+// threads that share a device, its stream and its scratch (as two threads of the Python layer do) would otherwise mix their launches,
+// and one would read what the other has written in between.  One lock for all devices: asking for the current one costs more than it.
+class MtbScratchTurn {
+ public:
+  MtbScratchTurn();
+  ~MtbScratchTurn();
+  MtbScratchTurn(const MtbScratchTurn&) = delete;
+  MtbScratchTurn& operator=(const MtbScratchTurn&) = delete;
+};
+
 #define MTB_REQUIRE(cond, ...) \
   do { if (!(cond)) return mtb_fail(MTB_ERR_INVALID, __VA_ARGS__); } while (0)
 

@@ -46,9 +46,11 @@ int forward_fp32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, i
                  float* y, int relu, void* workspace, long long workspace_bytes, void* stream) {
   const int* guard = nullptr;
   int guards = 0;
-  if (x && wt && y && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0, workspace, workspace_bytes))
-    if (int rc = mtb_split_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, (cudaStream_t)stream, &guard, &guards))
-      return rc;
+  if (!(x && wt && y && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0, workspace, workspace_bytes)))
+    return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream, nullptr, 0);
+  const MtbScratchTurn turn;
+  if (int rc = mtb_split_conv2d_forward_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, workspace, (cudaStream_t)stream, &guard, &guards))
+    return rc;
   return mtb_conv2d_forward_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, wt, bias, y, relu, nullptr, nullptr, stream, guard, guards);
 }
 
@@ -56,8 +58,10 @@ int dgrad_fp32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int
                void* workspace, long long workspace_bytes, void* stream) {
   const int* guard = nullptr;
   int guards = 0;
-  if (dy && wt && dx && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 1, workspace, workspace_bytes))
-    if (int rc = mtb_split_conv2d_dgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, workspace, (cudaStream_t)stream, &guard, &guards)) return rc;
+  if (!(dy && wt && dx && split_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 1, workspace, workspace_bytes)))
+    return mtb_conv2d_dgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream, nullptr, 0);
+  const MtbScratchTurn turn;
+  if (int rc = mtb_split_conv2d_dgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, workspace, (cudaStream_t)stream, &guard, &guards)) return rc;
   return mtb_conv2d_dgrad_simt(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, dy, wt, dx, stream, guard, guards);
 }
 
@@ -149,6 +153,7 @@ MTB_API int mtb_conv2d_dgrad_accumulates_in_place(int n, int cin, int h, int w, 
 
 MTB_API int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                  const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
+  const MtbScratchTurn turn;
   if (mtb_tc_conv2d_wgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw))
     return mtb_tc_conv2d_wgrad_f32(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, x, dy, dw, workspace, workspace_bytes, stream);
   const int* guard = nullptr;

@@ -63,6 +63,7 @@ MTB_API long long mtb_cross_entropy_workspace_bytes(int batch) { return (long lo
 // loss[0] = mean_b(-log softmax(logits[b])[target[b]]); logits row-major [B, C], target int64.
 MTB_API int mtb_cross_entropy_forward_f32(int batch, int classes, const float* logits, const long long* target, float* loss, void* workspace,
                                           long long workspace_bytes, void* stream) {
+  const MtbScratchTurn turn;
   MTB_REQUIRE(batch > 0 && classes > 0 && logits && target && loss && workspace, "cross_entropy_forward: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_cross_entropy_workspace_bytes(batch), "cross_entropy_forward: workspace too small");
   cudaStream_t st = (cudaStream_t)stream;

@@ -185,6 +185,7 @@ MTB_API long long mtb_colsum_workspace_bytes(int c) { return (long long)mtb_col_
 // N,H,W of a channels-last activation).
 MTB_API int mtb_colsum_f32(const float* a, long long rows, int c, float scale, float* out, void* workspace, long long workspace_bytes,
                            void* stream) {
+  const MtbScratchTurn turn;
   MTB_REQUIRE(a && out && workspace && rows > 0 && c > 0, "colsum: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_colsum_workspace_bytes(c), "colsum: workspace too small");
   cudaStream_t st = (cudaStream_t)stream;

@@ -2,6 +2,7 @@
 #include "common.cuh"
 #include <cstdarg>
 #include <cstring>
+#include <mutex>
 
 static thread_local char g_last_error[512] = "";
 
@@ -24,6 +25,10 @@ int mtb_sm_count() {
   }
   return cached[dev];
 }
+
+static std::mutex g_scratch_turn;
+MtbScratchTurn::MtbScratchTurn() { g_scratch_turn.lock(); }
+MtbScratchTurn::~MtbScratchTurn() { g_scratch_turn.unlock(); }
 
 int mtb_opt_in_smem(const void* kernel, int bytes, unsigned long long* done_mask) {
   int dev = 0;
