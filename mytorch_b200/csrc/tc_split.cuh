@@ -122,6 +122,7 @@ struct SplitCfg {
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kTurn + 1024;
   static constexpr uint32_t kTmemCols = BN == 32 ? 128 : BN == 64 ? 256 : 512;
   static constexpr int kCols = BN / 2;  // columns of an epilogue warp
+  static_assert(kSmemBytes <= 227 * 1024 && kStages <= 4 && kSplitAcc * BN <= (int)kTmemCols && kTmemCols <= 512);
 };
 
 __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float* r) {

@@ -45,6 +45,7 @@ def test_against_64_bits_and_the_other_kernels(n, cin, cout, h, w, k, stride, pa
         # an operand is off by 2^-22 at most, the term left out is 2^-22, a chain truncates 12 times, chains are added in FP32
         assert (np.abs(a - want) <= (18 + count / 32) * 2.0 ** -23 * size).all()
         err = lambda t: np.linalg.norm(t - want) / np.linalg.norm(want)
+        assert not np.array_equal(a, o)  # it was these kernels that ran
         assert err(a) <= max(err(o), 2.0e-7)  # 2e-7: what sums of some hundred terms, which these kernels are taken for, have in FP32
 
 
@@ -57,6 +58,7 @@ def test_several_groups_of_images(monkeypatch):
     monkeypatch.setenv("MTB_DISABLE_TC", "1")
     want, size = _run(x, wt, b, dy, 1, 1), _run(*(np.abs(t) for t in (x, wt, b, dy)), 1, 1)
     for a, o, m, count in zip(got, want, size, (33 * 9, 40 * 9, 70 * 64 * 64)):
+        assert not np.array_equal(a, o)
         terms = 18 + count / 32 + count  # both sides' rounding
         assert (np.abs(a - o) <= terms * 2.0 ** -23 * m).all()
 
@@ -114,3 +116,75 @@ def test_without_scratch_the_other_kernels_run():
     env.lib.conv2d_forward_f32(*args, xt, wtt, None, y, 0, None, 0, env.stream())
     want = g.host(g.op("conv2d")(xt, wtt, None, (1, 1), (1, 1)))
     assert np.abs(g.host(y) - want).max() <= 432 * 2.0 ** -23 * np.abs(x).max() * np.abs(wt).sum((1, 2, 3)).max()
+
+
+def test_price_and_packed_image_decide(monkeypatch):
+    """Without being forced: taken where the price says so, and not where one packed image is over the limit."""
+    b = np.zeros(82, np.float32)
+    x, wt, dy = _operands(32, 48, 82, 37, 37, 3, 1, 1)
+    got = _run(x, wt, b, dy, 1, 1)
+    monkeypatch.setenv("MTB_DISABLE_TC_SPLIT", "1")
+    assert not any(np.array_equal(a, o) for a, o in zip(got, _run(x, wt, b, dy, 1, 1)))
+    monkeypatch.delenv("MTB_DISABLE_TC_SPLIT")
+    x, wt, dy = _operands(1, 33, 34, 800, 700, 3, 1, 1)  # 287 MB packed
+    got = _run(x, wt, b[:34], dy, 1, 1)
+    monkeypatch.setenv("MTB_DISABLE_TC_SPLIT", "1")
+    assert all(np.array_equal(a, o) for a, o in zip(got, _run(x, wt, b[:34], dy, 1, 1)))
+
+
+@pytest.mark.parametrize("relu", [True, False])
+def test_with_batch_norm_and_residual(relu, monkeypatch):
+    """Convolution and BatchNorm with running statistics in one operator have the bits of the two; so have a residual and the ReLU."""
+    import gpu_util as g
+
+    x, wt, _ = _operands(8, 48, 82, 37, 37, 3, 1, 1)
+    rng = np.random.default_rng(4)
+    gamma, beta, mean = (g.dev(rng.standard_normal(82).astype(np.float32)) for _ in range(3))
+    var, res = g.dev(rng.uniform(0.5, 1.5, 82).astype(np.float32)), g.dev(rng.standard_normal((8, 82, 37, 37)).astype(np.float32))
+    xt, wtt, bt = g.dev(x), g.dev(wt), g.dev(rng.standard_normal(82).astype(np.float32))
+    one = g.op("conv2d_batch_norm")(xt, wtt, bt, (1, 1), (1, 1), gamma, beta, mean, var, 1e-5, relu, res if relu else None)
+    monkeypatch.setenv("MTB_DISABLE_TC_SPLIT", "1")
+    assert not np.array_equal(g.host(one), g.host(g.op("conv2d_batch_norm")(xt, wtt, bt, (1, 1), (1, 1), gamma, beta, mean, var, 1e-5, relu,
+                                                                            res if relu else None)))
+    monkeypatch.delenv("MTB_DISABLE_TC_SPLIT")
+    y = g.op("conv2d")(xt, wtt, bt, (1, 1), (1, 1))
+    norm = g.op("batch_norm2d")(y, gamma, beta, 1e-5, False, 0.1, mean, var)[0]
+    want = g.host(norm)
+    if relu:
+        want = np.maximum(want + g.host(res), 0)
+    assert np.array_equal(g.host(one), want)
+
+
+def test_data_gradient_added_to_another(monkeypatch):
+    import gpu_util as g
+
+    x, wt, dy = _operands(8, 48, 82, 37, 37, 3, 1, 1)
+    add = np.random.default_rng(3).standard_normal(x.shape).astype(np.float32)
+    xt, wtt, dyt = g.dev(x, True), g.dev(wt), g.dev(dy)
+    run = lambda **more: g.host(g.op("conv2d_backward")(dyt, xt, wtt, None, (1, 1), (1, 1), **more)[0])
+    dx = run()
+    assert np.array_equal(run(accumulate_dx=g.dev(add)), dx + add)
+    monkeypatch.setenv("MTB_DISABLE_TC_SPLIT", "1")
+    assert not np.array_equal(dx, run())
+
+
+def test_captured():
+    """Replays of a captured forward and backward pass on refilled inputs have the bits of eager calls."""
+    import gpu_util as g
+    from mytorch_b200.cuda_graph import StepGraph
+
+    x, wt, dy = _operands(8, 48, 82, 37, 37, 3, 1, 1)
+    xt, wtt, dyt = g.dev(x, True), g.dev(wt, True), g.dev(dy)
+
+    def step():
+        y = g.op("conv2d")(xt, wtt, None, (1, 1), (1, 1))
+        return [y, *g.op("conv2d_backward")(dyt, xt, wtt, None, (1, 1), (1, 1))[:2]]
+
+    graph = StepGraph(step)
+    out = graph.capture()
+    for scale in (1.0, 0.5, np.inf):
+        xt.copy_(g.dev((x * np.float32(scale)).astype(np.float32)))
+        graph.replay()
+        got = [g.host(t) for t in out]
+        assert all(np.array_equal(a, g.host(b), equal_nan=True) for a, b in zip(got, step()))
+    graph.destroy()
