@@ -1576,7 +1576,8 @@ WgradPlan wgrad_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int s
 // (pointers assumed 16-byte aligned), and, for the row-staged kernels, how their shared and tensor
 // memory is laid out against the furthest byte their copies write and their descriptors read.
 // Host code only: callable without a device (the SM count then defaults to 148).
-//   out[0..2]   path of forward, dgrad, wgrad: 0 CUDA-core, 1 im2col tcgen05, 2 row-staged tcgen05
+//   out[0..2]   path of forward, dgrad, wgrad: 0 FP32 (CUDA cores, or two-term products where scratch is passed and they pay), 1 im2col tcgen05,
+//               2 row-staged tcgen05
 //   out[3..9]   forward, row-staged: dynamic smem bytes, activation stage bytes, last byte written by
 //               the row copies, last byte read through a descriptor, TMEM columns, tiles per item,
 //               1 if the filter is resident
