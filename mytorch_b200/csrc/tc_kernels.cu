@@ -950,6 +950,7 @@ constexpr long long kMinIm2colBytes = 128 * 1024;
 }  // namespace
 
 #include "tc_conv_rows.cuh"
+#include "tc_conv_taps.cuh"
 
 // ------------------------------------------------------------------------------ host API
 
@@ -1090,6 +1091,13 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), gp.ns);
   const int bn = staged ? row_bn : gp.bn;
   if (stats_rows) *stats_rows = 0;
+  const TapsPlan taps = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout);
+  if (taps.ok &&
+      taps.ns <= (staged ? row_conv_ns(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32)) : gp.ns)) {
+    const bool with_stats = stats && stats_rows && !relu && cout % 32 == 0 && !getenv("MTB_DISABLE_CONV_STATS");
+    if (with_stats) *stats_rows = taps_stats_rows(taps);
+    return run_taps<B_KMAJOR>(taps, n, h, w, cin, cout, x, wt, bias, residual, relu, y, (cudaStream_t)stream, with_stats ? stats : nullptr, bn_eval);
+  }
   // the statistics and BatchNorm epilogues keep a CTA on one column tile: there must be a CTA for each
   const bool a_cta_per_column = (cout + bn - 1) / bn <= mtb_sm_count();
   if (bn_eval && !a_cta_per_column) {
@@ -1182,6 +1190,10 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb, class_plan.ns);
   const int bn = staged ? row_bn : class_plan.bn;
   cudaStream_t st = (cudaStream_t)stream;
+  const TapsPlan taps = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin);
+  if (taps.ok && addend != dx &&
+      taps.ns <= (staged ? row_conv_ns(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb) : class_plan.ns))
+    return run_taps<B_MNMAJOR>(taps, n, h, w, cout, cin, dy, wt, nullptr, addend, 0, dx, st);
   CUtensorMap mapB;
   const long long wcols = (long long)kh * kw * cin;
   const bool b_blocks = cin % 32 == 0;  // a tap's columns then are whole blocks
@@ -1570,6 +1582,32 @@ WgradPlan wgrad_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int s
 }
 
 }  // namespace
+
+// The same for the kernel that works in pairs of SMs (tc_conv_taps.cuh), which forward and data gradient take where its layout fits
+// and its price is lower.  out[0..8] forward, out[9..17] data gradient: form (1 or 2; 0: not taken), dynamic smem bytes, stage bytes, first and
+// (one past the) last byte written by the row copies, first and last byte read through a descriptor, image rows a stage, TMEM columns.
+MTB_API int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out) {
+  MTB_REQUIRE(out && n > 0 && cin > 0 && cout > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0, "conv2d_pair_plan: bad arguments");
+  for (int dir = 0; dir < 2; ++dir, out += 9) {
+    for (int i = 0; i < 9; ++i) out[i] = 0;
+    const int kc = dir ? cout : cin;
+    const TapsPlan q = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, kc, dir ? cin : cout);
+    if (!q.ok) continue;
+    out[0] = q.beside;
+    out[1] = (int)q.smem_bytes;
+    out[2] = (int)q.a_stage_bytes;
+    for (int col = 0; col < (q.rows ? 1 : q.Wp); ++col) {  // column of a tile's first position: whole rows start at 0
+      const int rows = q.rows ? q.rows + 2 : (col + 128) / q.Wp + 3, first = (q.origin - q.Wp - col) * 128, end = first + rows * q.Wp * 128;
+      if (col == 0 || first < out[3]) out[3] = first;
+      if (end > out[4]) out[4] = end;
+      if (rows > out[7]) out[7] = rows;
+    }
+    out[5] = (q.origin - q.Wp - (q.beside == 1 ? 1 : 0)) * 128;
+    out[6] = (q.origin + q.Wp + 127 + 1 + 1) * 128;
+    out[8] = kTapsBufs * q.beside * 64;
+  }
+  return MTB_OK;
+}
 
 // Which kernel family each of forward / data gradient / weight gradient can take for a shape: row-staged wherever
 // its layout fits (the launch then takes that or im2col, whichever is priced lower: row_conv_pays, wgrad_rows_pay)

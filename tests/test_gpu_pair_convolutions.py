@@ -1,0 +1,62 @@
+"""3x3 convolutions by pairs of SMs: tiles of whole image rows and tiles that start anywhere, image counts that leave the second CTA of a
+pair without work, one to four blocks of reduction channels, column tiles that end inside a tile, every epilogue, and what is added on
+boundaries of 4, 16 and 32 bytes; against 64-bit sums over operands as the copy engine rounds them."""
+import numpy as np
+import pytest
+
+from oracle import ops as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _product(x, w):
+    """Products of TF32 operands summed in 64 bits, and the same of the magnitudes."""
+    xp = np.pad(x, ((0, 0), (0, 0), (1, 1), (1, 1)))
+    h, wd = x.shape[2:]
+    return sum(np.einsum("nchw,oc->nohw", xp[:, :, a:a + h, b:b + wd], w[:, :, a, b], optimize=True) for a in range(3) for b in range(3))
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w", [
+    (20, 64, 64, 32, 32), (9, 32, 64, 19, 28), (5, 64, 80, 41, 56), (16, 96, 96, 30, 30), (17, 128, 128, 16, 16), (5, 128, 192, 28, 28),
+    (3, 64, 32, 64, 64), (200, 64, 64, 5, 4), (30, 128, 16, 13, 22), (2, 32, 48, 90, 81), (150, 96, 160, 8, 9)])
+def test_forward_and_data_gradient(n, cin, cout, h, w):
+    import gpu_util as g
+
+    from mytorch_b200.backends.cuda.env import CudaMemory, CudaMemoryView
+
+    rng = np.random.default_rng(n + cin + cout + w)
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)
+    x, wt, b, dy, add = f32(n, cin, h, w), f32(cout, cin, 3, 3), f32(cout), f32(n, cout, h, w), f32(n, cin, h, w)
+    rx, rw, rdy = (O.round_tf32(t).astype(np.float64) for t in (x, wt, dy))
+    xt, wtt, bt, s, p = g.dev(x, True), g.dev(wt), g.dev(b), (1, 1), (1, 1)
+
+    def check(got, want, magnitude, terms):  # products of TF32 operands are exact in FP32: what is left is the sum's rounding
+        assert (np.abs(got - want) <= (terms + 3) * 2.0 ** -23 * magnitude).all()
+
+    y = g.op("conv2d")(xt, wtt, bt, s, p)
+    yh = g.host(y)
+    check(yh, _product(rx, rw) + b[:, None, None], _product(abs(rx), abs(rw)) + abs(b)[:, None, None], 9 * cin)
+    # the same bits with statistics, and in the inference form
+    ys = g.op("conv2d")(xt, wtt, bt, s, p, bn_stats=True)
+    assert np.array_equal(g.host(ys), yh)
+    _, mean, var = g.op("batch_norm2d")(ys, None, None, 1e-5, True, 0.1, None, None)
+    y64, rows = yh.astype(np.float64), yh[:, 0].size
+    assert (np.abs(g.host(mean) - y64.mean((0, 2, 3))) <= rows * 2.0 ** -23 * np.abs(y64).mean((0, 2, 3))).all()
+    assert (np.abs(g.host(var) - y64.var((0, 2, 3))) <= rows * 2.0 ** -23 * (y64 ** 2).mean((0, 2, 3))).all()
+    res = g.dev(f32(*yh.shape))
+    vec = lambda lo, hi: g.dev(rng.uniform(lo, hi, cout).astype(np.float32))
+    gamma, beta, m, v = vec(0.5, 1.5), vec(-1, 1), vec(-1, 1), vec(0.5, 2)
+    plain = g.op("batch_norm2d")(y, gamma, beta, 1e-5, False, 0.1, m, v)[0]
+    assert np.array_equal(g.host(g.op("conv2d_batch_norm")(xt, wtt, bt, s, p, gamma, beta, m, v, 1e-5, True, res)), g.host(g.op("add_relu")(plain, res)))
+    if cout % 32:
+        return  # the data gradient then is none of this kernel's
+    turned = rw[:, :, ::-1, ::-1].transpose(1, 0, 2, 3)
+    dx = g.host(g.op("conv2d_backward")(g.dev(dy), xt, wtt, None, s, p)[0])
+    check(dx, _product(rdy, turned), _product(abs(rdy), abs(turned)), 9 * cout)
+    for start in (0, 16, 4):  # bytes past a boundary of 32
+        at = g.dev(add)
+        block = CudaMemory(0, at._native_array.nbytes + 32)
+        window = CudaMemoryView(block, start, at._native_array.nbytes, 0)
+        window.copy_from(at._native_array, window.nbytes)
+        at._native_array = window
+        assert np.array_equal(g.host(g.op("conv2d_backward")(g.dev(dy), xt, wtt, None, s, p, accumulate_dx=at)[0]), dx + add)
