@@ -901,9 +901,10 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_cons
     }
   }
 
-  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
+  // behind the barrier: see tc_wgrad_kernel
+  mtb_launch_dependents();
   if (abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
   }

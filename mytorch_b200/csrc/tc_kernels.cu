@@ -1491,9 +1491,12 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant_
     }
   }
 
-  mtb_launch_dependents();
   tc_fence_before();
   __syncthreads();
+  // Behind the barrier: the first thread's call counts for the CTA, and that of a producer that has nothing left to copy let the CTAs of
+  // the planes' addition take registers beside the main stream's kernels while this one still had its accumulators to store (ResNet-18
+  // step at 512 images 5.67 -> 5.47 ms, at 128 1925 -> 1903 us, ResNet-50 18.24 -> 18.16 ms).
+  mtb_launch_dependents();
   if (abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
   }
