@@ -114,6 +114,12 @@ int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
                               const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
                               const float* running_var, double eps, const float* residual, int relu, float* y, void* workspace,
                               long long workspace_bytes, void* stream);
+/* Inference: the same with a ReLU and a 2 x 2 max-pool of stride 2 behind it (mytorch/nn/max_pool.py:5-21), y [N,OH/2,OW/2,Cout] and its tie mask,
+ * where mtb_conv2d_bn_pool_takes answers 1 (small convolutions); the bits are those of the separate operators. */
+int mtb_conv2d_bn_pool_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
+int mtb_conv2d_bn_pool_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
+                                   const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
+                                   const float* running_var, double eps, float* y, unsigned short* mask, void* stream);
 /* dx[N,H,W,Cin]: every element is written (zeros where no window reaches); no atomics */
 int mtb_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                          const float* wt, float* dx, void* workspace, long long workspace_bytes, void* stream);

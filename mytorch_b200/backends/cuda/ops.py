@@ -227,10 +227,20 @@ def _conv_operands(env, input, weight, stride, padding, packed=None):
 
 
 @_reg("cuda", "conv2d_batch_norm")
-def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps, relu, residual=None):
-    """Inference: relu?(batch_norm2d(conv2d(input)) + residual) with running statistics, in the convolution's launch."""
+def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps, relu, residual=None, pool=False):
+    """Inference: relu?(batch_norm2d(conv2d(input)) + residual) with running statistics, in the convolution's launch.
+    ``pool``: with a ReLU and a 2x2 max-pool of stride 2 behind it; None where that takes more than one launch."""
     _f32(input, weight, bias, gamma, beta, running_mean, running_var, residual)
     env = _env(input)
+    if pool:
+        a = n, _, h, w, kh, kw, sh, sw, ph, pw, cout = _conv_args(input, weight, stride, padding)
+        # an image stem that is packed for the tensor cores is not a small convolution
+        if a[1] < _TC_CHANNELS and _stem_form(input.shape, weight.shape, stride, padding) is not None or not env.lib.conv2d_bn_pool_takes(*a):
+            return None
+        out = _new((n, cout, ((h + 2 * ph - kh) // sh + 1) // 2, ((w + 2 * pw - kw) // sw + 1) // 2), input)
+        out._pool_tiemask = mask = CudaMemory(input.device.index, out._native_array.nbytes // 2)
+        env.lib.conv2d_bn_pool_forward_f32(*a, input, weight, bias, gamma, beta, running_mean, running_var, float(eps), out, mask, env.stream())
+        return out
     a, x, wt, out = _conv_operands(env, input, weight, stride, padding)
     if residual is not None and residual.shape != out.shape:
         raise MismatchShapesError([out.shape, residual.shape])

@@ -14,6 +14,10 @@ int mtb_conv2d_dgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, 
                           void* stream, const int* guard, int guards);
 int mtb_conv2d_wgrad_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* dy, float* dw,
                           void* workspace, long long workspace_bytes, void* stream, const int* guard, int guards);
+// the same for a small convolution, followed by a ReLU and a 2 x 2 max-pool of stride 2 (mask: its tie mask)
+bool mtb_conv2d_bn_pool_simt_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
+int mtb_conv2d_bn_pool_simt(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x, const float* wt,
+                            const float* bias, const MtbBnEval& bn, float* y, unsigned short* mask, void* stream);
 // y = relu?(batch_norm(x) + residual) over [rows, c] with running statistics; x == y is allowed (batch_norm.cu)
 int mtb_bn_eval_apply(const float* x, float* y, long long rows, int c, const MtbBnEval& bn, const float* residual, int relu, cudaStream_t st);
 MTB_API int mtb_conv2d_dgrad_simt_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,

@@ -120,6 +120,18 @@ struct PatchK {
   }
 };
 
+// The same with the rows in the order in which a 2 x 2 max-pool of stride 2 reads the output pixels: four neighbouring rows are a
+// window (row-major), a last odd line or column of pixels belongs to none and is left out.
+struct PatchPoolK : PatchK {
+  FastDiv pool_w, pool_h;
+  __device__ __forceinline__ Row row(int i, bool valid, int) const {
+    if (!valid) return Row{nullptr, 0, 0};
+    unsigned c, r;
+    const unsigned n = pool_h.divmod(pool_w.divmod((unsigned)i >> 2, c), r);
+    return Row{x + (long long)n * d.H * d.W * d.Cin, (int)(2 * r + (i >> 1 & 1)) * d.SH - d.PH, (int)(2 * c + (i & 1)) * d.SW - d.PW};
+  }
+};
+
 // Data gradient.  The input pixels fall into SH*SW residue classes (one per blockIdx.z): pixel (i, j) of class (a, b)
 // is (start + s*i, ...) and only meets the taps a + s*t, from output row c0 + i - t: no multiplication is spent on
 // taps that cannot reach it.  k = (th, tw, co).
@@ -294,6 +306,7 @@ struct StageR {
 template <class Source> struct IsK { static constexpr bool value = false; };
 template <> struct IsK<DenseK> { static constexpr bool value = true; };
 template <> struct IsK<PatchK> { static constexpr bool value = true; };
+template <> struct IsK<PatchPoolK> { static constexpr bool value = true; };
 template <> struct IsK<DgradK> { static constexpr bool value = true; };
 template <class Source, int ROWS, int THREADS, int VEC>
 using Stage = std::conditional_t<IsK<Source>::value, StageK<Source, ROWS, THREADS, VEC>, StageR<Source, ROWS, THREADS, VEC>>;
@@ -321,6 +334,9 @@ struct Extra {
   float* pre;        // dense products of two operands along k only; not NULL: laid out like out, takes the value before the ReLU
 };
 struct NoExtra {};
+struct PoolExtra {  // with PatchPoolK
+  unsigned short* mask;  // per result, bit 2 * line + column of every pixel of the window that equals the maximum
+};
 template <int EXTRA>
 using ExtraOf = std::conditional_t<EXTRA == EXTRA_NONE, NoExtra, Extra>;
 
@@ -334,6 +350,12 @@ __device__ __forceinline__ float* out_row(const Out& o, int i, int z) {
   return o.out + r * o.ld;
 }
 
+__device__ __forceinline__ float bn_eval_value(const MtbBnEval& bn, int c, float v) {
+  const float rstd = 1.0f / sqrtf(bn.var[c] + bn.eps);
+  const float scale = bn.gamma ? bn.gamma[c] * rstd : rstd, beta = bn.beta ? bn.beta[c] : 0.f;
+  return (v - bn.mean[c]) * scale + beta;
+}
+
 // TAIL: with BatchNorm and the residual of Out (the cluster kernels, whose store is one loop)
 template <bool TAIL, int EXTRA>
 __device__ __forceinline__ void store4(const Out& o, const ExtraOf<EXTRA>& extra, float* row, int j, int N, bool vec, float4 v) {
@@ -342,11 +364,7 @@ __device__ __forceinline__ void store4(const Out& o, const ExtraOf<EXTRA>& extra
   for (int q = 0; q < 4; ++q) {
     if (o.bias && j + q < N) t[q] += o.bias[j + q];
     if constexpr (TAIL) {
-      if (o.bn.mean && j + q < N) {
-        const float rstd = 1.0f / sqrtf(o.bn.var[j + q] + o.bn.eps);
-        const float scale = o.bn.gamma ? o.bn.gamma[j + q] * rstd : rstd, beta = o.bn.beta ? o.bn.beta[j + q] : 0.f;
-        t[q] = (t[q] - o.bn.mean[j + q]) * scale + beta;
-      }
+      if (o.bn.mean && j + q < N) t[q] = bn_eval_value(o.bn, j + q, t[q]);
       if (o.residual && j + q < N) t[q] += o.residual[row - o.out + j + q];
     }
     if constexpr (EXTRA == EXTRA_PRE) {
@@ -394,9 +412,12 @@ using TableOf = std::conditional_t<std::is_same_v<SA, DgradK>, ClassTable, NoTab
 
 // blockIdx.z = class * slices + slice.  CLUSTER: the slices of a tile form a cluster and add up at the end;
 // otherwise slices > 1 only with planes of partials (Out::split_plane).
+template <class SA, int EXTRA>
+using LastParam = std::conditional_t<std::is_same_v<SA, PatchPoolK>, PoolExtra, ExtraOf<EXTRA>>;
+
 template <class T, class SA, int VA, class SB, int VB, bool CLUSTER, int EXTRA>
 __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB sb, Out o, const __grid_constant__ TableOf<SA> table, int M, int N, int K,
-                                                          int slices, int k_per_slice, const ExtraOf<EXTRA> extra) {
+                                                          int slices, int k_per_slice, const LastParam<SA, EXTRA> extra) {
   constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, THREADS = T::THREADS;
   constexpr int GM = TM / 4, GN = TN / 4;  // a thread's rows and columns come in groups of four, spread over the tile
   __shared__ float As[2][BK][BM + 4];
@@ -484,14 +505,44 @@ __global__ void __launch_bounds__(T::THREADS, T::kMinCtas) gemm_kernel(SA sa, SB
     cluster.sync();
     const int size = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     constexpr int kVecs = BN / 4;
-    for (int e = tid; e < (BM / size) * kVecs; e += THREADS) {
-      const int r = (e / kVecs) * size + rank, c = (e % kVecs) * 4;
-      float4 s = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], 0));
-      for (int q = 1; q < size; ++q) {  // rank order: the same sum every time
-        const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], q));
-        s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+    if constexpr (std::is_same_v<SA, PatchPoolK>) {  // CTA r finishes the windows r, r + size, ...: bias, BatchNorm and ReLU of four rows, their maximum
+      for (int e = tid; e < (BM / 4 / size) * kVecs; e += THREADS) {
+        const int u = (e / kVecs) * size + rank, c = (e % kVecs) * 4;
+        if (m0 + 4 * u >= M) continue;
+        float best[4];
+        unsigned ties[4] = {0u, 0u, 0u, 0u};
+        for (int w = 0; w < 4; ++w) {
+          float4 s = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[4 * u + w][c], 0));
+          for (int q = 1; q < size; ++q) {
+            const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[4 * u + w][c], q));
+            s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+          }
+          const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (n0 + c + q >= N) continue;
+            float t = v[q];
+            if (o.bias) t += o.bias[n0 + c + q];
+            t = fmaxf(bn_eval_value(o.bn, n0 + c + q, t), 0.f);
+            if (w == 0 || t > best[q]) { best[q] = t; ties[q] = 1u << w; }
+            else if (t == best[q]) ties[q] |= 1u << w;
+          }
+        }
+        const long long at = (long long)(m0 / 4 + u) * o.ld + n0 + c;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (n0 + c + q < N) { o.out[at + q] = best[q]; extra.mask[at + q] = (unsigned short)ties[q]; }
       }
-      if (m0 + r < M) store4<std::is_same_v<SA, PatchK>, EXTRA>(o, extra, out_row(o, m0 + r, z), n0 + c, N, vec, s);
+    } else {
+      for (int e = tid; e < (BM / size) * kVecs; e += THREADS) {
+        const int r = (e / kVecs) * size + rank, c = (e % kVecs) * 4;
+        float4 s = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], 0));
+        for (int q = 1; q < size; ++q) {  // rank order: the same sum every time
+          const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(&tile[r][c], q));
+          s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+        }
+        if (m0 + r < M) store4<std::is_same_v<SA, PatchK>, EXTRA>(o, extra, out_row(o, m0 + r, z), n0 + c, N, vec, s);
+      }
     }
     cluster.sync();  // nobody leaves while its tile is being read
   } else {
@@ -557,12 +608,12 @@ using TileXS = Tile<64, 32, 4, 4, 6>;
 
 template <int EXTRA, class T, class SA, int VA, class SB, int VB, bool CLUSTER>
 int launch_tile(const SA& sa, const SB& sb, const Out& o, const TableOf<SA>& table, int classes, int M, int N, int K, int slices, cudaStream_t st,
-                const char* name, const Extra& extra) {
+                const char* name, const std::conditional_t<std::is_same_v<SA, PatchPoolK>, PoolExtra, Extra>& extra) {
   int per = (K + slices - 1) / slices;
   per = (per + BK - 1) / BK * BK;
   if (per < BK) per = BK;
-  ExtraOf<EXTRA> with{};
-  if constexpr (EXTRA != EXTRA_NONE) with = extra;
+  LastParam<SA, EXTRA> with{};
+  if constexpr (EXTRA != EXTRA_NONE || std::is_same_v<SA, PatchPoolK>) with = extra;
   dim3 grid(mtb_div_up(M, T::BM), mtb_div_up(N, T::BN), classes * slices);
   MTB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "%s: grid too large", name);
   if constexpr (CLUSTER) {

@@ -72,10 +72,10 @@ class BatchNorm1d(BatchNorm2d):
         return y.reshape(x.shape)
 
 
-def inference_conv_norm(conv, norm, x, relu=False, residual=None):
+def inference_conv_norm(conv, norm, x, relu=False, residual=None, pool=False):
     """``norm(conv(x))``, then optionally ``+ residual``, then optionally ReLU, as one operator where that is possible: a
     convolution and a BatchNorm layer that normalises with its running statistics, on CUDA, with no gradient to record.
-    None elsewhere.  Same bits as the separate layers."""
+    None elsewhere.  Same bits as the separate layers.  ``pool``: with the ReLU, and a 2x2 max-pool of stride 2 behind it."""
     mean, device = norm.running_mean, x.device
     if norm.training or mean is None or device.type != "cuda":
         return None
@@ -92,4 +92,7 @@ def inference_conv_norm(conv, norm, x, relu=False, residual=None):
             return None
     if gamma is None or beta is None:
         gamma = beta = None
-    return dispatch(device, "conv2d_batch_norm")(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, relu, residual)
+    convolve = dispatch(device, "conv2d_batch_norm")
+    if pool:
+        return convolve(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, True, None, True)
+    return convolve(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, relu, residual)

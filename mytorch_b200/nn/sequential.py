@@ -3,15 +3,21 @@ from mytorch_b200.nn.conv import Conv2d
 from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu
 from mytorch_b200.nn.functional.linear import _linear_relu
 from mytorch_b200.nn.linear import Linear
+from mytorch_b200.nn.max_pool import MaxPool2d
 from mytorch_b200.nn.module import Module
 from mytorch_b200.nn.relu import ReLU
 
 _NORMS = (BatchNorm2d, BatchNormReLU2d)
 
 
+def _halves(layer):
+    """A 2x2 max-pool of stride 2 that runs the class's own forward."""
+    return type(layer) is MaxPool2d and layer.kernel_size == layer.stride == (2, 2) and layer.padding == (0, 0) and not layer._forward_replaced
+
+
 class Sequential(Module):
     """Layers one after the other.  Neighbours that exist as one operator with the same bits run as one on CUDA: BatchNorm2d +
-    ReLU, Linear + ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU) with running statistics.  A step of the
+    ReLU, Linear + ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU (+ MaxPool2d)) with running statistics.  A step of the
     MNIST example is 300 library calls of a few microseconds each, so every operator left out shows."""
 
     def __init__(self, *args):
@@ -20,7 +26,7 @@ class Sequential(Module):
             self.register_module(str(i), module)
 
     def forward(self, input):
-        layers = list(self._modules.values()) + [None, None]
+        layers = list(self._modules.values()) + [None, None, None]
         i = 0
         while layers[i] is not None:
             layer, after = layers[i], layers[i + 1]
@@ -28,6 +34,13 @@ class Sequential(Module):
             if kind is Conv2d and kind_after in _NORMS and not (after.training or layer._forward_replaced or after._forward_replaced):
                 behind = layers[i + 2]
                 relu = kind_after is BatchNorm2d and type(behind) is ReLU and not behind._forward_replaced
+                last = 3 if relu else 2
+                if (relu or kind_after is BatchNormReLU2d) and _halves(layers[i + last]):
+                    y = inference_conv_norm(layer, after, input, pool=True)
+                    if y is not None:
+                        input = y
+                        i += last + 1
+                        continue
                 y = inference_conv_norm(layer, after, input, relu or kind_after is BatchNormReLU2d)
                 if y is not None:
                     input = y
