@@ -951,6 +951,7 @@ constexpr long long kMinIm2colBytes = 128 * 1024;
 
 #include "tc_conv_rows.cuh"
 #include "tc_conv_taps.cuh"
+#include "tc_wgrad_pairs.cuh"
 
 // ------------------------------------------------------------------------------ host API
 
@@ -1676,6 +1677,11 @@ long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, in
     const long long b2 = (long long)rq.splits * q.Kw * cout * 4 + 256;
     if (b2 > bytes) bytes = b2;
   }
+  const WgradPairPlan pq = wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
+  if (wgrad_pairs_pay(pq, cin, cout)) {
+    const long long b2 = (long long)pq.splits * q.Kw * cout * 4 + 256;
+    if (b2 > bytes) bytes = b2;
+  }
   return bytes;
 }
 
@@ -1693,6 +1699,11 @@ bool mtb_tc_conv2d_wgrad_supported(int n, int cin, int h, int w, int kh, int kw,
 int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                             const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
+  const WgradPairPlan pq = wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
+  if (wgrad_pairs_pay(pq, cin, cout)) {
+    MTB_REQUIRE(workspace && workspace_bytes >= (long long)pq.splits * kh * kw * cin * cout * 4, "conv2d_wgrad: workspace too small");
+    return run_wgrad_pairs(pq, n, cin, h, w, cout, x, dy, dw, (float*)workspace, (cudaStream_t)stream);
+  }
   const WgradRowsPlan rq = wgrad_rows_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (wgrad_rows_pay(rq, cin, cout)) {
     MTB_REQUIRE(workspace && workspace_bytes >= (long long)rq.splits * kh * kw * cin * cout * 4, "conv2d_wgrad: workspace too small");
