@@ -17,8 +17,8 @@ def _product(x, w):
 
 
 @pytest.mark.parametrize("n,cin,cout,h,w", [
-    (20, 64, 64, 32, 32), (9, 32, 64, 19, 28), (5, 64, 80, 41, 56), (16, 96, 96, 30, 30), (17, 128, 128, 16, 16), (5, 128, 192, 28, 28),
-    (3, 64, 32, 64, 64), (200, 64, 64, 5, 4), (30, 128, 16, 13, 22), (2, 32, 48, 90, 81), (150, 96, 160, 8, 9)])
+    (20, 64, 64, 32, 32), (9, 64, 64, 19, 28), (5, 64, 80, 41, 56), (16, 96, 96, 30, 30), (17, 128, 128, 16, 16), (5, 128, 192, 28, 28),
+    (3, 64, 96, 64, 64), (200, 64, 64, 5, 4), (30, 128, 64, 13, 22), (2, 64, 112, 90, 81), (150, 96, 160, 8, 9)])
 def test_forward_and_data_gradient(n, cin, cout, h, w):
     import gpu_util as g
 

@@ -16,7 +16,7 @@ def test_copies_and_descriptors_stay_inside_their_stage():
                     assert lib.mtb_conv2d_pair_plan_f32(5, cin, h, w, 3, 3, 1, 1, 1, 1, cout, out) == 0
                     for kc, nout, o in ((cin, cout, 0), (cout, cin, 9)):
                         form, smem, stage, wfirst, wlast, rfirst, rlast, rows, tmem = out[o:o + 9]
-                        assert form == 0 or (kc % 32 == 0 and kc <= 128 and nout % 16 == 0)
+                        assert form == 0 or (kc % 32 == 0 and 64 <= kc <= 128 and nout % 16 == 0 and nout >= 64)
                         if form:
                             taken += 1
                             assert form in (1, 2) and smem <= 227 * 1024 - 4096 and stage % 1024 == 0
