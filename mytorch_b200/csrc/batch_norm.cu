@@ -10,21 +10,28 @@ MTB_API long long mtb_batch_norm2d_workspace_bytes(int n, int c, int h, int w);
 
 namespace {
 
-// The order in which a pass walks its rows.  All CTAs of a launch work on neighbouring groups of kGroup iterations (grid stride), so that what the
-// L2 holds at its end is one stretch of the tensor, and the pass behind it starts there: the normalise pass walks back to front behind a
-// convolution that wrote front to back, the backward's sums do so behind a data gradient, and dx then front to back.  A group's loads are
-// all issued before the first value is used or stored.  Walking front to back everywhere, before -> so (ResNet-50 step at 128 images,
-// ResNet-18 at 512, 128, 64): contiguous rows a CTA 18.50 ms, 5465, 1882, 1270 us; groups 18.13, 5406, 1854, 1246; groups and directions 18.08,
-// 5353, 1851, 1246.
+// The order in which a pass walks its rows, in groups of kGroup iterations whose loads are all issued before the first value is used or stored.
+// All CTAs work on neighbouring groups (grid stride), so that what the L2 holds at the end is one stretch of the tensor, and the pass behind it
+// starts there: the normalise pass walks back to front behind a convolution that wrote front to back, the backward's sums do so behind a data
+// gradient, and dx then front to back.  Single rows of a contiguous range a CTA -> groups, in these orders: ResNet-50 step at 128 images 18.50 -> 18.08 ms,
+// ResNet-18 at 512 5465 -> 5353 us (5406 without the turns), at 128 1882 -> 1851, at 64 (captured) 1270 -> 1246.  rows_per_block > 0: a CTA
+// takes that many rows one after the other; the sums do so up to 64 MB, which the L2 holds whole, and keep their order there.
 constexpr int kGroup = 4;
 struct RowWalk {
-  long long groups, at, step;
+  long long r, last, step, limit;  // first row of the group, of the last group, from group to group; end of the rows
   bool back;
-  __device__ __forceinline__ RowWalk(long long rows, int R, bool back_) : groups((rows + kGroup * R - 1) / (kGroup * R)), at(blockIdx.y), step(gridDim.y), back(back_) {}
-  __device__ __forceinline__ bool next(long long& group) {
-    if (at >= groups) return false;
-    group = back ? groups - 1 - at : at;
-    at += step;
+  __device__ __forceinline__ RowWalk(long long rows, int R, long long rows_per_block, bool back_) {
+    const long long group = (long long)kGroup * R;
+    back = back_ && rows_per_block == 0;
+    r = blockIdx.y * (rows_per_block ? rows_per_block : group);
+    step = rows_per_block ? group : group * gridDim.y;
+    limit = rows_per_block && r + rows_per_block < rows ? r + rows_per_block : rows;
+    last = (rows - 1) / group * group;
+  }
+  __device__ __forceinline__ bool next(long long& first) {
+    if (r >= limit) return false;
+    first = back ? last - r : r;
+    r += step;
     return true;
   }
 };
@@ -221,21 +228,21 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
   // Four rows are loaded before the first is stored: x may be y (an update in place), so the compiler would not do it.  BatchNorm,
   // ReLU and pooling of 256 x 128 x 56 x 56, forward and backward: 1073 -> 1050 us; ResNet-18 step at 512 images 5.84 -> 5.78 ms.
   constexpr int AHEAD = kGroup;
-  RowWalk walk(rows, R, true);
-  for (long long group; walk.next(group);) {
-    const long long r = group * (kGroup * R) + rsub;
+  RowWalk walk(rows, R, 0, true);
+  for (long long r; walk.next(r);) {
+    r += rsub;
     const long long off = r * C + (long long)cg * V, step = (long long)R * C;
     VecF<V> f[AHEAD], a[MODE == 2 ? AHEAD : 1];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (r + u * R < rows) {
+      if (r + u * R < walk.limit) {
         f[u] = vload<V>(x + off + u * step);
         if (MODE == 2) a[u] = vload<V>(res + off + u * step);
       }
     }
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (r + u * R >= rows) break;
+      if (r + u * R >= walk.limit) break;
       unsigned negative = 0;
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -256,7 +263,7 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
 // MODE 1 / 2: the forward output went through max(0, .) (MODE 2: after adding `res`) in the same pass;
 // the upstream gradient is first masked where the (recomputed, bit-identical) value was negative.
 template <int V, int MODE>
-__global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __restrict__ dy, const float* __restrict__ x, long long rows, int C, int L, const float* __restrict__ mean,
+__global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __restrict__ dy, const float* __restrict__ x, long long rows, int C, int L, long long rows_per_block, const float* __restrict__ mean,
                                                               const float* __restrict__ var, float eps, const float* __restrict__ gamma,
                                                               const float* __restrict__ beta, float* __restrict__ partial,
                                                               const float* __restrict__ res, const unsigned char* __restrict__ mask) {
@@ -277,14 +284,14 @@ __global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __rest
     bt[i] = (active && beta) ? beta[cg * V + i] : 0.f;
   }
   if (active) {
-    RowWalk walk(rows, R, true);
-    for (long long group; walk.next(group);) {
-      const long long r0 = group * (kGroup * R) + rsub;
+    RowWalk walk(rows, R, rows_per_block, true);
+    for (long long r0; walk.next(r0);) {
+      r0 += rsub;
       VecF<V> g[kGroup], f[kGroup], a[MODE == 2 ? kGroup : 1];
       unsigned negative[kGroup];
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) {
-        if (r0 + u * R < rows) {
+        if (r0 + u * R < walk.limit) {
           const long long off = (r0 + u * R) * C + (long long)cg * V;
           g[u] = vload<V>(dy + off);
           f[u] = vload<V>(x + off);
@@ -294,7 +301,7 @@ __global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __rest
       }
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) {
-        if (r0 + u * R >= rows) break;
+        if (r0 + u * R >= walk.limit) break;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
           float gi = g[u].v[i];
@@ -398,14 +405,14 @@ __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict_
     k3[i] = coef[2 * C + cg * V + i];
     bt[i] = beta ? beta[cg * V + i] : 0.f;
   }
-  RowWalk walk(rows, R, false);
-  for (long long group; walk.next(group);) {
-    const long long r0 = group * (kGroup * R) + rsub;
+  RowWalk walk(rows, R, 0, false);
+  for (long long r0; walk.next(r0);) {
+    r0 += rsub;
     VecF<V> g[kGroup], f[kGroup], a[MODE == 2 ? kGroup : 1];
     unsigned negative[kGroup];
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
-      if (r0 + u * R < rows) {
+      if (r0 + u * R < walk.limit) {
         const long long off = (r0 + u * R) * C + (long long)cg * V;
         g[u] = vload<V>(dy + off);
         f[u] = vload<V>(x + off);
@@ -415,7 +422,7 @@ __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict_
     }
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
-      if (r0 + u * R >= rows) break;
+      if (r0 + u * R >= walk.limit) break;
       const long long off = (r0 + u * R) * C + (long long)cg * V;
       VecF<V> m;
 #pragma unroll
@@ -526,7 +533,7 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
   ColCfg cfg = mtb_col_cfg(rows, c, aligned);
   dim3 grid(cfg.col_blocks, cfg.row_blocks);
 #define MTB_BN_PARTIAL(V_, M_) \
-  MTB_LAUNCH(bn_bwd_partial_kernel<V_, M_>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, mean, var, (float)eps, gamma, beta, \
+  MTB_LAUNCH(bn_bwd_partial_kernel<V_, M_>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta, \
              partial, res, mask)
   if (cfg.vec == 4) { if (mode == 3) MTB_BN_PARTIAL(4, 3); else if (mode == 2) MTB_BN_PARTIAL(4, 2); else if (mode == 1) MTB_BN_PARTIAL(4, 1); else MTB_BN_PARTIAL(4, 0); }
   else { if (mode == 2) MTB_BN_PARTIAL(1, 2); else if (mode == 1) MTB_BN_PARTIAL(1, 1); else MTB_BN_PARTIAL(1, 0); }
