@@ -162,6 +162,14 @@ int mtb_batch_norm2d_forward_f32(int n, int c, int h, int w, const float* x, con
 int mtb_batch_norm2d_forward_prestats_f32(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps,
                                           double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
                                           int relu, const float* stats, int stats_rows, void* workspace, long long workspace_bytes, void* stream);
+/* BatchNorm, ReLU and a 2 x 2 max-pool of stride 2 (mytorch/nn/batch_norm.py:123-135, relu.py:5-10, max_pool.py:5-21) as one operator; y [N,H/2,W/2,C] and
+ * its tie mask; c % 4 == 0, 16-byte aligned tensors, fewer than 2^29 elements.  The same bits as the operators one by one. */
+int mtb_batch_norm2d_relu_pool_forward_f32(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps, int training,
+                                           double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
+                                           unsigned short* tiemask, const float* stats, int stats_rows, void* workspace, long long workspace_bytes, void* stream);
+int mtb_batch_norm2d_relu_pool_backward_f32(int n, int c, int h, int w, const float* dy, const float* mean, const float* var, const float* x,
+                                            const unsigned short* tiemask, const float* gamma, const float* beta, double eps, float* dx, float* dgamma,
+                                            float* dbeta, void* workspace, long long workspace_bytes, void* stream);
 /* y = max(0, batch_norm(x) + residual): BatchNorm, shortcut addition and ReLU of a residual block's tail in
  * one normalise pass (the reference runs batch_norm2d, add_reference and relu_reference:
  * mytorch/nn/batch_norm.py:123-135, mytorch/tensor.py:292-300, mytorch/nn/relu.py:5-10).  stats / stats_rows as

@@ -238,7 +238,7 @@ constexpr unsigned HOST(I... i) { return (0u | ... | (1u << i)); }
   X(add_bias_rows_f32, LAUNCH, 0) X(binary_strided_f32, LAUNCH, HOST(2, 3, 4, 5)) X(resize_channels_f32, LAUNCH, 0) \
   X(pack_patches_f32, LAUNCH, 0) X(nchw_to_nhwc_f32, LAUNCH, 0) X(nhwc_to_nchw_f32, LAUNCH, 0) X(cast, LAUNCH, 0) \
   X(batch_norm2d_workspace_bytes, VALUE, 0) X(batch_norm2d_forward_f32, LAUNCH, 0) X(batch_norm2d_backward_f32, LAUNCH, 0) \
-  X(batch_norm2d_add_relu_forward_f32, LAUNCH, 0) X(batch_norm2d_add_relu_forward_masked_f32, LAUNCH, 0) \
+  X(batch_norm2d_relu_pool_forward_f32, LAUNCH, 0) X(batch_norm2d_relu_pool_backward_f32, LAUNCH, 0) X(batch_norm2d_add_relu_forward_f32, LAUNCH, 0) X(batch_norm2d_add_relu_forward_masked_f32, LAUNCH, 0) \
   X(batch_norm2d_add_relu_backward_masked_f32, LAUNCH, 0) X(batch_norm2d_add_relu_backward_f32, LAUNCH, 0) X(add_relu_f32, LAUNCH, 0) \
   X(add_relu_backward_f32, LAUNCH, 0) X(colsum_workspace_bytes, VALUE, 0) X(colsum_f32, LAUNCH, 0) X(colsum_noalloc_f32, LAUNCH, 0) \
   X(nhwc_spatial_sum_f32, LAUNCH, 0) X(nhwc_spatial_bcast_f32, LAUNCH, 0) X(sum_strided_f32, LAUNCH, HOST(3, 4, 6, 7)) \

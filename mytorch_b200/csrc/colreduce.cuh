@@ -66,3 +66,18 @@ __device__ __forceinline__ void vstore(float* p, const VecF<V>& r) {
   if (V == 4) *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1 % V], r.v[2 % V], r.v[3 % V]);
   else *p = r.v[0];
 }
+
+// n < 2^31 divided by a run-time constant: Granlund & Montgomery's round-up method.
+struct PoolDiv {
+  unsigned m, s, d;
+  PoolDiv() = default;
+  __host__ explicit PoolDiv(unsigned div) : m(0), s(0), d(div) {
+    while ((1ull << s) < d) ++s;
+    m = (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+  }
+  __device__ __forceinline__ unsigned divmod(unsigned n, unsigned& r) const {
+    const unsigned q = (unsigned)(((unsigned long long)__umulhi(n, m) + n) >> s);
+    r = n - q * d;
+    return q;
+  }
+};

@@ -115,24 +115,9 @@ __global__ void __launch_bounds__(256) maxpool2x2_fwd_kernel(const float4* __res
   }
 }
 
-// General windows of at most 16 elements, 4 channels per thread, 32-bit indices and a reciprocal instead of every division (n
-// < 2^31 divided by d: Granlund & Montgomery's round-up method).  A CTA takes 256 neighbouring float4 of one image row, so
+// General windows of at most 16 elements, 4 channels per thread, 32-bit indices and a reciprocal instead of every division (PoolDiv).  A CTA takes 256 neighbouring float4 of one image row, so
 // that what surrounds a window is still in L1.  Bound by HBM: 3x3/2 windows on 128 x 64 x 112x112 forward 240 -> 96 us,
 // backward 499 -> 204 us.
-struct PoolDiv {
-  unsigned m, s, d;
-  PoolDiv() = default;
-  __host__ explicit PoolDiv(unsigned div) : m(0), s(0), d(div) {
-    while ((1ull << s) < d) ++s;
-    m = (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
-  }
-  __device__ __forceinline__ unsigned divmod(unsigned n, unsigned& r) const {
-    const unsigned q = (unsigned)(((unsigned long long)__umulhi(n, m) + n) >> s);
-    r = n - q * d;
-    return q;
-  }
-};
-
 template <int KH, int KW, int SH, int SW>
 __global__ void __launch_bounds__(256) maxpool_fwd_vec_kernel(const float4* __restrict__ x, float4* __restrict__ y, uint2* __restrict__ mask, PoolDims d,
                                                                PoolDiv cv, PoolDiv ow_, PoolDiv oh_, unsigned total) {

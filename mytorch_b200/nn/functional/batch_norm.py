@@ -45,6 +45,31 @@ def _batch_norm2d_relu_backward(output_grad, mean, var, input, weight, bias, eps
     return dispatch(input.device, "batch_norm2d_relu_backward")(output_grad, mean, var, input, weight, bias, eps)
 
 
+def _batch_norm2d_relu_halved(input: Tensor, weight, bias, eps, training, momentum, running_mean, running_var):
+    """max_pool2d(relu(batch_norm2d(x)), 2, 2) as one operator on CUDA, None where it does not exist.  The reference runs three
+    (``mytorch/nn/batch_norm.py:123-135``, ``mytorch/nn/relu.py:5-10``, ``mytorch/nn/max_pool.py:5-21``); here neither the normalised
+    tensor nor its gradient is stored."""
+    requires_grad = input.requires_grad
+    channels = input.shape[1]
+    if weight is not None and bias is not None:
+        ok = (input.dtype == weight.dtype == bias.dtype and input.device == weight.device == bias.device
+              and weight.shape == (channels,) and bias.shape == (channels,))
+        if not ok:
+            return None  # the separate operators say what is wrong
+        requires_grad = requires_grad or weight.requires_grad or bias.requires_grad
+    made = dispatch(input.device, "batch_norm2d_relu_halved")(input, weight, bias, eps, training, momentum, running_mean, running_var)
+    if made is None:
+        return None
+    out, mean, var = made
+    out.requires_grad = requires_grad and not tracker.no_grad
+    return record("batch_norm2d_relu_halved", [input, weight, bias, eps], out, [mean, var])
+
+
+@tracker.register_backward_function("batch_norm2d_relu_halved")
+def _batch_norm2d_relu_halved_backward(output_grad, mean, var, input, weight, bias, eps):
+    return dispatch(input.device, "batch_norm2d_relu_halved_backward")(output_grad, mean, var, input, weight, bias, eps)
+
+
 def _batch_norm2d_add_relu(input: Tensor, residual: Tensor, weight, bias, eps, training, momentum, running_mean, running_var):
     """relu(batch_norm2d(x) + residual) as one operator: the tail of a residual block.  The reference runs
     three operators (``mytorch/nn/batch_norm.py:123-135``, ``mytorch/tensor.py:292-300``,

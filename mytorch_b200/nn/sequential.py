@@ -1,6 +1,6 @@
 from mytorch_b200.nn.batch_norm import BatchNorm2d, BatchNormReLU2d, inference_conv_norm
 from mytorch_b200.nn.conv import Conv2d
-from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu
+from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu, _batch_norm2d_relu_halved
 from mytorch_b200.nn.functional.linear import _linear_relu
 from mytorch_b200.nn.linear import Linear
 from mytorch_b200.nn.max_pool import MaxPool2d
@@ -17,8 +17,9 @@ def _halves(layer):
 
 class Sequential(Module):
     """Layers one after the other.  Neighbours that exist as one operator with the same bits run as one on CUDA: BatchNorm2d +
-    ReLU, Linear + ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU (+ MaxPool2d)) with running statistics.  A step of the
-    MNIST example is 300 library calls of a few microseconds each, so every operator left out shows."""
+    ReLU (+ MaxPool2d(2, 2)), Linear + ReLU, and, where nothing is differentiated, Conv2d + BatchNorm2d (+ ReLU (+ MaxPool2d(2, 2)))
+    with running statistics.  A step of the MNIST example is 300 library calls of a few microseconds each, so every operator left
+    out shows."""
 
     def __init__(self, *args):
         super().__init__()
@@ -47,6 +48,13 @@ class Sequential(Module):
                     i += 3 if relu else 2
                     continue
             if kind is BatchNorm2d and kind_after is ReLU and input.device.type == "cuda" and not (layer._forward_replaced or after._forward_replaced):
+                if _halves(layers[i + 2]):
+                    y = _batch_norm2d_relu_halved(input, layer.weight, layer.bias, layer.eps, layer.training, layer.momentum, layer.running_mean,
+                                                  layer.running_var)
+                    if y is not None:
+                        input = y
+                        i += 3
+                        continue
                 input = _batch_norm2d_relu(input, layer.weight, layer.bias, layer.eps, layer.training, layer.momentum, layer.running_mean,
                                            layer.running_var)
                 i += 2
