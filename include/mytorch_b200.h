@@ -162,9 +162,9 @@ int mtb_batch_norm2d_forward_f32(int n, int c, int h, int w, const float* x, con
 int mtb_batch_norm2d_forward_prestats_f32(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps,
                                           double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
                                           int relu, const float* stats, int stats_rows, void* workspace, long long workspace_bytes, void* stream);
-/* BatchNorm, ReLU and a 2 x 2 max-pool of stride 2 (mytorch/nn/batch_norm.py:123-135, relu.py:5-10, max_pool.py:5-21) as one operator; y [N,H/2,W/2,C] and
- * its tie mask; c % 4 == 0, 16-byte aligned tensors, fewer than 2^29 elements.  The same bits as the operators one by one. */
-int mtb_batch_norm2d_relu_pool_forward_f32(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps, int training,
+/* BatchNorm, ReLU and a max-pool of stride 2 (mytorch/nn/batch_norm.py:123-135, relu.py:5-10, max_pool.py:5-21) as one operator, window 2: 2 x 2, 3: 3 x 3 with
+ * padding 1 (backward: 2 x 2); y [N,OH,OW,C] and its tie mask; c % 4 == 0, 16-byte aligned tensors, fewer than 2^29 elements.  The same bits as the operators one by one. */
+int mtb_batch_norm2d_relu_pool_forward_f32(int n, int c, int h, int w, int window, const float* x, const float* gamma, const float* beta, double eps, int training,
                                            double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
                                            unsigned short* tiemask, const float* stats, int stats_rows, void* workspace, long long workspace_bytes, void* stream);
 int mtb_batch_norm2d_relu_pool_backward_f32(int n, int c, int h, int w, const float* dy, const float* mean, const float* var, const float* x,

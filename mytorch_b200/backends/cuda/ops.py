@@ -533,28 +533,32 @@ def cuda_batch_norm2d_relu_backward(output_grad, mean, var, x, weight, bias, eps
 
 
 @_reg("cuda", "batch_norm2d_relu_halved")
-def cuda_batch_norm2d_relu_halved(x, weight, bias, eps, training, momentum, running_mean, running_var):
-    """BatchNorm2d, ReLU and a 2x2 max-pool of stride 2: (y, mean, var), or None where the channels are no fours, no window fits or a tensor
-    starts off 16 bytes.  Same bits as the three operators."""
+def cuda_batch_norm2d_relu_halved(x, weight, bias, eps, training, momentum, running_mean, running_var, window=2):
+    """BatchNorm2d, ReLU and a max-pool of stride 2 (2x2, or 3x3 with padding 1: ``window``): (y, mean, var), or None where the
+    channels are no fours, no window fits or a tensor starts off 16 bytes.  Same bits as the three operators."""
     _f32(x, weight, bias, running_mean, running_var)
     n, c, h, w = x.shape
     if c % 4 or h < 2 or w < 2 or n * c * h * w >= 1 << 29 or not _aligned(x) or bias is not None and not _aligned(bias):
         return None
     env = _env(x)
-    y, mean, var = _new((n, c, h // 2, w // 2), x), _new((c,), x), _new((c,), x)
+    y, mean, var = _new((n, c, h // 2, w // 2) if window == 2 else (n, c, (h + 1) // 2, (w + 1) // 2), x), _new((c,), x), _new((c,), x)
     ws, ws_bytes = env.workspace(env.lib.batch_norm2d_workspace_bytes(n, c, h, w))
     use_batch_stats = bool(training) or running_mean is None or running_var is None
     pre = getattr(x, "_bn_partials", None) if use_batch_stats else None
     y._pool_tiemask = mean._pool_tiemask = mask = CudaMemory(x.device.index, y._native_array.nbytes // 2)
-    env.lib.batch_norm2d_relu_pool_forward_f32(n, c, h, w, x, weight, bias, float(eps), int(use_batch_stats), float(momentum), running_mean, running_var,
+    env.lib.batch_norm2d_relu_pool_forward_f32(n, c, h, w, window, x, weight, bias, float(eps), int(use_batch_stats), float(momentum), running_mean, running_var,
                                                y, mean, var, mask, pre[0] if pre else None, pre[1] if pre else 0, ws, ws_bytes, env.stream())
     return y, mean, var
 
 
 @_reg("cuda", "batch_norm2d_relu_halved_backward")
-def cuda_batch_norm2d_relu_halved_backward(output_grad, mean, var, x, weight, bias, eps):
+def cuda_batch_norm2d_relu_halved_backward(output_grad, mean, var, x, weight, bias, eps, window=2):
     env = _env(x)
     n, c, h, w = x.shape
+    if window == 3:
+        behind = _new(x.shape, x)
+        env.lib.max_pool2d_backward_f32(n, c, h, w, 3, 3, 2, 2, 1, 1, output_grad, mean._pool_tiemask, None, None, behind, env.stream())
+        return cuda_batch_norm2d_backward(behind, mean, var, x, weight, bias, eps, relu=True)
     dy, dx = output_grad, _new(x.shape, x)
     if not _aligned(dy):
         dy = _new(output_grad.shape, output_grad)

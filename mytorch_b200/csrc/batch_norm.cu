@@ -257,40 +257,57 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
   }
 }
 
-// y = max_pool(max(0, bn(x))) over 2 x 2 windows of stride 2, four channels of one window a thread, with the pool's tie mask (bit 2 * line + column of
-// every pixel that equals the maximum).  The normalised tensor is neither written nor read: S + S/4 instead of 3S + S/4
-// of traffic and a launch less, in backward the same.  The digit classifier's training step at 64 images, bound by the host: 60 launches -> 54,
-// 340 -> 316 us.
+// y = max_pool(max(0, bn(x))), four channels of one window a thread, with the pool's tie mask (bit WIN * line + column of every element that equals the
+// maximum).  WIN = 2: 2 x 2 windows of stride 2; 3: 3 x 3 windows of stride 2 with a border of one, whose values count as 0.  The normalised tensor is
+// neither written nor read (2 x 2: S + S/4 instead of 3S + S/4 of traffic), and a launch goes.  The digit classifier's training step at 64 images,
+// bound by the host, with the backward below: 60 launches -> 54, 340 -> 316 us.  64 channels of 128 x 112x112, 3 x 3: 233 -> 140 us.
+template <int WIN>
 __global__ void __launch_bounds__(256) bn_relu_pool_kernel(const float4* __restrict__ x, float4* __restrict__ y, uint2* __restrict__ mask, PoolDiv cv, PoolDiv ow_,
                                                             PoolDiv oh_, int H, int W, const float* __restrict__ mean, const float* __restrict__ scale,
                                                             const float* __restrict__ beta, unsigned total) {
   mtb_launch_dependents();
   mtb_wait_prior();
+  constexpr int PAD = WIN == 3 ? 1 : 0, N = WIN * WIN;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     unsigned cg, ow, oh;
     const unsigned n = oh_.divmod(ow_.divmod(cv.divmod(i, cg), ow), oh);
-    const float4* p = x + ((size_t)(n * H + 2 * oh) * W + 2 * ow) * cv.d + cg;
-    const float4 v[4] = {p[0], p[cv.d], p[(size_t)W * cv.d], p[(size_t)(W + 1) * cv.d]};
+    const int h0 = 2 * (int)oh - PAD, w0 = 2 * (int)ow - PAD;
+    float4 v[N];
+    bool in[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {  // all loads before the first comparison
+      const int h = h0 + k / WIN, w = w0 + k % WIN;
+      in[k] = PAD == 0 || ((unsigned)h < (unsigned)H && (unsigned)w < (unsigned)W);
+      if (in[k]) v[k] = __ldg(x + ((size_t)(n * H + h) * W + w) * cv.d + cg);
+    }
     const float4 mu = ld4(mean + 4 * cg), g = ld4(scale + 4 * cg), b = beta ? ld4(beta + 4 * cg) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 best;
-    unsigned ties[4];
-    auto one = [](float a, float b, float c, float d, float mu, float g, float beta, float& best, unsigned& m) {
-      a = fmaxf((a - mu) * g + beta, 0.f); b = fmaxf((b - mu) * g + beta, 0.f); c = fmaxf((c - mu) * g + beta, 0.f); d = fmaxf((d - mu) * g + beta, 0.f);
-      best = fmaxf(fmaxf(a, b), fmaxf(c, d));
-      m = (a == best ? 1u : 0u) | (b == best ? 2u : 0u) | (c == best ? 4u : 0u) | (d == best ? 8u : 0u);
-    };
-    one(v[0].x, v[1].x, v[2].x, v[3].x, mu.x, g.x, b.x, best.x, ties[0]);
-    one(v[0].y, v[1].y, v[2].y, v[3].y, mu.y, g.y, b.y, best.y, ties[1]);
-    one(v[0].z, v[1].z, v[2].z, v[3].z, mu.z, g.z, b.z, best.z, ties[2]);
-    one(v[0].w, v[1].w, v[2].w, v[3].w, mu.w, g.w, b.w, best.w, ties[3]);
+    float4 best = make_float4(0.f, 0.f, 0.f, 0.f);  // nothing behind a ReLU is less
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if (in[k]) {
+        v[k].x = fmaxf((v[k].x - mu.x) * g.x + b.x, 0.f); v[k].y = fmaxf((v[k].y - mu.y) * g.y + b.y, 0.f);
+        v[k].z = fmaxf((v[k].z - mu.z) * g.z + b.z, 0.f); v[k].w = fmaxf((v[k].w - mu.w) * g.w + b.w, 0.f);
+      } else {
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      best.x = fmaxf(best.x, v[k].x); best.y = fmaxf(best.y, v[k].y); best.z = fmaxf(best.z, v[k].z); best.w = fmaxf(best.w, v[k].w);
+    }
+    unsigned m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      m0 |= (v[k].x == best.x ? 1u : 0u) << k; m1 |= (v[k].y == best.y ? 1u : 0u) << k;
+      m2 |= (v[k].z == best.z ? 1u : 0u) << k; m3 |= (v[k].w == best.w ? 1u : 0u) << k;
+    }
     y[i] = best;
-    mask[i] = make_uint2(ties[0] | (ties[1] << 16), ties[2] | (ties[3] << 16));
+    mask[i] = make_uint2(m0 | (m1 << 16), m2 | (m3 << 16));
   }
 }
 
 // ---------------------------------------------------------------- backward
 
-// MODE 4: MODE 1 whose upstream gradient goes through the pool above first: dy and the tie mask have the shape of its result.
+// MODE 4: MODE 1 whose upstream gradient goes through a 2 x 2 max-pool of stride 2 first: dy and the tie mask have the shape of its result.  (For
+// 3 x 3 windows, up to four a pixel, both passes then wait for their windows: 64 channels of 128 x 112x112 380 and 503 us, against 102 for the
+// pool's own backward and 316 for two passes over what it writes.)
 struct PooledGradient {
   const unsigned short* mask;
   PoolDiv w, h;
@@ -542,11 +559,14 @@ int launch_normalize(const float* x, float* y, long long rows, int c, bool align
   return MTB_OK;
 }
 
+// What 2 x 2 windows of stride 2, and 3 x 3 ones with a border of one, leave of an extent.
+int pooled_extent(int size, int window) { return window == 2 ? size / 2 : (size + 1) / 2; }
+
 // mode 0: y = bn(x); 1: y = max(0, bn(x)); 2: y = max(0, bn(x) + res).  stats / stats_rows: batch statistics
 // prepared by the producer of x as partial rows (see mtb_conv2d_forward_stats_f32); 0 rows = compute them here.
 int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps, int training, double momentum,
                float* running_mean, float* running_var, float* y, float* mean, float* var, int mode, const float* res, unsigned char* mask,
-               const float* stats, int stats_rows, void* workspace, long long workspace_bytes, cudaStream_t st, unsigned short* ties = nullptr) {
+               const float* stats, int stats_rows, void* workspace, long long workspace_bytes, cudaStream_t st, unsigned short* ties = nullptr, int window = 0) {
   const MtbScratchTurn turn;
   MTB_REQUIRE(n > 0 && c > 0 && h > 0 && w > 0 && x && y && mean && var && workspace, "batch_norm2d_forward: bad arguments");
   MTB_REQUIRE(workspace_bytes >= mtb_batch_norm2d_workspace_bytes(n, c, h, w), "batch_norm2d_forward: workspace too small");
@@ -576,9 +596,13 @@ int bn_forward(int n, int c, int h, int w, const float* x, const float* gamma, c
     MTB_LAUNCH_CHECK("bn_eval_prep_kernel");
   }
   if (ties) {
-    const unsigned total = (unsigned)((long long)n * (h / 2) * (w / 2) * (c / 4));
-    MTB_LAUNCH(bn_relu_pool_kernel, mtb_stream_grid(total, 256), 256, 0, st, (const float4*)x, (float4*)y, (uint2*)ties, PoolDiv(c / 4), PoolDiv(w / 2), PoolDiv(h / 2),
-               h, w, mean, scale, beta, total);
+    const int oh = pooled_extent(h, window), ow = pooled_extent(w, window);
+    const unsigned total = (unsigned)((long long)n * oh * ow * (c / 4));
+    const int grid = mtb_stream_grid(total, 256);
+#define MTB_BN_POOL(W_) \
+  MTB_LAUNCH(bn_relu_pool_kernel<W_>, grid, 256, 0, st, (const float4*)x, (float4*)y, (uint2*)ties, PoolDiv(c / 4), PoolDiv(ow), PoolDiv(oh), h, w, mean, scale, beta, total)
+    if (window == 2) MTB_BN_POOL(2); else MTB_BN_POOL(3);
+#undef MTB_BN_POOL
     MTB_LAUNCH_CHECK("bn_relu_pool_kernel");
     return MTB_OK;
   }
@@ -722,25 +746,31 @@ MTB_API int mtb_batch_norm2d_add_relu_backward_masked_f32(int n, int c, int h, i
                      (cudaStream_t)stream);
 }
 
-// BatchNorm, ReLU and a 2 x 2 max-pool of stride 2 as one operator: y [n, h/2, w/2, c] and its tie mask; the normalised tensor is never stored.  c a
-// multiple of 4, the tensors 16-byte aligned, fewer than 2^31 / 4 elements.  stats / stats_rows as above.  Same bits as the operators one by one.
-MTB_API int mtb_batch_norm2d_relu_pool_forward_f32(int n, int c, int h, int w, const float* x, const float* gamma, const float* beta, double eps, int training,
-                                                   double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
+namespace {
+bool poolable(int n, int c, int h, int w, int window, const void* a, const void* b, const unsigned short* ties) {
+  return ties && n > 0 && c > 0 && c % 4 == 0 && h > 1 && w > 1 && (window == 2 || window == 3) && mtb_aligned16(a) && mtb_aligned16(b) &&
+         (reinterpret_cast<uintptr_t>(ties) & 7u) == 0 && (long long)n * h * w * c < (1LL << 29);
+}
+}  // namespace
+
+// BatchNorm, ReLU and a max-pool of stride 2 as one operator (window 2: 2 x 2; 3: 3 x 3 with a border of one): y [n, oh, ow, c] and its tie mask; the
+// normalised tensor is never stored.  c a multiple of 4, h and w at least 2, the tensors 16-byte aligned, fewer than 2^29 elements.
+// stats / stats_rows as above.  Same bits as the operators one by one.
+MTB_API int mtb_batch_norm2d_relu_pool_forward_f32(int n, int c, int h, int w, int window, const float* x, const float* gamma, const float* beta, double eps,
+                                                   int training, double momentum, float* running_mean, float* running_var, float* y, float* mean, float* var,
                                                    unsigned short* tiemask, const float* stats, int stats_rows, void* workspace, long long workspace_bytes,
                                                    void* stream) {
-  MTB_REQUIRE(tiemask && n > 0 && c > 0 && c % 4 == 0 && h > 1 && w > 1 && mtb_aligned16(x) && mtb_aligned16(y) && (reinterpret_cast<uintptr_t>(tiemask) & 7u) == 0 &&
-                  mtb_aligned16(beta) && mtb_aligned16(mean) && mtb_aligned16(workspace) && (long long)n * h * w * c < (1LL << 29),
+  MTB_REQUIRE(poolable(n, c, h, w, window, x, y, tiemask) && mtb_aligned16(beta) && mtb_aligned16(mean) && mtb_aligned16(workspace),
               "batch_norm2d_relu_pool_forward: four channels, whole windows and 16-byte alignment are required");
   return bn_forward(n, c, h, w, x, gamma, beta, eps, training, momentum, running_mean, running_var, y, mean, var, 1, nullptr, nullptr, stats, stats_rows, workspace,
-                    workspace_bytes, (cudaStream_t)stream, tiemask);
+                    workspace_bytes, (cudaStream_t)stream, tiemask, window);
 }
 
-// Its backward: dy and tiemask have the shape of y.
+// Its backward for 2 x 2 windows: dy and tiemask have the shape of y.
 MTB_API int mtb_batch_norm2d_relu_pool_backward_f32(int n, int c, int h, int w, const float* dy, const float* mean, const float* var, const float* x,
                                                     const unsigned short* tiemask, const float* gamma, const float* beta, double eps, float* dx, float* dgamma,
                                                     float* dbeta, void* workspace, long long workspace_bytes, void* stream) {
-  MTB_REQUIRE(tiemask && n > 0 && c > 0 && c % 4 == 0 && h > 1 && w > 1 && mtb_aligned16(x) && mtb_aligned16(dx) && mtb_aligned16(dy) &&
-                  (reinterpret_cast<uintptr_t>(tiemask) & 7u) == 0 && (long long)n * h * w * c < (1LL << 29),
+  MTB_REQUIRE(poolable(n, c, h, w, 2, x, dx, tiemask) && mtb_aligned16(dy),
               "batch_norm2d_relu_pool_backward: four channels, whole windows and 16-byte alignment are required");
   return bn_backward(n, c, h, w, dy, mean, var, x, gamma, beta, eps, 1, nullptr, nullptr, dx, nullptr, dgamma, dbeta, workspace, workspace_bytes,
                      (cudaStream_t)stream, tiemask);

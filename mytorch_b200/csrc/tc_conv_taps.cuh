@@ -446,7 +446,7 @@ struct TapsPlan {
 // 14x14 14.3 and 14.3).
 TapsPlan taps_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout) {
   TapsPlan r{};
-  if (getenv("MTB_DISABLE_TAPCONV")) return r;
+  if (getenv("MTB_DISABLE_PAIRCONV") || getenv("MTB_DISABLE_ROWCONV") || getenv("MTB_ROWCONV_MIN_ITEMS")) return r;  // the latter ask for other kernels
   if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || kc % 32 || kc < 64 || kc > 32 * kTapsMaxChunks || nout % 16 || nout < 64)
     return r;
   r.Wp = w + 2;

@@ -8,6 +8,7 @@ initialisation consumes one random draw per weight / bias tensor in creation ord
 import mytorch_b200.nn as nn
 import mytorch_b200.nn.functional as F
 from mytorch_b200.nn.batch_norm import inference_conv_norm
+from mytorch_b200.nn.functional.batch_norm import _batch_norm2d_relu_halved
 
 
 class Flatten(nn.Module):
@@ -148,9 +149,19 @@ class ResNet50(nn.Module):
         self.fc = nn.Linear(cin, num_classes, device=device)
 
     def forward(self, x):
-        x = self.maxpool(_conv_norm(self.conv1, self.bn1, x))
+        x = self._stem(x)
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(x.mean(dim=(2, 3)))
+
+    def _stem(self, x):
+        """maxpool(bn1(conv1(x))), the layers behind the convolution as one operator in training."""
+        norm, pool = self.bn1, self.maxpool
+        if (norm.training and x.device.type == "cuda" and type(norm) is nn.BatchNormReLU2d and type(pool) is nn.MaxPool2d
+                and (pool.kernel_size, pool.stride, pool.padding) == ((3, 3), (2, 2), (1, 1)) and not (norm._forward_replaced or pool._forward_replaced)):
+            x = self.conv1(x)
+            y = _batch_norm2d_relu_halved(x, norm.weight, norm.bias, norm.eps, True, norm.momentum, norm.running_mean, norm.running_var, 3)
+            return pool(norm(x)) if y is None else y
+        return pool(_conv_norm(self.conv1, norm, x))
 
 
 def bn_relu_pool(channels, device="cpu"):

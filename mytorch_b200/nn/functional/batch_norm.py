@@ -45,8 +45,8 @@ def _batch_norm2d_relu_backward(output_grad, mean, var, input, weight, bias, eps
     return dispatch(input.device, "batch_norm2d_relu_backward")(output_grad, mean, var, input, weight, bias, eps)
 
 
-def _batch_norm2d_relu_halved(input: Tensor, weight, bias, eps, training, momentum, running_mean, running_var):
-    """max_pool2d(relu(batch_norm2d(x)), 2, 2) as one operator on CUDA, None where it does not exist.  The reference runs three
+def _batch_norm2d_relu_halved(input: Tensor, weight, bias, eps, training, momentum, running_mean, running_var, window=2):
+    """max_pool2d(relu(batch_norm2d(x)), 2, 2) (``window`` 3: max_pool2d(.., 3, 2, 1)) as one operator on CUDA, None where it does not exist.  The reference runs three
     (``mytorch/nn/batch_norm.py:123-135``, ``mytorch/nn/relu.py:5-10``, ``mytorch/nn/max_pool.py:5-21``); here neither the normalised
     tensor nor its gradient is stored."""
     requires_grad = input.requires_grad
@@ -57,17 +57,17 @@ def _batch_norm2d_relu_halved(input: Tensor, weight, bias, eps, training, moment
         if not ok:
             return None  # the separate operators say what is wrong
         requires_grad = requires_grad or weight.requires_grad or bias.requires_grad
-    made = dispatch(input.device, "batch_norm2d_relu_halved")(input, weight, bias, eps, training, momentum, running_mean, running_var)
+    made = dispatch(input.device, "batch_norm2d_relu_halved")(input, weight, bias, eps, training, momentum, running_mean, running_var, window)
     if made is None:
         return None
     out, mean, var = made
     out.requires_grad = requires_grad and not tracker.no_grad
-    return record("batch_norm2d_relu_halved", [input, weight, bias, eps], out, [mean, var])
+    return record("batch_norm2d_relu_halved", [input, weight, bias, eps, window], out, [mean, var])
 
 
 @tracker.register_backward_function("batch_norm2d_relu_halved")
-def _batch_norm2d_relu_halved_backward(output_grad, mean, var, input, weight, bias, eps):
-    return dispatch(input.device, "batch_norm2d_relu_halved_backward")(output_grad, mean, var, input, weight, bias, eps)
+def _batch_norm2d_relu_halved_backward(output_grad, mean, var, input, weight, bias, eps, window):
+    return dispatch(input.device, "batch_norm2d_relu_halved_backward")(output_grad, mean, var, input, weight, bias, eps, window)
 
 
 def _batch_norm2d_add_relu(input: Tensor, residual: Tensor, weight, bias, eps, training, momentum, running_mean, running_var):

@@ -1,4 +1,4 @@
-"""BatchNorm2d + ReLU + 2x2 max-pool as one operator: the very bits of the three, forward (with the tie mask) and backward; odd extents, whose last line
+"""BatchNorm2d + ReLU + max-pool of stride 2 (2x2, or 3x3 with padding 1) as one operator: the very bits of the three, forward (with the tie mask) and backward; odd extents, whose last line
 and column no window holds, ties, one to many column blocks, running statistics, gradients off 16 bytes, and the layers of a Sequential."""
 import numpy as np
 import pytest
@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,c,h,w,training", [(64, 32, 28, 28, True), (5, 128, 7, 7, True), (3, 4, 2, 3, True), (2, 1028, 5, 4, True), (7, 36, 9, 2, False), (1, 64, 33, 31, True)])
-def test_same_bits_as_the_three_operators(n, c, h, w, training):
+@pytest.mark.parametrize("window", [2, 3])
+def test_same_bits_as_the_three_operators(n, c, h, w, training, window):
     import gpu_util as g
     from mytorch_b200.backends.cuda.env import CudaMemory, CudaMemoryView
 
@@ -15,16 +16,16 @@ def test_same_bits_as_the_three_operators(n, c, h, w, training):
     x = np.round(rng.standard_normal((n, c, h, w)) * 4).astype(np.float32) / 4  # ties
     vec = lambda lo, hi: rng.uniform(lo, hi, c).astype(np.float32)
     gamma, beta, rm, rv = vec(0.5, 1.5), vec(-0.5, 0.5), vec(-1, 1), vec(0.5, 2)
-    dy = rng.standard_normal((n, c, h // 2, w // 2)).astype(np.float32)
-    pool = ((2, 2), (2, 2), (0, 0))
+    dy = rng.standard_normal((n, c, h // 2, w // 2) if window == 2 else (n, c, (h + 1) // 2, (w + 1) // 2)).astype(np.float32)
+    pool = ((window, window), (2, 2), (window - 2, window - 2))
 
     def stats():
         return g.dev(rm), g.dev(rv)
 
     xt, gt, bt, dyt = g.dev(x, True), g.dev(gamma, True), g.dev(beta, True), g.dev(dy)
     running = stats()
-    y, mean, var = g.op("batch_norm2d_relu_halved")(xt, gt, bt, 1e-5, training, 0.1, *running)
-    dx, dg, db = g.op("batch_norm2d_relu_halved_backward")(dyt, mean, var, xt, gt, bt, 1e-5)
+    y, mean, var = g.op("batch_norm2d_relu_halved")(xt, gt, bt, 1e-5, training, 0.1, *running, window)
+    dx, dg, db = g.op("batch_norm2d_relu_halved_backward")(dyt, mean, var, xt, gt, bt, 1e-5, window)
     separate = stats()
     a, mean0, var0 = g.op("batch_norm2d_relu")(xt, gt, bt, 1e-5, training, 0.1, *separate)
     y0 = g.op("max_pool2d")(a, *pool)
@@ -35,10 +36,10 @@ def test_same_bits_as_the_three_operators(n, c, h, w, training):
     count = y._native_array.nbytes // 4
     assert np.array_equal(y._pool_tiemask.read((count,), np.uint16), y0._pool_tiemask.read((count,), np.uint16))
     block = CudaMemory(0, dyt._native_array.nbytes + 16)
-    window = CudaMemoryView(block, 4, dyt._native_array.nbytes, 0)
-    window.copy_from(dyt._native_array, window.nbytes)
-    dyt._native_array = window
-    assert np.array_equal(g.host(g.op("batch_norm2d_relu_halved_backward")(dyt, mean, var, xt, gt, bt, 1e-5)[0]), g.host(dx0))
+    off = CudaMemoryView(block, 4, dyt._native_array.nbytes, 0)
+    off.copy_from(dyt._native_array, off.nbytes)
+    dyt._native_array = off
+    assert np.array_equal(g.host(g.op("batch_norm2d_relu_halved_backward")(dyt, mean, var, xt, gt, bt, 1e-5, window)[0]), g.host(dx0))
 
 
 def test_shapes_that_keep_three_operators():
