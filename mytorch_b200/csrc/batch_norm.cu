@@ -16,7 +16,9 @@ namespace {
 // starts there: the normalise pass walks back to front behind a convolution that wrote front to back, the backward's sums do so behind a data
 // gradient, and dx then front to back.  Single rows of a contiguous range a CTA -> groups, in these orders: ResNet-50 step at 128 images 18.50 -> 18.08 ms,
 // ResNet-18 at 512 5465 -> 5353 us (5406 without the turns), at 128 1882 -> 1851, at 64 (captured) 1270 -> 1246.  rows_per_block > 0: a CTA
-// takes that many rows one after the other; the sums do so up to 64 MB, which the L2 holds whole, and keep their order there.
+// takes that many rows one after the other; the sums do so up to 64 MB, which the L2 holds whole, and keep their order there, and channels that
+// are no fours do, whose backward passes are bound by their instructions and take row after row (207 channels on 69 x 17x17 with ReLU and pool, forward
+// and backward: 114.9 us, in groups 117.6).
 constexpr int kGroup = 4;
 struct RowWalk {
   long long r, last, step, limit;  // first row of the group, of the last group, from group to group; end of the rows
@@ -203,7 +205,7 @@ __global__ void bn_eval_prep_kernel(int C, const float* __restrict__ gamma, floa
 // With var != NULL (running statistics) `scale` holds gamma, or is NULL, and the scale is computed here.
 // MODE 0: y = bn(x); 1: y = max(0, bn(x)); 2: y = max(0, bn(x) + res) (res has the shape of x)
 template <int V, int MODE>
-__global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float* y, long long rows, int C, int L, const float* __restrict__ mean,
+__global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float* y, long long rows, int C, int L, long long rows_per_block, const float* __restrict__ mean,
                                                             const float* __restrict__ scale, const float* __restrict__ beta,
                                                             const float* __restrict__ res, const float* __restrict__ var, float eps,
                                                             unsigned char* __restrict__ mask) {
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
   // Four rows are loaded before the first is stored: x may be y (an update in place), so the compiler would not do it.  BatchNorm,
   // ReLU and pooling of 256 x 128 x 56 x 56, forward and backward: 1073 -> 1050 us; ResNet-18 step at 512 images 5.84 -> 5.78 ms.
   constexpr int AHEAD = kGroup;
-  RowWalk walk(rows, R, 0, true);
+  RowWalk walk(rows, R, rows_per_block, true);
   for (long long r; walk.next(r);) {
     r += rsub;
     const long long off = r * C + (long long)cg * V, step = (long long)R * C;
@@ -365,7 +367,31 @@ __global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __rest
     gs[i] = (active && gamma) ? gamma[cg * V + i] * rstd[i] : rstd[i];
     bt[i] = (active && beta) ? beta[cg * V + i] : 0.f;
   }
-  if (active) {
+  auto add = [&](const VecF<V>& g, const VecF<V>& f, const VecF<V>& a, unsigned negative) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      float gi = g.v[i];
+      if (MODE == 3) {
+        if (negative >> i & 1u) gi = 0.f;
+      } else if (MODE) {
+        float t = (f.v[i] - mu[i]) * gs[i] + bt[i];
+        if (MODE == 2) t = t + a.v[i];
+        if (t < 0.f) gi = 0.f;
+      }
+      a0[i] += gi;
+      a1[i] += gi * ((f.v[i] - mu[i]) * rstd[i]);
+    }
+  };
+  if (V == 1 && active) {  // see RowWalk
+    const long long r0 = blockIdx.y * rows_per_block, r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+#pragma unroll 4
+    for (long long r = r0 + rsub; r < r1; r += R) {
+      const long long off = r * C + cg;
+      VecF<V> a;
+      if (MODE == 2) a = vload<V>(res + off);
+      add(load_gradient<V, MODE>(dy, r, C, cg, pool), vload<V>(x + off), a, 0u);
+    }
+  } else if (active) {
     RowWalk walk(rows, R, rows_per_block, true);
     for (long long r0; walk.next(r0);) {
       r0 += rsub;
@@ -384,19 +410,7 @@ __global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __rest
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) {
         if (r0 + u * R >= walk.limit) break;
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          float gi = g[u].v[i];
-          if (MODE == 3) {
-            if (negative[u] >> i & 1u) gi = 0.f;
-          } else if (MODE) {
-            float t = (f[u].v[i] - mu[i]) * gs[i] + bt[i];
-            if (MODE == 2) t = t + a[u].v[i];
-            if (t < 0.f) gi = 0.f;
-          }
-          a0[i] += gi;
-          a1[i] += gi * ((f[u].v[i] - mu[i]) * rstd[i]);
-        }
+        add(g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
       }
     }
   }
@@ -467,7 +481,7 @@ __global__ void __launch_bounds__(1024) bn_bwd_final_kernel(const float* __restr
 // MODES 2 and 3 also write the masked upstream gradient, which is the gradient of the added tensor, to dres.
 template <int V, int MODE>
 __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx,
-                                                         long long rows, int C, int L,
+                                                         long long rows, int C, int L, long long rows_per_block,
                                                          const float* __restrict__ mean, const float* __restrict__ coef,
                                                          const float* __restrict__ beta, const float* __restrict__ res, float* __restrict__ dres,
                                                          const unsigned char* __restrict__ mask, const GradientSource<MODE> pool) {
@@ -487,6 +501,36 @@ __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict_
     k3[i] = coef[2 * C + cg * V + i];
     bt[i] = beta ? beta[cg * V + i] : 0.f;
   }
+  auto store = [&](long long off, VecF<V>& g, const VecF<V>& f, const VecF<V>& a, unsigned negative) {
+    VecF<V> m;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      float gi = g.v[i];
+      if (MODE == 3) {
+        if (negative >> i & 1u) gi = 0.f;
+      } else if (MODE) {
+        float t = (f.v[i] - mu[i]) * k1[i] + bt[i];  // k1 = gamma / sigma, the forward's scale
+        if (MODE == 2) t = t + a.v[i];
+        if (t < 0.f) gi = 0.f;
+      }
+      m.v[i] = gi;
+      g.v[i] = k1[i] * (gi - k2[i] - (f.v[i] - mu[i]) * k3[i]);
+    }
+    vstore<V>(dx + off, g);
+    if (MODE == 2 || MODE == 3) vstore<V>(dres + off, m);
+  };
+  if (V == 1) {  // see RowWalk
+    const long long r0 = blockIdx.y * rows_per_block, r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+#pragma unroll 4
+    for (long long r = r0 + rsub; r < r1; r += R) {
+      const long long off = r * C + cg;
+      VecF<V> a;
+      if (MODE == 2) a = vload<V>(res + off);
+      VecF<V> g = load_gradient<V, MODE>(dy, r, C, cg, pool);
+      store(off, g, vload<V>(x + off), a, 0u);
+    }
+    return;
+  }
   RowWalk walk(rows, R, 0, false);
   for (long long r0; walk.next(r0);) {
     r0 += rsub;
@@ -505,23 +549,7 @@ __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict_
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
       if (r0 + u * R >= walk.limit) break;
-      const long long off = (r0 + u * R) * C + (long long)cg * V;
-      VecF<V> m;
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        float gi = g[u].v[i];
-        if (MODE == 3) {
-          if (negative[u] >> i & 1u) gi = 0.f;
-        } else if (MODE) {
-          float t = (f[u].v[i] - mu[i]) * k1[i] + bt[i];  // k1 = gamma / sigma, the forward's scale
-          if (MODE == 2) t = t + a[u].v[i];
-          if (t < 0.f) gi = 0.f;
-        }
-        m.v[i] = gi;
-        g[u].v[i] = k1[i] * (gi - k2[i] - (f[u].v[i] - mu[i]) * k3[i]);
-      }
-      vstore<V>(dx + off, g[u]);
-      if (MODE == 2 || MODE == 3) vstore<V>(dres + off, m);
+      store((r0 + u * R) * C + (long long)cg * V, g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
     }
   }
 }
@@ -551,7 +579,7 @@ int launch_normalize(const float* x, float* y, long long rows, int c, bool align
                      unsigned char* mask = nullptr) {
   ColCfg s = stream_cfg(rows, c, aligned);
   dim3 grid(s.col_blocks, s.row_blocks);
-#define MTB_BN_NORM(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_normalize_kernel<V_, M_>, grid, dim3(256), 0, st, x, y, rows, c, s.lanes, mean, scale, beta, res, var, eps, mask))
+#define MTB_BN_NORM(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_normalize_kernel<V_, M_>, grid, dim3(256), 0, st, x, y, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, scale, beta, res, var, eps, mask))
   if (s.vec == 4) { if (mode == 2) MTB_BN_NORM(4, 2); else if (mode == 1) MTB_BN_NORM(4, 1); else MTB_BN_NORM(4, 0); }
   else { if (mode == 2) MTB_BN_NORM(1, 2); else if (mode == 1) MTB_BN_NORM(1, 1); else MTB_BN_NORM(1, 0); }
 #undef MTB_BN_NORM
@@ -629,11 +657,11 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
   ColCfg cfg = mtb_col_cfg(rows, c, aligned);
   dim3 grid(cfg.col_blocks, cfg.row_blocks);
 #define MTB_BN_PARTIAL(V_, M_) \
-  MTB_LAUNCH(bn_bwd_partial_kernel<V_, M_>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta, \
+  MTB_LAUNCH(bn_bwd_partial_kernel<V_, M_>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) || cfg.vec == 1 ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta, \
              partial, res, mask, GradientSource<M_>{})
   const PooledGradient pooled{ties, PoolDiv(w), PoolDiv(h), (unsigned)(w / 2), (unsigned)(h / 2)};
   if (ties)
-    MTB_LAUNCH(bn_bwd_partial_kernel<4, 4>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta,
+    MTB_LAUNCH(bn_bwd_partial_kernel<4, 4>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) || cfg.vec == 1 ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta,
                partial, res, mask, pooled);
   else if (cfg.vec == 4) { if (mode == 3) MTB_BN_PARTIAL(4, 3); else if (mode == 2) MTB_BN_PARTIAL(4, 2); else if (mode == 1) MTB_BN_PARTIAL(4, 1); else MTB_BN_PARTIAL(4, 0); }
   else { if (mode == 2) MTB_BN_PARTIAL(1, 2); else if (mode == 1) MTB_BN_PARTIAL(1, 1); else MTB_BN_PARTIAL(1, 0); }
@@ -644,9 +672,9 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
   MTB_LAUNCH_CHECK("bn_bwd_final_kernel");
   ColCfg s = stream_cfg(rows, c, aligned);
   dim3 g2(s.col_blocks, s.row_blocks);
-#define MTB_BN_DX(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<V_, M_>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, mean, coef, beta, res, dres, mask, GradientSource<M_>{}))
+#define MTB_BN_DX(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<V_, M_>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, coef, beta, res, dres, mask, GradientSource<M_>{}))
   if (ties)
-    MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<4, 4>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, mean, coef, beta, res, dres, mask, pooled));
+    MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<4, 4>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, coef, beta, res, dres, mask, pooled));
   else if (s.vec == 4) { if (mode == 3) MTB_BN_DX(4, 3); else if (mode == 2) MTB_BN_DX(4, 2); else if (mode == 1) MTB_BN_DX(4, 1); else MTB_BN_DX(4, 0); }
   else { if (mode == 2) MTB_BN_DX(1, 2); else if (mode == 1) MTB_BN_DX(1, 1); else MTB_BN_DX(1, 0); }
 #undef MTB_BN_DX
