@@ -83,12 +83,13 @@ int mtb_conv2d_forward_simt(int n, int cin, int h, int w, int kh, int kw, int sh
 }
 
 namespace {
-// Rows, tile and reduction slices of the product whose rows are the pixels of 2 x 2 windows; false: no window, or a tile that is not a
-// cluster's (large products, which have better kernels and a pooling pass of their own).
+// Rows of the product whose rows are the pixels of 2 x 2 windows, and the tile and reduction slices of the convolution by itself (all pixels: a last odd line
+// or column must not change the order of a sum); false: no window, or a tile that is not a cluster's (large products, which have better kernels
+// and a pooling pass of their own).
 bool pooled_choice(const ConvDims& d, long long& rows, Choice& c) {
   rows = 4LL * d.N * (d.OH / 2) * (d.OW / 2);
   if (rows == 0) return false;
-  c = choose(rows, d.Cout, (long long)d.KH * d.KW * d.Cin, 1, 1);
+  c = choose((long long)d.N * d.OH * d.OW, d.Cout, (long long)d.KH * d.KW * d.Cin, 1, 1);
   return tile_info(c.tile).cluster;
 }
 }  // namespace

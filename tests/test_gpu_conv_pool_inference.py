@@ -45,3 +45,9 @@ def test_sequential_takes_it_only_for_the_class_s_own_layers():
         want = g.host(net(x).detach())  # gradients wanted: layer by layer
         with mt.no_grad():
             assert np.array_equal(g.host(net(x)), want)
+
+
+# odd extents, where the pixels in windows alone would be priced for another split of the reduction than all pixels
+@pytest.mark.parametrize("n,cin,cout,h,w", [(1, 32, 128, 25, 25), (1, 32, 128, 21, 29), (1, 32, 96, 25, 31)])
+def test_split_of_the_reduction_follows_from_all_pixels(n, cin, cout, h, w):
+    test_same_bits_as_separate_operators(n, cin, cout, h, w, 3, 1, 1, True)
