@@ -115,8 +115,10 @@ int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
                               const float* running_var, double eps, const float* residual, int relu, float* y, void* workspace,
                               long long workspace_bytes, void* stream);
 /* Inference: the same with a ReLU and a 2 x 2 max-pool of stride 2 behind it (mytorch/nn/max_pool.py:5-21), y [N,OH/2,OW/2,Cout] and its tie mask,
- * where mtb_conv2d_bn_pool_takes answers 1 (small convolutions); the bits are those of the separate operators. */
+ * where mtb_conv2d_bn_pool_takes answers 1 (small convolutions); the bits are those of the separate operators.  ..._scratch_bytes: -1 where that is so,
+ * else the scratch that mtb_conv2d_bn_forward_f32 reads for this shape (0: none). */
 int mtb_conv2d_bn_pool_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
+long long mtb_conv2d_bn_pool_scratch_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout);
 int mtb_conv2d_bn_pool_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                                    const float* wt, const float* bias, const float* gamma, const float* beta, const float* running_mean,
                                    const float* running_var, double eps, float* y, unsigned short* mask, void* stream);

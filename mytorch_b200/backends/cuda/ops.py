@@ -209,11 +209,19 @@ _BIAS_BESIDE_BYTES = 16 << 20
 def _conv_operands(env, input, weight, stride, padding, packed=None):
     """(arguments, input, filter, output tensor) of a forward convolution, the operands in the form its kernel reads.
     ``packed``: a list that takes the input as it was packed, if it was."""
+    return _operands_of(env, input, weight, *_conv_form(input, weight, stride, padding), packed)
+
+
+def _conv_form(input, weight, stride, padding):
+    """(arguments, how the input is packed or None) of a forward convolution."""
+    a = _conv_args(input, weight, stride, padding)
+    return a, _stem_form(input.shape, weight.shape, stride, padding) if a[1] < _TC_CHANNELS else None
+
+
+def _operands_of(env, input, weight, a, form, packed=None):
     x, wt = input, weight
-    a = _conv_args(x, wt, stride, padding)
     n, cin, h, w, kh, kw, sh, sw, ph, pw, cout = a
     oh, ow = (h + 2 * ph - kh) // sh + 1, (w + 2 * pw - kw) // sw + 1
-    form = _stem_form(x.shape, wt.shape, stride, padding) if cin < _TC_CHANNELS else None
     if form is not None:
         a = form[1]
         x = _stem_input(env, input, form)
@@ -233,20 +241,42 @@ def cuda_conv2d_batch_norm(input, weight, bias, stride, padding, gamma, beta, ru
     _f32(input, weight, bias, gamma, beta, running_mean, running_var, residual)
     env = _env(input)
     if pool:
-        a = n, _, h, w, kh, kw, sh, sw, ph, pw, cout = _conv_args(input, weight, stride, padding)
-        # an image stem that is packed for the tensor cores is not a small convolution
-        if a[1] < _TC_CHANNELS and _stem_form(input.shape, weight.shape, stride, padding) is not None or not env.lib.conv2d_bn_pool_takes(*a):
+        a, form = _conv_form(input, weight, stride, padding)
+        if form is not None or not env.lib.conv2d_bn_pool_takes(*a):
             return None
-        out = _new((n, cout, ((h + 2 * ph - kh) // sh + 1) // 2, ((w + 2 * pw - kw) // sw + 1) // 2), input)
-        out._pool_tiemask = mask = CudaMemory(input.device.index, out._native_array.nbytes // 2)
-        env.lib.conv2d_bn_pool_forward_f32(*a, input, weight, bias, gamma, beta, running_mean, running_var, float(eps), out, mask, env.stream())
-        return out
+        return _conv_bn_pooled(env, a, input, weight, bias, gamma, beta, running_mean, running_var, eps)
     a, x, wt, out = _conv_operands(env, input, weight, stride, padding)
     if residual is not None and residual.shape != out.shape:
         raise MismatchShapesError([out.shape, residual.shape])
     ws, ws_bytes = env.workspace(env.lib.conv2d_workspace_bytes(*a))
     env.lib.conv2d_bn_forward_f32(*a, x, wt, bias, gamma, beta, running_mean, running_var, float(eps),
                                   residual, int(bool(relu)), out, ws, ws_bytes, env.stream())
+    return out
+
+
+@_reg("cuda", "conv2d_batch_norm_halved")
+def cuda_conv2d_batch_norm_halved(input, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps):
+    """Inference: relu(batch_norm2d(conv2d(input))) with running statistics in the convolution's launch, and a 2x2 max-pool of stride 2 in the same
+    launch where that exists: (result, whether the pool is in it)."""
+    _f32(input, weight, bias, gamma, beta, running_mean, running_var)
+    env = _env(input)
+    a, form = _conv_form(input, weight, stride, padding)
+    scratch = 0  # an image stem that is packed for the tensor cores is not a small convolution, and takes none
+    if form is None:
+        scratch = env.lib.conv2d_bn_pool_scratch_bytes(*a)
+        if scratch < 0:
+            return _conv_bn_pooled(env, a, input, weight, bias, gamma, beta, running_mean, running_var, eps), True
+    a, x, wt, out = _operands_of(env, input, weight, a, form)
+    ws, ws_bytes = env.workspace(scratch) if scratch else (None, 0)
+    env.lib.conv2d_bn_forward_f32(*a, x, wt, bias, gamma, beta, running_mean, running_var, float(eps), None, 1, out, ws, ws_bytes, env.stream())
+    return out, False
+
+
+def _conv_bn_pooled(env, a, input, weight, bias, gamma, beta, running_mean, running_var, eps):
+    n, _, h, w, kh, kw, sh, sw, ph, pw, cout = a
+    out = _new((n, cout, ((h + 2 * ph - kh) // sh + 1) // 2, ((w + 2 * pw - kw) // sw + 1) // 2), input)
+    out._pool_tiemask = mask = CudaMemory(input.device.index, out._native_array.nbytes // 2)
+    env.lib.conv2d_bn_pool_forward_f32(*a, input, weight, bias, gamma, beta, running_mean, running_var, float(eps), out, mask, env.stream())
     return out
 
 

@@ -120,12 +120,18 @@ MTB_API int mtb_conv2d_bn_forward_f32(int n, int cin, int h, int w, int kh, int 
 // Inference: y = max_pool(max(0, batch_norm(conv(x)))) over 2 x 2 windows of stride 2, in one launch, where mtb_conv2d_bn_pool_takes answers 1:
 // the convolutions that the small tiles of the CUDA-core family take (also on tensors off 16 bytes, so that the answer follows from
 // the shape alone).  The bits, and the tie mask, are those of the separate operators.
-MTB_API int mtb_conv2d_bn_pool_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
+// mtb_conv2d_bn_pool_scratch_bytes answers both questions of a forward pass in one call: -1 where the pool goes along, else the scratch that
+// mtb_conv2d_bn_forward_f32 reads (0: none).
+MTB_API long long mtb_conv2d_bn_pool_scratch_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   const float* al = reinterpret_cast<const float*>(uintptr_t(256));
   if (n <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0 || !mtb_window_fits(h, ph, kh) || !mtb_window_fits(w, pw, kw)) return 0;
-  if (mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, al, al, al)) return 0;
-  if (split_scratch_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0) > 0) return 0;
-  return mtb_conv2d_bn_pool_simt_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout) ? 1 : 0;
+  const long long scratch = split_scratch_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, 0);
+  if (scratch > 0 || mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, al, al, al)) return scratch;
+  return mtb_conv2d_bn_pool_simt_takes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout) ? -1 : 0;
+}
+
+MTB_API int mtb_conv2d_bn_pool_takes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
+  return mtb_conv2d_bn_pool_scratch_bytes(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout) < 0 ? 1 : 0;
 }
 
 MTB_API int mtb_conv2d_bn_pool_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,

@@ -75,7 +75,9 @@ class BatchNorm1d(BatchNorm2d):
 def inference_conv_norm(conv, norm, x, relu=False, residual=None, pool=False):
     """``norm(conv(x))``, then optionally ``+ residual``, then optionally ReLU, as one operator where that is possible: a
     convolution and a BatchNorm layer that normalises with its running statistics, on CUDA, with no gradient to record.
-    None elsewhere.  Same bits as the separate layers.  ``pool``: with the ReLU, and a 2x2 max-pool of stride 2 behind it."""
+    None elsewhere.  Same bits as the separate layers.  ``pool``: the ReLU and a 2x2 max-pool of stride 2 follow; then (result, whether the
+    pool is in it: small convolutions), which one pass of these checks and one operator decide (the digit classifier on 16 images, where
+    no pool is taken: 70.6 us; asked first, and started again where refused, 80.4)."""
     mean, device = norm.running_mean, x.device
     if norm.training or mean is None or device.type != "cuda":
         return None
@@ -92,7 +94,6 @@ def inference_conv_norm(conv, norm, x, relu=False, residual=None, pool=False):
             return None
     if gamma is None or beta is None:
         gamma = beta = None
-    convolve = dispatch(device, "conv2d_batch_norm")
     if pool:
-        return convolve(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, True, None, True)
-    return convolve(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, relu, residual)
+        return dispatch(device, "conv2d_batch_norm_halved")(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps)
+    return dispatch(device, "conv2d_batch_norm")(x, weight, bias, conv.stride, conv.padding, gamma, beta, mean, var, norm.eps, relu, residual)

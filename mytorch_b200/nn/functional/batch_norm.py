@@ -51,6 +51,8 @@ def _batch_norm2d_relu_halved(input: Tensor, weight, bias, eps, training, moment
     tensor nor its gradient is stored."""
     requires_grad = input.requires_grad
     channels = input.shape[1]
+    if channels % 4:
+        return None
     if weight is not None and bias is not None:
         ok = (input.dtype == weight.dtype == bias.dtype and input.device == weight.device == bias.device
               and weight.shape == (channels,) and bias.shape == (channels,))

@@ -35,17 +35,15 @@ class Sequential(Module):
             if kind is Conv2d and kind_after in _NORMS and not (after.training or layer._forward_replaced or after._forward_replaced):
                 behind = layers[i + 2]
                 relu = kind_after is BatchNorm2d and type(behind) is ReLU and not behind._forward_replaced
-                last = 3 if relu else 2
-                if (relu or kind_after is BatchNormReLU2d) and _halves(layers[i + last]):
-                    y = inference_conv_norm(layer, after, input, pool=True)
-                    if y is not None:
-                        input = y
-                        i += last + 1
-                        continue
-                y = inference_conv_norm(layer, after, input, relu or kind_after is BatchNormReLU2d)
+                step = 3 if relu else 2
+                relu = relu or kind_after is BatchNormReLU2d
+                pooled = relu and _halves(layers[i + step])
+                y = inference_conv_norm(layer, after, input, relu, None, pooled)
                 if y is not None:
+                    if pooled:
+                        y, pooled = y
                     input = y
-                    i += 3 if relu else 2
+                    i += step + pooled
                     continue
             if kind is BatchNorm2d and kind_after is ReLU and input.device.type == "cuda" and not (layer._forward_replaced or after._forward_replaced):
                 if _halves(layers[i + 2]):

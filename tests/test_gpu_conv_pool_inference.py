@@ -51,3 +51,24 @@ def test_sequential_takes_it_only_for_the_class_s_own_layers():
 @pytest.mark.parametrize("n,cin,cout,h,w", [(1, 32, 128, 25, 25), (1, 32, 128, 21, 29), (1, 32, 96, 25, 31)])
 def test_split_of_the_reduction_follows_from_all_pixels(n, cin, cout, h, w):
     test_same_bits_as_separate_operators(n, cin, cout, h, w, 3, 1, 1, True)
+
+
+@pytest.mark.parametrize("batch", [1, 2, 16])
+def test_one_operator_call_per_convolution(batch, monkeypatch):
+    """Whether a convolution's pool goes along is the operator's own decision: no second attempt, with its checks, behind a refused one."""
+    import gpu_util as g
+    import mytorch_b200 as mt
+    import mytorch_b200.nn.batch_norm as B
+    from mytorch_b200.examples.mnist import CNN
+
+    mt.manual_seed(7)
+    net = CNN()
+    net.to(g.DEV)
+    net.eval()
+    x = g.dev(np.random.default_rng(batch).standard_normal((batch, 1, 28, 28)).astype(np.float32))
+    want = g.host(net(x).detach())  # gradients wanted: layer by layer
+    calls, dispatch = [], B.dispatch
+    monkeypatch.setattr(B, "dispatch", lambda device, name: calls.append(name) or dispatch(device, name))
+    with mt.no_grad():
+        assert np.array_equal(g.host(net(x)), want)
+    assert len(calls) == 3
