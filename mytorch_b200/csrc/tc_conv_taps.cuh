@@ -456,9 +456,10 @@ struct TapsPlan {
 // 14x14 14.3 and 14.3).
 TapsPlan taps_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout) {
   TapsPlan r{};
-  if (getenv("MTB_DISABLE_PAIRCONV") || getenv("MTB_DISABLE_ROWCONV") || getenv("MTB_ROWCONV_MIN_ITEMS")) return r;  // the latter ask for other kernels
   if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || kc % 32 || kc < 64 || kc > 32 * kTapsMaxChunks || nout % 16 || nout < 64)
     return r;
+  // behind what most layers fail: a look at the environment takes longer than all of that
+  if (getenv("MTB_DISABLE_PAIRCONV") || getenv("MTB_DISABLE_ROWCONV") || getenv("MTB_ROWCONV_MIN_ITEMS")) return r;  // the latter ask for other kernels
   r.Wp = w + 2;
   r.Hv = h + 1;
   if (r.Wp > 256 || r.Wp < 6) return r;  // rows the copy engine takes; at most 32 of them in a stage

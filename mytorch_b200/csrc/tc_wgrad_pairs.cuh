@@ -207,8 +207,8 @@ struct WgradPairPlan {
 
 WgradPairPlan wgrad_pair_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   WgradPairPlan r{};
+  if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || cin != 64 || cout % 4 || cout <= 32 || cout > 64) return r;
   if (getenv("MTB_DISABLE_PAIRCONV") || getenv("MTB_DISABLE_ROWCONV") || getenv("MTB_DISABLE_ROWWGRAD")) return r;  // the latter ask for other kernels
-  if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || cin % 64 || cout % 4) return r;
   r.Wp = w + 2;
   r.Hv = h + 1;
   if (r.Wp > 256 || (long long)n * r.Hv * r.Wp > 0x7ff00000LL) return r;
