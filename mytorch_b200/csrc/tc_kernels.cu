@@ -1678,7 +1678,7 @@ long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, in
     if (b2 > bytes) bytes = b2;
   }
   const WgradPairPlan pq = wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
-  if (wgrad_pairs_pay(pq, cin, cout)) {
+  if (wgrad_pairs_pay(pq)) {
     const long long b2 = (long long)pq.splits * q.Kw * cout * 4 + 256;
     if (b2 > bytes) bytes = b2;
   }
@@ -1700,9 +1700,9 @@ int mtb_tc_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
                             const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream) {
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   const WgradPairPlan pq = wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
-  if (wgrad_pairs_pay(pq, cin, cout)) {
+  if (wgrad_pairs_pay(pq)) {
     MTB_REQUIRE(workspace && workspace_bytes >= (long long)pq.splits * kh * kw * cin * cout * 4, "conv2d_wgrad: workspace too small");
-    return run_wgrad_pairs(pq, n, cin, h, w, cout, x, dy, dw, (float*)workspace, (cudaStream_t)stream);
+    return run_wgrad_pairs(pq, n, h, w, cout, x, dy, dw, (float*)workspace, (cudaStream_t)stream);
   }
   const WgradRowsPlan rq = wgrad_rows_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
   if (wgrad_rows_pay(rq, cin, cout)) {

@@ -22,15 +22,16 @@ namespace {
 using namespace tc;
 
 constexpr int kWgPairStages = 4;
+constexpr int kWgPairCin = 64;              // input channels: two blocks, one a CTA
 constexpr uint32_t kWgPairLead = 8 * 128;  // zeros around the X panel, which shifted reads of positions without a gradient reach
 constexpr int kWgPairCols = 192;           // of one accumulator; at 256 lies the second
 
 struct WgradPairParams {
   int Wp, Hv, H, W, rows;          // rows: image rows a stage
-  int Cin, Cout, ci_groups;        // pairs of input channel blocks
-  int stages, groups_total, groups_per_split, splits;
+  int Cout;                        // 33 to 64
+  int stages, groups_total, groups_per_split;
   uint32_t x_bytes, stage_bytes;   // X panel with its zeros; X and dY
-  float* partial;                  // [splits][9 * Cin][Cout]
+  float* partial;                  // [splits][9 * 64][Cout]
 };
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -72,9 +73,8 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
   const uint32_t tmem_base = tmem_slot;
   volatile int* abort_ptr = &abort_flag;
 
-  const int pair = (int)(blockIdx.x >> 1);
-  const int split = pair % p.splits, channels = pair / p.splits;
-  const int ci0 = (channels % p.ci_groups) * 64 + (int)rank * 32, co0 = (channels / p.ci_groups) * 64;
+  const int split = (int)(blockIdx.x >> 1);
+  const int ch0 = (int)rank * 32;  // this CTA's block of input channels, and of output channels
   const int g0 = split * p.groups_per_split;
   const int g1 = g0 + p.groups_per_split < p.groups_total ? g0 + p.groups_per_split : p.groups_total;
 
@@ -101,8 +101,8 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
         const int v = g * p.rows + (is_x ? lane : lane - p.rows - 1);
         const int img = v >= 0 ? v / p.Hv : -1, hrow = v - img * p.Hv;  // separators and images outside [0, N): zeros
         const uint32_t st = smem_base + stage * p.stage_bytes, full = smem_u32(&bar_full[stage]) & 0xFEFFFFFFu;
-        if (is_x) tma_load_4d_pair(st + kWgPairLead + (uint32_t)lane * row_bytes, &mapX, full, ci0, -1, hrow, img);
-        else tma_load_4d_pair(st + p.x_bytes + (uint32_t)(lane - p.rows) * row_bytes, &mapDY, full, co0 + (int)rank * 32, -1, hrow, img);
+        if (is_x) tma_load_4d_pair(st + kWgPairLead + (uint32_t)lane * row_bytes, &mapX, full, ch0, -1, hrow, img);
+        else tma_load_4d_pair(st + p.x_bytes + (uint32_t)(lane - p.rows) * row_bytes, &mapDY, full, ch0, -1, hrow, img);
       }
       ++filled;
       if (++stage == ST) { stage = 0; phase ^= 1u; }
@@ -152,12 +152,12 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
     const int quarter = warp & 3, half = (warp - 2) >> 2;  // tap kw; block of 32 output channels
     bool ok = lane != 0 || mbar_wait(smem_u32(&bar_tfull), 0, abort_ptr, 44);
     ok = __all_sync(0xffffffffu, ok);
-    const int c0 = co0 + 32 * half;
+    const int c0 = 32 * half;
     if (ok && quarter < 3 && c0 < p.Cout) {
       tc_fence_after();
       const bool vec_ok = (p.Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.partial) & 15u) == 0);
       const bool wide_ok = (p.Cout % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.partial) & 31u) == 0);
-      float* part = p.partial + (long long)split * 9 * p.Cin * p.Cout;
+      float* part = p.partial + (long long)split * 9 * kWgPairCin * p.Cout;
 #pragma unroll 1
       for (int j = 0; j < 3; ++j) {
         uint32_t r[32];
@@ -170,7 +170,7 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
 #pragma unroll
           for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) + __uint_as_float(t[k]));
         }
-        float* orow = part + ((long long)((2 - j) * 3 + quarter) * p.Cin + ci0 + lane) * p.Cout + c0;
+        float* orow = part + ((long long)((2 - j) * 3 + quarter) * kWgPairCin + ch0 + lane) * p.Cout + c0;
         if (vec_ok && c0 + 32 <= p.Cout) {
 #pragma unroll
           for (int k = 0; k < 32; k += 8)
@@ -201,13 +201,13 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
 
 struct WgradPairPlan {
   bool ok;
-  int Wp, Hv, rows, stages, ci_groups, co_groups, groups_total, groups_per_split, splits;
+  int Wp, Hv, rows, stages, groups_total, groups_per_split, splits;
   uint32_t x_bytes, stage_bytes, smem_bytes;
 };
 
 WgradPairPlan wgrad_pair_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   WgradPairPlan r{};
-  if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || cin != 64 || cout % 4 || cout <= 32 || cout > 64) return r;
+  if (kh != 3 || kw != 3 || sh != 1 || sw != 1 || ph != 1 || pw != 1 || cin != kWgPairCin || cout % 4 || cout <= 32 || cout > 64) return r;
   if (getenv("MTB_DISABLE_PAIRCONV") || getenv("MTB_DISABLE_ROWCONV") || getenv("MTB_DISABLE_ROWWGRAD")) return r;  // the latter ask for other kernels
   r.Wp = w + 2;
   r.Hv = h + 1;
@@ -223,11 +223,9 @@ WgradPairPlan wgrad_pair_plan(int n, int cin, int h, int w, int kh, int kw, int 
   r.stages = (int)(budget / r.stage_bytes);
   if (r.stages > kWgPairStages) r.stages = kWgPairStages;
   r.smem_bytes = 1024u + (uint32_t)r.stages * r.stage_bytes;
-  r.ci_groups = cin / 64;
-  r.co_groups = (cout + 63) / 64;
   const long long image_rows = (long long)n * r.Hv;
   r.groups_total = (int)((image_rows + r.rows - 1) / r.rows);
-  int splits = cluster_units(2) / 2 / (r.ci_groups * r.co_groups);
+  int splits = cluster_units(2) / 2;  // a pair each
   if (splits < 1) splits = 1;
   if (splits > r.groups_total) splits = r.groups_total;
   r.groups_per_split = (r.groups_total + splits - 1) / splits;
@@ -239,22 +237,22 @@ WgradPairPlan wgrad_pair_plan(int n, int cin, int h, int w, int kh, int kw, int 
 // Whether to take it where its layout fits.  Wider layers are near their best in the im2col kernel (128 -> 128 on 512 x 16x16 81 us and 85, on 128 x
 // 28x28 65 and 69).  Few positions a pair do not make up for its planes, one a pair: 1088 positions 27.7 us and 27.6, 840 23.6 and 25.6, 464
 // 19.5 and 21.4; 1624 37.9 and 31.8.
-bool wgrad_pairs_pay(const WgradPairPlan& r, int cin, int cout) {
-  return r.ok && cin == 64 && cout > 32 && cout <= 64 && r.groups_per_split * r.rows * r.Wp >= 1000;
+bool wgrad_pairs_pay(const WgradPairPlan& r) {
+  return r.ok && r.groups_per_split * r.rows * r.Wp >= 1000;
 }
 
-int run_wgrad_pairs(const WgradPairPlan& q, int n, int cin, int h, int w, int cout, const float* x, const float* dy, float* dw, float* partial, cudaStream_t st) {
+int run_wgrad_pairs(const WgradPairPlan& q, int n, int h, int w, int cout, const float* x, const float* dy, float* dw, float* partial, cudaStream_t st) {
   CUtensorMap mapX, mapDY;
-  if (int rc = tc::encode_rows_4d(&mapX, x, n, h, w, cin, 32, q.Wp, true)) return rc;
+  if (int rc = tc::encode_rows_4d(&mapX, x, n, h, w, kWgPairCin, 32, q.Wp, true)) return rc;
   if (int rc = tc::encode_rows_4d(&mapDY, dy, n, h, w, cout, 32, q.Wp, true)) return rc;
   WgradPairParams p{};
-  p.Wp = q.Wp; p.Hv = q.Hv; p.H = h; p.W = w; p.rows = q.rows; p.Cin = cin; p.Cout = cout; p.ci_groups = q.ci_groups;
-  p.stages = q.stages; p.groups_total = q.groups_total; p.groups_per_split = q.groups_per_split; p.splits = q.splits;
+  p.Wp = q.Wp; p.Hv = q.Hv; p.H = h; p.W = w; p.rows = q.rows; p.Cout = cout;
+  p.stages = q.stages; p.groups_total = q.groups_total; p.groups_per_split = q.groups_per_split;
   p.x_bytes = q.x_bytes; p.stage_bytes = q.stage_bytes; p.partial = partial;
   static unsigned long long configured = 0;
   if (int rc = mtb_opt_in_smem((const void*)tc_wgrad_pairs_kernel, (int)kTapsMaxSmem, &configured)) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * q.splits * q.ci_groups * q.co_groups);
+  cfg.gridDim = dim3(2 * q.splits);
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = q.smem_bytes;
   cfg.stream = st;
@@ -268,7 +266,7 @@ int run_wgrad_pairs(const WgradPairPlan& q, int n, int cin, int h, int w, int co
   cfg.numAttrs = 2;
   MTB_CUDA(cudaLaunchKernelEx(&cfg, tc_wgrad_pairs_kernel, mapX, mapDY, p));
   MTB_LAUNCH_CHECK("tc_wgrad_pairs_kernel");
-  const int Kw = 9 * cin;
+  const int Kw = 9 * kWgPairCin;
   dim3 rgrid((unsigned)((Kw + 3) / 4), (unsigned)((cout + 31) / 32));
   MTB_LAUNCH(wgrad_reduce_many_kernel, rgrid, dim3(32, 4, 8), 0, st, (const float*)partial, dw, Kw, cout, q.splits);
   MTB_LAUNCH_CHECK("wgrad_reduce_many_kernel");
