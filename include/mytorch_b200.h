@@ -139,8 +139,10 @@ int mtb_conv2d_dgrad_accumulates_in_place(int n, int cin, int h, int w, int kh, 
 /* Introspection, host code only (works without a GPU): which kernel family forward / dgrad / wgrad
  * would take for this shape and how the row-staged kernels lay out shared and tensor memory.
  * out: 25 ints, see the definition in csrc/tc_kernels.cu.  No counterpart in the reference. */
-int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* sizes); /* 18 ints */
 int mtb_conv2d_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out);
+/* The same for the kernel by pairs of SMs: its layout (18 ints), and whether forward and data gradient take it, with the prices (6 ints). */
+int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* sizes);
+int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* choice);
 /* dw[Cout,KH,KW,Cin]; needs mtb_conv2d_workspace_bytes() of workspace: split-K partials go there and are summed in a fixed order */
 int mtb_conv2d_wgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                          const float* dy, float* dw, void* workspace, long long workspace_bytes, void* stream);

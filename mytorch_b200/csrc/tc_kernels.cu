@@ -1078,12 +1078,41 @@ bool mtb_tc_conv2d_forward_supported(int n, int cin, int h, int w, int kh, int k
   return true;
 }
 
+namespace {
+// The kernel by pairs of SMs for a forward pass or (mn_major) a data gradient, and what the launch takes without it.  One price for all epilogues, without
+// the shared memory that some reserve in the other kernels: a layer's results are the same bits with every epilogue.
+struct PairChoice {
+  TapsPlan plan;
+  double other_ns;
+  bool taken;
+};
+PairChoice pair_choice(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int kc, int nout, bool mn_major) {
+  PairChoice r{taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, kc, nout), 0.0, false};
+  if (!r.plan.ok) return r;  // hence 3x3, stride 1, padding 1
+  const long long rows = (long long)n * h * w;
+  const int num_kb = 9 * (kc / 32), row_bn = pick_bn_for(nout, rows);
+  const RowConvPlan plan = row_conv_plan(n, h, w, kh, kw, sh, sw, ph, pw, kc, nout, row_bn);
+  const long long positions = (long long)n * plan.Hv * plan.Wp;
+  const GemmPlan gp = plan_gemm(nout, rows, num_kb, mn_major);
+  r.other_ns = row_conv_pays(plan, row_bn, positions, nout, num_kb, gp.ns) ? row_conv_ns(plan, row_bn, positions, nout, num_kb) : gp.ns;
+  r.taken = r.plan.ns <= r.other_ns;
+  return r;
+}
+}  // namespace
+
 // stats / stats_rows (both may be NULL): when given and the shape allows, the kernel also writes partial
 // rows [rows][3][cout] of per-channel (count, mean, M2) of y and *stats_rows receives their number;
 // *stats_rows == 0 means this launch did not produce statistics.
 int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* x,
                               const float* wt, const float* bias, float* y, int relu, void* workspace, long long workspace_bytes, void* stream,
                               float* stats, int* stats_rows, const MtbBnEval* bn_eval, const float* residual) {
+  if (stats_rows) *stats_rows = 0;
+  const PairChoice pairs = pair_choice(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout, false);
+  if (pairs.taken) {
+    const bool with_stats = stats && stats_rows && !relu && cout % 32 == 0 && !getenv("MTB_DISABLE_CONV_STATS");
+    if (with_stats) *stats_rows = taps_stats_rows(pairs.plan);
+    return run_taps<B_KMAJOR>(pairs.plan, n, h, w, cin, cout, x, wt, bias, residual, relu, y, (cudaStream_t)stream, with_stats ? stats : nullptr, bn_eval);
+  }
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   const long long M = (long long)n * oh * ow, K = (long long)kh * kw * cin;
   const int row_bn = pick_bn_for(cout, M);
@@ -1091,14 +1120,6 @@ int mtb_tc_conv2d_forward_f32(int n, int cin, int h, int w, int kh, int kw, int 
   const GemmPlan gp = plan_gemm(cout, M, (int)(K / 32), false);
   const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32), gp.ns);
   const int bn = staged ? row_bn : gp.bn;
-  if (stats_rows) *stats_rows = 0;
-  const TapsPlan taps = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, cin, cout);
-  if (taps.ok &&
-      taps.ns <= (staged ? row_conv_ns(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cout, (int)(K / 32)) : gp.ns)) {
-    const bool with_stats = stats && stats_rows && !relu && cout % 32 == 0 && !getenv("MTB_DISABLE_CONV_STATS");
-    if (with_stats) *stats_rows = taps_stats_rows(taps);
-    return run_taps<B_KMAJOR>(taps, n, h, w, cin, cout, x, wt, bias, residual, relu, y, (cudaStream_t)stream, with_stats ? stats : nullptr, bn_eval);
-  }
   // the statistics and BatchNorm epilogues keep a CTA on one column tile: there must be a CTA for each
   const bool a_cta_per_column = (cout + bn - 1) / bn <= mtb_sm_count();
   if (bn_eval && !a_cta_per_column) {
@@ -1180,6 +1201,10 @@ ClassAxis class_axis(int a, int size, int osize, int k, int s, int pad) {
 // other paths write dgrad and add afterwards.
 int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, const float* dy,
                             const float* wt, const float* addend, float* dx, void* workspace, long long workspace_bytes, void* stream) {
+  if (addend != dx) {
+    const PairChoice pairs = pair_choice(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin, true);
+    if (pairs.taken) return run_taps<B_MNMAJOR>(pairs.plan, n, h, w, cout, cin, dy, wt, nullptr, addend, 0, dx, (cudaStream_t)stream);
+  }
   const int oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   // one tile width for all residue classes (the weight tensor map is shared): the one the cost model picks
   // for a class-sized problem
@@ -1191,10 +1216,6 @@ int mtb_tc_conv2d_dgrad_f32(int n, int cin, int h, int w, int kh, int kw, int sh
   const bool staged = row_conv_pays(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb, class_plan.ns);
   const int bn = staged ? row_bn : class_plan.bn;
   cudaStream_t st = (cudaStream_t)stream;
-  const TapsPlan taps = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, cout, cin);
-  if (taps.ok && addend != dx &&
-      taps.ns <= (staged ? row_conv_ns(plan, row_bn, (long long)n * plan.Hv * plan.Wp, cin, class_kb) : class_plan.ns))
-    return run_taps<B_MNMAJOR>(taps, n, h, w, cout, cin, dy, wt, nullptr, addend, 0, dx, st);
   CUtensorMap mapB;
   const long long wcols = (long long)kh * kw * cin;
   const bool b_blocks = cin % 32 == 0;  // a tap's columns then are whole blocks
@@ -1587,32 +1608,6 @@ WgradPlan wgrad_plan(int n, int cin, int h, int w, int kh, int kw, int sh, int s
 
 }  // namespace
 
-// The same for the kernel that works in pairs of SMs (tc_conv_taps.cuh), which forward and data gradient take where its layout fits
-// and its price is lower.  out[0..8] forward, out[9..17] data gradient: form (1 or 2; 0: not taken), dynamic smem bytes, stage bytes, first and
-// (one past the) last byte written by the row copies, first and last byte read through a descriptor, image rows a stage, TMEM columns.
-MTB_API int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out) {
-  MTB_REQUIRE(out && n > 0 && cin > 0 && cout > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0, "conv2d_pair_plan: bad arguments");
-  for (int dir = 0; dir < 2; ++dir, out += 9) {
-    for (int i = 0; i < 9; ++i) out[i] = 0;
-    const int kc = dir ? cout : cin;
-    const TapsPlan q = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, kc, dir ? cin : cout);
-    if (!q.ok) continue;
-    out[0] = q.beside;
-    out[1] = (int)q.smem_bytes;
-    out[2] = (int)q.a_stage_bytes;
-    for (int col = 0; col < (q.rows ? 1 : q.Wp); ++col) {  // column of a tile's first position: whole rows start at 0
-      const int rows = q.rows ? q.rows + 2 : (col + 128) / q.Wp + 3, first = (q.origin - q.Wp - col) * 128, end = first + rows * q.Wp * 128;
-      if (col == 0 || first < out[3]) out[3] = first;
-      if (end > out[4]) out[4] = end;
-      if (rows > out[7]) out[7] = rows;
-    }
-    out[5] = (q.origin - q.Wp - (q.beside == 1 ? 1 : 0)) * 128;
-    out[6] = (q.origin + q.Wp + 127 + 1 + 1) * 128;
-    out[8] = kTapsBufs * q.beside * 64;
-  }
-  return MTB_OK;
-}
-
 // Which kernel family each of forward / data gradient / weight gradient can take for a shape: row-staged wherever
 // its layout fits (the launch then takes that or im2col, whichever is priced lower: row_conv_pays, wgrad_rows_pay)
 // (pointers assumed 16-byte aligned), and, for the row-staged kernels, how their shared and tensor
@@ -1664,6 +1659,48 @@ MTB_API int mtb_conv2d_plan_f32(int n, int cin, int h, int w, int kh, int kw, in
       out[23] = (int)(((q.Wp - 1) + (kWgRowsPB - 1) + 1) * 128);
       out[24] = kh * q.n_kwg * q.ncc_g * q.bn;
     }
+  }
+  return MTB_OK;
+}
+
+// How the kernel that works in pairs of SMs (tc_conv_taps.cuh) lays out a shape, wherever its layout fits (whether it is taken: mtb_conv2d_pair_choice_f32).
+// Host code only.  out[0..8] forward, out[9..17] data gradient: form (1 or 2; 0: does not fit), dynamic smem bytes, stage bytes, first and
+// (one past the) last byte written by the row copies, first and last byte read through a descriptor, image rows a stage, TMEM columns.
+MTB_API int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out) {
+  MTB_REQUIRE(out && n > 0 && cin > 0 && cout > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0, "conv2d_pair_plan: bad arguments");
+  for (int dir = 0; dir < 2; ++dir, out += 9) {
+    for (int i = 0; i < 9; ++i) out[i] = 0;
+    const int kc = dir ? cout : cin;
+    const TapsPlan q = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, kc, dir ? cin : cout);
+    if (!q.ok) continue;
+    out[0] = q.beside;
+    out[1] = (int)q.smem_bytes;
+    out[2] = (int)q.a_stage_bytes;
+    for (int col = 0; col < (q.rows ? 1 : q.Wp); ++col) {  // column of a tile's first position: whole rows start at 0
+      const int rows = q.rows ? q.rows + 2 : (col + 128) / q.Wp + 3, first = (q.origin - q.Wp - col) * 128, end = first + rows * q.Wp * 128;
+      if (col == 0 || first < out[3]) out[3] = first;
+      if (end > out[4]) out[4] = end;
+      if (rows > out[7]) out[7] = rows;
+    }
+    out[5] = (q.origin - q.Wp - (q.beside == 1 ? 1 : 0)) * 128;
+    out[6] = (q.origin + q.Wp + 127 + 1 + 1) * 128;
+    out[8] = kTapsBufs * q.beside * 64;
+  }
+  return MTB_OK;
+}
+
+// Whether forward and data gradient of a shape run by pairs of SMs (pointers assumed aligned, the gradient not in place), with the prices that decide.  Host code only.
+// out[0..2] forward, out[3..5] data gradient: taken, price in ns, price of the kernel that is taken otherwise.
+MTB_API int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out) {
+  MTB_REQUIRE(out && n > 0 && cin > 0 && cout > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0, "conv2d_pair_choice: bad arguments");
+  const float* al = reinterpret_cast<const float*>(uintptr_t(256));
+  for (int dir = 0; dir < 2; ++dir, out += 3) {
+    const PairChoice r = pair_choice(n, h, w, kh, kw, sh, sw, ph, pw, dir ? cout : cin, dir ? cin : cout, dir != 0);
+    const bool supported = dir ? mtb_tc_conv2d_dgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, al, al, al)
+                               : mtb_tc_conv2d_forward_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, al, al, al);
+    out[0] = r.taken && supported;
+    out[1] = (int)r.plan.ns;
+    out[2] = (int)r.other_ns;
   }
   return MTB_OK;
 }

@@ -60,3 +60,17 @@ def test_forward_and_data_gradient(n, cin, cout, h, w):
         window.copy_from(at._native_array, window.nbytes)
         at._native_array = window
         assert np.array_equal(g.host(g.op("conv2d_backward")(g.dev(dy), xt, wtt, None, s, p, accumulate_dx=at)[0]), dx + add)
+
+
+# 64 -> 64 on rows of 48 pixels: BatchNorm's coefficients leave the row-staged kernel no room for its whole filter, which must not decide between the kernels
+@pytest.mark.parametrize("n,h", [(1, 48), (2, 48), (4, 40), (4, 11)])
+def test_epilogue_does_not_choose_the_kernel(n, h):
+    import gpu_util as g
+
+    rng = np.random.default_rng(n + h)
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)
+    xt, wt, s, p = g.dev(f32(n, 64, h, 48)), g.dev(f32(64, 64, 3, 3)), (1, 1), (1, 1)
+    vec = lambda lo, hi: g.dev(rng.uniform(lo, hi, 64).astype(np.float32))
+    gamma, beta, m, v = vec(0.5, 1.5), vec(-1, 1), vec(-1, 1), vec(0.5, 2)
+    want = g.op("batch_norm2d")(g.op("conv2d")(xt, wt, None, s, p), gamma, beta, 1e-5, False, 0.1, m, v)[0]
+    assert np.array_equal(g.host(g.op("conv2d_batch_norm")(xt, wt, None, s, p, gamma, beta, m, v, 1e-5, False)), g.host(want))
