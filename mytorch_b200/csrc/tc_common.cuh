@@ -7,7 +7,6 @@
 // the kernel then tears down normally (TMEM is freed, the CTA exits).  Nothing traps.
 #pragma once
 #include "common.cuh"
-#include <cfloat>
 #include <cuda.h>
 
 // Status words of the tensor-core kernels (0 = fine).  One copy per translation unit that
@@ -381,11 +380,12 @@ struct LaneColSums {
   }
 };
 
-// The same for an epilogue with time to spare that stays on its 32 columns for many tiles: every lane runs Welford's update over its own rows, column by
-// column, on values from which the warp's first row has been taken (`pivot`, 32 floats of shared memory), and the lanes are merged with Chan's update
-// at the end.  Five operations a value and no exchange.  Neither a mean that is large against the spread nor a first row unlike the others costs
-// accuracy: relative error of the variance over 32 x 17 and 32 x 600 rows (mean^2 / variance 0 to 10^6, or first tile a thousand spreads away) 4e-8 and
-// 7e-8 (1.2e-7), against 7e-8 to 2.5e-6 and 4e-7 to 2e-6 of WarpColStats, and 7e-6, 7e-4 and 9e-2 of plain sums at ratios of 100, 10^4 and 10^6.
+// The same for an epilogue that stays on its 32 columns for many tiles: every lane runs Welford's update over its own rows, column by column (four operations a
+// value, two columns an instruction, no exchange), and the lanes are merged with Chan's update at the end.  Neither a mean that is large against the
+// spread nor first rows unlike the others cost accuracy.  Relative error of the variance over 32 x 17, 62 and 600 rows at mean^2 / variance of 0 to 100: 4e-8 to
+// 8e-8 (WarpColStats 7e-8 to 4e-7, plain sums 8e-6 and more at 100), at 10^4 and 10^6 5e-7 and 4e-6 (3e-7 to 5e-7 and 3e-6; 1e-3 and 1e-1), with a first tile a thousand spreads
+// away 8e-8 at most.  64 -> 64 on 50 x 7x6, one tile a CTA, and on 512 x 32x32: 8.35 us and 72.6, with plain sums 8.1 and 72.0.  (A merge by two
+// rounds of warp_transpose_sum takes 0.1 us more, one through shared memory 0.6, a first row taken from all values 1.0.)
 struct LaneColMoments {
   float cnt, inv;
   unsigned long long mean[16], m2[16];  // two columns each: one instruction updates both, with the rounding of two
@@ -412,39 +412,39 @@ struct LaneColMoments {
     inv = 1.f / cnt;
   }
   // columns c0 .. c0 + 15 (compile-time after unrolling) of the row that next_row() has counted
-  __device__ __forceinline__ void add(int c0, const float (&o)[16], const float* pivot) {
+  __device__ __forceinline__ void add(int c0, const float (&o)[16]) {
     const unsigned long long minus = pack(-1.f, -1.f), part = pack(inv, inv);
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) {
-      const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(pivot + c0 + j);
-#pragma unroll
-      for (int k = 0; k < 4; k += 2) {
-        const int c = (c0 + j + k) / 2;
-        const unsigned long long v = fma(k ? p.y : p.x, minus, pack(o[j + k], o[j + k + 1])), d = fma(mean[c], minus, v);
-        mean[c] = fma(d, part, mean[c]);
-        m2[c] = fma(d, fma(mean[c], minus, v), m2[c]);
-      }
+    for (int j = 0; j < 16; j += 2) {
+      const int c = (c0 + j) / 2;
+      const unsigned long long v = pack(o[j], o[j + 1]), d = fma(mean[c], minus, v);
+      mean[c] = fma(d, part, mean[c]);
+      m2[c] = fma(d, fma(mean[c], minus, v), m2[c]);
     }
   }
-  // one partial row [3][C] (count, mean, M2); bias (may be NULL) is added back to the mean
-  __device__ __forceinline__ void store(float* row, int C, int col0, int ncols, const float* pivot, const float* bias, int lane) {
-    float n = cnt, t[32];
+  // One partial row [3][C] (count, mean, M2); bias (may be NULL) is added back to the mean.  The exchanges are those of warp_transpose_sum.
+  __device__ __forceinline__ void store(float* row, int C, int col0, int ncols, const float* bias, int lane) const {
+    float n = cnt, m[32], q[32];
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
+    for (int k = 0; k < 32; ++k) { m[k] = at(mean, k); q[k] = at(m2, k); }
 #pragma unroll
-    for (int k = 0; k < 32; ++k) t[k] = cnt * at(mean, k);
-    const float sum = warp_transpose_sum(t, lane), mu = n > 0.f ? sum / n : 0.f;
+    for (int half = 16; half >= 1; half >>= 1) {
+      const bool upper = (lane & half) != 0;
+      const float nb = __shfl_xor_sync(0xffffffffu, n, half), both = n + nb, wb = both > 0.f ? __fdividef(nb, both) : 0.f, w = n * wb;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const float d = at(mean, k) - __shfl_sync(0xffffffffu, mu, k);
-      t[k] = fmaf(cnt * d, d, at(m2, k));
+      for (int k = 0; k < half; ++k) {
+        const float ma = upper ? m[k + half] : m[k], d = __shfl_xor_sync(0xffffffffu, upper ? m[k] : m[k + half], half) - ma;
+        const float qa = upper ? q[k + half] : q[k], qb = __shfl_xor_sync(0xffffffffu, upper ? q[k] : q[k + half], half);
+        m[k] = fmaf(d, wb, ma);
+        q[k] = fmaf(d * d, w, qa + qb);
+      }
+      n = both;
     }
-    const float q = warp_transpose_sum(t, lane);
     const int col = col0 + lane;
     if (col < ncols) {
       row[col] = n;
-      row[C + col] = n > 0.f ? (pivot[lane] + mu) + (bias ? bias[col] : 0.f) : 0.f;
-      row[2 * C + col] = q;
+      row[C + col] = m[0] + (bias ? bias[col] : 0.f);
+      row[2 * C + col] = q[0];
     }
   }
 };

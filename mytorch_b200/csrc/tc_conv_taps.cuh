@@ -136,7 +136,6 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   constexpr int BN = 64, DN = BESIDE * BN;  // output channels, accumulator columns
   extern __shared__ uint8_t smem_raw[];
   __shared__ alignas(16) BnColumns<BNORM ? BN : 4> bn_columns;
-  __shared__ alignas(16) float pivot[STATS ? 8 : 1][32];  // per epilogue warp, see LaneColMoments
   __shared__ alignas(16) float edge[2][2][4][32];  // what the next epilogue warp's first lane needs of this one's last (by half of the columns, tile parity)
   __shared__ uint64_t bar_afull[kTapsMaxStages], bar_aempty[kTapsMaxStages], bar_bfull[kTapsMaxChunks], bar_tfull[kTapsBufs], bar_tempty[kTapsBufs];
   __shared__ uint32_t tmem_slot;
@@ -291,8 +290,6 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     const int quarter = warp & 3, half = (warp - 2) >> 2, h0 = 32 * half;
     LaneColMoments moments;
     if constexpr (STATS) moments.reset();
-    float* const from = pivot[STATS ? warp - 2 : 0];
-    bool has_pivot = false;
     const int row = quarter * 32 + lane;
     const bool wide = (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0;                                   // 32-byte stores and loads;
     const uintptr_t add_low = p.addend ? reinterpret_cast<uintptr_t>(p.addend) & 31u : 0u;             // 16-byte ones, or single values
@@ -367,9 +364,7 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         }
         __syncwarp();
       }
-      unsigned rows_here = 0;
       if constexpr (STATS) {
-        rows_here = has_pivot ? 0u : __ballot_sync(0xffffffffu, valid);
         if (valid) moments.next_row();
       }
 #pragma unroll
@@ -381,17 +376,8 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
           if constexpr (BESIDE == 2) o[j] += __uint_as_float(__shfl_sync(0xffffffffu, side[16 * c + j], lane + 31));
         }
         const int c0 = 16 * c;
-        if constexpr (STATS) {
-          if (rows_here) {  // the warp's first row with an output
-            if (lane == __ffs(rows_here) - 1) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) from[c0 + j] = fabsf(o[j]) <= FLT_MAX ? o[j] : 0.f;
-            }
-            __syncwarp();
-          }
-        }
         if (valid && n0 + h0 + c0 < p.N) {
-          if constexpr (STATS) moments.add(c0, o, from);  // of the raw accumulator
+          if constexpr (STATS) moments.add(c0, o);  // of the raw accumulator
           if (p.bias) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) o[j] += __ldg(p.bias + n0 + h0 + c0 + j);
@@ -415,7 +401,6 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             st_row8(p.out + ooff + c0 + j, make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]), make_float4(o[j + 4], o[j + 5], o[j + 6], o[j + 7]), wide);
         }
       }
-      has_pivot = has_pivot || rows_here;
       valid = next_valid;
       ooff = next_off;
       if constexpr (!STATS) {
@@ -425,7 +410,7 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     }
     if constexpr (STATS) {
       float* srow = p.stats + (((long long)first * 2 + rank) * 4 + quarter) * 3 * p.N;
-      moments.store(srow, p.N, n0 + h0, p.N, from, p.bias, lane);
+      moments.store(srow, p.N, n0 + h0, p.N, p.bias, lane);
     }
   }
 
