@@ -478,8 +478,10 @@ TapsPlan taps_plan(int n, int h, int w, int kh, int kw, int sh, int sw, int ph, 
   r.pairs = (int)(items < most ? items : most) / r.n_tiles * r.n_tiles;
   const int per = r.pairs / r.n_tiles;
   const int waves = (r.m_items + per - 1) / per;
-  // Fitted to 31 shapes timed beside the other kernels: a stage takes 860 ns, with 3 us around them.  128 -> 128 on 16x16: 32 images 16.5 us
-  // (im2col kernel 16.4, data gradient 18.3), 64 images 20.5 (20.4), 100 images 24.6 (37).
+  // A price to hold against the other kernels' prices, not a time: launches take 6 us and 0.9 (two taps beside each other: 0.75) to 1.1 us a stage, the other
+  // kernels 2 to 3 us more than their prices, and more yet where those are high.  Of 207 shapes of 1 to 34 waves the forward pass so takes this kernel where it
+  // is over 3 % slower 6 times plain (two waves of 64 channels, 9.7 us against 8.9; 9 % at most), 28 with statistics (one wave, 0.4 to 0.8 us) and never with
+  // running statistics, the data gradient once; it does not where it would be that much faster 12, 15, 21 and 23 times.
   r.ns = 3000.0 + waves * (kc / 32) * 860.0;
   r.ok = true;
   return r;

@@ -1,6 +1,8 @@
 """3x3 convolutions by pairs of SMs: tiles of whole image rows and tiles that start anywhere, image counts that leave the second CTA of a
 pair without work, one to four blocks of reduction channels, column tiles that end inside a tile, every epilogue, and what is added on
 boundaries of 4, 16 and 32 bytes; against 64-bit sums over operands as the copy engine rounds them."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -74,3 +76,42 @@ def test_epilogue_does_not_choose_the_kernel(n, h):
     gamma, beta, m, v = vec(0.5, 1.5), vec(-1, 1), vec(-1, 1), vec(0.5, 2)
     want = g.op("batch_norm2d")(g.op("conv2d")(xt, wt, None, s, p), gamma, beta, 1e-5, False, 0.1, m, v)[0]
     assert np.array_equal(g.host(g.op("conv2d_batch_norm")(xt, wt, None, s, p, gamma, beta, m, v, 1e-5, False)), g.host(want))
+
+
+def _pairs(*shape):
+    """Whether (forward, data gradient) of n, cin, cout, h, w run by pairs of SMs."""
+    import gpu_util as g
+    import mytorch_b200 as mt
+    from mytorch_b200.backends.cuda.ops import _env
+
+    n, cin, cout, h, w = shape
+    out = (ctypes.c_int * 6)()
+    _env(mt.tensor(np.zeros(4, np.float32), device=g.DEV)).lib.conv2d_pair_choice_f32(n, cin, h, w, 3, 3, 1, 1, 1, 1, cout, out)
+    return bool(out[0]), bool(out[3])
+
+
+@pytest.mark.parametrize("shape", [
+    (20, 64, 64, 32, 32), (40, 64, 64, 19, 28), (5, 64, 80, 41, 56), (16, 96, 96, 30, 30), (17, 128, 128, 16, 16), (5, 128, 192, 28, 28),
+    (3, 64, 96, 64, 64), (200, 64, 64, 5, 4), (30, 128, 64, 13, 22), (2, 64, 112, 90, 81), (150, 96, 160, 8, 9)])
+def test_shapes_above_run_by_pairs(shape):
+    cout = shape[2]
+    # the data gradient reads blocks of 32 output channels, up to 128 of them
+    assert _pairs(*shape) == (True, cout % 32 == 0 and cout <= 128)
+
+
+def test_whole_rows_of_28_pixels():
+    test_forward_and_data_gradient(40, 64, 64, 19, 28)
+
+
+# input channels that are no blocks of 32: the filter's boxes reach into the next tap and past the last one
+@pytest.mark.parametrize("n,cin,cout,h,w", [(20, 80, 64, 32, 32), (12, 112, 128, 28, 28), (30, 80, 96, 13, 22), (9, 208, 64, 40, 41)])
+def test_data_gradient_of_odd_blocks(n, cin, cout, h, w):
+    import gpu_util as g
+
+    assert _pairs(n, cin, cout, h, w)[1]
+    rng = np.random.default_rng(n + cin)
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)
+    x, wt, dy = f32(n, cin, h, w), f32(cout, cin, 3, 3), f32(n, cout, h, w)
+    dx = g.host(g.op("conv2d_backward")(g.dev(dy), g.dev(x, True), g.dev(wt), None, (1, 1), (1, 1))[0])
+    rdy, turned = O.round_tf32(dy).astype(np.float64), O.round_tf32(wt).astype(np.float64)[:, :, ::-1, ::-1].transpose(1, 0, 2, 3)
+    assert (np.abs(dx - _product(rdy, turned)) <= (9 * cout + 3) * 2.0 ** -23 * _product(abs(rdy), abs(turned))).all()
