@@ -140,7 +140,8 @@ int mtb_conv2d_dgrad_accumulates_in_place(int n, int cin, int h, int w, int kh, 
  * would take for this shape and how the row-staged kernels lay out shared and tensor memory.
  * out: 25 ints, see the definition in csrc/tc_kernels.cu.  No counterpart in the reference. */
 int mtb_conv2d_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out);
-/* The same for the kernel by pairs of SMs: its layout (18 ints), and whether forward and data gradient take it, with the prices (6 ints). */
+/* The same for the kernel by pairs of SMs: its layout (18 ints), and whether forward, data gradient and weight gradient take it, with the prices of the
+ * first two (7 ints). */
 int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* sizes);
 int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* choice);
 /* dw[Cout,KH,KW,Cin]; needs mtb_conv2d_workspace_bytes() of workspace: split-K partials go there and are summed in a fixed order */

@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(1024) bn_bwd_final_kernel(const float* __restr
   coef[2 * C + c] = rstd * dg * inv_m;  // k3: (x - mean) * k3 = xhat * dgamma / m
 }
 
-// MODES 2 and 3 also write the masked upstream gradient, which is the gradient of the added tensor, to dres.
+// MODES 2 and 3 also write the masked upstream gradient, which is the gradient of the added tensor, to dres.  rows_per_block: of single rows (V = 1) alone.
 template <int V, int MODE>
 __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx,
                                                          long long rows, int C, int L, long long rows_per_block,
@@ -661,7 +661,7 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
              partial, res, mask, GradientSource<M_>{})
   const PooledGradient pooled{ties, PoolDiv(w), PoolDiv(h), (unsigned)(w / 2), (unsigned)(h / 2)};
   if (ties)
-    MTB_LAUNCH(bn_bwd_partial_kernel<4, 4>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) || cfg.vec == 1 ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta,
+    MTB_LAUNCH(bn_bwd_partial_kernel<4, 4>, grid, 256, 0, st, dy, x, rows, c, cfg.lanes, short_chain(rows, c) ? cfg.rows_per_block : 0, mean, var, (float)eps, gamma, beta,
                partial, res, mask, pooled);
   else if (cfg.vec == 4) { if (mode == 3) MTB_BN_PARTIAL(4, 3); else if (mode == 2) MTB_BN_PARTIAL(4, 2); else if (mode == 1) MTB_BN_PARTIAL(4, 1); else MTB_BN_PARTIAL(4, 0); }
   else { if (mode == 2) MTB_BN_PARTIAL(1, 2); else if (mode == 1) MTB_BN_PARTIAL(1, 1); else MTB_BN_PARTIAL(1, 0); }
@@ -672,9 +672,9 @@ int bn_backward(int n, int c, int h, int w, const float* dy, const float* mean, 
   MTB_LAUNCH_CHECK("bn_bwd_final_kernel");
   ColCfg s = stream_cfg(rows, c, aligned);
   dim3 g2(s.col_blocks, s.row_blocks);
-#define MTB_BN_DX(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<V_, M_>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, coef, beta, res, dres, mask, GradientSource<M_>{}))
+#define MTB_BN_DX(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<V_, M_>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.rows_per_block, mean, coef, beta, res, dres, mask, GradientSource<M_>{}))
   if (ties)
-    MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<4, 4>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, coef, beta, res, dres, mask, pooled));
+    MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_bwd_dx_kernel<4, 4>, g2, dim3(256), 0, st, dy, x, dx, rows, c, s.lanes, s.rows_per_block, mean, coef, beta, res, dres, mask, pooled));
   else if (s.vec == 4) { if (mode == 3) MTB_BN_DX(4, 3); else if (mode == 2) MTB_BN_DX(4, 2); else if (mode == 1) MTB_BN_DX(4, 1); else MTB_BN_DX(4, 0); }
   else { if (mode == 2) MTB_BN_DX(1, 2); else if (mode == 1) MTB_BN_DX(1, 1); else MTB_BN_DX(1, 0); }
 #undef MTB_BN_DX

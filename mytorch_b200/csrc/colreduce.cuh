@@ -3,8 +3,8 @@
 //
 // A CTA of 256 threads owns L column groups (L a power of two <= 256, each group VEC
 // channels wide) and R = 256 / L rows per iteration, so consecutive threads read
-// consecutive addresses.  Each CTA reduces a contiguous row range and writes one partial
-// row per quantity into scratch; a small second kernel combines the partials in a fixed
+// consecutive addresses.  Each CTA reduces a contiguous row range (BatchNorm's backward above
+// 64 MB: groups of rows strided over the grid) and writes one partial row per quantity into scratch; a small second kernel combines the partials in a fixed
 // order, so results are bit-reproducible (no float atomics).
 #pragma once
 #include "common.cuh"

@@ -208,7 +208,7 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             const int kh = lane / 3, j = lane % 3;
             const int tap = 3 * kh + (BESIDE == 2 && j < 2 ? (int)rank : j), c0 = n0 + 32 * (BESIDE == 2 && j < 2 ? j : (int)rank);
             const uint32_t dst = b_base + (uint32_t)(3 * cc + kh) * kTapsGroup + (uint32_t)j * 4096u;
-            const uint32_t bfull = smem_u32(&bar_bfull[cc]) & 0xFEFFFFFFu;
+            const uint32_t bfull = cluster_address(smem_u32(&bar_bfull[cc]), 0);
             if (BMODE == B_KMAJOR) tma_load_2d_pair(dst, &mapB, bfull, p.b_tap_x[tap] + cc * 32, c0);
             else tma_load_2d_pair(dst, &mapB, bfull, p.b_tap_x[tap] + c0, cc * 32);
           }
@@ -220,7 +220,7 @@ tc_conv_taps_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         // the tile's first position lies at the same place of every stage, whatever its column
         if (lane < nr)
           tma_load_4d_pair(smem_base + as * p.a_stage_bytes + (uint32_t)(p.origin - p.Wp - col) * 128u + (uint32_t)lane * row_bytes, &mapA,
-                           smem_u32(&bar_afull[as]) & 0xFEFFFFFFu, cc * 32, -1, hrow, img);
+                           cluster_address(smem_u32(&bar_afull[as]), 0), cc * 32, -1, hrow, img);
         ++filled;
         if (++as == ST) { as = 0; aphase ^= 1u; }
       }

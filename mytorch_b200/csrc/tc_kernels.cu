@@ -1689,8 +1689,8 @@ MTB_API int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int k
   return MTB_OK;
 }
 
-// Whether forward and data gradient of a shape run by pairs of SMs (pointers assumed aligned, the gradient not in place), with the prices that decide.  Host code only.
-// out[0..2] forward, out[3..5] data gradient: taken, price in ns, price of the kernel that is taken otherwise.
+// Whether forward, data gradient (pointers assumed aligned, the gradient not in place) and weight gradient of a shape run by pairs of SMs.  Host code only.
+// out[0..2] forward, out[3..5] data gradient: taken, and the prices that decide, in ns: this kernel's, and of the one that is taken otherwise.  out[6]: weight gradient taken.
 MTB_API int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* out) {
   MTB_REQUIRE(out && n > 0 && cin > 0 && cout > 0 && h > 0 && w > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0, "conv2d_pair_choice: bad arguments");
   const float* al = reinterpret_cast<const float*>(uintptr_t(256));
@@ -1702,6 +1702,8 @@ MTB_API int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int
     out[1] = (int)r.plan.ns;
     out[2] = (int)r.other_ns;
   }
+  out[0] = mtb_tc_conv2d_wgrad_supported(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout, al, al, al) &&
+           wgrad_pairs_pay(wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout));
   return MTB_OK;
 }
 

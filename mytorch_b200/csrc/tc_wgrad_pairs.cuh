@@ -100,7 +100,7 @@ tc_wgrad_pairs_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_con
         const bool is_x = lane < p.rows;
         const int v = g * p.rows + (is_x ? lane : lane - p.rows - 1);
         const int img = v >= 0 ? v / p.Hv : -1, hrow = v - img * p.Hv;  // separators and images outside [0, N): zeros
-        const uint32_t st = smem_base + stage * p.stage_bytes, full = smem_u32(&bar_full[stage]) & 0xFEFFFFFFu;
+        const uint32_t st = smem_base + stage * p.stage_bytes, full = cluster_address(smem_u32(&bar_full[stage]), 0);
         if (is_x) tma_load_4d_pair(st + kWgPairLead + (uint32_t)lane * row_bytes, &mapX, full, ch0, -1, hrow, img);
         else tma_load_4d_pair(st + p.x_bytes + (uint32_t)(lane - p.rows) * row_bytes, &mapDY, full, ch0, -1, hrow, img);
       }

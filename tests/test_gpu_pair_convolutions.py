@@ -85,7 +85,7 @@ def _pairs(*shape):
     from mytorch_b200.backends.cuda.ops import _env
 
     n, cin, cout, h, w = shape
-    out = (ctypes.c_int * 6)()
+    out = (ctypes.c_int * 7)()
     _env(mt.tensor(np.zeros(4, np.float32), device=g.DEV)).lib.conv2d_pair_choice_f32(n, cin, h, w, 3, 3, 1, 1, 1, 1, cout, out)
     return bool(out[0]), bool(out[3])
 

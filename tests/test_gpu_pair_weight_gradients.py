@@ -1,6 +1,8 @@
 """Weight gradients of 64 channels by pairs of SMs: image rows that are a multiple of 1, 2, 4 and 8 positions, last stages that end behind the last
 image, ranges of one stage and of odd and even counts, output channels that end inside a block; against 64-bit sums over operands as
 the copy engine rounds them."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -30,3 +32,15 @@ def test_weight_gradient(n, cout, h, w):
     # products of TF32 operands are exact in FP32; a sum loses at most its number of terms x 2^-23 of the sum of magnitudes
     assert (np.abs(dw - sums(rx, rdy)) <= n * h * w * 2.0 ** -23 * sums(abs(rx), abs(rdy))).all()
     assert np.linalg.norm(dw - sums(rx, rdy)) <= 5e-5 * np.linalg.norm(dw)
+
+
+@pytest.mark.parametrize("n,cout,h,w", [(70, 64, 32, 32), (131, 64, 32, 32), (24, 64, 56, 56), (40, 36, 45, 38), (100, 48, 29, 27), (9, 64, 100, 110), (33, 60, 50, 46),
+                                        (20, 64, 70, 62), (1000, 64, 7, 9)])
+def test_shapes_above_run_by_pairs(n, cout, h, w):
+    import gpu_util as g
+    import mytorch_b200 as mt
+    from mytorch_b200.backends.cuda.ops import _env
+
+    out = (ctypes.c_int * 7)()
+    _env(mt.tensor(np.zeros(4, np.float32), device=g.DEV)).lib.conv2d_pair_choice_f32(n, 64, h, w, 3, 3, 1, 1, 1, 1, cout, out)
+    assert out[6] == 1
