@@ -16,9 +16,9 @@ namespace {
 // starts there: the normalise pass walks back to front behind a convolution that wrote front to back, the backward's sums do so behind a data
 // gradient, and dx then front to back.  Single rows of a contiguous range a CTA -> groups, in these orders: ResNet-50 step at 128 images 18.50 -> 18.08 ms,
 // ResNet-18 at 512 5465 -> 5353 us (5406 without the turns), at 128 1882 -> 1851, at 64 (captured) 1270 -> 1246.  rows_per_block > 0: a CTA
-// takes that many rows one after the other; the sums do so up to 64 MB, which the L2 holds whole, and keep their order there, and channels that
-// are no fours do, whose backward passes are bound by their instructions and take row after row (207 channels on 69 x 17x17 with ReLU and pool, forward
-// and backward: 114.9 us, in groups 117.6).
+// takes that many rows one after the other; the sums do so up to 64 MB, which the L2 holds whole, and keep their order there.  Channels that are no fours
+// walk a CTA's rows without any of this: their passes are bound by their instructions (207 channels on 69 x 17x17 with ReLU and pool, forward
+// and backward: 114.9 us, the backward in groups 117.6; the forward of 150 channels on 30 x 50x50 40.4 us, in groups 42.3).
 constexpr int kGroup = 4;
 struct RowWalk {
   long long r, last, step, limit;  // first row of the group, of the last group, from group to group; end of the rows
@@ -231,21 +231,19 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
   // Four rows are loaded before the first is stored: x may be y (an update in place), so the compiler would not do it.  BatchNorm,
   // ReLU and pooling of 256 x 128 x 56 x 56, forward and backward: 1073 -> 1050 us; ResNet-18 step at 512 images 5.84 -> 5.78 ms.
   constexpr int AHEAD = kGroup;
-  RowWalk walk(rows, R, rows_per_block, true);
-  for (long long r; walk.next(r);) {
-    r += rsub;
+  auto group = [&](long long r, long long limit) {
     const long long off = r * C + (long long)cg * V, step = (long long)R * C;
     VecF<V> f[AHEAD], a[MODE == 2 ? AHEAD : 1];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (r + u * R < walk.limit) {
+      if (r + u * R < limit) {
         f[u] = vload<V>(x + off + u * step);
         if (MODE == 2) a[u] = vload<V>(res + off + u * step);
       }
     }
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (r + u * R >= walk.limit) break;
+      if (r + u * R >= limit) break;
       unsigned negative = 0;
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -256,6 +254,13 @@ __global__ void __launch_bounds__(256) bn_normalize_kernel(const float* x, float
       vstore<V>(y + off + u * step, f[u]);
       if (MODE == 2 && V == 4 && mask) mask[(off + u * step) / 4] = (unsigned char)negative;
     }
+  };
+  if (V == 1) {  // see RowWalk
+    const long long r0 = blockIdx.y * rows_per_block, r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+    for (long long r = r0 + rsub; r < r1; r += AHEAD * R) group(r, r1);
+  } else {
+    RowWalk walk(rows, R, 0, true);
+    for (long long r; walk.next(r);) group(r + rsub, walk.limit);
   }
 }
 
@@ -579,7 +584,7 @@ int launch_normalize(const float* x, float* y, long long rows, int c, bool align
                      unsigned char* mask = nullptr) {
   ColCfg s = stream_cfg(rows, c, aligned);
   dim3 grid(s.col_blocks, s.row_blocks);
-#define MTB_BN_NORM(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_normalize_kernel<V_, M_>, grid, dim3(256), 0, st, x, y, rows, c, s.lanes, s.vec == 1 ? s.rows_per_block : 0, mean, scale, beta, res, var, eps, mask))
+#define MTB_BN_NORM(V_, M_) MTB_CUDA(mtb_launch_after(short_chain(rows, c), bn_normalize_kernel<V_, M_>, grid, dim3(256), 0, st, x, y, rows, c, s.lanes, s.rows_per_block, mean, scale, beta, res, var, eps, mask))
   if (s.vec == 4) { if (mode == 2) MTB_BN_NORM(4, 2); else if (mode == 1) MTB_BN_NORM(4, 1); else MTB_BN_NORM(4, 0); }
   else { if (mode == 2) MTB_BN_NORM(1, 2); else if (mode == 1) MTB_BN_NORM(1, 1); else MTB_BN_NORM(1, 0); }
 #undef MTB_BN_NORM
