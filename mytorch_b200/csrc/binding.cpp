@@ -246,7 +246,7 @@ constexpr unsigned HOST(I... i) { return (0u | ... | (1u << i)); }
   X(max_pool2d_forward_f32, LAUNCH, 0) X(max_pool2d_backward_f32, LAUNCH, 0) X(max_pool2d_argmax_u8, LAUNCH, 0) \
   X(cross_entropy_workspace_bytes, VALUE, 0) X(cross_entropy_forward_f32, LAUNCH, 0) X(cross_entropy_backward_f32, LAUNCH, 0) \
   X(sgd_f32, LAUNCH, 0) X(sgd_multi_f32, LAUNCH, HOST(1, 2, 3, 4, 5)) X(pack_scale_f32, LAUNCH, HOST(1, 2, 3)) \
-  X(conv2d_workspace_bytes, VALUE, 0) X(conv2d_plan_f32, STATUS, HOST(11)) X(conv2d_pair_plan_f32, STATUS, HOST(11)) X(conv2d_pair_choice_f32, STATUS, HOST(11)) X(conv2d_forward_f32, LAUNCH, 0) \
+  X(conv2d_workspace_bytes, VALUE, 0) X(conv2d_plan_f32, STATUS, HOST(11)) X(conv2d_pair_plan_f32, STATUS, HOST(11)) X(conv2d_pair_choice_f32, STATUS, HOST(11)) X(conv2d_pair_smem_bytes, VALUE, 0) X(conv2d_forward_f32, LAUNCH, 0) \
   X(conv2d_stats_max_rows, VALUE, 0) X(conv2d_forward_stats_f32, LAUNCH, HOST(17)) X(conv2d_bn_forward_f32, LAUNCH, 0) X(conv2d_bn_pool_takes, VALUE, 0) X(conv2d_bn_pool_scratch_bytes, VALUE, 0) X(conv2d_bn_pool_forward_f32, LAUNCH, 0) \
   X(batch_norm2d_forward_prestats_f32, LAUNCH, 0) X(conv2d_dgrad_f32, LAUNCH, 0) X(conv2d_dgrad_add_f32, LAUNCH, 0) \
   X(conv2d_dgrad_accumulates_in_place, VALUE, 0) X(conv2d_wgrad_f32, LAUNCH, 0) X(gemm_f32, LAUNCH, 0) X(linear_relu_f32, LAUNCH, 0) X(tc_status, STATUS, HOST(0)) \

@@ -44,6 +44,11 @@ constexpr int kTapsMaxChunks = 4;    // blocks of 32 reduction channels: up to 1
 constexpr uint32_t kTapsGroup = 3u * 32u * 128u;  // one CTA's half of the three taps of a filter row, 32 reduction channels x 64 outputs
 constexpr int kTapsThreads = 32 * (2 + 8);  // producer, issuer, eight epilogue warps
 constexpr uint32_t kTapsMaxSmem = 227u * 1024u - 4096u;  // what is left beside the kernel's own shared variables
+// The least that a kernel by pairs of SMs takes: more than half of an SM's 228 KB (a CTA takes 1 KB beside its own), so that no SM holds CTAs of two of them.
+// Allocating tensor memory waits without a limit, and a pair holds what one CTA has got until the other has its own: two pairs of different streams (a data
+// gradient and the weight gradient beside it), each with its columns on one of two SMs, would wait for each other for good.
+// (The filter and two stages of this kernel are always more.)
+constexpr uint32_t kPairMinSmem = 114u * 1024u;
 
 struct TapsParams {
   long long Q;             // positions: N * Hv * Wp

@@ -1707,6 +1707,17 @@ MTB_API int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int
   return MTB_OK;
 }
 
+// Host code only: see kPairMinSmem for what it has to be.
+MTB_API long long mtb_conv2d_pair_smem_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction) {
+  if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || w <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0) return 0;
+  if (direction == 2) {
+    const WgradPairPlan q = wgrad_pair_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);
+    return q.ok ? q.smem_bytes : 0;
+  }
+  const TapsPlan q = taps_plan(n, h, w, kh, kw, sh, sw, ph, pw, direction ? cout : cin, direction ? cin : cout);
+  return q.ok ? q.smem_bytes : 0;
+}
+
 long long mtb_tc_conv2d_workspace_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout) {
   if (cin % 32) return 0;
   WgradPlan q = wgrad_plan(n, cin, h, w, kh, kw, sh, sw, ph, pw, cout);

@@ -223,6 +223,7 @@ WgradPairPlan wgrad_pair_plan(int n, int cin, int h, int w, int kh, int kw, int 
   r.stages = (int)(budget / r.stage_bytes);
   if (r.stages > kWgPairStages) r.stages = kWgPairStages;
   r.smem_bytes = 1024u + (uint32_t)r.stages * r.stage_bytes;
+  if (r.smem_bytes < kPairMinSmem) r.smem_bytes = kPairMinSmem;  // image rows of up to 9 pixels
   const long long image_rows = (long long)n * r.Hv;
   r.groups_total = (int)((image_rows + r.rows - 1) / r.rows);
   int splits = cluster_units(2) / 2;  // a pair each
