@@ -11,7 +11,7 @@ MTB_API long long mtb_batch_norm2d_workspace_bytes(int n, int c, int h, int w);
 
 namespace {
 
-// The order in which a pass walks its rows, in groups of kGroup iterations whose loads are all issued before the first value is used or stored.
+// The order in which a pass walks its rows, in groups of kGroup iterations whose loads are issued (forward all, backward see partial_ahead) before the first value is used or stored.
 // All CTAs work on neighbouring groups (grid stride), so that what the L2 holds at the end is one stretch of the tensor, and the pass behind it
 // starts there: the normalise pass walks back to front behind a convolution that wrote front to back, the backward's sums do so behind a data
 // gradient, and dx then front to back.  Single rows of a contiguous range a CTA -> groups, in these orders: ResNet-50 step at 128 images 18.50 -> 18.08 ms,
@@ -312,6 +312,15 @@ __global__ void __launch_bounds__(256) bn_relu_pool_kernel(const float4* __restr
 
 // ---------------------------------------------------------------- backward
 
+// Rows of a group whose loads are issued together (the order of the rows is the same).  The sums' grid is four CTAs an SM, in which four rows take 74 to 94
+// registers: two or three CTAs fit.  Two are as good as four, since the grid is two whole turns of them; three leave a second turn with a third of the CTAs.
+// BatchNorm by itself (MODE 0) had three so, and has four in 64 registers with two rows: backward of 60 x 64 x 33x33 17.1 -> 15.6 us, 60 x 132 x 33x33 37.7 ->
+// 36.4, 120 x 132 x 28x28 55.6 -> 52.3, 70 x 256 x 55x55 176.2 -> 170.6.  Behind a pool (MODE 4), whose loads are three and not neighbours, both passes are for
+// it: 67.8 -> 56.4 on 70 x 64 x 55x55, 242 -> 178 on 70 x 132 x 55x55, 257 -> 194 on 70 x 256 x 55x55.
+// With ReLU or addition two rows win 0 to 6 % alone and lose 0.3 to 1.3 % of a ResNet step, where weight gradients want the registers beside them.
+constexpr int partial_ahead(int mode) { return mode == 0 || mode == 4 ? 2 : kGroup; }
+constexpr int dx_ahead(int mode) { return mode == 4 ? 2 : kGroup; }
+
 // MODE 4: MODE 1 whose upstream gradient goes through a 2 x 2 max-pool of stride 2 first: dy and the tie mask have the shape of its result.  (For
 // 3 x 3 windows, up to four a pixel, both passes then wait for their windows: 64 channels of 128 x 112x112 380 and 503 us, against 102 for the
 // pool's own backward and 316 for two passes over what it writes.)
@@ -352,7 +361,7 @@ __device__ __forceinline__ VecF<V> load_gradient(const float* __restrict__ dy, l
 // MODE 1 / 2: the forward output went through max(0, .) (MODE 2: after adding `res`) in the same pass;
 // the upstream gradient is first masked where the (recomputed, bit-identical) value was negative.
 template <int V, int MODE>
-__global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __restrict__ dy, const float* __restrict__ x, long long rows, int C, int L, long long rows_per_block, const float* __restrict__ mean,
+__global__ void __launch_bounds__(256, partial_ahead(MODE) == 2 ? 4 : 0 /* as many as the compiler likes */) bn_bwd_partial_kernel(const float* __restrict__ dy, const float* __restrict__ x, long long rows, int C, int L, long long rows_per_block, const float* __restrict__ mean,
                                                               const float* __restrict__ var, float eps, const float* __restrict__ gamma,
                                                               const float* __restrict__ beta, float* __restrict__ partial,
                                                               const float* __restrict__ res, const unsigned char* __restrict__ mask, const GradientSource<MODE> pool) {
@@ -399,23 +408,27 @@ __global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const float* __rest
   } else if (active) {
     RowWalk walk(rows, R, rows_per_block, true);
     for (long long r0; walk.next(r0);) {
+      constexpr int AHEAD = partial_ahead(MODE);
       r0 += rsub;
-      VecF<V> g[kGroup], f[kGroup], a[MODE == 2 ? kGroup : 1];
-      unsigned negative[kGroup];
+#pragma unroll 1
+      for (int part = 0; part < kGroup / AHEAD; ++part, r0 += AHEAD * R) {
+        VecF<V> g[AHEAD], f[AHEAD], a[MODE == 2 ? AHEAD : 1];
+        unsigned negative[AHEAD];
 #pragma unroll
-      for (int u = 0; u < kGroup; ++u) {
-        if (r0 + u * R < walk.limit) {
-          const long long off = (r0 + u * R) * C + (long long)cg * V;
-          g[u] = load_gradient<V, MODE>(dy, r0 + u * R, C, cg * V, pool);
-          f[u] = vload<V>(x + off);
-          if (MODE == 2) a[u] = vload<V>(res + off);
-          negative[u] = MODE == 3 ? mask[off / 4] : 0u;
+        for (int u = 0; u < AHEAD; ++u) {
+          if (r0 + u * R < walk.limit) {
+            const long long off = (r0 + u * R) * C + (long long)cg * V;
+            g[u] = load_gradient<V, MODE>(dy, r0 + u * R, C, cg * V, pool);
+            f[u] = vload<V>(x + off);
+            if (MODE == 2) a[u] = vload<V>(res + off);
+            negative[u] = MODE == 3 ? mask[off / 4] : 0u;
+          }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < kGroup; ++u) {
-        if (r0 + u * R >= walk.limit) break;
-        add(g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
+        for (int u = 0; u < AHEAD; ++u) {
+          if (r0 + u * R >= walk.limit) break;
+          add(g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
+        }
       }
     }
   }
@@ -538,23 +551,27 @@ __global__ void __launch_bounds__(256) bn_bwd_dx_kernel(const float* __restrict_
   }
   RowWalk walk(rows, R, 0, false);
   for (long long r0; walk.next(r0);) {
+    constexpr int AHEAD = dx_ahead(MODE);
     r0 += rsub;
-    VecF<V> g[kGroup], f[kGroup], a[MODE == 2 ? kGroup : 1];
-    unsigned negative[kGroup];
+#pragma unroll 1
+    for (int part = 0; part < kGroup / AHEAD; ++part, r0 += AHEAD * R) {
+      VecF<V> g[AHEAD], f[AHEAD], a[MODE == 2 ? AHEAD : 1];
+      unsigned negative[AHEAD];
 #pragma unroll
-    for (int u = 0; u < kGroup; ++u) {
-      if (r0 + u * R < walk.limit) {
-        const long long off = (r0 + u * R) * C + (long long)cg * V;
-        g[u] = load_gradient<V, MODE>(dy, r0 + u * R, C, cg * V, pool);
-        f[u] = vload<V>(x + off);
-        if (MODE == 2) a[u] = vload<V>(res + off);
-        negative[u] = MODE == 3 ? mask[off / 4] : 0u;
+      for (int u = 0; u < AHEAD; ++u) {
+        if (r0 + u * R < walk.limit) {
+          const long long off = (r0 + u * R) * C + (long long)cg * V;
+          g[u] = load_gradient<V, MODE>(dy, r0 + u * R, C, cg * V, pool);
+          f[u] = vload<V>(x + off);
+          if (MODE == 2) a[u] = vload<V>(res + off);
+          negative[u] = MODE == 3 ? mask[off / 4] : 0u;
+        }
       }
-    }
 #pragma unroll
-    for (int u = 0; u < kGroup; ++u) {
-      if (r0 + u * R >= walk.limit) break;
-      store((r0 + u * R) * C + (long long)cg * V, g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
+      for (int u = 0; u < AHEAD; ++u) {
+        if (r0 + u * R >= walk.limit) break;
+        store((r0 + u * R) * C + (long long)cg * V, g[u], f[u], a[MODE == 2 ? u : 0], negative[u]);
+      }
     }
   }
 }
