@@ -143,7 +143,7 @@ int mtb_conv2d_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, in
 /* The same for the kernel by pairs of SMs: its layout (18 ints), and whether forward, data gradient and weight gradient take it, with the prices of the
  * first two (7 ints). */
 int mtb_conv2d_pair_plan_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* sizes);
-int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* choice);
+int mtb_conv2d_pair_choice_f32(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int* sizes);
 /* Dynamic shared memory of one of its CTAs in the forward pass (direction 0), data gradient (1) or weight gradient (2), 0 where its layout does not fit. */
 long long mtb_conv2d_pair_smem_bytes(int n, int cin, int h, int w, int kh, int kw, int sh, int sw, int ph, int pw, int cout, int direction);
 /* dw[Cout,KH,KW,Cin]; needs mtb_conv2d_workspace_bytes() of workspace: split-K partials go there and are summed in a fixed order */
